@@ -21,6 +21,7 @@
 #include <climits>
 
 #include "../../include/arbo.h"
+#include "launch.cuh"
 #include "sim_internal.h"
 
 namespace arbo {
@@ -57,12 +58,6 @@ __device__ __forceinline__ uint32_t lower_bound_f(const float* __restrict__ t, u
     }
     return lo;
 }
-
-// Programmatic dependent launch: wait for the previous kernel of the stream (its memory is
-// visible afterwards), and let the next kernel of the stream start its prologue early. Both are
-// no-ops when the kernels are launched without the programmatic-serialization attribute.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
 __device__ __forceinline__ Key load_key(const Ctrl* c)
 {
@@ -1590,25 +1585,6 @@ int launch_demog(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
     else if (U == 2) k_demog<2><<<grid, block, 0, st>>>(d, hblocks, koff);
     else k_demog<1><<<grid, block, 0, st>>>(d, hblocks, koff);
     return (int)cudaGetLastError();
-}
-
-// Launch with programmatic stream serialization: the kernel may start while the previous kernel
-// of the stream finishes; it calls griddepcontrol.wait before reading that kernel's results.
-template <typename... Args>
-static int launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
-                      Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 int launch_foi(const Dev& d, const Launch& l, cudaStream_t st, int collect_only, uint32_t koff)

@@ -14,11 +14,13 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
 
 #include "../../include/arbo.h"
+#include "launch.cuh"
 #include "philox.cuh"
 #include "sim_internal.h"
 #include "tc.cuh"
@@ -29,8 +31,9 @@ namespace {
 
 typedef __nv_bfloat16 bf16;
 
-enum Epi : int { kEpiHidden = 0, kEpiLinear = 1, kEpiBackward = 2, kEpiStore = 3 };
+enum Epi : int { kEpiHidden = 0, kEpiLinear = 1, kEpiBackward = 2, kEpiStore = 3, kEpiLoss = 4 };
 
+// One product C = A B^T and its epilogue.
 struct GemmArgs {
     const bf16* A;
     const bf16* B;
@@ -45,25 +48,39 @@ struct GemmArgs {
     uint32_t ldob;
     bf16* outt;          // [N][ldot] transposed copy
     uint32_t ldot;
-    uint32_t* err;       // bit 0: an mbarrier wait ran out
+    const float* target;  // [M][nout] (loss)
+    uint32_t nout;
+    float* loss;
+};
+
+// Column sums of a matrix given by its transposed copy (bias gradients): sums[c] = sum over n rows.
+struct ColumnSums {
+    const bf16* t;  // [cols][ld]
+    uint32_t ld, n, cols;
+    float* sums;
+};
+
+// What one launch of k_gemm_tn does: one or two independent products and optional column sums.
+struct GemmLaunch {
+    CUtensorMap map[2][2];  // A and B of each product
+    GemmArgs g[2];
+    uint32_t tn[2], tiles[2];
+    uint32_t stages, stage_size, acc_cols;  // operand ring; columns of one tensor-memory accumulator
+    ColumnSums cs;
+    uint32_t* err;  // bit 0: an mbarrier wait ran out
 };
 
 constexpr uint32_t kTileM = 128, kTileK = 64, kMaxStages = 8;
 constexpr uint32_t kMinTileN = 32, kMaxTileN = 256;
 constexpr uint32_t kStageBudget = 192 * 1024;  // shared memory of the operand ring
-constexpr uint32_t kEpiPitch = 36;             // floats per staged row of 32 columns (conflict-free 16-byte accesses)
-constexpr uint32_t kEpiBytes = 4 * 32 * kEpiPitch * 4;  // one staging tile per epilogue warp
+constexpr uint32_t kEpiWarps = 8;             // two per quarter of the 128 tensor-memory lanes
+constexpr uint32_t kEpiPitch = 20;             // words per staged row of 16 columns
+constexpr uint32_t kEpiBytes = kEpiWarps * 32 * kEpiPitch * 4;  // one staging block per epilogue warp
+constexpr uint32_t kGemmThreads = 64 + kEpiWarps * 32 + 64;
 
-__host__ __device__ constexpr uint32_t stage_bytes(uint32_t tn) { return (kTileM + tn) * kTileK * 2; }
-__host__ __device__ constexpr uint32_t ring_stages(uint32_t tn, uint32_t nk)
-{
-    uint32_t n = kStageBudget / stage_bytes(tn);
-    if (n > kMaxStages) n = kMaxStages;
-    return n < nk ? n : nk;
-}
 // Dynamic shared memory: the ring, the epilogue's staging and 1 KB of alignment slack.
-constexpr uint32_t gemm_smem(uint32_t tn, uint32_t nk) { return ring_stages(tn, nk) * stage_bytes(tn) + kEpiBytes + 1024; }
 constexpr uint32_t kGemmSmemMax = kStageBudget + kEpiBytes + 1024;
+static_assert(kGemmSmemMax <= 232448 - 256, "dynamic and static shared memory of one CTA");
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float dsilu(float z)
@@ -78,48 +95,40 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
            ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
 }
 
-// The epilogue's copies between a warp's 32 x 32 block (one row per lane) and row-major global
-// memory, through the warp's staging tile so that a warp instruction touches whole rows of the
-// block: 128-byte FP32 rows (four per instruction) and 64-byte BF16 rows (eight per instruction).
-// `rows` and `cols` are the live rows and columns of the block (cols 16 or 32).
-__device__ __forceinline__ void block_store_f32(float* st, const float (&v)[32], float* out, uint32_t ld, uint32_t rows,
-                                                uint32_t cols, uint32_t lane)
+// The epilogue's copies between a warp's block of 32 rows (one per lane) and 16 columns and row-major
+// global memory, through the warp's staging block, so that a warp instruction touches whole sectors:
+// eight 64-byte FP32 rows or sixteen 32-byte BF16 rows. `rows` is the number of live rows.
+__device__ __forceinline__ void block_store_f32(float* st, const float (&v)[16], float* out, uint32_t ld, uint32_t rows,
+                                                uint32_t lane)
 {
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < 4; ++k)
         *reinterpret_cast<float4*>(st + lane * kEpiPitch + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     __syncwarp();
-    const uint32_t c = (lane & 7u) * 4;
+    const uint32_t c = (lane & 3u) * 4;
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-        const uint32_t r = it * 4 + (lane >> 3);
-        if (r < rows && c < cols)
+    for (int it = 0; it < 4; ++it) {
+        const uint32_t r = it * 8 + (lane >> 2);
+        if (r < rows)
             *reinterpret_cast<float4*>(out + (size_t)r * ld + c) = *reinterpret_cast<const float4*>(st + r * kEpiPitch + c);
     }
     __syncwarp();
 }
 
-__device__ __forceinline__ void block_fetch_f32(float4 (&f)[8], const float* in, uint32_t ld, uint32_t rows, uint32_t cols,
-                                                uint32_t lane)
+__device__ __forceinline__ void block_fetch_f32(float4 (&f)[4], const float* in, uint32_t ld, uint32_t rows, uint32_t lane)
 {
-    const uint32_t c = (lane & 7u) * 4;
+    const uint32_t c = (lane & 3u) * 4;
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-        const uint32_t r = it * 4 + (lane >> 3);
-        f[it] = (r < rows && c < cols) ? *reinterpret_cast<const float4*>(in + (size_t)r * ld + c)
-                                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int it = 0; it < 4; ++it) {
+        const uint32_t r = it * 8 + (lane >> 2);
+        f[it] = r < rows ? *reinterpret_cast<const float4*>(in + (size_t)r * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 
-__device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[8], float (&v)[32], uint32_t lane)
+__device__ __forceinline__ void block_row_f32(const float* st, float (&v)[16], uint32_t lane)
 {
-    const uint32_t c = (lane & 7u) * 4;
 #pragma unroll
-    for (int it = 0; it < 8; ++it)
-        *reinterpret_cast<float4*>(st + (it * 4 + (lane >> 3)) * kEpiPitch + c) = f[it];
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < 4; ++k) {
         const float4 x = *reinterpret_cast<const float4*>(st + lane * kEpiPitch + 4 * k);
         v[4 * k] = x.x;
         v[4 * k + 1] = x.y;
@@ -129,48 +138,109 @@ __device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[8]
     __syncwarp();
 }
 
+__device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[4], float (&v)[16], uint32_t lane)
+{
+    const uint32_t c = (lane & 3u) * 4;
+#pragma unroll
+    for (int it = 0; it < 4; ++it) *reinterpret_cast<float4*>(st + (it * 8 + (lane >> 2)) * kEpiPitch + c) = f[it];
+    __syncwarp();
+    block_row_f32(st, v, lane);
+}
+
 // The block as BF16: row-major to `out`, transposed to `outt` (column n of the block at outt + n * ldt,
 // the lane's row advancing along it). w[j] packs columns 2j and 2j+1 of the lane's row; neighbouring
 // lanes swap halves so that each store of the transposed copy carries two rows of one column. Rows come
 // in pairs: the products with a transposed copy have a multiple of 16 of them.
-__device__ __forceinline__ void block_store_bf16(float* st, const uint32_t (&w)[16], bf16* out, uint32_t ld, bf16* outt,
-                                                 uint32_t ldt, uint32_t rows, uint32_t cols, uint32_t lane)
+__device__ __forceinline__ void block_store_bf16(float* st, const uint32_t (&w)[8], bf16* out, uint32_t ld, bf16* outt,
+                                                 uint32_t ldt, uint32_t rows, uint32_t lane)
 {
     uint32_t* sw = reinterpret_cast<uint32_t*>(st);
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        *reinterpret_cast<uint4*>(sw + lane * 20 + 4 * k) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+    for (int k = 0; k < 2; ++k)
+        *reinterpret_cast<uint4*>(sw + lane * 12 + 4 * k) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
     __syncwarp();
-    const uint32_t c = lane & 3u;
+    const uint32_t c = lane & 1u;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const uint32_t r = it * 8 + (lane >> 2);
-        if (r < rows && 8 * c < cols)
-            *reinterpret_cast<uint4*>(out + (size_t)r * ld + 8 * c) = *reinterpret_cast<const uint4*>(sw + r * 20 + 4 * c);
+    for (int it = 0; it < 2; ++it) {
+        const uint32_t r = it * 16 + (lane >> 1);
+        if (r < rows)
+            *reinterpret_cast<uint4*>(out + (size_t)r * ld + 8 * c) = *reinterpret_cast<const uint4*>(sw + r * 12 + 4 * c);
     }
     __syncwarp();
-    const uint32_t odd = lane & 1u;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < 8; ++j) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, w[j], 1);
-        const uint32_t v = odd ? __byte_perm(other, w[j], 0x7632) : __byte_perm(w[j], other, 0x5410);
-        if (lane < rows && (uint32_t)(2 * j) < cols)
-            *reinterpret_cast<uint32_t*>(outt + (size_t)(2 * j + odd) * ldt + lane - odd) = v;
+        const uint32_t v = c ? __byte_perm(other, w[j], 0x7632) : __byte_perm(w[j], other, 0x5410);
+        if (lane < rows) *reinterpret_cast<uint32_t*>(outt + (size_t)(2 * j + c) * ldt + lane - c) = v;
     }
 }
 
-// Persistent, warp-specialised product: each CTA (192 threads) walks output tiles of kTileM x tn
-// (tn = 32, 64, 128 or 256) in a grid-stride loop.
+// Column sums by the warps w, w + nw, ... of the launch, four columns at a time so that a warp keeps
+// 32 loads in flight. Each column is summed by lane-strided rows, then across the lanes.
+__device__ __forceinline__ void column_sums(const ColumnSums& cs, uint32_t w, uint32_t nw, uint32_t lane)
+{
+    for (uint32_t c = 4 * w; c < cs.cols; c += 4 * nw) {  // cols is a multiple of 16
+        const bf16* t = cs.t + (size_t)c * cs.ld;
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (uint32_t r0 = lane; r0 < cs.n; r0 += 256) {
+            bf16 x[4][8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    x[q][k] = r0 + 32 * k < cs.n ? t[(size_t)q * cs.ld + r0 + 32 * k] : __float2bfloat16_rn(0.0f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] += __bfloat162float(x[q][k]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+            if (lane == 0) cs.sums[c + q] = s[q];
+        }
+    }
+}
+
+// Tile t of a launch: which product, and where in it.
+struct TileAt {
+    uint32_t q, m0, n0, nt, tn, nk;
+};
+__device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
+{
+    TileAt x;
+    x.q = t >= p.tiles[0] ? 1u : 0u;
+    const uint32_t i = x.q ? t - p.tiles[0] : t;
+    const GemmArgs& g = p.g[x.q];
+    const uint32_t mtiles = (g.M + kTileM - 1) / kTileM;
+    x.tn = p.tn[x.q];
+    x.m0 = (i % mtiles) * kTileM;
+    x.n0 = (i / mtiles) * x.tn;
+    x.nt = min(x.tn, g.N - x.n0);
+    x.nk = (g.K + kTileK - 1) / kTileK;
+    return x;
+}
+
+// Persistent, warp-specialised product: each CTA (384 threads) walks output tiles of kTileM x tn
+// (tn = 32, 64, 128 or 256) in a grid-stride loop over the tiles of one or two independent products.
 //   warp 0, one thread: TMA producer. Each 64-wide K chunk of A and B is one box per operand in
 //     the 128-byte-swizzled K-major layout; up to eight chunks are in flight ("full" / "empty"
 //     mbarriers per stage), which for the narrow tiles is the whole K of a 512-wide layer.
 //   warp 1, one thread: issues the four K=16 tcgen05 products of each chunk into one of two
 //     tensor-memory accumulators (tile parity), commits each chunk to the stage's "empty" barrier
 //     and each finished tile to the accumulator's "full" barrier.
-//   warps 2-5: epilogue. Warp w reads tensor-memory lanes 32*(w mod 4) .. +31 with tcgen05.ld, 32
-//     columns at a time, applies the fused epilogue and writes whole rows through shared memory
-//     (block_store_*), then releases the accumulator ("empty", four arrivals), so the products of
-//     the next tile overlap the epilogue of this one.
+//   warps 2-9: epilogue. Warp w reads tensor-memory lanes 32*(w mod 4) .. +31 with tcgen05.ld, 16
+//     columns at a time (two warps share a lane quarter's columns: the activations are some fifty
+//     instructions an output; with one warp the 4096 x 1024 layer took 42 us, with two 29, with
+//     four 26 but the small layers 0.8 us more each),
+//     applies the fused epilogue and writes whole sectors through shared memory (block_store_*), then
+//     releases the accumulator ("empty"), so the products of the next tile overlap the epilogue of
+//     this one.
+//   warps 10-11: the launch's column sums (bias gradients), beside the products.
+// The backward pass of a layer is one launch: its weight gradient, the signal of the layer below and
+// its bias gradient all read the same dZ. Launched with programmatic serialization: barriers and
+// tensor memory are set up while the previous launch ends. The next launch is let in only after this
+// CTA holds its tensor memory, so a later CTA can never take columns that an earlier one waits for.
 // Every wait is bounded; a role that runs out records the error and stops, which bounds the waits
 // of the others; tensor memory is freed at the end in every case.
 //
@@ -180,19 +250,16 @@ __device__ __forceinline__ void block_store_bf16(float* st, const uint32_t (&w)[
 // instruction (32 rows apart) and tiles of 128 columns the first took 41.7 us and a
 // training step of the second shape 85 us a product; now 10.7 and 34 us (profiler, cold caches), and the
 // fit network's training step 573 -> 245 us.
-__global__ void __launch_bounds__(192, 1) k_gemm_tn(const __grid_constant__ CUtensorMap mapA,
-                                                   const __grid_constant__ CUtensorMap mapB, GemmArgs g, uint32_t tn)
+__global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_constant__ GemmLaunch p)
 {
     extern __shared__ uint8_t smem_raw[];
     __shared__ unsigned long long full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t aBytes = kTileM * kTileK * 2, stageBytes = stage_bytes(tn);
-    const uint32_t mtiles = (g.M + kTileM - 1) / kTileM, ntiles = (g.N + tn - 1) / tn, tiles = mtiles * ntiles;
-    const uint32_t nk = (g.K + kTileK - 1) / kTileK;
-    const uint32_t S = ring_stages(tn, nk);
-    if (warp == 0) tc_alloc(&tmem_slot, 2 * tn);
+    constexpr uint32_t aBytes = kTileM * kTileK * 2;
+    const uint32_t tiles = p.tiles[0] + p.tiles[1], S = p.stages;
+    if (warp == 0) tc_alloc(&tmem_slot, 2 * p.acc_cols);
     if (tid == 0) {
         for (uint32_t s = 0; s < S; ++s) {
             tc_bar_init(&full[s], 1);
@@ -200,25 +267,28 @@ __global__ void __launch_bounds__(192, 1) k_gemm_tn(const __grid_constant__ CUte
         }
         for (uint32_t a = 0; a < 2; ++a) {
             tc_bar_init(&acc_full[a], 1);
-            tc_bar_init(&acc_empty[a], 4);
+            tc_bar_init(&acc_empty[a], kEpiWarps);
         }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    griddep_launch_dependents();
+    griddep_wait();
     bool ok = true;
     if (warp == 0 && lane == 0) {  // producer
         uint32_t s = 0, round = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-            const uint32_t m0 = (t % mtiles) * kTileM, n0 = (t / mtiles) * tn;
-            for (uint32_t c = 0; c < nk && ok; ++c) {
+            const TileAt x = tile_at(p, t);
+            const uint32_t bytes = aBytes + x.tn * kTileK * 2;
+            for (uint32_t c = 0; c < x.nk && ok; ++c) {
                 if (round > 0) ok = tc_bar_wait(&empty[s], (round - 1) & 1u);
                 if (!ok) break;
-                uint8_t* sa = smem + s * stageBytes;
-                tc_bar_expect_tx(&full[s], stageBytes);
-                tc_tma_load_2d(sa, &mapA, (int32_t)(c * kTileK), (int32_t)m0, &full[s]);
-                tc_tma_load_2d(sa + aBytes, &mapB, (int32_t)(c * kTileK), (int32_t)n0, &full[s]);
+                uint8_t* sa = smem + s * p.stage_size;
+                tc_bar_expect_tx(&full[s], bytes);
+                tc_tma_load_2d(sa, &p.map[x.q][0], (int32_t)(c * kTileK), (int32_t)x.m0, &full[s]);
+                tc_tma_load_2d(sa + aBytes, &p.map[x.q][1], (int32_t)(c * kTileK), (int32_t)x.n0, &full[s]);
                 if (++s == S) {
                     s = 0;
                     ++round;
@@ -228,17 +298,18 @@ __global__ void __launch_bounds__(192, 1) k_gemm_tn(const __grid_constant__ CUte
     } else if (warp == 1 && lane == 0) {  // tensor-core issuer
         uint32_t s = 0, round = 0, li = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++li) {
-            const uint32_t n0 = (t / mtiles) * tn, nt = min(tn, g.N - n0), a = li & 1u;
+            const TileAt x = tile_at(p, t);
+            const uint32_t a = li & 1u, K = p.g[x.q].K;
             if (li >= 2) ok = tc_bar_wait(&acc_empty[a], ((li >> 1) - 1) & 1u);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t idesc = tc_idesc_bf16(kTileM, nt), d = tmem + a * tn;
-            for (uint32_t c = 0; c < nk; ++c) {
+            const uint32_t idesc = tc_idesc_bf16(kTileM, x.nt), d = tmem + a * p.acc_cols;
+            for (uint32_t c = 0; c < x.nk; ++c) {
                 ok = tc_bar_wait(&full[s], round & 1u);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t sa = tc_smem(smem + s * stageBytes), sb = sa + aBytes;
-                const uint32_t ks = min(4u, (g.K - c * kTileK + 15) / 16);
+                const uint32_t sa = tc_smem(smem + s * p.stage_size), sb = sa + aBytes;
+                const uint32_t ks = min(4u, (K - c * kTileK + 15) / 16);
                 for (uint32_t kk = 0; kk < ks; ++kk)
                     tc_mma(d, tc_desc_sw128(sa + kk * 32), tc_desc_sw128(sb + kk * 32), idesc, c > 0 || kk > 0);
                 tc_commit(&empty[s]);
@@ -249,59 +320,99 @@ __global__ void __launch_bounds__(192, 1) k_gemm_tn(const __grid_constant__ CUte
             }
             tc_commit(&acc_full[a]);
         }
-    } else if (warp >= 2) {  // epilogue
-        const uint32_t quarter = warp & 3u;
-        float* st = reinterpret_cast<float*>(smem + S * stageBytes) + quarter * 32 * kEpiPitch;
+    } else if (warp >= 2 && warp < 2 + kEpiWarps) {  // epilogue
+        const uint32_t quarter = warp & 3u, part = (warp - 2) >> 2;
+        float* st = reinterpret_cast<float*>(smem + S * p.stage_size) + (warp - 2) * 32 * kEpiPitch;
+        constexpr uint32_t kStep = 16 * (kEpiWarps / 4);  // columns between a warp's blocks
         uint32_t li = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++li) {
-            const uint32_t m0 = (t % mtiles) * kTileM, n0 = (t / mtiles) * tn, nt = min(tn, g.N - n0), a = li & 1u;
-            const uint32_t r0 = m0 + quarter * 32, row = r0 + lane;
+            const TileAt x = tile_at(p, t);
+            const GemmArgs& g = p.g[x.q];
+            const uint32_t a = li & 1u, n0 = x.n0, nt = x.nt;
+            const uint32_t r0 = x.m0 + quarter * 32;
             const uint32_t rows = r0 < g.M ? min(32u, g.M - r0) : 0u;
-            float4 zf[8];  // pre-activations of the next block, in flight while the current one is done
-            if (g.epi == kEpiBackward)
-                block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n0, g.ldz, rows, min(32u, nt), lane);
+            float4 zf[4];  // pre-activations of the next block, in flight while the current one is done
+            if (g.epi == kEpiBackward && part * 16 < nt)
+                block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n0 + part * 16, g.ldz, rows, lane);
+            float e2 = 0.0f;
             ok = __all_sync(0xffffffffu, tc_bar_wait(&acc_full[a], (li >> 1) & 1u));  // warp-uniform
             if (!ok) break;
             tc_fence_after();
-            for (uint32_t c0 = 0; c0 < nt; c0 += 32) {
-                const uint32_t n = n0 + c0, cols = min(32u, nt - c0);
-                float v[32], z[32];
-                uint32_t w[16];
-                tc_ld32(tmem + a * tn + ((quarter * 32u) << 16) + c0, v);
+            for (uint32_t c0 = part * 16; c0 < nt; c0 += kStep) {
+                const uint32_t n = n0 + c0;
+                float v[16], z[16];
+                uint32_t w[8];
+                if (g.epi == kEpiLoss) {  // targets of the block, two rows per instruction
+#pragma unroll
+                    for (int it = 0; it < 16; ++it) {
+                        const uint32_t r = 2 * it + (lane >> 4), c = n + (lane & 15u);
+                        z[it] = (r < rows && c < g.nout) ? g.target[(size_t)(r0 + r) * g.nout + c] : 0.0f;
+                    }
+                }
+                tc_ld16(tmem + a * p.acc_cols + ((quarter * 32u) << 16) + c0, v);
+                if (g.epi == kEpiHidden || g.epi == kEpiLinear || g.epi == kEpiLoss) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + n) + k);
+                        v[4 * k] += b.x;
+                        v[4 * k + 1] += b.y;
+                        v[4 * k + 2] += b.z;
+                        v[4 * k + 3] += b.w;
+                    }
+                }
                 if (g.epi == kEpiHidden) {
+                    block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, lane);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] += (uint32_t)j < cols ? __ldg(&g.bias[n + j]) : 0.0f;
-                    block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, cols, lane);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) w[j] = pack_bf16(silu(v[2 * j]), silu(v[2 * j + 1]));
+                    for (int j = 0; j < 8; ++j) w[j] = pack_bf16(silu(v[2 * j]), silu(v[2 * j + 1]));
                 } else if (g.epi == kEpiBackward) {
                     block_spread_f32(st, zf, z, lane);
-                    if (c0 + 32 < nt)
-                        block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n + 32, g.ldz, rows, min(32u, nt - c0 - 32), lane);
+                    if (c0 + kStep < nt)
+                        block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n + kStep, g.ldz, rows, lane);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
+                    for (int j = 0; j < 8; ++j)
                         w[j] = pack_bf16(v[2 * j] * dsilu(z[2 * j]), v[2 * j + 1] * dsilu(z[2 * j + 1]));
-                } else {
-                    if (g.epi == kEpiLinear) {
+                } else if (g.epi == kEpiLoss) {
+                    // Mean squared error over the real outputs and its gradient 2 (Y - T) / (rows * nout).
+                    const float cells = (float)(g.M * g.nout);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] += (uint32_t)j < cols ? __ldg(&g.bias[n + j]) : 0.0f;
+                    for (int it = 0; it < 16; ++it) st[(2 * it + (lane >> 4)) * kEpiPitch + (lane & 15u)] = z[it];
+                    __syncwarp();
+                    block_row_f32(st, z, lane);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        float grad = 0.0f;
+                        if (lane < rows && n + j < g.nout) {
+                            const float e = v[j] - z[j];
+                            e2 += e * e;
+                            grad = 2.0f * e / cells;
+                        }
+                        v[j] = grad;
                     }
-                    block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, cols, lane);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
+                } else {
+                    block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, lane);
                 }
-                if (g.epi == kEpiHidden || g.epi == kEpiBackward)
+                if (g.epi == kEpiHidden || g.epi == kEpiBackward || g.epi == kEpiLoss)
                     block_store_bf16(st, w, g.outb + (size_t)r0 * g.ldob + n, g.ldob, g.outt + (size_t)n * g.ldot + r0,
-                                     g.ldot, rows, cols, lane);
+                                     g.ldot, rows, lane);
+            }
+            if (g.epi == kEpiLoss) {
+                for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+                if (lane == 0 && e2 != 0.0f) atomicAdd(g.loss, e2 / (float)(g.M * g.nout));
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) tc_bar_arrive(&acc_empty[a]);
         }
+    } else if (warp >= 2 + kEpiWarps && p.cs.cols) {
+        column_sums(p.cs, blockIdx.x * 2 + (warp - 2 - kEpiWarps), gridDim.x * 2, lane);
     }
-    if (!ok) atomicOr(g.err, 1u);
+    if (!ok) atomicOr(p.err, 1u);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tc_dealloc(tmem, 2 * tn);
+    if (warp == 0) tc_dealloc(tmem, 2 * p.acc_cols);
 }
 
 // Tensor map of a row-major BF16 matrix [rows][ld] whose first `cols` columns are the operand:
@@ -332,46 +443,79 @@ int tensor_map(CUtensorMap* map, const bf16* base, uint32_t rows, uint32_t cols,
     return ARBO_OK;
 }
 
-// Columns per tile of an M x N x K product on num_sm SMs. A CTA's time on a tile is modelled as a
-// fixed part, its operand loads (128 + tn rows of 128 bytes per K chunk) and its epilogue (32
-// columns at a time); the tiles fill whole waves of SMs, so the narrow tiles win while the wide
-// ones leave SMs idle (a 256 x 512 layer: 32 tiles of 32 columns instead of 8 of 128) and the wide
-// ones once every SM has work (fewer operand loads per output).
-uint32_t tile_cols(uint32_t M, uint32_t N, uint32_t K, uint32_t num_sm)
+uint32_t tile_count(const GemmArgs& g, uint32_t tn)
 {
-    const uint64_t mt = (M + kTileM - 1) / kTileM, nk = (K + kTileK - 1) / kTileK;
-    uint32_t best = kMinTileN;
-    uint64_t best_cost = ~0ull;
-    for (uint32_t tn = kMinTileN; tn <= kMaxTileN; tn *= 2) {
-        const uint64_t tiles = mt * ((N + tn - 1) / tn), waves = (tiles + num_sm - 1) / num_sm;
-        const uint64_t cost = 2000 + waves * (nk * (128 + tn) * 2 + 500 * (tn / 32));
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = tn;
+    return ((g.M + kTileM - 1) / kTileM) * ((g.N + tn - 1) / tn);
+}
+
+// Model of a CTA's time on one tile (cycles): its operand loads, (128 + tn) rows of 128 bytes per K
+// chunk, and its epilogue, 32 columns at a time.
+uint64_t tile_cost(const GemmArgs& g, uint32_t tn)
+{
+    return (uint64_t)((g.K + kTileK - 1) / kTileK) * (kTileM + tn) * 2 + 500ull * (tn / 32);
+}
+
+// Columns per tile of each of the n products of a launch on num_sm SMs: the pair with the smallest
+// modelled time. Narrow tiles win while wide ones leave SMs idle (a 256 x 512 layer: 32 tiles of 32
+// columns instead of 8 of 128), wide ones once every SM has work (fewer operand loads per output):
+// the step of a 1024-wide network at 4,096 rows took 570, 522, 496 and 450 us with forward tiles and
+// backward pairs of 32, 64, 128 and 256 columns, and 480 us with the long weight-gradient tiles first.
+void choose_tiles(const GemmArgs* g, uint32_t n, uint32_t num_sm, uint32_t (&tn)[2])
+{
+    uint64_t best = ~0ull;
+    for (uint32_t a = kMinTileN; a <= kMaxTileN; a *= 2)
+        for (uint32_t b = kMinTileN; b <= (n > 1 ? kMaxTileN : kMinTileN); b *= 2) {
+            const uint64_t ca = tile_cost(g[0], a), cb = n > 1 ? tile_cost(g[1], b) : 0;
+            const uint64_t ta = tile_count(g[0], a), tb = n > 1 ? tile_count(g[1], b) : 0;
+            const uint64_t waves = (ta + tb + num_sm - 1) / num_sm;
+            // One product fills whole waves; two of different cost fill the gaps of each other.
+            const uint64_t cost = waves <= 1 ? std::max(ca, cb)
+                                  : n == 1   ? waves * ca
+                                             : (ta * ca + tb * cb) / num_sm + std::max(ca, cb) / 2;
+            if (cost < best) {
+                best = cost;
+                tn[0] = a;
+                tn[1] = b;
+            }
         }
+}
+
+// Launches one or two independent products (g[i]: C = A B^T with its epilogue) and optional column
+// sums on persistent CTAs, at most one per SM. Returns a cudaError_t (invalid value when a tensor map
+// cannot be built; the reason is then in arbo_last_error).
+int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* err, cudaStream_t st, uint32_t num_sm,
+                bool pdl)
+{
+    GemmLaunch p{};
+    uint32_t nk = 0;
+    choose_tiles(g, n, num_sm, p.tn);
+    for (uint32_t i = 0; i < n; ++i) {
+        p.g[i] = g[i];
+        p.tiles[i] = tile_count(g[i], p.tn[i]);
+        if (tensor_map(&p.map[i][0], g[i].A, g[i].M, g[i].K, g[i].lda, kTileM) ||
+            tensor_map(&p.map[i][1], g[i].B, g[i].N, g[i].K, g[i].ldb, p.tn[i]))
+            return (int)cudaErrorInvalidValue;
+        p.acc_cols = std::max(p.acc_cols, p.tn[i]);
+        nk = std::max(nk, (g[i].K + kTileK - 1) / kTileK);
     }
-    return best;
+    p.stage_size = (kTileM + p.acc_cols) * kTileK * 2;
+    p.stages = std::min({kStageBudget / p.stage_size, kMaxStages, nk * (p.tiles[0] + p.tiles[1] > num_sm ? 2u : 1u)});
+    p.cs = cs;
+    p.err = err;
+    // CTAs without a tile only add column sums (eight columns each pass).
+    const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 7) / 8), num_sm);
+    return launch_pdl(k_gemm_tn, dim3(ctas), dim3(kGemmThreads),
+                      p.stages * p.stage_size + kEpiBytes + 1024, st, pdl, p);
 }
 
-// Launches C = A B^T with the epilogue of g on min(tiles, SMs) persistent CTAs. Returns a
-// cudaError_t (invalid value when a tensor map cannot be built; the reason is then in arbo_last_error).
-int gemm_launch(const GemmArgs& g, cudaStream_t st, uint32_t num_sm)
-{
-    const uint32_t mt = (g.M + kTileM - 1) / kTileM;
-    const uint32_t tn = tile_cols(g.M, g.N, g.K, num_sm);
-    CUtensorMap ma, mb;
-    if (tensor_map(&ma, g.A, g.M, g.K, g.lda, kTileM) || tensor_map(&mb, g.B, g.N, g.K, g.ldb, tn))
-        return (int)cudaErrorInvalidValue;
-    const uint32_t tiles = mt * ((g.N + tn - 1) / tn);
-    k_gemm_tn<<<tiles < num_sm ? tiles : num_sm, 192, gemm_smem(tn, (g.K + kTileK - 1) / kTileK), st>>>(ma, mb, g, tn);
-    return (int)cudaGetLastError();
-}
-
-// Inputs: FP32 [n][nin] -> BF16 [n][ldx] (zero padded) and transposed [ldx][ldt].
+// Inputs: FP32 [n][nin] -> BF16 [n][ldx] (zero padded) and transposed [ldx][ldt]; the loss is zeroed
+// for the sums of the last layer's epilogue.
 __global__ void k_stage_input(const float* __restrict__ x, uint32_t n, uint32_t nin, uint32_t ldx, bf16* xb, bf16* xt,
-                              uint32_t ldt)
+                              uint32_t ldt, float* loss)
 {
+    griddep_launch_dependents();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *loss = 0.0f;
     if (i >= n * ldx) return;
     const uint32_t r = i / ldx, c = i - r * ldx;
     const bf16 v = __float2bfloat16_rn(c < nin ? x[(size_t)r * nin + c] : 0.0f);
@@ -379,66 +523,59 @@ __global__ void k_stage_input(const float* __restrict__ x, uint32_t n, uint32_t 
     xt[(size_t)c * ldt + r] = v;
 }
 
-// Mean squared error over the real outputs and its gradient dL/dY = 2 (Y - T) / (n * nout).
-__global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t, uint32_t n, uint32_t nout,
-                       uint32_t ldy, bf16* dy, bf16* dyt, uint32_t ldt, float* loss)
+// One parameter array of the optimiser: a layer's weights [rows][cols] with their BF16 copy and its
+// transpose [cols][rows], or its bias (rows 1, no copies). `first` is its first 32 x 32 block.
+struct AdamArray {
+    float *w, *m, *v;
+    const float* g;
+    bf16 *wb, *wt;
+    uint32_t rows, cols, first;
+};
+
+// Adam (Kingma & Ba 2015) on FP32 master weights, all arrays of the network in one launch: one block
+// of 256 threads per 32 x 32 weights, the transposed copy written through shared memory. One launch
+// per array, each thread writing its own transposed element, took 48 us of the fit network's step
+// (ten launches of 3-6 us) and 70 us of a 1024-wide network's. Nothing is updated when a wait of this
+// step's products ran out (*err != 0).
+__global__ void __launch_bounds__(256) k_adam(const AdamArray* __restrict__ arrays, uint32_t count, float lr, float b1,
+                                              float b2, float eps, float c1, float c2, const uint32_t* err)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float e2 = 0.0f;
-    if (i < n * ldy) {
-        const uint32_t r = i / ldy, c = i - r * ldy;
-        float g = 0.0f;
-        if (c < nout) {
-            const float e = y[(size_t)r * ldy + c] - t[(size_t)r * nout + c];
-            e2 = e * e;
-            g = 2.0f * e / (float)(n * nout);
+    __shared__ uint16_t tile[32][33];
+    uint32_t lo = 0, hi = count - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (arrays[mid].first <= blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const AdamArray a = arrays[lo];
+    griddep_wait();
+    if (*err) return;
+    const uint32_t cb = (a.cols + 31) / 32, k = blockIdx.x - a.first;
+    const uint32_t r0 = (k / cb) * 32, col = (k % cb) * 32 + (threadIdx.x & 31u);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t rr = (threadIdx.x >> 5) + 8 * j, r = r0 + rr;
+        if (r >= a.rows || col >= a.cols) continue;
+        const size_t i = (size_t)r * a.cols + col;
+        const float gi = a.g[i];
+        const float mi = b1 * a.m[i] + (1.0f - b1) * gi;
+        const float vi = b2 * a.v[i] + (1.0f - b2) * gi * gi;
+        a.m[i] = mi;
+        a.v[i] = vi;
+        const float wi = a.w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        a.w[i] = wi;
+        if (a.wb) {
+            const bf16 b = __float2bfloat16_rn(wi);
+            a.wb[i] = b;
+            tile[rr][threadIdx.x & 31u] = __bfloat16_as_ushort(b);
         }
-        const bf16 gb = __float2bfloat16_rn(g);
-        dy[(size_t)r * ldy + c] = gb;
-        dyt[(size_t)c * ldt + r] = gb;
     }
-    // One atomic per block: one per warp kept the kernel at 96 us on 4096 x 480 outputs (61,440
-    // additions to one address).
-    __shared__ float part[8];
-    for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = e2;
+    if (!a.wb) return;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.0f;
-        for (uint32_t w = 0; w < 8; ++w) s += part[w];
-        if (s != 0.0f) atomicAdd(loss, s / (float)(n * nout));
-    }
-}
-
-// Bias gradient: db[c] = sum over rows of dZ, from the transposed copy (one warp per column).
-__global__ void k_bias_grad(const bf16* __restrict__ dzt, uint32_t ldt, uint32_t n, uint32_t cols, float* db)
-{
-    const uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (uint32_t r = lane; r < n; r += 32) s += __bfloat162float(dzt[(size_t)c * ldt + r]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) db[c] = s;
-}
-
-// Adam (Kingma & Ba 2015) on FP32 master weights; writes the BF16 copy and its transpose.
-__global__ void k_adam(float* w, float* m, float* v, const float* __restrict__ g, uint32_t count, uint32_t rows,
-                       uint32_t cols, bf16* wb, bf16* wt, float lr, float b1, float b2, float eps, float c1, float c2)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) {
-        const uint32_t r = i / cols, c = i - r * cols;
-        const bf16 b = __float2bfloat16_rn(wi);
-        wb[i] = b;
-        wt[(size_t)c * rows + r] = b;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t cc = (threadIdx.x >> 5) + 8 * j, c = (k % cb) * 32 + cc, r = r0 + (threadIdx.x & 31u);
+        if (c < a.cols && r < a.rows)
+            a.wt[(size_t)c * a.rows + r] = __ushort_as_bfloat16(tile[threadIdx.x & 31u][cc]);
     }
 }
 
@@ -480,64 +617,91 @@ struct arbo_mlp {
     uint32_t* err = nullptr;
     uint32_t steps = 0;
     uint32_t num_sm = 152;
+    AdamArray* adam = nullptr;         // device table of the optimiser's arrays
+    uint32_t adam_arrays = 0, adam_blocks = 0;
     std::vector<void*> allocs;
 };
 
 namespace {
 
-int mlp_gemm(arbo_mlp* n, const bf16* A, uint32_t lda, const bf16* B, uint32_t ldb, uint32_t M, uint32_t N,
-             uint32_t K, int epi, const float* bias, const float* zprev, uint32_t ldz, float* outf, uint32_t ldof,
-             bf16* outb, uint32_t ldob, bf16* outt, uint32_t ldot, cudaStream_t st)
+// train: the last layer's epilogue goes straight to the loss and its gradient (no outputs kept).
+int mlp_forward(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
 {
-    GemmArgs g{A, B, lda, ldb, M, N, K, epi, bias, zprev, ldz, outf, ldof, outb, ldob, outt, ldot, n->err};
-    return gemm_launch(g, st, n->num_sm);
-}
-
-int mlp_forward(arbo_mlp* n, uint32_t rows, cudaStream_t st)
-{
-    const uint32_t ld = n->maxb;
-    k_stage_input<<<(rows * n->dim[0] + 255) / 256, 256, 0, st>>>(n->xin, rows, n->nin, n->dim[0], n->x, n->xt, ld);
-    const bf16* a = n->x;
-    for (uint32_t l = 0; l < n->L; ++l) {
+    const uint32_t ld = n->maxb, L = n->L;
+    k_stage_input<<<(rows * n->dim[0] + 255) / 256, 256, 0, st>>>(n->xin, rows, n->nin, n->dim[0], n->x, n->xt, ld, n->loss);
+    int e = (int)cudaGetLastError();
+    for (uint32_t l = 0; l < L && !e; ++l) {
         const uint32_t in = n->dim[l], out = n->dim[l + 1];
-        int e;
-        if (l + 1 < n->L)
-            e = mlp_gemm(n, a, in, n->wb[l], in, rows, out, in, kEpiHidden, n->b[l], nullptr, 0, n->z[l], out, n->h[l],
-                         out, n->ht[l], ld, st);
-        else
-            e = mlp_gemm(n, a, in, n->wb[l], in, rows, out, in, kEpiLinear, n->b[l], nullptr, 0, n->y, out, nullptr, 0,
-                         nullptr, 0, st);
-        if (e) return e;
-        if (l + 1 < n->L) a = n->h[l];
+        GemmArgs g{};
+        g.A = l == 0 ? n->x : n->h[l - 1];
+        g.B = n->wb[l];
+        g.lda = g.ldb = in;
+        g.M = rows;
+        g.N = out;
+        g.K = in;
+        g.bias = n->b[l];
+        g.ldof = g.ldob = out;
+        g.ldot = ld;
+        if (l + 1 < L) {
+            g.epi = kEpiHidden;
+            g.outf = n->z[l];
+            g.outb = n->h[l];
+            g.outt = n->ht[l];
+        } else if (train) {
+            g.epi = kEpiLoss;
+            g.outb = n->d0;
+            g.outt = n->d0t;
+            g.target = n->tin;
+            g.nout = n->nout;
+            g.loss = n->loss;
+        } else {
+            g.epi = kEpiLinear;
+            g.outf = n->y;
+        }
+        e = gemm_launch(&g, 1, ColumnSums{}, n->err, st, n->num_sm, true);
     }
-    return 0;
+    return e;
 }
 
+// One launch per layer: dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}) (M = rows, N = in, K = out), dW_l =
+// dZ_l^T H_{l-1} (M = out, N = in, K = rows) and db_l = column sums of dZ_l.
 int mlp_backward(arbo_mlp* n, uint32_t rows, cudaStream_t st)
 {
     const uint32_t ld = n->maxb, L = n->L;
-    cudaMemsetAsync(n->loss, 0, 4, st);
-    const uint32_t outw = n->dim[L];
-    k_loss<<<(rows * outw + 255) / 256, 256, 0, st>>>(n->y, n->tin, rows, n->nout, outw, n->d0, n->d0t, ld, n->loss);
     bf16 *dz = n->d0, *dzt = n->d0t, *nd = n->d1, *ndt = n->d1t;
-    for (uint32_t l = L; l-- > 0;) {
+    int e = 0;
+    for (uint32_t l = L; l-- > 0 && !e;) {
         const uint32_t in = n->dim[l], out = n->dim[l + 1];
-        const bf16* hprevt = l == 0 ? n->xt : n->ht[l - 1];
-        // dW_l = dZ^T H_{l-1}: M = out, N = in, K = rows.
-        int e = mlp_gemm(n, dzt, ld, hprevt, ld, out, in, rows, kEpiStore, nullptr, nullptr, 0, n->dw[l], in, nullptr,
-                         0, nullptr, 0, st);
-        if (e) return e;
-        k_bias_grad<<<(out + 7) / 8, 256, 0, st>>>(dzt, ld, rows, out, n->db[l]);
+        GemmArgs g[2] = {};
+        GemmArgs& w = g[l > 0 ? 1 : 0];
+        w.A = dzt;
+        w.B = l == 0 ? n->xt : n->ht[l - 1];
+        w.lda = w.ldb = ld;
+        w.M = out;
+        w.N = in;
+        w.K = rows;
+        w.epi = kEpiStore;
+        w.outf = n->dw[l];
+        w.ldof = in;
         if (l > 0) {
-            // dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}): M = rows, N = in, K = out.
-            e = mlp_gemm(n, dz, out, n->wt[l], out, rows, in, out, kEpiBackward, nullptr, n->z[l - 1], in, nullptr, 0,
-                         nd, in, ndt, ld, st);
-            if (e) return e;
-            std::swap(dz, nd);
-            std::swap(dzt, ndt);
+            g[0].A = dz;
+            g[0].B = n->wt[l];
+            g[0].lda = g[0].ldb = out;
+            g[0].M = rows;
+            g[0].N = in;
+            g[0].K = out;
+            g[0].epi = kEpiBackward;
+            g[0].zprev = n->z[l - 1];
+            g[0].ldz = g[0].ldob = in;
+            g[0].outb = nd;
+            g[0].outt = ndt;
+            g[0].ldot = ld;
         }
+        e = gemm_launch(g, l > 0 ? 2 : 1, ColumnSums{dzt, ld, rows, out, n->db[l]}, n->err, st, n->num_sm, true);
+        std::swap(dz, nd);
+        std::swap(dzt, ndt);
     }
-    return (int)cudaGetLastError();
+    return e;
 }
 
 int mlp_upload(arbo_mlp* n, const float* x, const float* t, uint32_t rows, cudaStream_t st)
@@ -652,6 +816,21 @@ int arbo_mlp_create(uint32_t n_in, uint32_t hidden, uint32_t hidden_layers, uint
         arbo_mlp_destroy(n);
         return ufail(ARBO_ERR_ALLOC, "arbo_mlp_create: device allocation failed");
     }
+    std::vector<AdamArray> arrays;
+    for (uint32_t l = 0; l < n->L; ++l) {
+        const uint32_t in = n->dim[l], o = n->dim[l + 1];
+        arrays.push_back({n->w[l], n->mw[l], n->vw[l], n->dw[l], n->wb[l], n->wt[l], o, in, n->adam_blocks});
+        n->adam_blocks += ((o + 31) / 32) * ((in + 31) / 32);
+        arrays.push_back({n->b[l], n->mb[l], n->vb[l], n->db[l], nullptr, nullptr, 1, o, n->adam_blocks});
+        n->adam_blocks += (o + 31) / 32;
+    }
+    n->adam_arrays = (uint32_t)arrays.size();
+    n->adam = (AdamArray*)alloc(arrays.size() * sizeof(AdamArray));
+    if (!n->adam) {
+        arbo_mlp_destroy(n);
+        return ufail(ARBO_ERR_ALLOC, "arbo_mlp_create: device allocation failed");
+    }
+    UCUDA(cudaMemcpy(n->adam, arrays.data(), arrays.size() * sizeof(AdamArray), cudaMemcpyHostToDevice));
     UCUDA(cudaDeviceSynchronize());
     *out = n;
     return ARBO_OK;
@@ -682,7 +861,7 @@ int arbo_mlp_forward(arbo_mlp* n, const float* x, uint32_t rows, float* y, void*
     cudaStream_t st = (cudaStream_t)stream;
     int e = mlp_upload(n, x, nullptr, rows, st);
     if (e) return e;
-    if ((e = mlp_forward(n, rows, st))) return ufail(ARBO_ERR_CUDA, std::string("forward: ") + cudaGetErrorString((cudaError_t)e));
+    if ((e = mlp_forward(n, rows, false, st))) return ufail(ARBO_ERR_CUDA, std::string("forward: ") + cudaGetErrorString((cudaError_t)e));
     const uint32_t w = n->dim[n->L];
     if (w == n->nout) {
         UCUDA(cudaMemcpyAsync(y, n->y, (size_t)rows * w * 4, cudaMemcpyDeviceToHost, st));
@@ -699,7 +878,7 @@ int arbo_mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t row
     cudaStream_t st = (cudaStream_t)stream;
     int e = mlp_upload(n, x, t, rows, st);
     if (e) return e;
-    if ((e = mlp_forward(n, rows, st)) || (e = mlp_backward(n, rows, st)))
+    if ((e = mlp_forward(n, rows, true, st)) || (e = mlp_backward(n, rows, st)))
         return ufail(ARBO_ERR_CUDA, std::string("forward/backward: ") + cudaGetErrorString((cudaError_t)e));
     if (loss) UCUDA(cudaMemcpyAsync(loss, n->loss, 4, cudaMemcpyDeviceToHost, st));
     return mlp_check_err(n, st);
@@ -713,13 +892,7 @@ int arbo_mlp_train_step(arbo_mlp* n, const float* x, const float* t, uint32_t ro
     n->steps += 1;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.0f - std::pow(b1, (float)n->steps), c2 = 1.0f - std::pow(b2, (float)n->steps);
-    for (uint32_t l = 0; l < n->L; ++l) {
-        const uint32_t in = n->dim[l], o = n->dim[l + 1], cnt = in * o;
-        k_adam<<<(cnt + 255) / 256, 256, 0, st>>>(n->w[l], n->mw[l], n->vw[l], n->dw[l], cnt, o, in, n->wb[l], n->wt[l],
-                                                  lr, b1, b2, eps, c1, c2);
-        k_adam<<<(o + 255) / 256, 256, 0, st>>>(n->b[l], n->mb[l], n->vb[l], n->db[l], o, 1, o, nullptr, nullptr, lr, b1,
-                                                b2, eps, c1, c2);
-    }
+    k_adam<<<n->adam_blocks, 256, 0, st>>>(n->adam, n->adam_arrays, lr, b1, b2, eps, c1, c2, n->err);
     UCUDA(cudaGetLastError());
     return ARBO_OK;
 }
@@ -781,17 +954,26 @@ int arbo_tc_gemm(const float* a, const float* b, uint32_t M, uint32_t N, uint32_
     cudaMemcpy(da, ha.data(), ha.size() * 2, cudaMemcpyHostToDevice);
     cudaMemcpy(db, hb.data(), hb.size() * 2, cudaMemcpyHostToDevice);
     cudaMemset(derr, 0, 4);
-    GemmArgs g{da, db, K, K, M, N, K, kEpiStore, nullptr, nullptr, 0, dc, N, nullptr, 0, nullptr, 0, derr};
+    GemmArgs g{};
+    g.A = da;
+    g.B = db;
+    g.lda = g.ldb = K;
+    g.M = M;
+    g.N = g.ldof = N;
+    g.K = K;
+    g.epi = kEpiStore;
+    g.outf = dc;
     int sms = 152, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    int le = gemm_launch(g, nullptr, (uint32_t)sms);
+    auto product = [&]() { return gemm_launch(&g, 1, ColumnSums{}, derr, nullptr, (uint32_t)sms, false); };
+    int le = product();
     const std::string map_err = le ? std::string(arbo_last_error()) : std::string();
     cudaEventRecord(e0);
-    for (uint32_t r = 0; r < reps && !le; ++r) le = gemm_launch(g, nullptr, (uint32_t)sms);
+    for (uint32_t r = 0; r < reps && !le; ++r) le = product();
     cudaEventRecord(e1);
     cudaError_t ce = cudaEventSynchronize(e1);
     float t = 0;
