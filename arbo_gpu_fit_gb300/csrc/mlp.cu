@@ -74,8 +74,8 @@ struct GemmLaunch {
 constexpr uint32_t kTileM = 128, kTileK = 64, kMaxStages = 8;
 constexpr uint32_t kMinTileN = 32, kMaxTileN = 256;
 constexpr uint32_t kStageBudget = 192 * 1024;  // shared memory of the operand ring
-constexpr uint32_t kEpiWarps = 8;             // two per quarter of the 128 tensor-memory lanes
-constexpr uint32_t kEpiPitch = 20;             // words per staged row of 16 columns
+constexpr uint32_t kEpiWarps = 16;  // four per quarter of the 128 tensor-memory lanes
+constexpr uint32_t kEpiPitch = 12;  // words per staged row of 8 columns
 constexpr uint32_t kEpiBytes = kEpiWarps * 32 * kEpiPitch * 4;  // one staging block per epilogue warp
 constexpr uint32_t kGemmThreads = 64 + kEpiWarps * 32 + 64;
 
@@ -96,40 +96,40 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
            ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
 }
 
-// The epilogue's copies between a warp's block of 32 rows (one per lane) and 16 columns and row-major
-// global memory, through the warp's staging block, so that a warp instruction touches whole sectors:
-// eight 64-byte FP32 rows or sixteen 32-byte BF16 rows. `rows` is the number of live rows.
-__device__ __forceinline__ void block_store_f32(float* st, const float (&v)[16], float* out, uint32_t ld, uint32_t rows,
+// The epilogue's copies between a warp's block of 32 rows (one per lane) and 8 columns and row-major
+// FP32 memory, through the warp's staging block, so that a warp instruction touches sixteen whole
+// 32-byte sectors. `rows` is the number of live rows.
+__device__ __forceinline__ void block_store_f32(float* st, const float (&v)[8], float* out, uint32_t ld, uint32_t rows,
                                                 uint32_t lane)
 {
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 2; ++k)
         *reinterpret_cast<float4*>(st + lane * kEpiPitch + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     __syncwarp();
-    const uint32_t c = (lane & 3u) * 4;
+    const uint32_t c = (lane & 1u) * 4;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const uint32_t r = it * 8 + (lane >> 2);
+    for (int it = 0; it < 2; ++it) {
+        const uint32_t r = it * 16 + (lane >> 1);
         if (r < rows)
             *reinterpret_cast<float4*>(out + (size_t)r * ld + c) = *reinterpret_cast<const float4*>(st + r * kEpiPitch + c);
     }
     __syncwarp();
 }
 
-__device__ __forceinline__ void block_fetch_f32(float4 (&f)[4], const float* in, uint32_t ld, uint32_t rows, uint32_t lane)
+__device__ __forceinline__ void block_fetch_f32(float4 (&f)[2], const float* in, uint32_t ld, uint32_t rows, uint32_t lane)
 {
-    const uint32_t c = (lane & 3u) * 4;
+    const uint32_t c = (lane & 1u) * 4;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const uint32_t r = it * 8 + (lane >> 2);
+    for (int it = 0; it < 2; ++it) {
+        const uint32_t r = it * 16 + (lane >> 1);
         f[it] = r < rows ? *reinterpret_cast<const float4*>(in + (size_t)r * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 
-__device__ __forceinline__ void block_row_f32(const float* st, float (&v)[16], uint32_t lane)
+__device__ __forceinline__ void block_row_f32(const float* st, float (&v)[8], uint32_t lane)
 {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 2; ++k) {
         const float4 x = *reinterpret_cast<const float4*>(st + lane * kEpiPitch + 4 * k);
         v[4 * k] = x.x;
         v[4 * k + 1] = x.y;
@@ -139,11 +139,11 @@ __device__ __forceinline__ void block_row_f32(const float* st, float (&v)[16], u
     __syncwarp();
 }
 
-__device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[4], float (&v)[16], uint32_t lane)
+__device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[2], float (&v)[8], uint32_t lane)
 {
-    const uint32_t c = (lane & 3u) * 4;
+    const uint32_t c = (lane & 1u) * 4;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) *reinterpret_cast<float4*>(st + (it * 8 + (lane >> 2)) * kEpiPitch + c) = f[it];
+    for (int it = 0; it < 2; ++it) *reinterpret_cast<float4*>(st + (it * 16 + (lane >> 1)) * kEpiPitch + c) = f[it];
     __syncwarp();
     block_row_f32(st, v, lane);
 }
@@ -152,51 +152,40 @@ __device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[4]
 // the lane's row advancing along it). w[j] packs columns 2j and 2j+1 of the lane's row; neighbouring
 // lanes swap halves so that each store of the transposed copy carries two rows of one column. Rows come
 // in pairs: the products with a transposed copy have a multiple of 16 of them.
-__device__ __forceinline__ void block_store_bf16(float* st, const uint32_t (&w)[8], bf16* out, uint32_t ld, bf16* outt,
-                                                 uint32_t ldt, uint32_t rows, uint32_t lane)
+__device__ __forceinline__ void block_store_bf16(const uint32_t (&w)[4], bf16* out, uint32_t ld, bf16* outt, uint32_t ldt,
+                                                 uint32_t rows, uint32_t lane)
 {
-    uint32_t* sw = reinterpret_cast<uint32_t*>(st);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        *reinterpret_cast<uint4*>(sw + lane * 12 + 4 * k) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
-    __syncwarp();
+    if (lane < rows) *reinterpret_cast<uint4*>(out + (size_t)lane * ld) = make_uint4(w[0], w[1], w[2], w[3]);
     const uint32_t c = lane & 1u;
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const uint32_t r = it * 16 + (lane >> 1);
-        if (r < rows)
-            *reinterpret_cast<uint4*>(out + (size_t)r * ld + 8 * c) = *reinterpret_cast<const uint4*>(sw + r * 12 + 4 * c);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 4; ++j) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, w[j], 1);
         const uint32_t v = c ? __byte_perm(other, w[j], 0x7632) : __byte_perm(w[j], other, 0x5410);
         if (lane < rows) *reinterpret_cast<uint32_t*>(outt + (size_t)(2 * j + c) * ldt + lane - c) = v;
     }
 }
 
-// Column sums by the warps w, w + nw, ... of the launch, four columns at a time so that a warp keeps
-// 32 loads in flight. Each column is summed by lane-strided rows, then across the lanes.
+// Column sums by the warps w, w + nw, ... of the launch, two columns at a time so that a warp keeps
+// 16 loads in flight. Each column is summed by lane-strided rows, then across the lanes.
 __device__ __forceinline__ void column_sums(const ColumnSums& cs, uint32_t w, uint32_t nw, uint32_t lane)
 {
-    for (uint32_t c = 4 * w; c < cs.cols; c += 4 * nw) {  // cols is a multiple of 16
+    for (uint32_t c = 2 * w; c < cs.cols; c += 2 * nw) {  // cols is a multiple of 16
         const bf16* t = cs.t + (size_t)c * cs.ld;
-        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float s[2] = {0.0f, 0.0f};
         for (uint32_t r0 = lane; r0 < cs.n; r0 += 256) {
-            bf16 x[4][8];
+            bf16 x[2][8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
+            for (int q = 0; q < 2; ++q)
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
                     x[q][k] = r0 + 32 * k < cs.n ? t[(size_t)q * cs.ld + r0 + 32 * k] : __float2bfloat16_rn(0.0f);
 #pragma unroll
             for (int k = 0; k < 8; ++k)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) s[q] += __bfloat162float(x[q][k]);
+                for (int q = 0; q < 2; ++q) s[q] += __bfloat162float(x[q][k]);
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < 2; ++q) {
             for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
             if (lane == 0) cs.sums[c + q] = s[q];
         }
@@ -222,7 +211,7 @@ __device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
     return x;
 }
 
-// Persistent, warp-specialised product: each CTA (384 threads) walks output tiles of kTileM x tn
+// Persistent, warp-specialised product: each CTA (640 threads) walks output tiles of kTileM x tn
 // (tn = 32, 64, 128 or 256) in a grid-stride loop over the tiles of one or two independent products.
 //   warp 0, one thread: TMA producer. Each 64-wide K chunk of A and B is one box per operand in
 //     the 128-byte-swizzled K-major layout; up to eight chunks are in flight ("full" / "empty"
@@ -230,14 +219,13 @@ __device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
 //   warp 1, one thread: issues the four K=16 tcgen05 products of each chunk into one of two
 //     tensor-memory accumulators (tile parity), commits each chunk to the stage's "empty" barrier
 //     and each finished tile to the accumulator's "full" barrier.
-//   warps 2-9: epilogue. Warp w reads tensor-memory lanes 32*(w mod 4) .. +31 with tcgen05.ld, 16
-//     columns at a time (two warps share a lane quarter's columns: the activations are some fifty
-//     instructions an output; with one warp the 4096 x 1024 layer took 42 us, with two 29, with
-//     four 26 but the small layers 0.8 us more each),
+//   warps 2-17: epilogue. Warp w reads tensor-memory lanes 32*(w mod 4) .. +31 with tcgen05.ld, 8
+//     columns at a time (four warps share a lane quarter's columns: the activation's exponential and
+//     division are one long chain per output, which only other warps hide),
 //     applies the fused epilogue and writes whole sectors through shared memory (block_store_*), then
 //     releases the accumulator ("empty"), so the products of the next tile overlap the epilogue of
 //     this one.
-//   warps 10-11: the launch's column sums (bias gradients), beside the products.
+//   warps 18-19: the launch's column sums (bias gradients), beside the products.
 // The backward pass of a layer is one launch: its weight gradient, the signal of the layer below and
 // its bias gradient all read the same dZ. Launched with programmatic serialization: barriers and
 // tensor memory are set up while the previous launch ends. The next launch is let in only after this
@@ -324,7 +312,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
     } else if (warp >= 2 && warp < 2 + kEpiWarps) {  // epilogue
         const uint32_t quarter = warp & 3u, part = (warp - 2) >> 2;
         float* st = reinterpret_cast<float*>(smem + S * p.stage_size) + (warp - 2) * 32 * kEpiPitch;
-        constexpr uint32_t kStep = 16 * (kEpiWarps / 4);  // columns between a warp's blocks
+        constexpr uint32_t kStep = 8 * (kEpiWarps / 4);  // columns between a warp's blocks
         uint32_t li = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++li) {
             const TileAt x = tile_at(p, t);
@@ -332,28 +320,28 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
             const uint32_t a = li & 1u, n0 = x.n0, nt = x.nt;
             const uint32_t r0 = x.m0 + quarter * 32;
             const uint32_t rows = r0 < g.M ? min(32u, g.M - r0) : 0u;
-            float4 zf[4];  // pre-activations of the next block, in flight while the current one is done
-            if (g.epi == kEpiBackward && part * 16 < nt)
-                block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n0 + part * 16, g.ldz, rows, lane);
+            float4 zf[2];  // pre-activations of the next block, in flight while the current one is done
+            if (g.epi == kEpiBackward && part * 8 < nt)
+                block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n0 + part * 8, g.ldz, rows, lane);
             float e2 = 0.0f;
             ok = __all_sync(0xffffffffu, tc_bar_wait(&acc_full[a], (li >> 1) & 1u));  // warp-uniform
             if (!ok) break;
             tc_fence_after();
-            for (uint32_t c0 = part * 16; c0 < nt; c0 += kStep) {
+            for (uint32_t c0 = part * 8; c0 < nt; c0 += kStep) {
                 const uint32_t n = n0 + c0;
-                float v[16], z[16];
-                uint32_t w[8];
-                if (g.epi == kEpiLoss) {  // targets of the block, two rows per instruction
+                float v[8], z[8];
+                uint32_t w[4];
+                if (g.epi == kEpiLoss) {  // targets of the block, four rows per instruction
 #pragma unroll
-                    for (int it = 0; it < 16; ++it) {
-                        const uint32_t r = 2 * it + (lane >> 4), c = n + (lane & 15u);
+                    for (int it = 0; it < 8; ++it) {
+                        const uint32_t r = 4 * it + (lane >> 3), c = n + (lane & 7u);
                         z[it] = (r < rows && c < g.nout) ? g.target[(size_t)(r0 + r) * g.nout + c] : 0.0f;
                     }
                 }
-                tc_ld16(tmem + a * p.acc_cols + ((quarter * 32u) << 16) + c0, v);
+                tc_ld8(tmem + a * p.acc_cols + ((quarter * 32u) << 16) + c0, v);
                 if (g.epi == kEpiHidden || g.epi == kEpiLinear || g.epi == kEpiLoss) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int k = 0; k < 2; ++k) {
                         const float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + n) + k);
                         v[4 * k] += b.x;
                         v[4 * k + 1] += b.y;
@@ -364,23 +352,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
                 if (g.epi == kEpiHidden) {
                     block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, lane);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) w[j] = pack_bf16(silu(v[2 * j]), silu(v[2 * j + 1]));
+                    for (int j = 0; j < 4; ++j) w[j] = pack_bf16(silu(v[2 * j]), silu(v[2 * j + 1]));
                 } else if (g.epi == kEpiBackward) {
                     block_spread_f32(st, zf, z, lane);
                     if (c0 + kStep < nt)
                         block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n + kStep, g.ldz, rows, lane);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
+                    for (int j = 0; j < 4; ++j)
                         w[j] = pack_bf16(v[2 * j] * dsilu(z[2 * j]), v[2 * j + 1] * dsilu(z[2 * j + 1]));
                 } else if (g.epi == kEpiLoss) {
                     // Mean squared error over the real outputs and its gradient 2 (Y - T) / (rows * nout).
                     const float cells = (float)(g.M * g.nout);
 #pragma unroll
-                    for (int it = 0; it < 16; ++it) st[(2 * it + (lane >> 4)) * kEpiPitch + (lane & 15u)] = z[it];
+                    for (int it = 0; it < 8; ++it) st[(4 * it + (lane >> 3)) * kEpiPitch + (lane & 7u)] = z[it];
                     __syncwarp();
                     block_row_f32(st, z, lane);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
+                    for (int j = 0; j < 8; ++j) {
                         float grad = 0.0f;
                         if (lane < rows && n + j < g.nout) {
                             const float e = v[j] - z[j];
@@ -390,12 +378,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
                         v[j] = grad;
                     }
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
+                    for (int j = 0; j < 4; ++j) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
                 } else {
                     block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, lane);
                 }
                 if (g.epi == kEpiHidden || g.epi == kEpiBackward || g.epi == kEpiLoss)
-                    block_store_bf16(st, w, g.outb + (size_t)r0 * g.ldob + n, g.ldob, g.outt + (size_t)n * g.ldot + r0,
+                    block_store_bf16(w, g.outb + (size_t)r0 * g.ldob + n, g.ldob, g.outt + (size_t)n * g.ldot + r0,
                                      g.ldot, rows, lane);
             }
             if (g.epi == kEpiLoss) {
@@ -503,8 +491,8 @@ int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* e
     p.stages = std::min({kStageBudget / p.stage_size, kMaxStages, nk * (p.tiles[0] + p.tiles[1] > num_sm ? 2u : 1u)});
     p.cs = cs;
     p.err = err;
-    // CTAs without a tile only add column sums (eight columns each pass).
-    const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 7) / 8), num_sm);
+    // CTAs without a tile only add column sums (four columns each pass).
+    const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 3) / 4), num_sm);
     return launch_pdl(k_gemm_tn, dim3(ctas), dim3(kGemmThreads),
                       p.stages * p.stage_size + kEpiBytes + 1024, st, pdl, p);
 }

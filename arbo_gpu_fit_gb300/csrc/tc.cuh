@@ -96,20 +96,17 @@ __device__ __forceinline__ bool tc_bar_wait(unsigned long long* bar, uint32_t pa
     return false;
 }
 
-// Sixteen consecutive FP32 accumulator columns of the calling thread's tensor-memory lane.
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16])
+// Eight consecutive FP32 accumulator columns of the calling thread's tensor-memory lane.
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8])
 {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // One arrival on `bar` that also announces `bytes` of asynchronous transfers for its current phase.
