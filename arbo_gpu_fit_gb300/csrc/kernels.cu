@@ -68,6 +68,21 @@ __device__ __forceinline__ Key load_key(const Ctrl* c)
     return k;
 }
 
+// The step a body works on: its number, its winner epoch and the random key of the simulation.
+struct StepAt {
+    uint32_t t, epoch;
+    Key key;
+};
+
+__device__ __forceinline__ StepAt load_step(const Ctrl* c, uint32_t koff)
+{
+    StepAt at;
+    at.t = c->t + koff;
+    at.epoch = c->epoch + koff;
+    at.key = load_key(c);
+    return at;
+}
+
 __device__ __forceinline__ void counter_dec(uint32_t* p, Ctrl* ctrl)
 {
     if (atomicSub(p, 1u) == 0u) atomicOr(&ctrl->err, ARBO_DEVERR_COUNTER);
@@ -642,7 +657,8 @@ __device__ __forceinline__ void split_events(const Dev& d, uint32_t* trans, floa
 // one per lane: each lane reads its pair's counters, adds them to the warp's series sums and
 // splits the pair's events both ways; then the 32 lanes spread the flattened events of the warp's
 // 128 (pair, kind) entries, four per Philox call. No block barrier: a warp is a chain of two
-// dependent round trips and its draws, so the more warps in flight the better.
+// dependent round trips and its draws, so the more warps in flight the better. With kWait, the wait
+// for the previous kernel stands between the loads of static data and those of its results.
 struct __align__(16) FoiWarpSmem {
     uint32_t to[32][8];                      // CSR row of each lane's source community (degree <= 8)
     uint32_t cnt[32][4];                     // events of (lane, kind): 0 HM local, 1 HM long, 2 MH local, 3 MH long
@@ -652,11 +668,12 @@ struct __align__(16) FoiWarpSmem {
     uint32_t sum[3 * ARBO_MAX_STRAINS + 2];  // series sums: infected, incidence, infectious mosquitoes; humans, mosquitoes
 };
 
-__device__ __forceinline__ void foi_warp(const Dev& d, uint32_t p0, int collect_only, uint32_t koff, FoiWarpSmem& sh)
+template <bool kWait>
+__device__ __forceinline__ void foi_warp(const Dev& d, uint32_t p0, int collect_only, const StepAt& at, FoiWarpSmem& sh)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t t = d.ctrl->t + koff;
-    const Key key = load_key(d.ctrl);
+    const uint32_t t = at.t;
+    const Key key = at.key;
     const uint32_t row = collect_only ? 0u : t + 1;
     const uint32_t SP = d.S * d.P, S = d.S, P = d.P;
     const uint32_t p = p0 + lane;
@@ -680,7 +697,7 @@ __device__ __forceinline__ void foi_warp(const Dev& d, uint32_t p0, int collect_
             rm = draw4(key, kFoiMH, p, t);
         }
     }
-    griddep_wait();
+    if (kWait) griddep_wait();
     __syncwarp();  // the sums are zeroed
     if (valid) {
         uint32_t ih = d.infh[p], im = d.infm[p], ic = d.inc[p];
@@ -789,7 +806,8 @@ __global__ void __launch_bounds__(512) k_foi(Dev d, int collect_only, uint32_t k
     FoiWarpSmem& sh = reinterpret_cast<FoiWarpSmem*>(foi_dyn)[warp];
     const uint32_t SP = d.S * d.P;
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
-    for (uint32_t g = blockIdx.x * W + warp; 32 * g < SP; g += gridDim.x * W) foi_warp(d, 32 * g, collect_only, koff, sh);
+    const StepAt at = load_step(d.ctrl, koff);
+    for (uint32_t g = blockIdx.x * W + warp; 32 * g < SP; g += gridDim.x * W) foi_warp<true>(d, 32 * g, collect_only, at, sh);
 }
 
 // ------------------------------------------------------------------ infection draws
@@ -839,6 +857,7 @@ __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key
 
 // Per-warp tables of the infection pass: one community and its events of every serotype
 // flattened into one index space.
+constexpr uint32_t kIntroScan = 1024;   // humans of a community up to which failed introductions look at all of them
 constexpr uint32_t kTargetCache = 128;  // items whose targets Phase A keeps for Phase C
 
 struct InfectWarpSmem {
@@ -864,7 +883,7 @@ __device__ __forceinline__ uint32_t item_position(const uint32_t* start, uint32_
 //   A: every event whose target is eligible at the start of the pass bids its serial order
 //      (serotype position j, event index) for the target with atomicMin; the targets of the first
 //      kTargetCache items are kept in shared memory for phase C;
-//   B: external introductions (cpp/nepidemic.cu:261-309) in serial order, 32 attempts at a time;
+//   B: external introductions (cpp/nepidemic.cu:261-309) in serial order, 32 attempts at a time, then 128;
 //   C: each event that won its target applies its infection.
 // This reproduces the serial loops of nmTransmission / mnTransmission (cpp/mepidemic.cu:143-246,
 // cpp/nepidemic.cu:146-319): a target is infected by the first eligible event in serial order.
@@ -872,12 +891,13 @@ __device__ __forceinline__ uint32_t item_position(const uint32_t* start, uint32_
 // other warp reads or writes them during the pass and warp barriers order the phases. One warp
 // per community with no block barrier: the pass is a chain of dependent round trips per
 // community, so the more communities in flight per SM the better.
-__device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, uint32_t koff, InfectWarpSmem& sh)
+template <bool kWait>
+__device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t t = d.ctrl->t + koff;
-    const uint32_t hiword = ~(d.ctrl->epoch + koff);
-    const Key key = load_key(d.ctrl);
+    const uint32_t t = at.t;
+    const uint32_t hiword = ~at.epoch;
+    const Key key = at.key;
     const uint32_t S = d.S, P = d.P;
     const float ext = __fdiv_rn(d.extInf, (float)P);
     // Static loads and keyed draws first; the event counts and alive mosquitoes written by the
@@ -888,7 +908,7 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, uint32_t k
     // One draw per lane in one pass: introduction counts (lanes < S), first serotypes (8, 9).
     const U4 rd = draw4(key, lane < S ? (uint32_t)kIntroCount : lane == 8 ? (uint32_t)kInfMStart : (uint32_t)kInfHStart,
                         lane < S ? pl : c, t);
-    griddep_wait();
+    if (kWait) griddep_wait();
     const uint32_t mc = d.mcnt[c];
     uint32_t kh = lane < S ? d.transh[pl] : 0u;
     uint32_t km = lane < S ? d.transm[pl] : 0u;
@@ -961,38 +981,62 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, uint32_t k
     __syncwarp();
     // Phase B
     if (any_intro) {
+        uint32_t avail = 0xFFu;  // bit s clear: no human of the community can take serotype s
+        bool scanned = false;
         for (uint32_t j = 0; j < S; ++j) {
             const uint32_t s = (s0h + j) % S, ph = s * P + c;
             uint32_t left = __shfl_sync(kFull, ne, s);
-            if (left == 0) continue;
-            uint32_t a0 = 0;
-            while (left > 0 && a0 < d.maxIntro) {
-                const uint32_t a = a0 + lane;
-                bool elig = false;
-                uint32_t i = 0;
-                unsigned long long okey = 0;
-                uint32_t im = 0;
-                if (a < d.maxIntro) {
-                    const U4 r = draw4(key, kIntroTarget, ph, t, a >> 2);
-                    i = nbase + bounded(r.v[a & 3], ns);
-                    okey = order_key(hiword, j, 1, a);
-                    im = __ldcg(&d.n_imm[i]);
-                    elig = __ldcg(&d.n_status[i]) == 0 && !((im >> s) & 1u) && __ldcg(&d.winh[i]) > okey;
+            uint32_t a0 = (avail >> s) & 1u ? 0u : d.maxIntro;
+            // The first 32 attempts one per lane (most introductions find someone there), later ones
+            // 128 at a time, four to a lane and to a Philox call.
+            for (uint32_t per = 1; left > 0 && a0 < d.maxIntro; per = 4) {
+                uint32_t i[4], im[4], elig = 0;
+                const uint32_t av = a0 + per * lane;  // a0 is a multiple of four
+                const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {
+                    i[q] = im[q] = 0;
+                    if (q < per && av + q < d.maxIntro) {
+                        i[q] = nbase + bounded(per == 1 ? r.v[av & 3] : r.v[q], ns);
+                        im[q] = __ldcg(&d.n_imm[i[q]]);
+                        if (__ldcg(&d.n_status[i[q]]) == 0 && !((im[q] >> s) & 1u) &&
+                            __ldcg(&d.winh[i[q]]) > order_key(hiword, j, 1, av + q))
+                            elig |= 1u << q;
+                    }
                 }
-                const unsigned bal = __ballot_sync(kFull, elig);
-                if (!bal) {
-                    a0 += 32;
-                    continue;
-                }
-                const uint32_t pl2 = __ffs(bal) - 1;
-                if (lane == pl2) {
-                    d.winh[i] = okey;
-                    infect_human(d, i, s, draw4(key, kIntroExposed, ph, t, a), t, im, __ldcg(&d.n_born[i]),
-                                 __ldcg(&d.n_dtime[i]));
+                // The eligible attempts in order; a human taken by one is lost to the later ones.
+                while (left > 0) {
+                    const unsigned bal = __ballot_sync(kFull, elig != 0);
+                    if (!bal) break;
+                    const uint32_t first = __ffs(bal) - 1;
+                    uint32_t q = elig ? __ffs(elig) - 1 : 0;
+                    const uint32_t iq = q == 0 ? i[0] : q == 1 ? i[1] : q == 2 ? i[2] : i[3];
+                    const uint32_t mq = q == 0 ? im[0] : q == 1 ? im[1] : q == 2 ? im[2] : im[3];
+                    const uint32_t taken = __shfl_sync(kFull, iq, first);
+                    if (lane == first) {
+                        d.winh[iq] = order_key(hiword, j, 1, av + q);
+                        infect_human(d, iq, s, draw4(key, kIntroExposed, ph, t, av + q), t, mq, __ldcg(&d.n_born[iq]),
+                                     __ldcg(&d.n_dtime[iq]));
+                    }
+#pragma unroll
+                    for (q = 0; q < 4; ++q)
+                        if (i[q] == taken) elig &= ~(1u << q);
+                    left -= 1;
                 }
                 __syncwarp();
-                left -= 1;
-                a0 = a0 + pl2 + 1;
+                a0 += 32 * per;
+                if (left > 0 && !scanned && ns <= kIntroScan) {
+                    // Is there anyone left to infect? In a small population the attempts would else run
+                    // to their limit (1,000) in every community that is immune, 32 a round trip: once a small
+                    // population was immune its step took 42 us (2,000 humans) and 27 us (10,000), now 18
+                    // and 19; 512 instances of 1e4 humans 300 -> 255 us.
+                    scanned = true;
+                    uint32_t open = 0;
+                    for (uint32_t h = lane; h < ns; h += 32)
+                        if (__ldcg(&d.n_status[nbase + h]) == 0) open |= ~(uint32_t)__ldcg(&d.n_imm[nbase + h]);
+                    avail = __reduce_or_sync(kFull, open & 0xFFu);
+                }
+                if (!((avail >> s) & 1u)) break;
             }
             if (left > 0 && lane == 0) atomicAdd(&d.ctrl->diag[1], 1u);
         }
@@ -1080,7 +1124,8 @@ __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
     extern __shared__ __align__(16) unsigned char infect_dyn[];
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
-    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp(d, c, koff, sh);
+    const StepAt at = load_step(d.ctrl, koff);
+    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp<true>(d, c, at, sh);
 }
 
 // ------------------------------------------------------------------ batched steps
@@ -1189,7 +1234,7 @@ __global__ void __launch_bounds__(512) k_foi_batch(BatchDev bd, int collect_only
     }
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
     batch_warp_items(bd, bd.foi_off, bd.foi_run, wdev,
-                     [&](const Dev& d, uint32_t item) { foi_warp(d, 32 * item, collect_only, koff, sh); });
+                     [&](const Dev& d, uint32_t item) { foi_warp<true>(d, 32 * item, collect_only, load_step(d.ctrl, koff), sh); });
 }
 
 // Infection pass of a batch: one warp per community over the concatenated communities of all
@@ -1202,7 +1247,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
     unsigned long long* wdev =
         reinterpret_cast<unsigned long long*>(infect_dyn + K * sizeof(InfectWarpSmem)) + warp * (sizeof(Dev) / 8);
     batch_warp_items(bd, bd.infect_off, bd.infect_run, wdev,
-                     [&](const Dev& d, uint32_t c) { infect_warp(d, c, koff, sh); });
+                     [&](const Dev& d, uint32_t c) { infect_warp<true>(d, c, load_step(d.ctrl, koff), sh); });
 }
 
 static_assert(16 * (sizeof(InfectWarpSmem) + sizeof(Dev)) <= 48 * 1024 && 16 * (sizeof(FoiWarpSmem) + sizeof(Dev)) <= 48 * 1024,
