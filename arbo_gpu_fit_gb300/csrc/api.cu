@@ -102,14 +102,17 @@ void apply_rates(const arbo_sim_param& p, Dev& d)
     d.mInit = std::min<uint32_t>((uint32_t)p.mInitialInf, d.M);
 }
 
-uint32_t comm_of_host(const std::vector<uint32_t>& loc, uint32_t P, uint32_t i)
+// For each block of `block` agents the community of its first agent, the largest c with loc[c] <= i,
+// | kTileSpans when the block holds agents of later communities too.
+std::vector<uint32_t> block_communities(const std::vector<uint32_t>& loc, uint32_t P, uint32_t agents, uint32_t block)
 {
-    uint32_t lo = 0, hi = P;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (loc[mid] <= i) lo = mid; else hi = mid;
+    std::vector<uint32_t> out(cdiv(agents, block));
+    uint32_t c = 0;
+    for (uint32_t b = 0; b < out.size(); ++b) {
+        while (c + 1 < P && loc[c + 1] <= b * block) ++c;
+        out[b] = c | (loc[c + 1] < std::min((b + 1) * block, agents) ? kTileSpans : 0u);
     }
-    return lo;
+    return out;
 }
 
 // Death-age tables of one species: CDF per integer age and the inverse bucket table.
@@ -453,6 +456,14 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
         minv[k] = a;
     }
     minv[4097] = (uint32_t)cdfm.size();
+    // Per bucket the first age and the CDF there; 2 (any PLE) when no age step lies in the bucket.
+    std::vector<uint2> mlut(4097);
+    for (uint32_t k = 0; k <= 4096; ++k) {
+        const uint32_t lo = minv[k], hi = minv[k + 1];
+        const float at = hi == lo ? 2.0f : cdfm[lo];
+        mlut[k].x = lo | (hi - lo > 1 ? kLutWide : 0u);
+        std::memcpy(&mlut[k].y, &at, 4);
+    }
     std::vector<uint32_t> minvh(65538);
     for (uint32_t k = 0, a = 0; k <= 65536; ++k) {
         const float thr = (float)k / 65536.0f;
@@ -492,14 +503,14 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     std::vector<Item> items = {
         {(void**)&d.n_born, Np * 4}, {(void**)&d.n_dtime, Np * 4}, {(void**)&d.n_next, Np * 4}, {(void**)&d.n_status, Np}, {(void**)&d.n_exposed, Np * 4},
         {(void**)&d.n_recovery, Np * 4}, {(void**)&d.n_ple, Np * 4}, {(void**)&d.n_strain, Np}, {(void**)&d.n_imm, Np},
-        {(void**)&d.m_born, Mp * 4}, {(void**)&d.m_dtime, Mp * 4}, {(void**)&d.m_state, Mp}, {(void**)&d.m_exposed, Mp * 4},
-        {(void**)&d.m_ple, Mp * 4}, {(void**)&d.m_strain, Mp}, {(void**)&d.ledger, (size_t)d.tiles * 4},
+        {(void**)&d.m_code, Mp}, {(void**)&d.m_stat, Mp}, {(void**)&d.m_life, Mp * sizeof(Life)}, {(void**)&d.m_exposed, Mp * 4},
+        {(void**)&d.m_strain, Mp}, {(void**)&d.ledger, (size_t)d.tiles * 4},
         {(void**)&d.nloc, (P + 1) * 4}, {(void**)&d.mloc, (P + 1) * 4}, {(void**)&d.nsize, P * 4},
         {(void**)&d.msize, P * 4}, {(void**)&d.tcomm, (size_t)d.tiles * 4}, {(void**)&d.csr_loc, (P + 1) * 4},
         {(void**)&d.csr_to, std::max<size_t>(csr->nnz, 1) * 4}, {(void**)&d.infh, SP * 4}, {(void**)&d.infm, SP * 4},
         {(void**)&d.inc, SP * 4}, {(void**)&d.ncnt, P * 4}, {(void**)&d.mcnt, P * 4}, {(void**)&d.transh, SP * 4},
-        {(void**)&d.transm, SP * 4}, {(void**)&d.cdfh, cdfh.size() * 4}, {(void**)&d.cdfm, cdfm.size() * 4}, {(void**)&d.minv, minv.size() * 4}, {(void**)&d.minvh, minvh.size() * 4},
-        {(void**)&d.hcomm, (size_t)((N + 127) / 128) * 4},
+        {(void**)&d.transm, SP * 4}, {(void**)&d.cdfh, cdfh.size() * 4}, {(void**)&d.cdfm, cdfm.size() * 4}, {(void**)&d.minv, minv.size() * 4}, {(void**)&d.mlut, mlut.size() * sizeof(uint2)}, {(void**)&d.minvh, minvh.size() * 4},
+        {(void**)&d.hcomm, (size_t)cdiv(N, kHumanBlock) * 4},
         {(void**)&d.survh, survh.size() * 4}, {(void**)&d.survm, survm.size() * 4}, {(void**)&d.etab, R * 4},
         {(void**)&d.winh, Np * 8}, {(void**)&d.winm, Mp * 8}, {(void**)&d.s_ninc, R * S * 4},
         {(void**)&d.s_ninf, R * S * 4}, {(void**)&d.s_one, R * S * 4}, {(void**)&d.s_ncount, R * 4},
@@ -521,8 +532,7 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
         off += align256(it.bytes);
     }
 
-    std::vector<uint32_t> tcomm(d.tiles);
-    for (uint32_t b = 0; b < d.tiles; ++b) tcomm[b] = comm_of_host(s->mloc, P, b * kTile);
+    const std::vector<uint32_t> tcomm = block_communities(s->mloc, P, M, kTile);
     auto fail_free = [&](int code) {
         arbo_sim_destroy(s);
         return code;
@@ -546,9 +556,9 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     UP(d.cdfh, cdfh.data(), cdfh.size() * 4);
     UP(d.cdfm, cdfm.data(), cdfm.size() * 4);
     UP(d.minv, minv.data(), minv.size() * 4);
+    UP(d.mlut, mlut.data(), mlut.size() * sizeof(uint2));
     UP(d.minvh, minvh.data(), minvh.size() * 4);
-    std::vector<uint32_t> hcomm((N + 127) / 128);
-    for (uint32_t b = 0; b < hcomm.size(); ++b) hcomm[b] = comm_of_host(s->nloc, P, b * 128);
+    const std::vector<uint32_t> hcomm = block_communities(s->nloc, P, N, kHumanBlock);
     UP(d.hcomm, hcomm.data(), hcomm.size() * 4);
     UP(d.survh, survh.data(), survh.size() * 4);
     UP(d.survm, survm.data(), survm.size() * 4);
@@ -884,16 +894,37 @@ static int census_ptr(arbo_sim* s, arbo_census_field f, void** ptr, size_t* coun
     case ARBO_CENSUS_N_RECOVERY: *ptr = d.n_recovery; *elem = 4; break;
     case ARBO_CENSUS_N_STRAIN: *ptr = d.n_strain; *elem = 1; break;
     case ARBO_CENSUS_N_DEATH_AGE: *ptr = d.n_dtime; *elem = 4; *packed = 3; break;
-    case ARBO_CENSUS_M_AGE: *ptr = d.m_born; *elem = 4; *packed = 3; break;
-    case ARBO_CENSUS_M_DEAD: *ptr = d.m_state; *elem = 1; *packed = 1; break;
+    case ARBO_CENSUS_M_AGE: *ptr = d.m_life; *elem = 4; *packed = 3; break;
+    case ARBO_CENSUS_M_DEAD: *ptr = d.m_code; *elem = 1; *packed = 1; break;
     case ARBO_CENSUS_M_EXPOSED: *ptr = d.m_exposed; *elem = 4; break;
-    case ARBO_CENSUS_M_STATUS: *ptr = d.m_state; *elem = 1; *packed = 2; break;
-    case ARBO_CENSUS_M_PLE: *ptr = d.m_ple; *elem = 4; break;
+    case ARBO_CENSUS_M_STATUS: *ptr = d.m_stat; *elem = 1; *packed = 2; break;
+    case ARBO_CENSUS_M_PLE: *ptr = d.m_life; *elem = 4; *packed = 4; break;
     case ARBO_CENSUS_M_STRAIN: *ptr = d.m_strain; *elem = 1; break;
-    case ARBO_CENSUS_M_DEATH_AGE: *ptr = d.m_dtime; *elem = 4; *packed = 3; break;
+    case ARBO_CENSUS_M_DEATH_AGE: *ptr = d.m_life; *elem = 4; *packed = 3; break;
     default: return fail(ARBO_ERR_INVALID, "unknown census field");
     }
     *count = f <= ARBO_CENSUS_N_DEATH_AGE ? d.N : d.M;
+    return ARBO_OK;
+}
+
+// One field of the mosquitoes' life records (0 PLE, 1 birth time, 2 death time) between host and
+// device, through a device array of M values.
+static int life_field(arbo_sim* s, int field, void* host, bool store, void* stream)
+{
+    const size_t bytes = (size_t)s->d.M * 4;
+    cudaStream_t st = (cudaStream_t)stream;
+    CUDA_TRY(cudaSetDevice(s->device));
+    void* buf = nullptr;
+    cudaError_t e = cudaMalloc(&buf, bytes);
+    if (e != cudaSuccess)
+        return fail(ARBO_ERR_ALLOC, std::string("cudaMalloc of a census field: ") + cudaGetErrorString(e));
+    if (store) e = cudaMemcpyAsync(buf, host, bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = (cudaError_t)launch_life_field(s->d, field, buf, store, stream);
+    if (e == cudaSuccess && !store) e = cudaMemcpyAsync(host, buf, bytes, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(buf);
+    if (e != cudaSuccess) return fail(ARBO_ERR_CUDA, std::string("census field: ") + cudaGetErrorString(e));
+    (store ? s->h2d : s->d2h) += bytes;
     return ARBO_OK;
 }
 
@@ -910,11 +941,16 @@ static int census_derived(arbo_sim* s, arbo_census_field f, int32_t* out, size_t
     const bool human = f == ARBO_CENSUS_N_AGE || f == ARBO_CENSUS_N_DEATH_AGE;
     std::vector<int32_t> born(count), dtime(count);
     std::vector<uint8_t> state;
-    if ((e = copy_out(s, born.data(), human ? d.n_born : d.m_born, count * 4, stream))) return e;
-    if ((e = copy_out(s, dtime.data(), human ? d.n_dtime : d.m_dtime, count * 4, stream))) return e;
+    if (human) {
+        if ((e = copy_out(s, born.data(), d.n_born, count * 4, stream))) return e;
+        if ((e = copy_out(s, dtime.data(), d.n_dtime, count * 4, stream))) return e;
+    } else {
+        if ((e = life_field(s, 1, born.data(), false, stream))) return e;
+        if ((e = life_field(s, 2, dtime.data(), false, stream))) return e;
+    }
     if (f == ARBO_CENSUS_M_AGE) {
         state.resize(count);
-        if ((e = copy_out(s, state.data(), d.m_state, count, stream))) return e;
+        if ((e = copy_out(s, state.data(), d.m_code, count, stream))) return e;
     }
     const int32_t tn = (int32_t)now;
     for (size_t i = 0; i < count; ++i) {
@@ -939,6 +975,7 @@ int arbo_sim_get_census(arbo_sim* s, arbo_census_field f, void* host, size_t byt
     if (e) return e;
     if (bytes != count * elem) return fail(ARBO_ERR_INVALID, "census size mismatch: expected " + std::to_string(count * elem));
     if (packed == 3) return census_derived(s, f, (int32_t*)host, count, stream);
+    if (packed == 4) return life_field(s, 0, host, false, stream);
     e = copy_out(s, host, ptr, bytes, stream);
     if (e || !packed) return e;
     uint8_t* h = (uint8_t*)host;
@@ -977,6 +1014,34 @@ static int refresh_human_next(arbo_sim* s, void* stream)
     return ARBO_OK;
 }
 
+// Recomputes every mosquito slot's event code from its dead flag (dead[i], or the present code's when
+// dead is null), status, life and exposed age (after a census write that changed any of them).
+static int refresh_mosquito_code(arbo_sim* s, const uint8_t* dead, void* stream)
+{
+    const Dev& d = s->d;
+    const size_t M = d.M;
+    std::vector<uint8_t> code(M), stat(M);
+    std::vector<Life> life(M);
+    std::vector<int32_t> ex(M);
+    uint32_t err = 0, now = 0;
+    int e;
+    if ((e = arbo_sim_status(s, stream, &err, &now)) || (e = copy_out(s, code.data(), d.m_code, M, stream)) ||
+        (e = copy_out(s, stat.data(), d.m_stat, M, stream)) ||
+        (e = copy_out(s, life.data(), d.m_life, M * sizeof(Life), stream)) ||
+        (e = copy_out(s, ex.data(), d.m_exposed, M * 4, stream)))
+        return e;
+    for (size_t i = 0; i < M; ++i) {
+        const uint32_t st = stat[i] & 3u;
+        if (dead ? dead[i] != 0 : (code[i] & kDead) != 0) code[i] = (uint8_t)(kDead | (st ? kDeep : 0u));
+        else code[i] = mosq_code(mosq_next(st, life[i].dtime, life[i].born, ex[i]), (int32_t)now, st != 0);
+    }
+    cudaStream_t cs = (cudaStream_t)stream;
+    CUDA_TRY(cudaMemcpyAsync(d.m_code, code.data(), M, cudaMemcpyHostToDevice, cs));
+    CUDA_TRY(cudaStreamSynchronize(cs));
+    s->h2d += M;
+    return ARBO_OK;
+}
+
 int arbo_sim_set_census(arbo_sim* s, arbo_census_field f, const void* host, size_t bytes, void* stream)
 {
     if (!s || !host) return fail(ARBO_ERR_INVALID, "null argument");
@@ -996,20 +1061,18 @@ int arbo_sim_set_census(arbo_sim* s, arbo_census_field f, const void* host, size
         s->h2d += bytes;
         if (f == ARBO_CENSUS_N_STATUS || f == ARBO_CENSUS_N_EXPOSED || f == ARBO_CENSUS_N_RECOVERY)
             return refresh_human_next(s, stream);
+        if (f == ARBO_CENSUS_M_EXPOSED) return refresh_mosquito_code(s, nullptr, stream);
         return ARBO_OK;
     }
+    if (packed == 4) return life_field(s, 0, const_cast<void*>(host), true, stream);
+    if (packed == 1) return refresh_mosquito_code(s, (const uint8_t*)host, stream);
     std::vector<uint8_t> cur(count);
-    e = copy_out(s, cur.data(), ptr, count, stream);
-    if (e) return e;
     const uint8_t* h = (const uint8_t*)host;
-    for (size_t i = 0; i < count; ++i) {
-        if (packed == 1) cur[i] = (uint8_t)((cur[i] & 3u) | (h[i] ? kDead : 0u));
-        else cur[i] = (uint8_t)((cur[i] & kDead) | (h[i] & 3u));
-    }
+    for (size_t i = 0; i < count; ++i) cur[i] = (uint8_t)(h[i] & 3u);
     CUDA_TRY(cudaMemcpyAsync(ptr, cur.data(), count, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     s->h2d += count;
-    return ARBO_OK;
+    return refresh_mosquito_code(s, nullptr, stream);
 }
 
 int arbo_sim_dims(const arbo_sim* s, uint32_t* n, uint32_t* m, uint32_t* p, uint32_t* strains, uint32_t* max_time,
@@ -1389,6 +1452,7 @@ Dev batch_desc(const arbo_batch* b, size_t i)
     d.minvh = h.minvh;
     d.cdfm = m.cdfm;
     d.minv = m.minv;
+    d.mlut = m.mlut;
     return d;
 }
 

@@ -2,8 +2,8 @@
 //
 // One step is three launches (captured in a CUDA graph by the host):
 //   k_demog   human and mosquito demographic passes over the whole census (HBM stream: a
-//             human's next event time, a mosquito slot's state byte and death time; ages are
-//             birth times, so a survivor without a transition writes nothing), per-tile
+//             human's next event time, a mosquito slot's event code; ages are birth times,
+//             so a survivor without a transition writes nothing), per-tile
 //             mosquito recruitment, counter deltas; replaces nBlockBirthDeath + resetIncidence
 //             + mBlockBirthDeath (cpp/ndemographic.cu:32-120, cpp/mdemographic.cu:22-150).
 //   k_foi     per (serotype, community): the series row of the next time point, then the
@@ -113,107 +113,111 @@ __device__ __forceinline__ int32_t death_age_inv(const float* __restrict__ cdf, 
     return lo >= n ? INT_MAX : (int32_t)lo;
 }
 
-// Community of human i: start from the community of its 128-agent block and walk forward.
+// The same for mosquitoes with the bucket's first age and the CDF there in one load: a bucket of 1/4096
+// holds at most one age step except in the far tail (ages past 60 at a mean of 10 days), where the
+// search runs.
+__device__ __forceinline__ int32_t death_age_lut(const Dev& d, float ple)
+{
+    const uint2 e = __ldg(&d.mlut[(uint32_t)(ple * 4096.0f)]);
+    if (e.x & kLutWide) return death_age_inv(d.cdfm, d.minv, d.am, ple, 4096.0f);
+    const uint32_t a = e.x + (__uint_as_float(e.y) >= ple ? 0u : 1u);
+    return a >= d.am ? INT_MAX : (int32_t)a;
+}
+
+// Per-warp shared staging of the demographic pass.
+struct QuadSmem {
+    uint4 code[32];
+    union {
+        uint8_t slot[kQuad][kTile];    // reborn slot offsets by rank
+        uint16_t deep[kQuad * kTile];  // slots with a deep event; a human pass's agents with an event due
+    };
+};
+
+// Community of human i.
 __device__ __forceinline__ uint32_t human_comm(const uint32_t* __restrict__ nloc, const uint32_t* __restrict__ hcomm,
                                                uint32_t P, uint32_t i)
 {
-    uint32_t c = __ldg(&hcomm[i >> 7]);
-    while (c + 1 < P && __ldg(&nloc[c + 1]) <= i) ++c;
+    const uint32_t h = __ldg(&hcomm[i / kHumanBlock]);
+    uint32_t c = h & ~kTileSpans;
+    if (h & kTileSpans)
+        while (c + 1 < P && __ldg(&nloc[c + 1]) <= i) ++c;
     return c;
 }
 
-// Rare per-human path, in the step that reaches time tn at or after the human's next event time:
-// a transition of an exposed or infectious human or a death with rebirth. `ex` / `rec` are its
-// exposed and recovery ages and `born` its birth time (its age is tn - born). Returns the new
-// status byte in the low word and the human's new next event time in the high word.
-__device__ __noinline__ unsigned long long human_slow(uint32_t i, uint32_t st, int32_t tn, int32_t dtime, int32_t born,
-                                                      int32_t ex, int32_t rec, uint32_t t,
-                                                      const uint32_t* __restrict__ nloc,
-                                                      const uint32_t* __restrict__ hcomm, uint32_t P,
-                                                      const uint8_t* n_strain, float* n_ple, int32_t* n_born,
-                                                      int32_t* n_dtime, uint8_t* n_imm, uint32_t* infh, uint32_t* inc,
-                                                      const float* __restrict__ cdfh,
-                                                      const uint32_t* __restrict__ minvh, uint32_t ah, Key key,
-                                                      Ctrl* ctrl)
+// Human i in the step that reaches time tn, at or after its next event time: a transition of an
+// exposed or infectious human, a death with rebirth, or (after a census write) neither yet.
+__device__ __noinline__ void human_due(const Dev& d, const Key key, uint32_t i, int32_t tn)
 {
-    auto pack = [](uint32_t status, int32_t next) {
-        return ((unsigned long long)(uint32_t)next << 32) | status;
-    };
-    if (tn < dtime) {
+    uint32_t st = d.n_status[i];
+    const int32_t dt = d.n_dtime[i], born = d.n_born[i], ex = d.n_exposed[i], rec = d.n_recovery[i];
+    const uint32_t s = d.n_strain[i], c = human_comm(d.nloc, d.hcomm, d.P, i);
+    if (tn < dt) {
         const int32_t a = tn - born;
-        if (st == 2) {
-            if (rec < a) {
-                const uint32_t c = human_comm(nloc, hcomm, P, i);
-                counter_dec(&infh[n_strain[i] * P + c], ctrl);
-                return pack(0, dtime);
-            }
-        } else if (st == 1) {
-            if (ex < a) {
-                const uint32_t c = human_comm(nloc, hcomm, P, i);
-                const uint32_t s = n_strain[i];
-                atomicAdd(&inc[s * P + c], 1u);
-                atomicAdd(&infh[s * P + c], 1u);
-                return pack(2, human_next(2, dtime, born, rec));
-            }
+        if (st == 2 && rec < a) {
+            counter_dec(&d.infh[s * d.P + c], d.ctrl);
+            d.n_status[i] = (uint8_t)(st = 0);
+        } else if (st == 1 && ex < a) {
+            atomicAdd(&d.inc[s * d.P + c], 1u);
+            atomicAdd(&d.infh[s * d.P + c], 1u);
+            d.n_status[i] = (uint8_t)(st = 2);
         }
-        return pack(st, human_next(st, dtime, born, st == 1 ? ex : rec));
+        d.n_next[i] = human_next(st, dt, born, st == 1 ? ex : rec);
+        return;
     }
-    if (st == 2) {
-        const uint32_t c = human_comm(nloc, hcomm, P, i);
-        counter_dec(&infh[n_strain[i] * P + c], ctrl);
-    }
-    const U4 r = draw4(key, kHumanRebirth, i >> 2, t);
+    if (st == 2) counter_dec(&d.infh[s * d.P + c], d.ctrl);
+    const U4 r = draw4(key, kHumanRebirth, i >> 2, (uint32_t)(tn - 1));
     const float ple = u01(r.v[i & 3]);
-    const int32_t dt = death_time(tn, death_age_inv(cdfh, minvh, ah, ple, 65536.0f));
-    n_ple[i] = ple;
-    n_born[i] = tn;
-    n_dtime[i] = dt;
-    n_imm[i] = 0;
-    return pack(0, dt);
+    const int32_t nd = death_time(tn, death_age_inv(d.cdfh, d.minvh, d.ah, ple, 65536.0f));
+    d.n_ple[i] = ple;
+    d.n_born[i] = tn;
+    d.n_dtime[i] = nd;
+    d.n_next[i] = nd;
+    d.n_imm[i] = 0;
+    d.n_status[i] = 0;
 }
 
-// Human pass over groups of four (cpp/ndemographic.cu:32-105): ageing is implicit in the birth
-// times, and each human's next event time (its death, or its exposed-to-infectious or recovery
-// step, whichever comes first) is kept up to date by every writer of its status, so the pass
-// streams only that time. A group with an event due loads its status, times and ages in one round
-// trip and takes the slow path for the humans whose event is due.
+// Human pass of one warp over U rows of 32 groups of four, `stride` groups apart (g0: this lane's
+// first group; cpp/ndemographic.cu:32-105): ageing is implicit in the birth times, and each human's
+// next event time (its death, or its exposed-to-infectious or recovery step, whichever comes first)
+// is kept up to date by every writer of its status, so the pass streams only that time. The agents
+// with an event due are listed and taken one per lane: their status, times and ages are one round
+// trip for the whole warp. Worked off by the lane that streamed them, four agents in turn and each
+// kind of event by itself, the chain of the last warps set the end of the pass (a step of 5e4 agents
+// 18.9 -> 15.0 us, of 7 M 34 -> 28 us, with the mosquitoes' deep events taken the same way).
 template <int U>
-__device__ __forceinline__ void demog_humans(const Dev& d, const Key key, uint32_t g0, uint32_t stride, uint32_t t)
+__device__ __forceinline__ void demog_humans(const Dev& d, const Key key, uint32_t g0, uint32_t stride, uint32_t t,
+                                             QuadSmem& sm)
 {
+    const uint32_t lane = threadIdx.x & 31u;
     int4 X[U];
-    bool ok[U];
     const int32_t tn = (int32_t)t + 1;
+    int32_t first = INT_MAX;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const uint32_t g = g0 + u * stride;
-        ok[u] = g < d.nvec;
-        if (ok[u]) X[u] = __ldcs(reinterpret_cast<const int4*>(d.n_next) + g);
+        X[u] = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);  // as padding
+        if (g < d.nvec) X[u] = __ldcs(reinterpret_cast<const int4*>(d.n_next) + g);
+        first = min(first, min(min(X[u].x, X[u].y), min(X[u].z, X[u].w)));
     }
+    if (!__any_sync(kFull, tn >= first)) return;
+    uint32_t n = 0;
+    const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        if (!ok[u]) continue;
-        if (tn < X[u].x && tn < X[u].y && tn < X[u].z && tn < X[u].w) continue;  // nothing due (padding: INT_MAX)
-        const uint32_t g = g0 + u * stride;
-        const uint32_t sw = reinterpret_cast<const unsigned int*>(d.n_status)[g];
-        const int4 D = reinterpret_cast<const int4*>(d.n_dtime)[g], B = reinterpret_cast<const int4*>(d.n_born)[g];
-        const int4 E = reinterpret_cast<const int4*>(d.n_exposed)[g], R = reinterpret_cast<const int4*>(d.n_recovery)[g];
-        const int32_t xv[4] = {X[u].x, X[u].y, X[u].z, X[u].w}, dd[4] = {D.x, D.y, D.z, D.w};
-        const int32_t bv[4] = {B.x, B.y, B.z, B.w}, ev[4] = {E.x, E.y, E.z, E.w}, rv[4] = {R.x, R.y, R.z, R.w};
-        int32_t nx[4] = {xv[0], xv[1], xv[2], xv[3]};
-        uint32_t nsw = sw;
+        const int32_t x[4] = {X[u].x, X[u].y, X[u].z, X[u].w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (tn < xv[k]) continue;
-            const uint32_t st = (sw >> (8 * k)) & 0xFFu;
-            const unsigned long long res =
-                human_slow(4 * g + k, st, tn, dd[k], bv[k], ev[k], rv[k], t, d.nloc, d.hcomm, d.P, d.n_strain, d.n_ple,
-                           d.n_born, d.n_dtime, d.n_imm, d.infh, d.inc, d.cdfh, d.minvh, d.ah, key, d.ctrl);
-            nsw = (nsw & ~(0xFFu << (8 * k))) | (((uint32_t)res & 0xFFu) << (8 * k));
-            nx[k] = (int32_t)(uint32_t)(res >> 32);
+            const unsigned bal = __ballot_sync(kFull, tn >= x[k]);
+            if (tn >= x[k]) sm.deep[n + __popc(bal & below)] = (uint16_t)((u << 7) | (lane << 2) | k);
+            n += __popc(bal);
         }
-        if (nsw != sw) reinterpret_cast<unsigned int*>(d.n_status)[g] = nsw;
-        reinterpret_cast<int4*>(d.n_next)[g] = make_int4(nx[0], nx[1], nx[2], nx[3]);
     }
+    __syncwarp();
+    for (uint32_t j = lane; j < n; j += 32) {
+        const uint32_t e = sm.deep[j];
+        human_due(d, key, 4 * (g0 - lane + (e >> 7) * stride) + (e & 127u), tn);
+    }
+    __syncwarp();
 }
 
 __device__ __forceinline__ uint32_t slot_comm(const Dev& d, uint32_t c0, uint32_t i)
@@ -223,21 +227,38 @@ __device__ __forceinline__ uint32_t slot_comm(const Dev& d, uint32_t c0, uint32_
     return c;
 }
 
-// Rare per-mosquito counter change (death of an infectious mosquito, or E->I).
-__device__ __noinline__ void mosq_counter(uint32_t* infm, const uint8_t* m_strain, const uint32_t* __restrict__ mloc,
-                                          const uint32_t* __restrict__ tcomm, uint32_t P, uint32_t i, int add, Ctrl* ctrl)
+// Community of mosquito slot i.
+__device__ __forceinline__ uint32_t mosq_comm(const Dev& d, uint32_t i)
 {
-    uint32_t c = __ldg(&tcomm[i / kTile]);
-    while (c + 1 < P && __ldg(&mloc[c + 1]) <= i) ++c;
-    uint32_t* p = &infm[m_strain[i] * P + c];
-    if (add > 0) atomicAdd(p, 1u); else counter_dec(p, ctrl);
+    const uint32_t c = __ldg(&d.tcomm[i / kTile]);
+    return (c & kTileSpans) ? slot_comm(d, c & ~kTileSpans, i) : c;
 }
 
+// A live slot whose event is due in the step that reaches time tn and is not the plain death of a
+// susceptible mosquito: its death, its latent-to-infectious transition, or neither yet. Returns its
+// new code.
+__device__ __noinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn)
+{
+    const int4 r = *reinterpret_cast<const int4*>(d.m_life + i);  // ple, born, dtime
+    uint32_t st = d.m_stat[i] & 3u;
+    const int32_t ex = d.m_exposed[i];
+    const uint32_t s = d.m_strain[i], c = mosq_comm(d, i);
+    if (tn >= r.z) {
+        if (st == 2) counter_dec(&d.infm[s * d.P + c], d.ctrl);
+        return st ? (uint32_t)(kDead | kDeep) : (uint32_t)kDead;
+    }
+    if (st == 1 && ex < tn - r.y) {
+        st = 2;
+        d.m_stat[i] = 2;
+        atomicAdd(&d.infm[s * d.P + c], 1u);
+    }
+    return mosq_code(mosq_next(st, r.z, r.y, ex), tn, st != 0);
+}
 
-// Bit 7 of each byte of x gathered into a 4-bit mask (byte k -> bit k).
+// Bit 7 of each byte of x (the other bits zero) gathered into a 4-bit mask (byte k -> bit k).
 __device__ __forceinline__ uint32_t nibble7(uint32_t x)
 {
-    return (((x >> 7) & 0x01010101u) * 0x01020408u) >> 24;
+    return ((x >> 7) * 0x01020408u) >> 24;
 }
 
 __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
@@ -245,237 +266,172 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
     return i == 0 ? v.v[0] : i == 1 ? v.v[1] : i == 2 ? v.v[2] : v.v[3];
 }
 
-// Per-warp shared staging of the mosquito pass: reborn slot offsets by rank and the Philox
-// outputs of the groups of four reborn slots, for the four tiles of a quad.
-struct QuadSmem {
-    uint4 draw[kQuad][32];
-    uint8_t slot[kQuad][kTile];
-};
-
-// The m lowest set bits of a 4-bit mask, from 64-bit tables of sixteen 4-bit entries.
-__host__ __device__ constexpr uint32_t keep_low_bits(uint32_t mask, uint32_t m)
-{
-    uint32_t out = 0;
-    for (uint32_t b = 0; b < 4; ++b)
-        if (((mask >> b) & 1u) && m > 0) {
-            out |= 1u << b;
-            --m;
-        }
-    return out;
-}
-__host__ __device__ constexpr unsigned long long keep_low_table(uint32_t m)
-{
-    unsigned long long v = 0;
-    for (uint32_t mask = 0; mask < 16; ++mask) v |= (unsigned long long)keep_low_bits(mask, m) << (4 * mask);
-    return v;
-}
-__device__ __forceinline__ uint32_t keep_low(uint32_t mask, uint32_t m)
-{
-    constexpr unsigned long long L1 = keep_low_table(1), L2 = keep_low_table(2), L3 = keep_low_table(3);
-    if (m == 0) return 0u;
-    if (m >= 4) return mask;
-    const unsigned long long lut = m == 1 ? L1 : m == 2 ? L2 : L3;
-    return (uint32_t)(lut >> (4 * mask)) & 0xFu;
-}
-
-// One warp, tiles 4q..4q+3; lane l holds slots 4l..4l+3 of each tile. Per tile: deaths (an
-// alive slot dies when the new time reaches its death time), the birth quota (cpp/mdemographic.cu:104-129) from the carried dead count, rebirth of
-// the lowest-index dead slots, the net change of each community's alive count. The quota draws
-// of the four tiles come from one Philox call; the r-th reborn slot of tile b takes component
-// r&3 of the call keyed (b, t, r>>2). Per-tile counts of the four tiles travel packed in the
-// four bytes of one word (at most 128 per tile), so one warp reduction or scan serves all four.
-// Slot-owner lanes test their slots, clear the state bytes of their reborn slots and post each
-// reborn slot's offset under its rank; one lane per group of four reborn slots then draws the
-// group, and one lane per reborn slot writes the newborn's PLE, birth time and death time.
+// One warp, tiles 4q..4q+3; lane l holds the codes of slots 16(l mod 8) .. +15 of tile 4q + l/8, four
+// words. Per tile: deaths (a live slot dies in the step that reaches its death time), the birth quota
+// (cpp/mdemographic.cu:104-129) from the carried dead count, rebirth of the lowest-index dead slots, the
+// net change of each community's alive count. The quota draws of the four tiles come from one Philox
+// call; the r-th reborn slot of tile b takes component r&3 of the call keyed (b, t, r>>2).
+//
+// What bounds it: instruction issue. The whole test of a slot is a byte compare (three instructions for
+// four slots): its code holds the low bits of its next event time, and a susceptible mosquito's event is
+// its death, so nothing else is read. Before, a slot's state byte and 4-byte death time were streamed
+// and tested one slot at a time (1,150 warp instructions a quad); demographic phase of 14 M agents 60 ->
+// 42 us, of 128 instances of 7e4 agents 79 -> 42 us (with the human pass above). Owner lanes post the offset of each
+// reborn slot under its rank; one lane per reborn slot then draws its PLE and writes its life record
+// (one sector instead of three) and its code, which the owners write back with one 16-byte store.
 __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
-                                                   QuadSmem& sm, uint32_t (&SW)[kQuad], const int4 (&D)[kQuad])
+                                                   QuadSmem& sm, const uint4 A)
 {
-    const uint32_t b0 = q * kQuad;
     const int32_t tn = (int32_t)t + 1;
-    const uint32_t bl = b0 + lane;
-    const bool tile_lane = lane < kQuad && bl < d.tiles;
-    const int32_t led = tile_lane ? d.ledger[bl] : 0;
-    const uint32_t cl = tile_lane ? __ldg(&d.tcomm[bl]) : 0u;
-    const uint32_t cl_end = tile_lane ? __ldg(&d.mloc[cl + 1]) : 0u;
+    const uint32_t u = lane >> 3, seg = lane & 7u, b = q * kQuad + u;
+    const bool live = b < d.tiles;
+    const int32_t led = live ? d.ledger[b] : 0;
+    const uint32_t c0 = live ? __ldg(&d.tcomm[b]) : 0u;
+    const float target = __ldg(&d.etab[t + 1]);
     const U4 rq = draw4(key, kMosquitoTile, q, t);
 
-    uint32_t deadm = 0, diedm = 0;  // 4 bits per tile
-    uint32_t chg = 0;               // bit u: state word of tile u changed
-    uint32_t ndp = 0, diedp = 0;    // packed per-tile counts of this lane: dead after deaths, died now
+    uint32_t aw[4] = {A.x, A.y, A.z, A.w}, z[4], deep = 0;
+    const uint32_t now4 = ((uint32_t)tn & 63u) * 0x01010101u;
 #pragma unroll
-    for (uint32_t u = 0; u < kQuad; ++u) {
-        const uint32_t sw = SW[u];
-        // Byte-parallel masks of the four state bytes (bit 7 of a byte: dead or padding; padding
-        // bytes, 0xFF, exist only in the last tile).
-        const uint32_t alive4 = ~sw & 0x80808080u;
-        uint32_t dead4 = sw & 0x80808080u;
-        if (b0 + u == d.tiles - 1) dead4 &= ~__vcmpeq4(sw, 0xFFFFFFFFu);
-        const uint32_t al0 = (alive4 >> 7) & 1u, al1 = (alive4 >> 15) & 1u, al2 = (alive4 >> 23) & 1u,
-                       al3 = alive4 >> 31;
-        const uint32_t dim = (al0 & (uint32_t)(tn >= D[u].x)) | ((al1 & (uint32_t)(tn >= D[u].y)) << 1) |
-                             ((al2 & (uint32_t)(tn >= D[u].z)) << 2) | ((al3 & (uint32_t)(tn >= D[u].w)) << 3);
-        const uint32_t dm = nibble7(dead4) | dim;
-        const uint32_t stat4 = sw & 0x03030303u;
-        uint32_t rm = nibble7(((stat4 | (stat4 >> 1)) & (alive4 >> 7)) << 7);
-        uint32_t ns = sw | (((dim * 0x00204081u) & 0x01010101u) << 7);
-        const uint32_t g = (b0 + u) * 32 + lane;
-        // Rare: deaths of infectious mosquitoes and latent-to-infectious transitions.
-        while (rm) {
-            const int k = __ffs(rm) - 1;
-            rm &= rm - 1;
-            const uint32_t i = 4 * g + k;
-            const uint32_t st = (ns >> (8 * k)) & 0xFFu;
-            if (st & kDead) {
-                if ((st & 3u) == 2u) mosq_counter(d.infm, d.m_strain, d.mloc, d.tcomm, d.P, i, -1, d.ctrl);
-            } else if ((st & 3u) == 1u) {
-                if (d.m_exposed[i] < tn - d.m_born[i]) {
-                    ns = (ns & ~(0x3u << (8 * k))) | (2u << (8 * k));
-                    mosq_counter(d.infm, d.m_strain, d.mloc, d.tcomm, d.P, i, +1, d.ctrl);
-                }
-            }
-        }
-        if (ns != sw) chg |= 1u << u;
-        SW[u] = ns;
-        deadm |= dm << (4 * u);
-        diedm |= dim << (4 * u);
-        ndp |= (uint32_t)__popc(dm) << (8 * u);
-        diedp |= (uint32_t)__popc(dim) << (8 * u);
+    for (int j = 0; j < 4; ++j) {
+        // Bytes with code == now: the sum reaches bit 7 in every other byte (no carry between bytes).
+        z[j] = ~((((aw[j] & 0x3F3F3F3Fu) ^ now4) + 0x7F7F7F7Fu) | aw[j]) & 0x80808080u;
+        deep |= z[j] & (aw[j] << 1);
     }
-    // Deaths per tile (packed) and the birth quotas: lane u computes tile b0+u.
-    const uint32_t died_all = __reduce_add_sync(kFull, diedp);
-    int births_l = 0;
-    if (tile_lane) {
-        const uint32_t start = bl * kTile;
+    bool chg = (z[0] | z[1] | z[2] | z[3]) != 0;
+    uint32_t dead[4] = {0, 0, 0, 0};  // died in the deep path
+    if (__any_sync(kFull, deep != 0)) {
+        // One lane per deep event of the quad, whoever owns its slot: its loads are one round trip.
+        uint32_t zd[4], m = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            zd[j] = z[j] & (aw[j] << 1);
+            z[j] &= ~zd[j];
+            m |= nibble7(zd[j]) << (4 * j);
+        }
+        const uint32_t cnt = __popc(m);
+        uint32_t at = cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, at, off);
+            if (lane >= (uint32_t)off) at += y;
+        }
+        const uint32_t total = __shfl_sync(kFull, at, 31);
+        for (at -= cnt; m; m &= m - 1) sm.deep[at++] = (uint16_t)(16 * lane + __ffs(m) - 1);
+        sm.code[lane] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
+        __syncwarp();
+        for (uint32_t j = lane; j < total; j += 32) {
+            const uint32_t o = sm.deep[j];
+            reinterpret_cast<uint8_t*>(sm.code)[o] = (uint8_t)mosq_deep(d, q * kQuad * kTile + o, tn);
+        }
+        __syncwarp();
+        const uint4 B = sm.code[lane];
+        aw[0] = B.x, aw[1] = B.y, aw[2] = B.z, aw[3] = B.w;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dead[j] = zd[j] & aw[j];
+    }
+    // Plain deaths become kDead exactly; died: both kinds.
+    uint32_t dm = 0, died = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        aw[j] = (aw[j] & ~((z[j] >> 7) * 0xFFu)) | z[j];
+        z[j] |= dead[j];
+        uint32_t dj = aw[j] & 0x80808080u;
+        if (b == d.tiles - 1) dj &= ~__vcmpeq4(aw[j], 0xFFFFFFFFu);  // padding is in the last tile only
+        dm |= nibble7(dj) << (4 * j);
+        died |= z[j] >> (7 - j);  // byte k, bit j
+    }
+    if (!live) dm = 0;
+    // Counts of the tile's eight lanes: exclusive dead count before this lane's slots (slot order) and
+    // the tile's totals, dead in the low and died in the high half.
+    const uint32_t own = (uint32_t)__popc(dm) | ((uint32_t)__popc(died) << 16);
+    uint32_t incl = own;
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, off, 8);
+        if (seg >= (uint32_t)off) incl += y;
+    }
+    const uint32_t excl = (incl - own) & 0xFFFFu, tot = __shfl_sync(kFull, incl, 7, 8);
+    const uint32_t dead_tot = tot & 0xFFFFu, died_tot = tot >> 16;
+    // The quota, by every lane of the tile alike.
+    uint32_t nb = 0;
+    if (live) {
+        const uint32_t start = b * kTile;
         const uint32_t bt = (d.M - start) < kTile ? (d.M - start) : kTile;
-        const uint32_t L = (uint32_t)led + ((died_all >> (8 * lane)) & 0xFFu);
+        const uint32_t L = (uint32_t)led + died_tot;
         const float fbt = (float)bt;
-        float x = __fmul_rn(__ldg(&d.etab[t + 1]), fbt);
+        float x = __fmul_rn(target, fbt);
         x = __fdiv_rn(x, (float)d.M);
         x = __fsub_rn(x, fbt);
         x = __fadd_rn(x, (float)L);
-        births_l = (int)resolve(x, pick4(rq, lane));
-        d.ledger[bl] = (int32_t)L - births_l;
+        const int births = (int)resolve(x, pick4(rq, u));
+        if (seg == 0) d.ledger[b] = (int32_t)L - births;
+        nb = births > 0 ? min((uint32_t)births, dead_tot) : 0u;
     }
-    // Ranks of dead slots (slot order): packed exclusive scan of the per-lane dead counts.
-    uint32_t incl = ndp;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, incl, off);
-        if (lane >= (uint32_t)off) incl += y;
-    }
-    const uint32_t excl = incl - ndp;
-    const uint32_t tot = __shfl_sync(kFull, incl, 31);
-    uint32_t bornp = 0, nb_pack = 0, gtot = 0, gst = 0;
-#pragma unroll
-    for (uint32_t u = 0; u < kQuad; ++u) {
-        const int bu = __shfl_sync(kFull, births_l, u);
-        const uint32_t total = (tot >> (8 * u)) & 0xFFu;
-        const uint32_t nb = (bu > 0 && b0 + u < d.tiles) ? min((uint32_t)bu, total) : 0u;
-        nb_pack |= nb << (8 * u);
-        gst |= gtot << (8 * u);
-        gtot += (nb + 3) >> 2;
-        const uint32_t pre = (excl >> (8 * u)) & 0xFFu;
-        const uint32_t dm = (deadm >> (4 * u)) & 0xFu;
-        const uint32_t born = keep_low(dm, nb > pre ? nb - pre : 0u);
-        if (born) {
-            uint32_t bm = born, r = pre;
-            while (bm) {
-                const int k = __ffs(bm) - 1;
-                bm &= bm - 1;
-                sm.slot[u][r++] = (uint8_t)(4 * lane + k);
-            }
-            SW[u] &= ~(((born * 0x00204081u) & 0x01010101u) * 0xFFu);
+    const uint32_t mine = min(nb > excl ? nb - excl : 0u, own & 0xFFFFu);
+    // The lowest `mine` dead slots of the lane, posted under their ranks.
+    uint32_t born = 0;
+    {
+        uint32_t m = dm;
+        for (uint32_t r = excl, n = mine; n; --n, ++r) {
+            const uint32_t low = m & (0u - m);
+            sm.slot[u][r] = (uint8_t)(16 * seg + 31 - __clz(low));
+            m ^= low;
         }
-        if (born || ((chg >> u) & 1u)) reinterpret_cast<unsigned int*>(d.m_state)[(b0 + u) * 32 + lane] = SW[u];
-        bornp |= (uint32_t)__popc(born) << (8 * u);
+        born = dm ^ m;
     }
-    // Alive count per community: one atomic per tile when the tile lies in one community.
-    const uint32_t born_all = __reduce_add_sync(kFull, bornp);
-    const bool single_l = tile_lane && cl_end >= min((bl + 1) * kTile, d.M);
-    if (single_l) {
-        const int net = (int)((born_all >> (8 * lane)) & 0xFFu) - (int)((died_all >> (8 * lane)) & 0xFFu);
-        if (net != 0) atomicAdd(&d.mcnt[cl], (unsigned)net);
-    }
-    const unsigned single = __ballot_sync(kFull, single_l);
+    chg |= born != 0;
+    if (live && (c0 & kTileSpans)) {
+        // A tile across communities: the net change slot by slot.
+        uint32_t died16 = 0;
 #pragma unroll
-    for (uint32_t u = 0; u < kQuad; ++u) {
-        if (b0 + u >= d.tiles || ((single >> u) & 1u)) continue;  // warp-uniform
-        const uint32_t g = (b0 + u) * 32 + lane;
-        const uint32_t c0 = __ldg(&d.tcomm[b0 + u]);
-        const uint32_t dim = (diedm >> (4 * u)) & 0xFu;
-        const uint32_t pre = (excl >> (8 * u)) & 0xFFu, nb = (nb_pack >> (8 * u)) & 0xFFu;
-        const uint32_t born = keep_low((deadm >> (4 * u)) & 0xFu, nb > pre ? nb - pre : 0u);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int net = (int)((born >> k) & 1u) - (int)((dim >> k) & 1u);
-            if (net != 0) atomicAdd(&d.mcnt[slot_comm(d, c0, 4 * g + k)], (unsigned)net);
+        for (int j = 0; j < 4; ++j) died16 |= nibble7(z[j]) << (4 * j);
+        for (uint32_t m = born ^ died16; m; m &= m - 1) {
+            const uint32_t k = __ffs(m) - 1;
+            atomicAdd(&d.mcnt[slot_comm(d, c0 & ~kTileSpans, b * kTile + 16 * seg + k)], ((born >> k) & 1u) ? 1u : ~0u);
         }
+    } else if (seg == 0 && nb != died_tot) {
+        atomicAdd(&d.mcnt[c0], nb - died_tot);  // one atomic per tile
     }
-    // Draw groups: lane gi computes the Philox call of reborn group gi of the quad.
-    for (uint32_t gi = lane; gi < gtot; gi += 32) {
-        uint32_t u = 0;
-#pragma unroll
-        for (uint32_t v = 1; v < kQuad; ++v)
-            if (gi >= ((gst >> (8 * v)) & 0xFFu) && ((nb_pack >> (8 * v)) & 0xFFu)) u = v;
-        const uint32_t r4 = gi - ((gst >> (8 * u)) & 0xFFu);
-        const U4 v4 = draw4(key, kMosquitoRebirth, b0 + u, t, r4);
-        sm.draw[u][r4] = make_uint4(v4.v[0], v4.v[1], v4.v[2], v4.v[3]);
-    }
-    __syncwarp();
-    // Rank lanes: reborn slot j of the quad (tile u, rank r).
-    const uint32_t rtot = (nb_pack & 0xFFu) + ((nb_pack >> 8) & 0xFFu) + ((nb_pack >> 16) & 0xFFu) + (nb_pack >> 24);
-    for (uint32_t j = lane; j < rtot; j += 32) {
-        uint32_t u = 0, base = 0;
-#pragma unroll
-        for (uint32_t v = 0; v + 1 < kQuad; ++v) {
-            const uint32_t nbv = (nb_pack >> (8 * v)) & 0xFFu;
-            if (u == v && j >= base + nbv) {
-                base += nbv;
-                u = v + 1;
-            }
+    const uint32_t n0 = __shfl_sync(kFull, nb, 0), n1 = n0 + __shfl_sync(kFull, nb, 8), n2 = n1 + __shfl_sync(kFull, nb, 16);
+    const uint32_t rtot = n2 + __shfl_sync(kFull, nb, 24);
+    if (rtot) {
+        sm.code[lane] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
+        __syncwarp();
+        uint8_t* codes = reinterpret_cast<uint8_t*>(sm.code);
+        for (uint32_t j = lane; j < rtot; j += 32) {
+            const uint32_t v = (j >= n0 ? 1u : 0u) + (j >= n1 ? 1u : 0u) + (j >= n2 ? 1u : 0u);
+            const uint32_t r = j - (v == 0 ? 0u : v == 1 ? n0 : v == 2 ? n1 : n2);
+            const U4 x = draw4(key, kMosquitoRebirth, q * kQuad + v, t, r >> 2);
+            const float ple = u01(pick4(x, r & 3u));
+            const uint32_t o = v * kTile + sm.slot[v][r], i = q * kQuad * kTile + o;
+            const int32_t dt = death_time(tn, death_age_lut(d, ple));
+            *reinterpret_cast<int4*>(d.m_life + i) = make_int4(__float_as_int(ple), tn, dt, 0);
+            if (codes[o] & kDeep) d.m_stat[i] = 0;
+            codes[o] = mosq_code(dt, tn, false);
         }
-        const uint32_t r = j - base;
-        const uint32_t i = (b0 + u) * kTile + sm.slot[u][r];
-        const uint4 v4 = sm.draw[u][r >> 2];
-        const uint32_t c = r & 3u;
-        const float ple = u01(c == 0 ? v4.x : c == 1 ? v4.y : c == 2 ? v4.z : v4.w);
-        d.m_ple[i] = ple;
-        d.m_born[i] = tn;
-        d.m_dtime[i] = death_time(tn, death_age_inv(d.cdfm, d.minv, d.am, ple, 4096.0f));
+        __syncwarp();
+        if (chg) reinterpret_cast<uint4*>(d.m_code)[q * 32 + lane] = sm.code[lane];
+        __syncwarp();
+    } else if (chg) {
+        reinterpret_cast<uint4*>(d.m_code)[q * 32 + lane] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
     }
-    __syncwarp();
 }
 
-// Quad with its census words loaded straight from global memory.
+// Quad with its codes loaded straight from global memory.
 __device__ __forceinline__ void demog_mosquito_quad(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
                                                     QuadSmem& sm)
 {
-    const uint32_t b0 = q * kQuad;
-    uint32_t SW[kQuad];
-    int4 D[kQuad];
-#pragma unroll
-    for (uint32_t u = 0; u < kQuad; ++u) {
-        if (b0 + u < d.tiles) {
-            const uint32_t g = (b0 + u) * 32 + lane;
-            SW[u] = __ldcs(reinterpret_cast<const unsigned int*>(d.m_state) + g);
-            D[u] = __ldcs(reinterpret_cast<const int4*>(d.m_dtime) + g);
-        } else {
-            SW[u] = 0xFFFFFFFFu;
-            D[u] = make_int4(0, 0, 0, 0);
-        }
-    }
-    mosquito_quad_core(d, key, q, lane, t, sm, SW, D);
+    uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
+    if (q * kQuad + (lane >> 3) < d.tiles) A = reinterpret_cast<const uint4*>(d.m_code)[q * 32 + lane];
+    mosquito_quad_core(d, key, q, lane, t, sm, A);
 }
 
 // ------------------------------------------------------------------ TMA-staged pipeline
 
-// One warp's double buffer of quad census words, filled by bulk asynchronous copies.
-struct MosqStage {
-    uint32_t state[kQuad * 32];
-    int4 dtime[kQuad * 32];
-};
+// One warp's double buffer of quad codes, filled by bulk asynchronous copies.
 struct TmaWarpSmem {
-    MosqStage stage[2];
+    uint4 stage[2][32];
     QuadSmem qs;
     unsigned long long mbar[2];
 };
@@ -524,16 +480,15 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
     return false;
 }
 
-// Lane 0 starts the three copies of quad q into `st`.
-__device__ __forceinline__ void issue_quad(const Dev& d, uint32_t q, MosqStage& st, unsigned long long* bar)
+// Lane 0 starts the copy of quad q into `st`.
+__device__ __forceinline__ void issue_quad(const Dev& d, uint32_t q, uint4* st, unsigned long long* bar)
 {
     const uint32_t b0 = q * kQuad;
     const uint32_t nt = min(kQuad, d.tiles - b0);
     // Order the warp's earlier generic reads of this buffer before the asynchronous writes.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(bar, nt * kTile * 5);
-    bulk_load(st.state, d.m_state + (size_t)b0 * kTile, nt * kTile, bar);
-    bulk_load(st.dtime, d.m_dtime + (size_t)b0 * kTile, nt * kTile * 4, bar);
+    mbar_expect_tx(bar, nt * kTile);
+    bulk_load(st, d.m_code + (size_t)b0 * kTile, nt * kTile, bar);
 }
 
 // Persistent demographic pass with TMA staging. Every warp first walks chunks of 32*U human
@@ -559,7 +514,7 @@ __global__ void __launch_bounds__(128, 4) k_demog_tma(Dev d, uint32_t koff)
     }
     __syncwarp();
     const uint32_t hchunks = (d.nvec + 32 * U - 1) / (32 * U);
-    for (uint32_t ch = gw; ch < hchunks; ch += nw) demog_humans<U>(d, key, ch * 32 * U + lane, 32, t);
+    for (uint32_t ch = gw; ch < hchunks; ch += nw) demog_humans<U>(d, key, ch * 32 * U + lane, 32, t, ws.qs);
     uint32_t phase = 0;  // bit s: parity to wait for on stage s
     uint32_t i = 0;
     for (uint32_t q = gw; q < quads; q += nw, ++i) {
@@ -575,22 +530,10 @@ __global__ void __launch_bounds__(128, 4) k_demog_tma(Dev d, uint32_t koff)
             }
             break;
         }
-        const MosqStage& st = ws.stage[sidx];
-        const uint32_t b0 = q * kQuad;
-        uint32_t SW[kQuad];
-        int4 D[kQuad];
-#pragma unroll
-        for (uint32_t u = 0; u < kQuad; ++u) {
-            if (b0 + u < d.tiles) {
-                SW[u] = st.state[u * 32 + lane];
-                D[u] = st.dtime[u * 32 + lane];
-            } else {
-                SW[u] = 0xFFFFFFFFu;
-                D[u] = make_int4(0, 0, 0, 0);
-            }
-        }
+        uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
+        if (q * kQuad + (lane >> 3) < d.tiles) A = ws.stage[sidx][lane];
         __syncwarp();  // every lane has its words before the buffer is refilled next iteration
-        mosquito_quad_core(d, key, q, lane, t, ws.qs, SW, D);
+        mosquito_quad_core(d, key, q, lane, t, ws.qs, A);
     }
     griddep_launch_dependents();
 }
@@ -602,11 +545,11 @@ __device__ __forceinline__ void demog_block(const Dev& d, uint32_t b, uint32_t h
 {
     const uint32_t t = d.ctrl->t + koff;
     const Key key = load_key(d.ctrl);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     if (b < hblocks) {
-        demog_humans<U>(d, key, b * blockDim.x * U + threadIdx.x, blockDim.x, t);
+        demog_humans<U>(d, key, b * blockDim.x * U + threadIdx.x, blockDim.x, t, wsm[warp]);
     } else {
         const uint32_t wpb = blockDim.x >> 5;
-        const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
         const uint32_t q = (b - hblocks) * wpb + warp;
         if (q * kQuad < d.tiles) demog_mosquito_quad(d, key, q, lane, t, wsm[warp]);
     }
@@ -832,7 +775,7 @@ __device__ __forceinline__ void infect_human(const Dev& d, uint32_t i, uint32_t 
 // Target of mosquito event e: the first alive slot of its attempt sequence (dead slots are
 // retried, cpp/mepidemic.cu:206-235). Returns UINT_MAX when the attempts run out. The four
 // candidates of one Philox call are loaded together (one memory round trip) and the first alive
-// one in attempt order is taken; its state byte is left in *state. `first` is the draw of the
+// one in attempt order is taken; its status is left in *state (a live slot without kDeep is susceptible). `first` is the draw of the
 // first four attempts (the caller computes it together with other lanes' draws).
 __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key, uint32_t pidx, uint32_t e,
                                                     uint32_t base, uint32_t size, uint32_t t, uint32_t* state,
@@ -844,11 +787,11 @@ __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key
 #pragma unroll
         for (int q = 0; q < 4; ++q) slot[q] = base + bounded(r.v[q], size);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) st[q] = (a + q < d.maxTarget) ? __ldcg(&d.m_state[slot[q]]) : (uint32_t)kDead;
+        for (int q = 0; q < 4; ++q) st[q] = (a + q < d.maxTarget) ? __ldcg(&d.m_code[slot[q]]) : (uint32_t)kDead;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             if (!(st[q] & kDead)) {
-                *state = st[q];
+                *state = (st[q] & kDeep) ? __ldcg(&d.m_stat[slot[q]]) & 3u : 0u;
                 return slot[q];
             }
     }
@@ -1100,17 +1043,19 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
                                       ? sh.target[it].x
                                       : mosquito_target(d, key, pm, idx, mbase, ms, t, &st, draw4(key, kInfMTarget, pm, t, idx));
             unsigned long long wk = 0;
-            int32_t bn = 0;
-            if (slot != UINT_MAX) {  // winner key and birth time in one round trip
+            int4 life = make_int4(0, 0, 0, 0);
+            if (slot != UINT_MAX) {  // winner key and life record in one round trip
                 wk = __ldcg(&d.winm[slot]);
-                bn = __ldcg(&d.m_born[slot]);
+                life = __ldcg(reinterpret_cast<const int4*>(d.m_life + slot));
             }
             if (slot != UINT_MAX && wk == order_key(hiword, j, 0, idx)) {
                 const U4 r = draw4(key, kInfMExposed, pm, t, idx >> 2);
-                d.m_state[slot] = 1;
+                d.m_stat[slot] = 1;
                 d.m_strain[slot] = (uint8_t)sm;
-                const int32_t age = (int32_t)t + 1 - bn;
-                d.m_exposed[slot] = (int32_t)resolve(__fadd_rn((float)age, d.mExposed), r.v[idx & 3]);
+                const int32_t age = (int32_t)t + 1 - life.y;
+                const int32_t ex = (int32_t)resolve(__fadd_rn((float)age, d.mExposed), r.v[idx & 3]);
+                d.m_exposed[slot] = ex;
+                d.m_code[slot] = mosq_code(mosq_next(1, life.z, life.y, ex), (int32_t)t + 1, true);
             }
         }
     }
@@ -1211,7 +1156,7 @@ __global__ void __launch_bounds__(256, 4) k_demog_batch(BatchDev bd, uint32_t ko
             const uint32_t local = it - lo, hw = __ldg(&bd.demog_h[inst]);
             const uint32_t t = d.ctrl->t + koff;
             const Key key = load_key(d.ctrl);
-            if (local < hw) demog_humans<U>(d, key, local * 32 * U + lane, 32, t);
+            if (local < hw) demog_humans<U>(d, key, local * 32 * U + lane, 32, t, wsm[warp]);
             else demog_mosquito_quad(d, key, local - hw, lane, t, wsm[warp]);
         }
     }
@@ -1329,42 +1274,38 @@ __global__ void k_init_humans(Dev d)
 __device__ __forceinline__ void init_mosquito_tile(const Dev& d, const Key& key, uint32_t b, uint32_t lane)
 {
     const float alive_p = __fdiv_rn(__ldg(&d.etab[0]), (float)d.M);
-    const uint32_t c0 = __ldg(&d.tcomm[b]);
+    const uint32_t c0 = __ldg(&d.tcomm[b]) & ~kTileSpans;
+    uint32_t codes = 0;
     uint32_t ndead = 0, ndead0 = 0;  // dead slots of the tile; of them, in the tile's first community
     for (int k = 0; k < 4; ++k) {
         const uint32_t i = 4 * (b * 32 + lane) + k;
-        if (i >= d.M) {
-            d.m_state[i] = kPad;
-            d.m_born[i] = 0;
-            d.m_dtime[i] = INT_MIN;
-            d.m_ple[i] = 0.0f;
-            d.m_strain[i] = 0;
-            d.m_exposed[i] = 0;
-            continue;
-        }
-        const U4 r = draw4(key, kInitMosquito, i, 0);
+        d.m_stat[i] = 0;
         d.m_strain[i] = 0;
         d.m_exposed[i] = 0;
-        if (!(u01(r.v[0]) < alive_p)) {
-            d.m_state[i] = kDead;
-            d.m_born[i] = 0;
-            d.m_ple[i] = 0.0f;
-            d.m_dtime[i] = INT_MIN;  // never alive: age 0, death age 0
-            ndead += 1;
-            const uint32_t cc = slot_comm(d, c0, i);
-            if (cc == c0) ndead0 += 1;
-            else atomicSub(&d.mcnt[cc], 1u);
-        } else {
-            const float randCSF = __fmul_rn(__ldg(&d.survm[d.dm]), u01(r.v[1]));
-            const uint32_t a = lower_bound_f(d.survm, d.dm + 1, randCSF);
-            const float base = cdf_at(d.cdfm, d.am, a != 0 ? (int32_t)a - 1 : 0);
-            const float ple = __fadd_rn(__fmul_rn(__fsub_rn(1.0f, base), u01(r.v[2])), base);
-            d.m_state[i] = 0;
-            d.m_born[i] = -(int32_t)a;
-            d.m_ple[i] = ple;
-            d.m_dtime[i] = death_time(-(int32_t)a, death_age_inv(d.cdfm, d.minv, d.am, ple, 4096.0f));
+        Life life{0.0f, 0, INT_MIN, 0};  // padding, or never alive: age 0, death age 0
+        uint32_t code = kPad;
+        if (i < d.M) {
+            const U4 r = draw4(key, kInitMosquito, i, 0);
+            if (!(u01(r.v[0]) < alive_p)) {
+                code = kDead;
+                ndead += 1;
+                const uint32_t cc = slot_comm(d, c0, i);
+                if (cc == c0) ndead0 += 1;
+                else atomicSub(&d.mcnt[cc], 1u);
+            } else {
+                const float randCSF = __fmul_rn(__ldg(&d.survm[d.dm]), u01(r.v[1]));
+                const uint32_t a = lower_bound_f(d.survm, d.dm + 1, randCSF);
+                const float base = cdf_at(d.cdfm, d.am, a != 0 ? (int32_t)a - 1 : 0);
+                life.ple = __fadd_rn(__fmul_rn(__fsub_rn(1.0f, base), u01(r.v[2])), base);
+                life.born = -(int32_t)a;
+                life.dtime = death_time(-(int32_t)a, death_age_lut(d, life.ple));
+                code = mosq_code(life.dtime, 0, false);
+            }
         }
+        codes |= code << (8 * k);
+        d.m_life[i] = life;
     }
+    reinterpret_cast<uint32_t*>(d.m_code)[b * 32 + lane] = codes;
     // One atomic per tile for its first community (a community's alive count would otherwise
     // take one same-address atomic per dead slot).
     const uint32_t tile_dead = __reduce_add_sync(kFull, ndead);
@@ -1411,11 +1352,12 @@ __device__ __forceinline__ void seed_one(const Dev& d, const Key& key, uint32_t 
     }
     if (j < d.mInit) {
         const uint32_t i = seed_perm(key, 1, d.M, j);
-        const uint8_t st = d.m_state[i];
-        if ((st & kDead) && !(d.quirks & ARBO_QUIRK_SEED_DEAD_MOSQUITO)) return;
+        const uint8_t code = d.m_code[i];
+        if ((code & kDead) && !(d.quirks & ARBO_QUIRK_SEED_DEAD_MOSQUITO)) return;
         const U4 r = draw4(key, kSeedMosquito, j, 0);
         const uint32_t s = bounded(r.v[0], d.S);
-        d.m_state[i] = (uint8_t)((st & kDead) | 2u);
+        d.m_stat[i] = 2;
+        d.m_code[i] = (code & kDead) ? (uint8_t)(kDead | kDeep) : mosq_code(d.m_life[i].dtime, 0, true);
         d.m_strain[i] = (uint8_t)s;
         atomicAdd(&d.infm[s * d.P + comm_of(d.mloc, d.P, i)], 1u);
     }
@@ -1555,24 +1497,41 @@ __global__ void k_export_mosquitoes(Dev d, arbo_census_export x)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.M) return;
     const int32_t now = (int32_t)d.ctrl->t;
-    const uint32_t st = d.m_state[i];
+    const bool dead = (d.m_code[i] & kDead) != 0;
+    const Life life = d.m_life[i];
     if (x.m_age) {
         // Alive: steps since birth; dead: the age it died at (0 for a slot dead since initialisation).
-        const int32_t b = d.m_born[i], dt = d.m_dtime[i];
+        const int32_t b = life.born, dt = life.dtime;
         int32_t a = now - b;
-        if (st & kDead) a = dt == INT_MIN ? 0 : max(dt, max(b, 0) + 1) - b;
+        if (dead) a = dt == INT_MIN ? 0 : max(dt, max(b, 0) + 1) - b;
         x.m_age[i] = (uint16_t)a;
     }
-    if (x.m_dead) x.m_dead[i] = (st & kDead) ? 1 : 0;
+    if (x.m_dead) x.m_dead[i] = dead ? 1 : 0;
     if (x.m_exposed) x.m_exposed[i] = (uint16_t)d.m_exposed[i];
-    if (x.m_infect_status) x.m_infect_status[i] = (uint8_t)(st & 3u);
-    if (x.m_ple) x.m_ple[i] = d.m_ple[i];
+    if (x.m_infect_status) x.m_infect_status[i] = (uint8_t)(d.m_stat[i] & 3u);
+    if (x.m_ple) x.m_ple[i] = life.ple;
     if (x.m_strain) x.m_strain[i] = d.m_strain[i];
-    if (x.m_sub_population) x.m_sub_population[i] = slot_comm(d, __ldg(&d.tcomm[i / kTile]), i);
+    if (x.m_sub_population) x.m_sub_population[i] = mosq_comm(d, i);
     if (x.m_sub_pop_index) x.m_sub_pop_index[i] = i;
 }
 
+// One field of the life records to or from an array of M values.
+__global__ void k_life_field(Dev d, int field, int32_t* array, int store)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.M) return;
+    int32_t* f = reinterpret_cast<int32_t*>(d.m_life + i) + field;
+    if (store) *f = array[i];
+    else array[i] = *f;
+}
+
 }  // namespace
+
+int launch_life_field(const Dev& d, int field, void* array, bool store, void* stream)
+{
+    k_life_field<<<cdiv(d.M, 256), 256, 0, (cudaStream_t)stream>>>(d, field, (int32_t*)array, store ? 1 : 0);
+    return (int)cudaGetLastError();
+}
 
 int launch_export(const Dev& d, const arbo_census_export& x, void* stream)
 {

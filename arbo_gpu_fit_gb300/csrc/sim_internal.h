@@ -4,9 +4,10 @@
 //   humans   (N padded to a multiple of 4 agents):  birth time i32, death time i32, next
 //            event time i32, status u8, exposed i32, recovery i32, ple f32, strain u8,
 //            immunity u8.
-//   mosquito (M padded to whole 128-slot tiles):     birth time i32, death time i32, state u8
-//            (bits 0-1 status, bit 7 dead), exposed i32, ple f32, strain u8; tile dead
-//            count i32 per tile. Exposed and recovery hold ages, as in the reference.
+//   mosquito (M padded to whole 128-slot tiles):     event code u8 (dead flag and the low bits of
+//            the next event time, mosq_code), status u8, life record 16 B (ple f32, birth time
+//            i32, death time i32), exposed i32, strain u8; tile dead count i32 per tile.
+//            Exposed and recovery hold ages, as in the reference.
 //   The census is community-sorted: community c owns the contiguous index range
 //   [loc[c], loc[c+1]) of each species, so infection draws hit contiguous ranges and a
 //   128-slot tile spans one or two communities.
@@ -28,7 +29,14 @@
 namespace arbo {
 
 constexpr uint8_t kPad = 0xFF;        // status byte of a padding agent
-constexpr uint8_t kDead = 0x80;       // mosquito state: dead flag
+// Event code of a mosquito slot: what the demographic pass streams, one byte a slot. Bit 7: dead. Of a
+// live slot, bits 0-5 are the low bits of the time of the step in which something happens to it, and
+// kDeep says that this is not simply the death of a susceptible mosquito (it is infected, or its
+// death lies more than kCodeAhead steps away and is looked at again then). Of a dead slot kDeep says
+// that its status byte is not zero. A dead slot is exactly kDead or kDead | kDeep.
+constexpr uint8_t kDead = 0x80;
+constexpr uint8_t kDeep = 0x40;
+constexpr int32_t kCodeAhead = 62;
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 // Death time of an agent born at time `born` with death age `dage` (INT_MAX: never dies).
@@ -47,6 +55,34 @@ __host__ __device__ inline int32_t human_next(uint32_t st, int32_t dtime, int32_
     const int32_t tr = born + when + 1;
     return tr < dtime ? tr : dtime;
 }
+
+// Code of a live slot at time `now` (its steps up to the one that reached `now` are done) whose next
+// event is at time `next`: the step that reaches `next`, the coming one if that is past already.
+__host__ __device__ inline uint8_t mosq_code(int32_t next, int32_t now, bool deep)
+{
+    const int32_t e = next > now ? next : now + 1;
+    const bool far = e > now + kCodeAhead;
+    return (uint8_t)(((uint32_t)(far ? now + kCodeAhead : e) & 63u) | (deep || far ? kDeep : 0u));
+}
+
+// Next event time of a live mosquito of status st: its death or, latent (1), the first step whose new
+// age exceeds its exposed age, whichever comes first.
+__host__ __device__ inline int32_t mosq_next(uint32_t st, int32_t dtime, int32_t born, int32_t exposed)
+{
+    if (st != 1) return dtime;
+    const long long tr = (long long)born + exposed + 1;
+    return tr < dtime ? (tr < INT_MIN ? INT_MIN : (int32_t)tr) : dtime;
+}
+
+// A mosquito slot's life: one 16-byte record, so that a birth writes one sector.
+struct __align__(16) Life {
+    float ple;
+    int32_t born, dtime, unused;
+};
+
+constexpr uint32_t kLutWide = 0x80000000u;    // mlut: several ages in the bucket, search the CDF
+constexpr uint32_t kTileSpans = 0x80000000u;  // tcomm, hcomm: the tile or block spans several communities
+constexpr uint32_t kHumanBlock = 32;
 
 constexpr uint32_t kQuad = 4;  // consecutive recruitment tiles handled by one warp
 constexpr uint32_t kTile = 128;       // mosquito recruitment tile (slots)
@@ -71,10 +107,10 @@ struct Dev {
     // parameters
     float biting, mnSuccess, nmSuccess, recovery, mExposed, nExposed, extInf, longDist, noDist, seroPrev;
     uint32_t maxIntro, maxTarget, quirks, recordSpatial, nInit, mInit;
-    // Ages are kept as birth and death times, so that the demographic pass reads the status
-    // byte and the death time of an agent and writes nothing for a survivor without a
-    // transition: age at time t = t - born; the agent dies in the step that reaches time
-    // t >= dtime (its age then reaches its death age; INT_MAX: never).
+    // Ages are kept as birth and death times, so that the demographic pass reads only when the
+    // next event of an agent is due and writes nothing for an agent without one: age at time
+    // t = t - born; the agent dies in the step that reaches time t >= dtime (its age then reaches
+    // its death age; INT_MAX: never).
     // humans (n_next: next demographic event time, human_next; the pass reads only this)
     int32_t* n_born;
     int32_t* n_dtime;
@@ -87,11 +123,10 @@ struct Dev {
     uint8_t* n_imm;
     // mosquitoes (a dead slot keeps the times of its last life; a slot dead since
     // initialisation has dtime == INT_MIN)
-    int32_t* m_born;
-    int32_t* m_dtime;
-    uint8_t* m_state;
+    uint8_t* m_code;
+    uint8_t* m_stat;
+    Life* m_life;
     int32_t* m_exposed;
-    float* m_ple;
     uint8_t* m_strain;
     int32_t* ledger;
     // communities and network
@@ -99,8 +134,8 @@ struct Dev {
     uint32_t* mloc;   // [P+1]
     uint32_t* nsize;  // [P]
     uint32_t* msize;  // [P]
-    uint32_t* tcomm;  // [tiles] community of each mosquito tile's first slot
-    uint32_t* hcomm;  // [ceil(N/128)] community of each 128-human block's first agent
+    uint32_t* tcomm;  // [tiles] community of each mosquito tile's first slot | kTileSpans
+    uint32_t* hcomm;  // community of each block of kHumanBlock humans' first agent | kTileSpans
     uint32_t* csr_loc;
     uint32_t* csr_to;
     // counters
@@ -115,6 +150,7 @@ struct Dev {
     float* cdfh;
     float* cdfm;
     uint32_t* minv;   // [4098] first mosquito age with CDF >= k/4096 (table size if none)
+    uint2* mlut;      // [4097] {first age with CDF >= k/4096 | kLutWide, CDF at it as bits} (death_age_lut)
     uint32_t* minvh;  // [65538] first human age with CDF >= k/65536 (table size if none)
     float* survh;
     float* survm;
@@ -171,6 +207,8 @@ int demog_tma_blocks_per_sm(uint32_t unroll);
 int launch_step(const Dev& d, const Launch& l, void* stream, void* events, uint32_t koff);
 // Adds n to the step counter and the winner epoch (one thread).
 int launch_advance(const Dev& d, uint32_t n, void* stream);
+// field 0, 1, 2: PLE, birth time, death time of every slot, between the life records and an array.
+int launch_life_field(const Dev& d, int field, void* array, bool store, void* stream);
 // Writes the census in the reference's types into the caller's buffers (arbo_sim_export_census).
 int launch_export(const Dev& d, const arbo_census_export& x, void* stream);
 uint32_t launches_per_step();
