@@ -127,6 +127,7 @@ __device__ __forceinline__ int32_t death_age_lut(const Dev& d, float ple)
 // Per-warp shared staging of the demographic pass.
 struct QuadSmem {
     uint4 code[32];
+    uint4 draw[32];  // rebirth draws of ranks 4s .. 4s+3 of tile u, by the lane 8u + s that made them
     union {
         uint8_t slot[kQuad][kTile];    // reborn slot offsets by rank
         uint16_t deep[kQuad * kTile];  // slots with a deep event; a human pass's agents with an event due
@@ -266,6 +267,31 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
     return i == 0 ? v.v[0] : i == 1 ? v.v[1] : i == 2 ? v.v[2] : v.v[3];
 }
 
+// What a quad needs that does not depend on its codes, made while they are on their way: the tile's
+// carried dead count and community, the expected mosquitoes and the tile's quota draw, and the draws of
+// the first 32 births of each tile (left in the staging), which are keyed by rank and not by slot.
+struct QuadStart {
+    int32_t led;
+    uint32_t c0;
+    float target;
+    uint32_t quota;
+};
+
+__device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
+                                                QuadSmem& sm)
+{
+    const uint32_t u = lane >> 3, b = q * kQuad + u;
+    const bool live = b < d.tiles;
+    QuadStart at;
+    at.led = live ? d.ledger[b] : 0;
+    at.c0 = live ? __ldg(&d.tcomm[b]) : 0u;
+    at.target = __ldg(&d.etab[t + 1]);
+    at.quota = pick4(draw4(key, kMosquitoTile, q, t), u);
+    const U4 r = draw4(key, kMosquitoRebirth, b, t, lane & 7u);
+    sm.draw[lane] = make_uint4(r.v[0], r.v[1], r.v[2], r.v[3]);
+    return at;
+}
+
 // One warp, tiles 4q..4q+3; lane l holds the codes of slots 16(l mod 8) .. +15 of tile 4q + l/8, four
 // words. Per tile: deaths (a live slot dies in the step that reaches its death time), the birth quota
 // (cpp/mdemographic.cu:104-129) from the carried dead count, rebirth of the lowest-index dead slots, the
@@ -280,15 +306,12 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
 // reborn slot under its rank; one lane per reborn slot then draws its PLE and writes its life record
 // (one sector instead of three) and its code, which the owners write back with one 16-byte store.
 __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
-                                                   QuadSmem& sm, const uint4 A)
+                                                   QuadSmem& sm, const QuadStart& at, const uint4 A)
 {
     const int32_t tn = (int32_t)t + 1;
     const uint32_t u = lane >> 3, seg = lane & 7u, b = q * kQuad + u;
     const bool live = b < d.tiles;
-    const int32_t led = live ? d.ledger[b] : 0;
-    const uint32_t c0 = live ? __ldg(&d.tcomm[b]) : 0u;
-    const float target = __ldg(&d.etab[t + 1]);
-    const U4 rq = draw4(key, kMosquitoTile, q, t);
+    const uint32_t c0 = at.c0;
 
     uint32_t aw[4] = {A.x, A.y, A.z, A.w}, z[4], deep = 0;
     const uint32_t now4 = ((uint32_t)tn & 63u) * 0x01010101u;
@@ -358,13 +381,13 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
     if (live) {
         const uint32_t start = b * kTile;
         const uint32_t bt = (d.M - start) < kTile ? (d.M - start) : kTile;
-        const uint32_t L = (uint32_t)led + died_tot;
+        const uint32_t L = (uint32_t)at.led + died_tot;
         const float fbt = (float)bt;
-        float x = __fmul_rn(target, fbt);
+        float x = __fmul_rn(at.target, fbt);
         x = __fdiv_rn(x, (float)d.M);
         x = __fsub_rn(x, fbt);
         x = __fadd_rn(x, (float)L);
-        const int births = (int)resolve(x, pick4(rq, u));
+        const int births = (int)resolve(x, at.quota);
         if (seg == 0) d.ledger[b] = (int32_t)L - births;
         nb = births > 0 ? min((uint32_t)births, dead_tot) : 0u;
     }
@@ -402,8 +425,10 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
         for (uint32_t j = lane; j < rtot; j += 32) {
             const uint32_t v = (j >= n0 ? 1u : 0u) + (j >= n1 ? 1u : 0u) + (j >= n2 ? 1u : 0u);
             const uint32_t r = j - (v == 0 ? 0u : v == 1 ? n0 : v == 2 ? n1 : n2);
-            const U4 x = draw4(key, kMosquitoRebirth, q * kQuad + v, t, r >> 2);
-            const float ple = u01(pick4(x, r & 3u));
+            uint32_t x;
+            if (r < 32) x = reinterpret_cast<const uint32_t*>(sm.draw)[32 * v + r];
+            else x = pick4(draw4(key, kMosquitoRebirth, q * kQuad + v, t, r >> 2), r & 3u);
+            const float ple = u01(x);
             const uint32_t o = v * kTile + sm.slot[v][r], i = q * kQuad * kTile + o;
             const int32_t dt = death_time(tn, death_age_lut(d, ple));
             *reinterpret_cast<int4*>(d.m_life + i) = make_int4(__float_as_int(ple), tn, dt, 0);
@@ -418,13 +443,17 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
     }
 }
 
-// Quad with its codes loaded straight from global memory.
+// Quad with its codes loaded straight from global memory. With kWait, the wait for the previous kernel
+// stands between what does not depend on it and the codes, which its infections change.
+template <bool kWait>
 __device__ __forceinline__ void demog_mosquito_quad(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
                                                     QuadSmem& sm)
 {
+    const QuadStart at = quad_start(d, key, q, lane, t, sm);
+    if (kWait) griddep_wait();
     uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
     if (q * kQuad + (lane >> 3) < d.tiles) A = reinterpret_cast<const uint4*>(d.m_code)[q * 32 + lane];
-    mosquito_quad_core(d, key, q, lane, t, sm, A);
+    mosquito_quad_core(d, key, q, lane, t, sm, at, A);
 }
 
 // ------------------------------------------------------------------ TMA-staged pipeline
@@ -533,7 +562,7 @@ __global__ void __launch_bounds__(128, 4) k_demog_tma(Dev d, uint32_t koff)
         uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
         if (q * kQuad + (lane >> 3) < d.tiles) A = ws.stage[sidx][lane];
         __syncwarp();  // every lane has its words before the buffer is refilled next iteration
-        mosquito_quad_core(d, key, q, lane, t, ws.qs, A);
+        mosquito_quad_core(d, key, q, lane, t, ws.qs, quad_start(d, key, q, lane, t, ws.qs), A);
     }
     griddep_launch_dependents();
 }
@@ -547,11 +576,12 @@ __device__ __forceinline__ void demog_block(const Dev& d, uint32_t b, uint32_t h
     const Key key = load_key(d.ctrl);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     if (b < hblocks) {
+        griddep_wait();
         demog_humans<U>(d, key, b * blockDim.x * U + threadIdx.x, blockDim.x, t, wsm[warp]);
     } else {
         const uint32_t wpb = blockDim.x >> 5;
         const uint32_t q = (b - hblocks) * wpb + warp;
-        if (q * kQuad < d.tiles) demog_mosquito_quad(d, key, q, lane, t, wsm[warp]);
+        if (q * kQuad < d.tiles) demog_mosquito_quad<true>(d, key, q, lane, t, wsm[warp]);
     }
 }
 
@@ -560,7 +590,7 @@ __device__ __forceinline__ void demog_block(const Dev& d, uint32_t b, uint32_t h
 // the last wave they fill the SMs that the mosquito blocks leave idle (2.4 waves of mosquito blocks
 // on the large workload). Same results either way; 34.6-34.8 against 36.4-37.5 us mid-epidemic.
 template <int U>
-__global__ void __launch_bounds__(256, 4) k_demog(Dev d, uint32_t hblocks, uint32_t koff)
+__global__ void __launch_bounds__(256, 6) k_demog(Dev d, uint32_t hblocks, uint32_t koff)
 {
     __shared__ QuadSmem wsm[8];
     const uint32_t mblocks = gridDim.x - hblocks;
@@ -1070,6 +1100,7 @@ __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
+    griddep_launch_dependents();  // the next step's demographic pass may be scheduled; it waits for this grid
     for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp<true>(d, c, at, sh);
 }
 
@@ -1125,7 +1156,7 @@ __device__ __forceinline__ void batch_warp_items(const BatchDev& bd, const uint3
 // private copy of its current instance's descriptor in shared memory: no block-wide barrier
 // anywhere.
 template <int U>
-__global__ void __launch_bounds__(256, 4) k_demog_batch(BatchDev bd, uint32_t koff)
+__global__ void __launch_bounds__(256, 5) k_demog_batch(BatchDev bd, uint32_t koff)
 {
     __shared__ QuadSmem wsm[8];
     __shared__ __align__(16) unsigned long long wdev[8][sizeof(Dev) / 8];
@@ -1157,7 +1188,7 @@ __global__ void __launch_bounds__(256, 4) k_demog_batch(BatchDev bd, uint32_t ko
             const uint32_t t = d.ctrl->t + koff;
             const Key key = load_key(d.ctrl);
             if (local < hw) demog_humans<U>(d, key, local * 32 * U + lane, 32, t, wsm[warp]);
-            else demog_mosquito_quad(d, key, local - hw, lane, t, wsm[warp]);
+            else demog_mosquito_quad<false>(d, key, local - hw, lane, t, wsm[warp]);
         }
     }
     griddep_launch_dependents();
@@ -1585,10 +1616,11 @@ int launch_demog(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
     const uint32_t quads = cdiv(d.tiles, kQuad);
     const uint32_t mblocks = cdiv(quads, l.demogBlock / 32);
     const dim3 grid(hblocks + mblocks), block(l.demogBlock);
-    if (U == 4) k_demog<4><<<grid, block, 0, st>>>(d, hblocks, koff);
-    else if (U == 2) k_demog<2><<<grid, block, 0, st>>>(d, hblocks, koff);
-    else k_demog<1><<<grid, block, 0, st>>>(d, hblocks, koff);
-    return (int)cudaGetLastError();
+    // Inside a graph the previous kernel is the last step's infection pass, which leaves the step
+    // control, the dead counts and the tables alone, so the pass may begin before it ends. At a graph's
+    // first step it is the kernel that advances the step control.
+    return launch_pdl(U == 4 ? k_demog<4> : U == 2 ? k_demog<2> : k_demog<1>, grid, block, 0, st, l.pdl && koff > 0, d,
+                      hblocks, koff);
 }
 
 int launch_foi(const Dev& d, const Launch& l, cudaStream_t st, int collect_only, uint32_t koff)
