@@ -881,7 +881,12 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
     // One draw per lane in one pass: introduction counts (lanes < S), first serotypes (8, 9).
     const U4 rd = draw4(key, lane < S ? (uint32_t)kIntroCount : lane == 8 ? (uint32_t)kInfMStart : (uint32_t)kInfHStart,
                         lane < S ? pl : c, t);
-    if (kWait) griddep_wait();
+    if (kWait) {
+        griddep_wait();
+        // Only now may the next step's demographic pass be scheduled: before its own wait it reads the
+        // dead counts, which this step's pass (finished before the grid waited for) writes.
+        griddep_launch_dependents();
+    }
     const uint32_t mc = d.mcnt[c];
     uint32_t kh = lane < S ? d.transh[pl] : 0u;
     uint32_t km = lane < S ? d.transm[pl] : 0u;
@@ -1100,7 +1105,6 @@ __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
-    griddep_launch_dependents();  // the next step's demographic pass may be scheduled; it waits for this grid
     for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp<true>(d, c, at, sh);
 }
 
@@ -1616,9 +1620,9 @@ int launch_demog(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
     const uint32_t quads = cdiv(d.tiles, kQuad);
     const uint32_t mblocks = cdiv(quads, l.demogBlock / 32);
     const dim3 grid(hblocks + mblocks), block(l.demogBlock);
-    // Inside a graph the previous kernel is the last step's infection pass, which leaves the step
-    // control, the dead counts and the tables alone, so the pass may begin before it ends. At a graph's
-    // first step it is the kernel that advances the step control.
+    // Within a run of steps the previous kernel is the last step's infection pass, which leaves the step
+    // control, the dead counts and the tables alone, so the pass may begin before it ends. At a run's
+    // first step (koff 0) it may be the kernel that advances the step control.
     return launch_pdl(U == 4 ? k_demog<4> : U == 2 ? k_demog<2> : k_demog<1>, grid, block, 0, st, l.pdl && koff > 0, d,
                       hblocks, koff);
 }
