@@ -33,6 +33,14 @@ int fail(int code, const std::string& msg)
         if (e_ != cudaSuccess) return fail(ARBO_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// Steps that a handle or batch launches kernel by kernel before it captures graphs: the three launches
+// of a step take the host less time (about 8 us) than the step takes the device, while a 64-step graph
+// costs half a millisecond to make, again after every change of parameters. What is left of a call
+// after its whole graphs is launched the same way (as one-step graphs each step paid for a graph launch
+// and could not overlap the one before: 30 steps of 1.2e4 agents with initialisation and results 775 ->
+// 662 us, and 440 to 500 us less for the first run of a handle).
+constexpr uint32_t kDirectSteps = 256;
+
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Human bi-Weibull CDF at an integer age (cpp/ndemographic.cu:13-29), in double, rounded once.
@@ -136,8 +144,8 @@ struct arbo_sim {
     std::vector<uint32_t> nsize, msize, nloc, mloc;
     std::vector<float> etab;
     cudaStream_t cap = nullptr;
-    cudaGraphExec_t gmulti = nullptr, gone = nullptr;
-    uint32_t gsteps = 0;
+    cudaGraphExec_t gmulti = nullptr;
+    uint32_t direct = 0;  // steps launched kernel by kernel since the parameters changed
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     int device = 0;
     uint64_t seed = 0;
@@ -597,7 +605,6 @@ int arbo_sim_destroy(arbo_sim* s)
     if (!s) return ARBO_OK;
     cudaSetDevice(s->device);
     if (s->gmulti) cudaGraphExecDestroy(s->gmulti);
-    if (s->gone) cudaGraphExecDestroy(s->gone);
     for (int k = 0; k < 4; ++k)
         if (s->ev[k]) cudaEventDestroy(s->ev[k]);
     for (cudaEvent_t e : s->step_ev) cudaEventDestroy(e);
@@ -658,8 +665,8 @@ static void param_change_host(arbo_sim* s, const arbo_sim_param& p)
     apply_rates(p, s->d);
     fill_expected(p, s->d.M, s->d.T, s->etab);
     if (s->gmulti) cudaGraphExecDestroy(s->gmulti);
-    if (s->gone) cudaGraphExecDestroy(s->gone);
-    s->gmulti = s->gone = nullptr;
+    s->gmulti = nullptr;
+    s->direct = 0;
     s->version += 1;
 }
 
@@ -755,23 +762,23 @@ int arbo_sim_step(arbo_sim* s, uint32_t nsteps, void* stream)
         }
         return ARBO_OK;
     }
-    if (n >= G && !s->gmulti) {
-        const int e = capture_graph(s, G, &s->gmulti);
-        if (e) return e;
-    }
-    while (n >= G) {
-        CUDA_TRY(cudaGraphLaunch(s->gmulti, st));
-        n -= G;
-        s->host_t += G;
-    }
-    if (n > 0 && !s->gone) {
-        const int e = capture_graph(s, 1, &s->gone);
-        if (e) return e;
-    }
     while (n > 0) {
-        CUDA_TRY(cudaGraphLaunch(s->gone, st));
-        n -= 1;
-        s->host_t += 1;
+        const uint32_t chunk = std::min(n, G);
+        if (chunk == G && s->direct >= kDirectSteps) {
+            if (!s->gmulti) {
+                const int e = capture_graph(s, G, &s->gmulti);
+                if (e) return e;
+            }
+            CUDA_TRY(cudaGraphLaunch(s->gmulti, st));
+        } else {
+            int e = 0;
+            for (uint32_t k = 0; k <= chunk && !e; ++k)
+                e = k < chunk ? launch_step(s->d, s->l, st, nullptr, k) : launch_advance(s->d, chunk, st);
+            if (e) return fail(ARBO_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString((cudaError_t)e));
+            s->direct += chunk;
+        }
+        n -= chunk;
+        s->host_t += chunk;
     }
     return ARBO_OK;
 }
@@ -1396,7 +1403,8 @@ struct arbo_batch {
     void* stage = nullptr;                    // pinned staging of arbo_batch_set_params
     size_t stage_bytes = 0;
     cudaStream_t cap = nullptr;
-    cudaGraphExec_t gmulti = nullptr, gone = nullptr;
+    cudaGraphExec_t gmulti = nullptr;
+    uint32_t direct = 0;  // steps launched kernel by kernel since the launch shapes changed
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> step_ev;
     void* flush = nullptr;
@@ -1418,8 +1426,8 @@ int arch_knobs_ok(const arbo_arch_param& a)
 void batch_drop_graphs(arbo_batch* b)
 {
     if (b->gmulti) cudaGraphExecDestroy(b->gmulti);
-    if (b->gone) cudaGraphExecDestroy(b->gone);
-    b->gmulti = b->gone = nullptr;
+    b->gmulti = nullptr;
+    b->direct = 0;
 }
 
 // Instances with equal death-age tables (equal life-expectancy parameters and run lengths, as
@@ -1838,17 +1846,20 @@ int arbo_batch_step(arbo_batch* b, uint32_t nsteps, void* stream)
         }
         return ARBO_OK;
     }
-    if (n >= G && !b->gmulti && (e = batch_capture(b, G, &b->gmulti))) return e;
-    while (n >= G) {
-        CUDA_TRY(cudaGraphLaunch(b->gmulti, st));
-        n -= G;
-        batch_advance_host(b, G);
-    }
-    if (n > 0 && !b->gone && (e = batch_capture(b, 1, &b->gone))) return e;
     while (n > 0) {
-        CUDA_TRY(cudaGraphLaunch(b->gone, st));
-        n -= 1;
-        batch_advance_host(b, 1);
+        const uint32_t chunk = std::min(n, G);
+        if (chunk == G && b->direct >= kDirectSteps) {
+            if (!b->gmulti && (e = batch_capture(b, G, &b->gmulti))) return e;
+            CUDA_TRY(cudaGraphLaunch(b->gmulti, st));
+        } else {
+            e = 0;
+            for (uint32_t k = 0; k <= chunk && !e; ++k)
+                e = k < chunk ? launch_step_batch(b->bd, b->l, st, nullptr, k) : launch_advance_batch(b->bd, chunk, st);
+            if (e) return fail(ARBO_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString((cudaError_t)e));
+            b->direct += chunk;
+        }
+        n -= chunk;
+        batch_advance_host(b, chunk);
     }
     return ARBO_OK;
 }
