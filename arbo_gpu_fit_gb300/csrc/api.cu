@@ -1405,6 +1405,8 @@ struct arbo_batch {
     cudaStream_t cap = nullptr;
     cudaGraphExec_t gmulti = nullptr;
     uint32_t direct = 0;  // steps launched kernel by kernel since the launch shapes changed
+    bool phase_shapes = false;  // the caller chose launch shapes of the per-phase kernels
+    uint32_t cluster = 0;       // CTAs per simulation of k_steps (0: the per-phase kernels)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> step_ev;
     void* flush = nullptr;
@@ -1462,6 +1464,44 @@ Dev batch_desc(const arbo_batch* b, size_t i)
     d.minv = m.minv;
     d.mlut = m.mlut;
     return d;
+}
+
+// Steps per launch of k_steps.
+constexpr uint32_t kClusterSteps = 128;
+
+// Whether `a` chooses launch shapes of the per-phase kernels (the human unroll aside, which chain
+// batches set for them): a caller who does gets those kernels.
+bool chooses_shapes(const arbo_arch_param& a)
+{
+    arbo_arch_param q;
+    arbo_arch_param_query(&q, -1);
+    return a.demogBlock != q.demogBlock || a.foiBlock != q.foiBlock || a.infectBlock != q.infectBlock ||
+           a.graphSteps != q.graphSteps || a.demogPipeline != q.demogPipeline;
+}
+
+// CTAs per simulation when the batch's steps run as one cluster per simulation (k_steps), or 0 for the
+// per-phase kernels. C: the largest cluster of which all the simulations' fit the device at once.
+// A step takes a cluster about 13 us plus 0.45 us per 1,000 work units of its simulation (agents, and
+// 300 per community for the infection pass) and CTA, 0.85 us once CTAs share SMs, and the device as a
+// whole 0.003 us per 1,000 units; the per-phase kernels take 35 us and the same throughput. Measured, us
+// per step, clusters against per-phase kernels: 8 simulations of 7e4 agents 17 and 38, 32 of them 20 and
+// 41, 128 of them 51 and 65, 200 of them 100 and 91, 304 of them 120 and 130; 32 of 2.1e5 agents 37 and
+// 50; 64 of 4e4 to 4e5 agents 92 and 67. The line falls where one simulation is much larger than the
+// others (its cluster works alone) or there are more than fit at once.
+uint32_t batch_cluster(const arbo_batch* b)
+{
+    if (b->phase_shapes) return 0;
+    const uint32_t n = (uint32_t)b->sims.size();
+    const uint32_t C = steps_cluster(n);
+    if (!C) return 0;
+    double total = 0.0, most = 0.0;
+    for (const arbo_sim* s : b->sims) {
+        const double units = ((double)s->d.N + s->d.M + 300.0 * s->d.P) / 1000.0;
+        total += units;
+        most = std::max(most, units);
+    }
+    const double per = n * C <= b->l.numSM ? 0.45 : 0.85;
+    return 13.0 + std::max(per * most / C, 0.003 * total) < 35.0 + 0.003 * total ? C : 0;
 }
 
 // Block counts of every instance for the launch shapes of `a`; descriptors and tables uploaded.
@@ -1569,6 +1609,7 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     b->bd = bd;
     b->l = l;
     b->arch = a;
+    b->cluster = batch_cluster(b);
     return ARBO_OK;
 }
 
@@ -1706,6 +1747,7 @@ int arbo_batch_create(arbo_sim* const* sims, uint32_t n, const arbo_arch_param* 
         return bail(fail(ARBO_ERR_CUDA, "cudaStreamCreate"));
     for (int k = 0; k < 4; ++k)
         if (cudaEventCreate(&b->ev[k]) != cudaSuccess) return bail(fail(ARBO_ERR_CUDA, "cudaEventCreate"));
+    b->phase_shapes = chooses_shapes(arch ? *arch : sims[0]->arch);
     const int e = batch_configure(b, arch ? *arch : sims[0]->arch);
     if (e) return bail(e);
     *out = b;
@@ -1743,7 +1785,11 @@ int arbo_batch_set_arch(arbo_batch* b, const arbo_arch_param* arch)
     if (!b || !arch) return fail(ARBO_ERR_INVALID, "null argument");
     CUDA_TRY(cudaSetDevice(b->device));
     CUDA_TRY(cudaDeviceSynchronize());  // graphs of the old shape may still run
-    return batch_configure(b, *arch);
+    const bool before = b->phase_shapes;
+    b->phase_shapes = chooses_shapes(*arch);
+    const int e = batch_configure(b, *arch);
+    if (e) b->phase_shapes = before;
+    return e;
 }
 
 int arbo_batch_get_arch(const arbo_batch* b, arbo_arch_param* arch, uint32_t grids[3])
@@ -1845,6 +1891,13 @@ int arbo_batch_step(arbo_batch* b, uint32_t nsteps, void* stream)
             batch_advance_host(b, 1);
         }
         return ARBO_OK;
+    }
+    while (n > 0 && b->cluster) {
+        const uint32_t chunk = std::min(n, kClusterSteps);
+        e = launch_steps(b->bd.devs, b->bd.n, b->cluster, chunk, st);
+        if (e) return fail(ARBO_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString((cudaError_t)e));
+        n -= chunk;
+        batch_advance_host(b, chunk);
     }
     while (n > 0) {
         const uint32_t chunk = std::min(n, G);

@@ -217,6 +217,12 @@ uint32_t launches_per_step();
 // code. Returns the cudaError_t as int.
 int preload_step_kernels(const Launch& l);
 
+// Many whole steps of the n simulations of descriptors devs in one launch, one cluster of C CTAs each
+// (C as steps_cluster(n) gives it: the largest of 16, 8, 4, 2, 1 with all n clusters resident at
+// once on the current device; 0 when there is none).
+int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t nsteps, void* stream);
+uint32_t steps_cluster(uint32_t n);
+
 // Batched steps (see BatchDev); the block shapes come from l, the grids from bd.
 int launch_step_batch(const BatchDev& bd, const Launch& l, void* stream, void* events, uint32_t koff);
 int launch_advance_batch(const BatchDev& bd, uint32_t n, void* stream);
