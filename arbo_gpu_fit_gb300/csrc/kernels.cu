@@ -127,6 +127,7 @@ __device__ __forceinline__ int32_t death_age_lut(const Dev& d, float ple)
 // Per-warp shared staging of the demographic pass.
 struct QuadSmem {
     uint4 code[32];
+    uint32_t c0[kQuad], end[kQuad];  // community of each tile's first slot, and the slot where it ends
     uint4 draw[32];  // rebirth draws of ranks 4s .. 4s+3 of tile u, by the lane 8u + s that made them
     union {
         uint8_t slot[kQuad][kTile];    // reborn slot offsets by rank
@@ -221,6 +222,12 @@ __device__ __forceinline__ void demog_humans(const Dev& d, const Key key, uint32
     __syncwarp();
 }
 
+// Community of slot i at or after community c, which ends at slot `end` (both move on).
+__device__ __forceinline__ void comm_forward(const Dev& d, uint32_t i, uint32_t& c, uint32_t& end)
+{
+    while (i >= end) end = __ldg(&d.mloc[++c + 1]);
+}
+
 __device__ __forceinline__ uint32_t slot_comm(const Dev& d, uint32_t c0, uint32_t i)
 {
     uint32_t c = c0;
@@ -237,13 +244,14 @@ __device__ __forceinline__ uint32_t mosq_comm(const Dev& d, uint32_t i)
 
 // A live slot whose event is due in the step that reaches time tn and is not the plain death of a
 // susceptible mosquito: its death, its latent-to-infectious transition, or neither yet. Returns its
-// new code.
-__device__ __noinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn)
+// new code. c and end: the community of its tile's first slot and where that ends.
+__device__ __noinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn, uint32_t c, uint32_t end)
 {
     const int4 r = *reinterpret_cast<const int4*>(d.m_life + i);  // ple, born, dtime
     uint32_t st = d.m_stat[i] & 3u;
     const int32_t ex = d.m_exposed[i];
-    const uint32_t s = d.m_strain[i], c = mosq_comm(d, i);
+    const uint32_t s = d.m_strain[i];
+    comm_forward(d, i, c, end);
     if (tn >= r.z) {
         if (st == 2) counter_dec(&d.infm[s * d.P + c], d.ctrl);
         return st ? (uint32_t)(kDead | kDeep) : (uint32_t)kDead;
@@ -272,7 +280,7 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
 // the first 32 births of each tile (left in the staging), which are keyed by rank and not by slot.
 struct QuadStart {
     int32_t led;
-    uint32_t c0;
+    uint32_t c0, end;
     float target;
     uint32_t quota;
 };
@@ -285,6 +293,11 @@ __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uin
     QuadStart at;
     at.led = live ? d.ledger[b] : 0;
     at.c0 = live ? __ldg(&d.tcomm[b]) : 0u;
+    at.end = (at.c0 & kTileSpans) ? __ldg(&d.mloc[(at.c0 & ~kTileSpans) + 1]) : ~0u;
+    if ((lane & 7u) == 0) {
+        sm.c0[u] = at.c0 & ~kTileSpans;
+        sm.end[u] = at.end;
+    }
     at.target = __ldg(&d.etab[t + 1]);
     at.quota = pick4(draw4(key, kMosquitoTile, q, t), u);
     const U4 r = draw4(key, kMosquitoRebirth, b, t, lane & 7u);
@@ -345,7 +358,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
         __syncwarp();
         for (uint32_t j = lane; j < total; j += 32) {
             const uint32_t o = sm.deep[j];
-            reinterpret_cast<uint8_t*>(sm.code)[o] = (uint8_t)mosq_deep(d, q * kQuad * kTile + o, tn);
+            reinterpret_cast<uint8_t*>(sm.code)[o] = (uint8_t)mosq_deep(d, q * kQuad * kTile + o, tn, sm.c0[o / kTile], sm.end[o / kTile]);
         }
         __syncwarp();
         const uint4 B = sm.code[lane];
@@ -409,9 +422,11 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
         uint32_t died16 = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) died16 |= nibble7(z[j]) << (4 * j);
+        uint32_t c = c0 & ~kTileSpans, end = at.end;
         for (uint32_t m = born ^ died16; m; m &= m - 1) {
             const uint32_t k = __ffs(m) - 1;
-            atomicAdd(&d.mcnt[slot_comm(d, c0 & ~kTileSpans, b * kTile + 16 * seg + k)], ((born >> k) & 1u) ? 1u : ~0u);
+            comm_forward(d, b * kTile + 16 * seg + k, c, end);
+            atomicAdd(&d.mcnt[c], ((born >> k) & 1u) ? 1u : ~0u);
         }
     } else if (seg == 0 && nb != died_tot) {
         atomicAdd(&d.mcnt[c0], nb - died_tot);  // one atomic per tile
