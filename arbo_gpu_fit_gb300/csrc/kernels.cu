@@ -850,20 +850,31 @@ constexpr uint32_t kTargetCache = 128;  // items whose targets Phase A keeps for
 
 struct InfectWarpSmem {
     uint4 target[kTargetCache];         // per item: four human targets, or a mosquito slot in .x
-    uint32_t hstart[ARBO_MAX_STRAINS];  // first item of serotype position j, human groups
-    uint32_t mstart[ARBO_MAX_STRAINS];  // first item of serotype position j, mosquito events
-    uint32_t kh[ARBO_MAX_STRAINS];      // human events by position
-    uint32_t km[ARBO_MAX_STRAINS];      // mosquito events by position
+    // First item of each serotype position and events by position, humans (groups of four) and
+    // mosquitoes; positions past the last serotype start at UINT_MAX.
+    uint4 hstart[2], mstart[2];
+    uint32_t kh[ARBO_MAX_STRAINS], km[ARBO_MAX_STRAINS];
 };
+static_assert(ARBO_MAX_STRAINS == 8, "tables of eight serotype positions");
 
-// Serotype position of item `rel` of a table of starts (the last position whose start is <= rel;
-// positions without items share the next one's start).
-__device__ __forceinline__ uint32_t item_position(const uint32_t* start, uint32_t S, uint32_t rel)
+// Serotype position of item `rel` and its number within it, from a table of starts: the last position
+// whose start is <= rel (positions without items share the next one's start).
+__device__ __forceinline__ uint32_t item_position(const uint4* start, uint32_t rel, uint32_t* idx)
 {
-    uint32_t j = 0;
-    while (j + 1 < S && start[j + 1] <= rel) ++j;
+    const uint4 a = start[0], b = start[1];
+    const uint32_t s[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t j = 0, at = 0;
+#pragma unroll
+    for (uint32_t k = 1; k < 8; ++k)
+        if (s[k] <= rel) {
+            j = k;
+            at = s[k];
+        }
+    *idx = rel - at;
     return j;
 }
+
+__device__ __forceinline__ uint32_t wrap(uint32_t x, uint32_t n) { return x >= n ? x - n : x; }
 
 // Infection draws of community c, by one warp. Lanes 0..S-1 read the community's event counts
 // and draw its introduction counts, lanes 8 and 9 the first serotypes; the events (groups of
@@ -923,32 +934,53 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
         if (ns) sv = bounded(rd.v[0], S);
     }
     const uint32_t s0m = __shfl_sync(kFull, sv, 8), s0h = __shfl_sync(kFull, sv, 9);
-    uint32_t H = 0, Mt = 0;
-    for (uint32_t j = 0; j < S; ++j) {
-        const uint32_t khj = __shfl_sync(kFull, kh, (s0h + j) % S);
-        const uint32_t kmj = __shfl_sync(kFull, km, (s0m + j) % S);
-        if (lane == 0) {
-            sh.hstart[j] = H;
-            sh.mstart[j] = Mt;
-            sh.kh[j] = khj;
-            sh.km[j] = kmj;
+    // Lane j: serotype position j (the j-th serotype from the first of each species).
+    const uint32_t hs = wrap(s0h + (lane & 7u), S), ms_ = wrap(s0m + (lane & 7u), S);
+    uint32_t khj = __shfl_sync(kFull, kh, hs), kmj = __shfl_sync(kFull, km, ms_), nej = __shfl_sync(kFull, ne, hs);
+    if (lane >= S) khj = kmj = nej = 0;
+    uint32_t hi = (khj + 3) >> 2, mi = kmj;
+    const uint32_t h0 = hi, m0 = mi;
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, hi, off), x = __shfl_up_sync(kFull, mi, off);
+        if (lane >= (uint32_t)off) {
+            hi += y;
+            mi += x;
         }
-        H += (khj + 3) >> 2;
-        Mt += kmj;
     }
+    if (lane < 8) {
+        reinterpret_cast<uint32_t*>(sh.hstart)[lane] = lane < S ? hi - h0 : UINT_MAX;
+        reinterpret_cast<uint32_t*>(sh.mstart)[lane] = lane < S ? mi - m0 : UINT_MAX;
+        sh.kh[lane] = khj;
+        sh.km[lane] = kmj;
+    }
+    const uint32_t H = __shfl_sync(kFull, hi, 7), Mt = __shfl_sync(kFull, mi, 7);
+    const unsigned intro = __ballot_sync(kFull, nej != 0);  // positions with introductions
     __syncwarp();
     const uint32_t items = H + Mt;
-    const bool any_intro = __any_sync(kFull, ne != 0);
-    if (items == 0 && !any_intro) return;
+    if (items == 0 && !intro) return;
+    // The first introduction's first 32 attempts load everything but the bids together with the events'
+    // targets: nothing before them changes it.
+    uint32_t ii = 0, iim = 0, ist = 1;
+    int32_t ibn = 0, idt = 0;
+    if (intro && lane < d.maxIntro) {
+        const uint32_t ph = wrap(s0h + __ffs(intro) - 1, S) * P + c;
+        const U4 r = draw4(key, kIntroTarget, ph, t, lane >> 2);
+        ii = nbase + bounded(pick4(r, lane & 3u), ns);
+        iim = __ldcg(&d.n_imm[ii]);
+        ist = __ldcg(&d.n_status[ii]);
+        ibn = __ldcg(&d.n_born[ii]);
+        idt = __ldcg(&d.n_dtime[ii]);
+    }
 
     // Phase A. Human groups and mosquito events draw their targets in one pass (the first four
     // attempts of a mosquito event).
     for (uint32_t it = lane; it < items; it += 32) {
         const bool hum = it < H;
         const uint32_t rel = hum ? it : it - H;
-        const uint32_t j = item_position(hum ? sh.hstart : sh.mstart, S, rel);
-        const uint32_t idx = rel - (hum ? sh.hstart[j] : sh.mstart[j]);
-        const uint32_t sp = ((hum ? s0h : s0m) + j) % S, pp = sp * P + c;
+        uint32_t idx;
+        const uint32_t j = item_position(hum ? sh.hstart : sh.mstart, rel, &idx);
+        const uint32_t sp = wrap((hum ? s0h : s0m) + j, S), pp = sp * P + c;
         const U4 r = draw4(key, hum ? (uint32_t)kInfHTarget : (uint32_t)kInfMTarget, pp, t, idx);
         if (hum) {
             const uint32_t s = sp, k = sh.kh[j];
@@ -973,28 +1005,47 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
     }
     __syncwarp();
     // Phase B
-    if (any_intro) {
+    if (intro) {
         uint32_t avail = 0xFFu;  // bit s clear: no human of the community can take serotype s
         bool scanned = false;
-        for (uint32_t j = 0; j < S; ++j) {
-            const uint32_t s = (s0h + j) % S, ph = s * P + c;
-            uint32_t left = __shfl_sync(kFull, ne, s);
+        for (unsigned left_pos = intro; left_pos; left_pos &= left_pos - 1) {
+            const uint32_t j = __ffs(left_pos) - 1, s = wrap(s0h + j, S), ph = s * P + c;
+            uint32_t left = __shfl_sync(kFull, nej, j);
             uint32_t a0 = (avail >> s) & 1u ? 0u : d.maxIntro;
             // The first 32 attempts one per lane (most introductions find someone there), later ones
             // 128 at a time, four to a lane and to a Philox call.
             for (uint32_t per = 1; left > 0 && a0 < d.maxIntro; per = 4) {
                 uint32_t i[4], im[4], elig = 0;
+                int32_t bn = 0, dt = 0;  // times of the lane's one attempt
                 const uint32_t av = a0 + per * lane;  // a0 is a multiple of four
-                const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
+                if (per == 1) {
+                    i[1] = i[2] = i[3] = im[1] = im[2] = im[3] = 0;
+                    if (left_pos != intro) {
+                        const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
+                        ii = nbase + bounded(pick4(r, av & 3u), ns);
+                        if (av < d.maxIntro) {
+                            iim = __ldcg(&d.n_imm[ii]);
+                            ist = __ldcg(&d.n_status[ii]);
+                            ibn = __ldcg(&d.n_born[ii]);
+                            idt = __ldcg(&d.n_dtime[ii]);
+                        }
+                    }
+                    i[0] = ii, im[0] = iim, bn = ibn, dt = idt;
+                    if (av < d.maxIntro && ist == 0 && !((iim >> s) & 1u) &&
+                        __ldcg(&d.winh[ii]) > order_key(hiword, j, 1, av))
+                        elig = 1;
+                } else {
+                    const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
 #pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {
-                    i[q] = im[q] = 0;
-                    if (q < per && av + q < d.maxIntro) {
-                        i[q] = nbase + bounded(per == 1 ? r.v[av & 3] : r.v[q], ns);
-                        im[q] = __ldcg(&d.n_imm[i[q]]);
-                        if (__ldcg(&d.n_status[i[q]]) == 0 && !((im[q] >> s) & 1u) &&
-                            __ldcg(&d.winh[i[q]]) > order_key(hiword, j, 1, av + q))
-                            elig |= 1u << q;
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        i[q] = im[q] = 0;
+                        if (av + q < d.maxIntro) {
+                            i[q] = nbase + bounded(r.v[q], ns);
+                            im[q] = __ldcg(&d.n_imm[i[q]]);
+                            if (__ldcg(&d.n_status[i[q]]) == 0 && !((im[q] >> s) & 1u) &&
+                                __ldcg(&d.winh[i[q]]) > order_key(hiword, j, 1, av + q))
+                                elig |= 1u << q;
+                        }
                     }
                 }
                 // The eligible attempts in order; a human taken by one is lost to the later ones.
@@ -1008,8 +1059,11 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
                     const uint32_t taken = __shfl_sync(kFull, iq, first);
                     if (lane == first) {
                         d.winh[iq] = order_key(hiword, j, 1, av + q);
-                        infect_human(d, iq, s, draw4(key, kIntroExposed, ph, t, av + q), t, mq, __ldcg(&d.n_born[iq]),
-                                     __ldcg(&d.n_dtime[iq]));
+                        if (per != 1) {
+                            bn = __ldcg(&d.n_born[iq]);
+                            dt = __ldcg(&d.n_dtime[iq]);
+                        }
+                        infect_human(d, iq, s, draw4(key, kIntroExposed, ph, t, av + q), t, mq, bn, dt);
                     }
 #pragma unroll
                     for (q = 0; q < 4; ++q)
@@ -1038,8 +1092,9 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
     // Phase C
     for (uint32_t it = lane; it < items; it += 32) {
         if (it < H) {
-            const uint32_t j = item_position(sh.hstart, S, it), idx = it - sh.hstart[j];
-            const uint32_t s = (s0h + j) % S, ph = s * P + c, k = sh.kh[j];
+            uint32_t idx;
+            const uint32_t j = item_position(sh.hstart, it, &idx);
+            const uint32_t s = wrap(s0h + j, S), ph = s * P + c, k = sh.kh[j];
             uint32_t tg[4];
             if (it < kTargetCache) {
                 const uint4 v = sh.target[it];
@@ -1086,8 +1141,9 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
                 infect_human(d, tq, s, draw4(key, kInfHExposed, ph, t, e), t, iq, bq, dq);
             }
         } else {
-            const uint32_t rel = it - H, j = item_position(sh.mstart, S, rel), idx = rel - sh.mstart[j];
-            const uint32_t sm = (s0m + j) % S, pm = sm * P + c;
+            uint32_t idx;
+            const uint32_t rel = it - H, j = item_position(sh.mstart, rel, &idx);
+            const uint32_t sm = wrap(s0m + j, S), pm = sm * P + c;
             uint32_t st = 0;
             const uint32_t slot = it < kTargetCache
                                       ? sh.target[it].x
@@ -1098,8 +1154,8 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
                 wk = __ldcg(&d.winm[slot]);
                 life = __ldcg(reinterpret_cast<const int4*>(d.m_life + slot));
             }
+            const U4 r = draw4(key, kInfMExposed, pm, t, idx >> 2);  // while they are on their way
             if (slot != UINT_MAX && wk == order_key(hiword, j, 0, idx)) {
-                const U4 r = draw4(key, kInfMExposed, pm, t, idx >> 2);
                 d.m_stat[slot] = 1;
                 d.m_strain[slot] = (uint8_t)sm;
                 const int32_t age = (int32_t)t + 1 - life.y;
