@@ -1540,7 +1540,7 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
         }
         const uint64_t hb = cdiv(d.nvec, (uint64_t)32 * a.demogUnroll);  // warp items
         const uint64_t mb = cdiv(d.tiles, kQuad);
-        const uint64_t fb = cdiv((uint64_t)d.S * d.P, 32);  // force of infection: warps of 32 pairs
+        const uint64_t fb = foi_items(d.S, d.P);  // force of infection: warp items
         const uint64_t ib = d.P;  // the infection kernel takes communities, one warp each
         if (demog_off[i] + hb + mb >= (1ull << 31) || foi_off[i] + fb >= (1ull << 31) ||
             infect_off[i] + ib >= (1ull << 31))

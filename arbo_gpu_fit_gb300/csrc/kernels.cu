@@ -127,7 +127,7 @@ __device__ __forceinline__ int32_t death_age_lut(const Dev& d, float ple)
 // Per-warp shared staging of the demographic pass.
 struct QuadSmem {
     uint4 code[32];
-    uint32_t c0[kQuad], end[kQuad];  // community of each tile's first slot, and the slot where it ends
+    uint32_t c0[kQuad], end[kQuad], end2[kQuad];  // community of each tile's first slot; where it and the next end
     uint4 draw[32];  // rebirth draws of ranks 4s .. 4s+3 of tile u, by the lane 8u + s that made them
     union {
         uint8_t slot[kQuad][kTile];    // reborn slot offsets by rank
@@ -222,9 +222,11 @@ __device__ __forceinline__ void demog_humans(const Dev& d, const Key key, uint32
     __syncwarp();
 }
 
-// Community of slot i at or after community c, which ends at slot `end` (both move on).
-__device__ __forceinline__ void comm_forward(const Dev& d, uint32_t i, uint32_t& c, uint32_t& end)
+// Community of slot i at or after community c, which ends at slot `end`, the next one at `end2` (c and
+// end move on; few tiles reach into a third community).
+__device__ __forceinline__ void comm_forward(const Dev& d, uint32_t i, uint32_t& c, uint32_t& end, uint32_t end2)
 {
+    if (i >= end && end < end2) ++c, end = end2;
     while (i >= end) end = __ldg(&d.mloc[++c + 1]);
 }
 
@@ -244,14 +246,14 @@ __device__ __forceinline__ uint32_t mosq_comm(const Dev& d, uint32_t i)
 
 // A live slot whose event is due in the step that reaches time tn and is not the plain death of a
 // susceptible mosquito: its death, its latent-to-infectious transition, or neither yet. Returns its
-// new code. c and end: the community of its tile's first slot and where that ends.
-__device__ __noinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn, uint32_t c, uint32_t end)
+// new code. c, end, end2: the community of its tile's first slot and where that and the next one end.
+__device__ __noinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn, uint32_t c, uint32_t end, uint32_t end2)
 {
     const int4 r = *reinterpret_cast<const int4*>(d.m_life + i);  // ple, born, dtime
     uint32_t st = d.m_stat[i] & 3u;
     const int32_t ex = d.m_exposed[i];
     const uint32_t s = d.m_strain[i];
-    comm_forward(d, i, c, end);
+    comm_forward(d, i, c, end, end2);
     if (tn >= r.z) {
         if (st == 2) counter_dec(&d.infm[s * d.P + c], d.ctrl);
         return st ? (uint32_t)(kDead | kDeep) : (uint32_t)kDead;
@@ -280,7 +282,7 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
 // the first 32 births of each tile (left in the staging), which are keyed by rank and not by slot.
 struct QuadStart {
     int32_t led;
-    uint32_t c0, end;
+    uint32_t c0, end, end2;
     float target;
     uint32_t quota;
 };
@@ -293,10 +295,15 @@ __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uin
     QuadStart at;
     at.led = live ? d.ledger[b] : 0;
     at.c0 = live ? __ldg(&d.tcomm[b]) : 0u;
-    at.end = (at.c0 & kTileSpans) ? __ldg(&d.mloc[(at.c0 & ~kTileSpans) + 1]) : ~0u;
+    at.end = at.end2 = ~0u;
+    if (at.c0 & kTileSpans) {
+        at.end = __ldg(&d.mloc[(at.c0 & ~kTileSpans) + 1]);
+        at.end2 = __ldg(&d.mloc[(at.c0 & ~kTileSpans) + 2]);
+    }
     if ((lane & 7u) == 0) {
         sm.c0[u] = at.c0 & ~kTileSpans;
         sm.end[u] = at.end;
+        sm.end2[u] = at.end2;
     }
     at.target = __ldg(&d.etab[t + 1]);
     at.quota = pick4(draw4(key, kMosquitoTile, q, t), u);
@@ -358,7 +365,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
         __syncwarp();
         for (uint32_t j = lane; j < total; j += 32) {
             const uint32_t o = sm.deep[j];
-            reinterpret_cast<uint8_t*>(sm.code)[o] = (uint8_t)mosq_deep(d, q * kQuad * kTile + o, tn, sm.c0[o / kTile], sm.end[o / kTile]);
+            reinterpret_cast<uint8_t*>(sm.code)[o] = (uint8_t)mosq_deep(d, q * kQuad * kTile + o, tn, sm.c0[o / kTile], sm.end[o / kTile], sm.end2[o / kTile]);
         }
         __syncwarp();
         const uint4 B = sm.code[lane];
@@ -425,7 +432,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
         uint32_t c = c0 & ~kTileSpans, end = at.end;
         for (uint32_t m = born ^ died16; m; m &= m - 1) {
             const uint32_t k = __ffs(m) - 1;
-            comm_forward(d, b * kTile + 16 * seg + k, c, end);
+            comm_forward(d, b * kTile + 16 * seg + k, c, end, at.end2);
             atomicAdd(&d.mcnt[c], ((born >> k) & 1u) ? 1u : ~0u);
         }
     } else if (seg == 0 && nb != died_tot) {
@@ -641,114 +648,128 @@ __device__ __forceinline__ void split_events(const Dev& d, uint32_t* trans, floa
     *nlong = lng;
 }
 
-// Series row + force of infection, by one warp for 32 consecutive (serotype, community) pairs,
-// one per lane: each lane reads its pair's counters, adds them to the warp's series sums and
-// splits the pair's events both ways; then the 32 lanes spread the flattened events of the warp's
-// 128 (pair, kind) entries, four per Philox call. No block barrier: a warp is a chain of two
-// dependent round trips and its draws, so the more warps in flight the better. With kWait, the wait
-// for the previous kernel stands between the loads of static data and those of its results.
+// A count at or above 2^31 is a counter that went below zero (counter_dec records
+// ARBO_DEVERR_COUNTER when that happens): it is read as 0, so that an inconsistent state cannot turn
+// into an unbounded number of events.
+__device__ __forceinline__ uint32_t checked_count(uint32_t x, uint32_t* bad)
+{
+    *bad |= x & 0x80000000u;
+    return (x & 0x80000000u) ? 0u : x;
+}
+
+// Series row of the step and the reset of the incidence counters, by one warp for one serotype and 256
+// consecutive communities (item s * series_chunks + chunk): its loads are one round trip, then one
+// reduction and one atomic per series. Beside the force of infection and not in it: summed by the warps
+// that spread the events, the row stood between their counters and their events.
+__device__ __forceinline__ uint32_t series_chunks(uint32_t P) { return (P + 255) / 256; }
+
+template <bool kWait>
+__device__ __forceinline__ void foi_series(const Dev& d, uint32_t item, int collect_only, const StepAt& at)
+{
+    const uint32_t lane = threadIdx.x & 31u, S = d.S, P = d.P, chunks = series_chunks(P);
+    const uint32_t s = item / chunks, c0 = (item - s * chunks) * 256 + lane;
+    const uint32_t row = collect_only ? 0u : at.t + 1;
+    uint32_t humans = 0;
+    if (s == 0)
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+            if (c0 + 32 * k < P) humans += __ldg(&d.ncnt[c0 + 32 * k]);
+    if (kWait) griddep_wait();
+    uint32_t ih[8], im[8], ic[8], mc[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t c = c0 + 32 * k;
+        const bool ok = c < P;
+        ih[k] = ok ? d.infh[s * P + c] : 0u;
+        im[k] = ok ? d.infm[s * P + c] : 0u;
+        ic[k] = ok ? d.inc[s * P + c] : 0u;
+        mc[k] = ok && s == 0 ? d.mcnt[c] : 0u;
+    }
+    uint32_t si = 0, sm = 0, sc = 0, mosq = 0, bad = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t c = c0 + 32 * k;
+        if (ic[k]) d.inc[s * P + c] = 0u;
+        const uint32_t x = checked_count(ih[k], &bad);
+        si += x;
+        sm += checked_count(im[k], &bad);
+        sc += checked_count(ic[k], &bad);
+        mosq += checked_count(mc[k], &bad);
+        if (c == 0) d.s_one[row * S + s] = x;
+        if (d.recordSpatial && c < P) d.s_spatial[(size_t)row * S * P + s * P + c] = x;
+    }
+    if (bad) atomicOr(&d.ctrl->err, ARBO_DEVERR_COUNTER);
+    si = __reduce_add_sync(kFull, si);
+    sc = __reduce_add_sync(kFull, sc);
+    sm = __reduce_add_sync(kFull, sm);
+    if (lane == 0 && si) atomicAdd(&d.s_ninf[row * S + s], si);
+    if (lane == 1 && sc) atomicAdd(&d.s_ninc[row * S + s], sc);
+    if (lane == 2 && sm) atomicAdd(&d.s_minf[row * S + s], sm);
+    if (s == 0) {
+        humans = __reduce_add_sync(kFull, humans);
+        mosq = __reduce_add_sync(kFull, mosq);
+        if (lane == 3 && humans) atomicAdd(&d.s_ncount[row], humans);
+        if (lane == 4 && mosq) atomicAdd(&d.s_mcount[row], mosq);
+    }
+}
+
+// Force of infection, by one warp for kFoiPairs consecutive (serotype, community) pairs: lane l splits
+// the events of pair l mod 16 in one direction (below 16 human to mosquito, else mosquito to human);
+// then the 32 lanes spread the flattened events of the warp's 64 (lane, kind) entries, four per Philox
+// call. No block barrier: a warp is a chain of two dependent round trips and its draws, so the more warps
+// in flight the better. With kWait, the wait for the previous kernel stands between the loads of static
+// data and those of its results.
+constexpr uint32_t kFoiPairs = 16;
+
 struct __align__(16) FoiWarpSmem {
-    uint32_t to[32][8];                      // CSR row of each lane's source community (degree <= 8)
-    uint32_t cnt[32][4];                     // events of (lane, kind): 0 HM local, 1 HM long, 2 MH local, 3 MH long
-    uint32_t kofs[32][4];                    // first group of four of (lane, kind) in the warp's space
-    uint32_t base[33];                       // first group of each lane; base[32] = groups in the warp
-    uint32_t loc[32], deg[32];
-    uint32_t sum[3 * ARBO_MAX_STRAINS + 2];  // series sums: infected, incidence, infectious mosquitoes; humans, mosquitoes
+    uint32_t to[kFoiPairs][8];  // CSR row of each pair's source community (degree <= 8)
+    uint32_t base[33];          // first group of four events of each lane; base[32]: groups in the warp
+    uint32_t local[32], far[32];  // a lane's events to neighbours and to any community
+    uint32_t loc[kFoiPairs], deg[kFoiPairs], row[kFoiPairs];  // CSR row, its length, first counter of the serotype
+    uint32_t pad[3];
 };
 
 template <bool kWait>
-__device__ __forceinline__ void foi_warp(const Dev& d, uint32_t p0, int collect_only, const StepAt& at, FoiWarpSmem& sh)
+__device__ __forceinline__ void foi_events(const Dev& d, uint32_t p0, const StepAt& at, FoiWarpSmem& sh)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t t = at.t;
-    const Key key = at.key;
-    const uint32_t row = collect_only ? 0u : t + 1;
-    const uint32_t SP = d.S * d.P, S = d.S, P = d.P;
-    const uint32_t p = p0 + lane;
-    const bool valid = p < SP;
-    if (lane < 3 * ARBO_MAX_STRAINS + 2) sh.sum[lane] = 0;
-    uint32_t nk[4] = {0, 0, 0, 0};
-    uint32_t s = 0, c = 0, ncc = 0, loc = 0, deg = 0;
-    U4 rh, rm;
+    const uint32_t lane = threadIdx.x & 31u, SP = d.S * d.P, P = d.P;
+    const uint32_t slot = lane & (kFoiPairs - 1), p = p0 + slot;
+    const bool hm = lane < kFoiPairs, valid = p < SP;
+    uint32_t ncc = 0, loc = 0, deg = 0, s = 0, c = 0;
+    U4 r;
     if (valid) {
-        // Loads of static data and the keyed draws run before the wait on the demographic kernel
-        // (programmatic dependent launch); the counters it writes are read after.
         s = p / P;
         c = p - s * P;
         ncc = __ldg(&d.ncnt[c]);
         loc = __ldg(&d.csr_loc[c]);
         deg = __ldg(&d.csr_loc[c + 1]) - loc;
-        if (!collect_only && deg <= 8)
-            for (uint32_t q = 0; q < deg; ++q) sh.to[lane][q] = __ldg(&d.csr_to[loc + q]);
-        if (!collect_only) {
-            rh = draw4(key, kFoiHM, p, t);
-            rm = draw4(key, kFoiMH, p, t);
+        if (deg <= 8)  // the two lanes of a pair fetch every second neighbour
+            for (uint32_t q = hm ? 0u : 1u; q < deg; q += 2) sh.to[slot][q] = __ldg(&d.csr_to[loc + q]);
+        if (hm) {
+            sh.loc[slot] = loc;
+            sh.deg[slot] = deg;
+            sh.row[slot] = s * P;
         }
+        r = draw4(at.key, hm ? kFoiHM : kFoiMH, p, at.t);
     }
     if (kWait) griddep_wait();
-    __syncwarp();  // the sums are zeroed
+    uint32_t nlocal = 0, nfar = 0;
     if (valid) {
-        uint32_t ih = d.infh[p], im = d.infm[p], ic = d.inc[p];
-        uint32_t mcc = d.mcnt[c];
-        if (ic) d.inc[p] = 0u;
-        // A count at or above 2^31 is a counter that went below zero (counter_dec records
-        // ARBO_DEVERR_COUNTER when that happens): it is read as 0, so that an inconsistent state
-        // cannot turn into an unbounded number of events.
-        if ((ih | im | ic | mcc) & 0x80000000u) {
-            atomicOr(&d.ctrl->err, ARBO_DEVERR_COUNTER);
-            ih = (ih & 0x80000000u) ? 0u : ih;
-            im = (im & 0x80000000u) ? 0u : im;
-            ic = (ic & 0x80000000u) ? 0u : ic;
-            mcc = (mcc & 0x80000000u) ? 0u : mcc;
-        }
-        if (ih) atomicAdd(&sh.sum[s], ih);
-        if (ic) atomicAdd(&sh.sum[ARBO_MAX_STRAINS + s], ic);
-        if (im) atomicAdd(&sh.sum[2 * ARBO_MAX_STRAINS + s], im);
-        if (c == 0) d.s_one[row * S + s] = ih;
-        if (s == 0) {
-            atomicAdd(&sh.sum[3 * ARBO_MAX_STRAINS], ncc);
-            atomicAdd(&sh.sum[3 * ARBO_MAX_STRAINS + 1], mcc);
-        }
-        if (d.recordSpatial) d.s_spatial[(size_t)row * SP + p] = ih;
-        if (!collect_only && (ih | im)) {
-            if (ih > 0) {  // human -> mosquito (cpp/nepidemic.cu:28-142)
-                const float ratio = __fdiv_rn((float)mcc, (float)ncc);
-                float x = __fmul_rn(ratio, d.biting);
-                x = __fmul_rn(x, d.nmSuccess);
-                x = __fmul_rn(x, (float)ih);
-                split_events(d, d.transm, x, rh, p, deg, &nk[0], &nk[1]);
-            }
-            if (im > 0) {  // mosquito -> human (cpp/mepidemic.cu:28-138)
-                float x = __fmul_rn(d.biting, d.mnSuccess);
-                x = __fmul_rn(x, (float)im);
-                split_events(d, d.transh, x, rm, p, deg, &nk[2], &nk[3]);
-            }
+        uint32_t bad = 0;
+        const uint32_t inf = checked_count(hm ? d.infh[p] : d.infm[p], &bad);
+        const uint32_t mcc = checked_count(hm ? d.mcnt[c] : 0u, &bad);
+        if (bad) atomicOr(&d.ctrl->err, ARBO_DEVERR_COUNTER);
+        if (inf) {
+            // Human to mosquito (cpp/nepidemic.cu:28-142), mosquito to human (cpp/mepidemic.cu:28-138).
+            float x = hm ? __fmul_rn(__fmul_rn(__fdiv_rn((float)mcc, (float)ncc), d.biting), d.nmSuccess)
+                         : __fmul_rn(d.biting, d.mnSuccess);
+            x = __fmul_rn(x, (float)inf);
+            split_events(d, hm ? d.transm : d.transh, x, r, p, deg, &nlocal, &nfar);
         }
     }
-    __syncwarp();
-    if (lane < 3 * S) {
-        const uint32_t kind = lane / S, ss = lane - kind * S;
-        const uint32_t v = sh.sum[kind * ARBO_MAX_STRAINS + ss];
-        uint32_t* dst = kind == 0 ? d.s_ninf : kind == 1 ? d.s_ninc : d.s_minf;
-        if (v) atomicAdd(&dst[row * S + ss], v);
-    } else if (lane == 3 * S) {
-        if (sh.sum[3 * ARBO_MAX_STRAINS]) atomicAdd(&d.s_ncount[row], sh.sum[3 * ARBO_MAX_STRAINS]);
-        if (sh.sum[3 * ARBO_MAX_STRAINS + 1]) atomicAdd(&d.s_mcount[row], sh.sum[3 * ARBO_MAX_STRAINS + 1]);
-    }
-    if (collect_only) {
-        __syncwarp();  // the sums are read before the warp's next pairs zero them
-        return;
-    }
-    // Groups of four events: per lane over its four kinds, then an exclusive scan over the lanes.
-    uint32_t own = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        sh.cnt[lane][k] = nk[k];
-        sh.kofs[lane][k] = own;
-        own += (nk[k] + 3) >> 2;
-    }
-    sh.loc[lane] = loc;
-    sh.deg[lane] = deg;
+    const uint32_t own = ((nlocal + 3) >> 2) + ((nfar + 3) >> 2);
+    sh.local[lane] = nlocal;
+    sh.far[lane] = nfar;
     uint32_t v = own;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -756,46 +777,57 @@ __device__ __forceinline__ void foi_warp(const Dev& d, uint32_t p0, int collect_
         if (lane >= (uint32_t)off) v += y;
     }
     sh.base[lane] = v - own;
-    if (lane == 31) sh.base[32] = v;
     __syncwarp();
-    const uint32_t G = sh.base[32];
+    const uint32_t G = __shfl_sync(kFull, v, 31);
     for (uint32_t gi = lane; gi < G; gi += 32) {
-        uint32_t lo = 0, hi = 31;  // last lane whose first group is <= gi
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (sh.base[mid] <= gi) lo = mid; else hi = mid - 1;
-        }
-        const uint32_t owner = lo, rel = gi - sh.base[owner];
-        const uint32_t kind = rel >= sh.kofs[owner][3] ? 3u : rel >= sh.kofs[owner][2] ? 2u : rel >= sh.kofs[owner][1] ? 1u : 0u;
-        const uint32_t r4 = rel - sh.kofs[owner][kind];
-        const uint32_t po = p0 + owner, so = po / P;
-        const uint32_t n = sh.cnt[owner][kind];
-        const uint32_t stream = kind == 0 ? kFoiHMLocal : kind == 1 ? kFoiHMLong : kind == 2 ? kFoiMHLocal : kFoiMHLong;
-        uint32_t* trans = kind < 2 ? d.transm : d.transh;
-        const U4 r = draw4(key, stream, po, t, r4);
-        const uint32_t lo_ = sh.loc[owner], dg = sh.deg[owner];
+        uint32_t o = 0;  // last lane whose first group is <= gi
 #pragma unroll
-        for (int qq = 0; qq < 4; ++qq) {
-            if (4 * r4 + qq >= n) break;
-            const uint32_t nb = (kind & 1u) ? 0u : bounded(r.v[qq], dg);
-            const uint32_t dest = (kind & 1u) ? bounded(r.v[qq], P) : (dg <= 8 ? sh.to[owner][nb] : __ldg(&d.csr_to[lo_ + nb]));
-            atomicAdd(&trans[so * P + dest], 1u);
+        for (uint32_t half = 16; half; half >>= 1)
+            if (sh.base[o + half] <= gi) o += half;
+        const uint32_t rel = gi - sh.base[o], nl = sh.local[o], gl = (nl + 3) >> 2;
+        const bool far = rel >= gl, human = o < kFoiPairs;
+        const uint32_t r4 = far ? rel - gl : rel, n = far ? sh.far[o] : nl, q = o & (kFoiPairs - 1);
+        const uint32_t stream = human ? (far ? kFoiHMLong : kFoiHMLocal) : (far ? kFoiMHLong : kFoiMHLocal);
+        uint32_t* trans = (human ? d.transm : d.transh) + sh.row[q];
+        const U4 x = draw4(at.key, stream, p0 + q, at.t, r4);
+        const uint32_t dg = sh.deg[q];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (4 * r4 + e >= n) break;
+            uint32_t dest;
+            if (far) dest = bounded(x.v[e], P);
+            else {
+                const uint32_t nb = bounded(x.v[e], dg);
+                dest = dg <= 8 ? sh.to[q][nb] : __ldg(&d.csr_to[sh.loc[q] + nb]);
+            }
+            atomicAdd(&trans[dest], 1u);
         }
     }
     __syncwarp();  // the tables are reused for the warp's next pairs
 }
 
-// Warp w of block b takes pairs 32 * (b * W + w), then every gridDim.x * W warps further
-// (W = blockDim.x / 32; W per-warp tables in dynamic shared memory).
+// Items of the pass of one simulation: the event items first, then those of the series row.
+__device__ __forceinline__ uint32_t foi_event_items(const Dev& d) { return (d.S * d.P + kFoiPairs - 1) / kFoiPairs; }
+
+template <bool kWait>
+__device__ __forceinline__ void foi_item(const Dev& d, uint32_t item, int collect_only, const StepAt& at, FoiWarpSmem& sh)
+{
+    const uint32_t ev = foi_event_items(d);
+    if (item >= ev) foi_series<kWait>(d, item - ev, collect_only, at);
+    else if (!collect_only) foi_events<kWait>(d, kFoiPairs * item, at, sh);
+}
+
+// Warp w of block b takes item b * W + w, then every gridDim.x * W further (W = blockDim.x / 32; W
+// per-warp tables in dynamic shared memory).
 __global__ void __launch_bounds__(512) k_foi(Dev d, int collect_only, uint32_t koff)
 {
     extern __shared__ __align__(16) unsigned char foi_dyn[];
     const uint32_t warp = threadIdx.x >> 5, W = blockDim.x >> 5;
     FoiWarpSmem& sh = reinterpret_cast<FoiWarpSmem*>(foi_dyn)[warp];
-    const uint32_t SP = d.S * d.P;
+    const uint32_t items = foi_event_items(d) + d.S * series_chunks(d.P);
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t g = blockIdx.x * W + warp; 32 * g < SP; g += gridDim.x * W) foi_warp<true>(d, 32 * g, collect_only, at, sh);
+    for (uint32_t g = blockIdx.x * W + warp; g < items; g += gridDim.x * W) foi_item<true>(d, g, collect_only, at, sh);
 }
 
 // ------------------------------------------------------------------ infection draws
@@ -1269,8 +1301,7 @@ __global__ void __launch_bounds__(256, 5) k_demog_batch(BatchDev bd, uint32_t ko
     griddep_launch_dependents();
 }
 
-// Force-of-infection pass of a batch: one warp per 32 consecutive (serotype, community) pairs of
-// an instance (bd.foi_off counts these warp items), in runs of bd.foi_run items per warp. With
+// Force-of-infection pass of a batch: one warp per item of an instance (foi_item; bd.foi_off counts them), in runs of bd.foi_run items per warp. With
 // collect_only, only series row 0 of every instance (the end of its initialisation).
 __global__ void __launch_bounds__(512) k_foi_batch(BatchDev bd, int collect_only, uint32_t koff)
 {
@@ -1285,7 +1316,7 @@ __global__ void __launch_bounds__(512) k_foi_batch(BatchDev bd, int collect_only
     }
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
     batch_warp_items(bd, bd.foi_off, bd.foi_run, wdev,
-                     [&](const Dev& d, uint32_t item) { foi_warp<true>(d, 32 * item, collect_only, load_step(d.ctrl, koff), sh); });
+                     [&](const Dev& d, uint32_t item) { foi_item<true>(d, item, collect_only, load_step(d.ctrl, koff), sh); });
 }
 
 // Infection pass of a batch: one warp per community over the concatenated communities of all
@@ -1360,15 +1391,15 @@ __global__ void __launch_bounds__(kStepsWarps * 32, 2) k_steps(const Dev* devs, 
     // Neighbouring warps of the cluster's order sit on different SMs.
     const uint32_t rank = cluster_rank(), w = warp * C + rank, nw = kStepsWarps * C;
     StepAt at = load_step(d.ctrl, 0);
-    const uint32_t quads = (d.tiles + kQuad - 1) / kQuad, hw = (d.nvec + 31) / 32, SP = d.S * d.P;
+    const uint32_t quads = (d.tiles + kQuad - 1) / kQuad, hw = (d.nvec + 31) / 32;
+    const uint32_t foi = foi_event_items(d) + d.S * series_chunks(d.P);
     for (uint32_t k = 0; k < nsteps; ++k, ++at.t, ++at.epoch) {
         for (uint32_t it = w; it < quads + hw; it += nw) {
             if (it < quads) demog_mosquito_quad<false>(d, at.key, it, lane, at.t, scratch.demog);
             else demog_humans<1>(d, at.key, (it - quads) * 32 + lane, 32, at.t, scratch.demog);
         }
         cluster_barrier();
-        for (uint32_t g = w; 32 * g < SP; g += nw)
-            foi_warp<false>(d, 32 * g, 0, at, scratch.foi);
+        for (uint32_t g = w; g < foi; g += nw) foi_item<false>(d, g, 0, at, scratch.foi);
         cluster_barrier();
         for (uint32_t c = w; c < d.P; c += nw) infect_warp<false>(d, c, at, scratch.infect);
         cluster_barrier();
@@ -1761,11 +1792,11 @@ int launch_demog(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
                       hblocks, koff);
 }
 
+uint32_t foi_items(uint32_t S, uint32_t P) { return cdiv((uint64_t)S * P, kFoiPairs) + S * cdiv(P, 256); }
+
 int launch_foi(const Dev& d, const Launch& l, cudaStream_t st, int collect_only, uint32_t koff)
 {
-    const uint32_t SP = d.S * d.P;
-    const uint32_t pairs = 32 * (l.foiBlock / 32);  // one warp per 32 pairs
-    return launch_pdl(k_foi, dim3(cdiv(SP, pairs)), dim3(l.foiBlock), foi_smem(l.foiBlock, false), st,
+    return launch_pdl(k_foi, dim3(cdiv(foi_items(d.S, d.P), l.foiBlock / 32)), dim3(l.foiBlock), foi_smem(l.foiBlock, false), st,
                       l.pdl && !collect_only, d, collect_only, koff);
 }
 

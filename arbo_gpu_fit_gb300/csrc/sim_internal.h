@@ -178,7 +178,7 @@ struct BatchDev {
     const uint32_t* demog_off;   // [n+1] demographic warp items (32*U-lane human groups, mosquito quads)
     const uint32_t* demog_h;     // [n] human warp items of each instance (the rest are quads)
     uint32_t* work;              // demographic item counter (zero between steps)
-    const uint32_t* foi_off;     // [n+1] force-of-infection warp items (32 (serotype, community) pairs each)
+    const uint32_t* foi_off;     // [n+1] force-of-infection warp items (foi_items)
     const uint32_t* infect_off;  // [n+1] communities (the infection kernel runs one warp per community)
     const uint32_t* init_off[4];  // [n+1] each: 256-thread blocks of the batched initialisation kernels
                                   // (humans, mosquito tiles, seeds, counter and series reset)
@@ -202,6 +202,8 @@ int launch_init(const Dev& d, const Launch& l, void* stream);
 // Resident CTAs per SM of the demographic kernel for the given unroll and block size.
 int demog_blocks_per_sm(uint32_t unroll, uint32_t block);
 int demog_tma_blocks_per_sm(uint32_t unroll);
+// Warp items of the force-of-infection kernel for S serotypes and P communities.
+uint32_t foi_items(uint32_t S, uint32_t P);
 // One time step at offset koff from ctrl->t (the step counter advances only through
 // launch_advance); with events != null, records cudaEvent_t events[0..3] around the three kernels.
 int launch_step(const Dev& d, const Launch& l, void* stream, void* events, uint32_t koff);
