@@ -148,7 +148,7 @@ __device__ __forceinline__ uint32_t human_comm(const uint32_t* __restrict__ nloc
 
 // Human i in the step that reaches time tn, at or after its next event time: a transition of an
 // exposed or infectious human, a death with rebirth, or (after a census write) neither yet.
-__device__ __noinline__ void human_due(const Dev& d, const Key key, uint32_t i, int32_t tn)
+__device__ __forceinline__ void human_due(const Dev& d, const Key key, uint32_t i, int32_t tn)
 {
     uint32_t st = d.n_status[i];
     const int32_t dt = d.n_dtime[i], born = d.n_born[i], ex = d.n_exposed[i], rec = d.n_recovery[i];
@@ -247,7 +247,7 @@ __device__ __forceinline__ uint32_t mosq_comm(const Dev& d, uint32_t i)
 // A live slot whose event is due in the step that reaches time tn and is not the plain death of a
 // susceptible mosquito: its death, its latent-to-infectious transition, or neither yet. Returns its
 // new code. c, end, end2: the community of its tile's first slot and where that and the next one end.
-__device__ __noinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn, uint32_t c, uint32_t end, uint32_t end2)
+__device__ __forceinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn, uint32_t c, uint32_t end, uint32_t end2)
 {
     const int4 r = *reinterpret_cast<const int4*>(d.m_life + i);  // ple, born, dtime
     uint32_t st = d.m_stat[i] & 3u;
