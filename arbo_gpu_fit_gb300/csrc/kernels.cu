@@ -128,7 +128,7 @@ __device__ __forceinline__ int32_t death_age_lut(const Dev& d, float ple)
 struct QuadSmem {
     uint4 code[32];
     uint32_t c0[kQuad], end[kQuad], end2[kQuad];  // community of each tile's first slot; where it and the next end
-    uint4 draw[32];  // rebirth draws of ranks 4s .. 4s+3 of tile u, by the lane 8u + s that made them
+    uint4 draw[32];  // rebirth draws of ranks 4s .. 4s+3 of tile u, by the lane 8u + s that made them; 31: quota draws
     union {
         uint8_t slot[kQuad][kTile];    // reborn slot offsets by rank
         uint16_t deep[kQuad * kTile];  // slots with a deep event; a human pass's agents with an event due
@@ -278,13 +278,12 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
 }
 
 // What a quad needs that does not depend on its codes, made while they are on their way: the tile's
-// carried dead count and community, the expected mosquitoes and the tile's quota draw, and the draws of
-// the first 32 births of each tile (left in the staging), which are keyed by rank and not by slot.
+// carried dead count and community, the expected mosquitoes, and (left in the staging) the quad's quota
+// draws and the draws of the first 28 births of each tile, which are keyed by rank and not by slot.
 struct QuadStart {
     int32_t led;
     uint32_t c0, end, end2;
     float target;
-    uint32_t quota;
 };
 
 __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
@@ -306,8 +305,8 @@ __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uin
         sm.end2[u] = at.end2;
     }
     at.target = __ldg(&d.etab[t + 1]);
-    at.quota = pick4(draw4(key, kMosquitoTile, q, t), u);
-    const U4 r = draw4(key, kMosquitoRebirth, b, t, lane & 7u);
+    const bool quota = lane == 31;  // one Philox call a lane: the last one makes the quota draws
+    const U4 r = draw4(key, quota ? kMosquitoTile : kMosquitoRebirth, quota ? q : b, t, quota ? 0u : lane & 7u);
     sm.draw[lane] = make_uint4(r.v[0], r.v[1], r.v[2], r.v[3]);
     return at;
 }
@@ -398,6 +397,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
     const uint32_t dead_tot = tot & 0xFFFFu, died_tot = tot >> 16;
     // The quota, by every lane of the tile alike.
     uint32_t nb = 0;
+    __syncwarp();
     if (live) {
         const uint32_t start = b * kTile;
         const uint32_t bt = (d.M - start) < kTile ? (d.M - start) : kTile;
@@ -407,7 +407,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
         x = __fdiv_rn(x, (float)d.M);
         x = __fsub_rn(x, fbt);
         x = __fadd_rn(x, (float)L);
-        const int births = (int)resolve(x, at.quota);
+        const int births = (int)resolve(x, reinterpret_cast<const uint32_t*>(sm.draw)[31 * 4 + u]);
         if (seg == 0) d.ledger[b] = (int32_t)L - births;
         nb = births > 0 ? min((uint32_t)births, dead_tot) : 0u;
     }
@@ -448,7 +448,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
             const uint32_t v = (j >= n0 ? 1u : 0u) + (j >= n1 ? 1u : 0u) + (j >= n2 ? 1u : 0u);
             const uint32_t r = j - (v == 0 ? 0u : v == 1 ? n0 : v == 2 ? n1 : n2);
             uint32_t x;
-            if (r < 32) x = reinterpret_cast<const uint32_t*>(sm.draw)[32 * v + r];
+            if (r < 28) x = reinterpret_cast<const uint32_t*>(sm.draw)[32 * v + r];
             else x = pick4(draw4(key, kMosquitoRebirth, q * kQuad + v, t, r >> 2), r & 3u);
             const float ple = u01(x);
             const uint32_t o = v * kTile + sm.slot[v][r], i = q * kQuad * kTile + o;
