@@ -589,6 +589,8 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     s->l.demogBlocksPerSM = (uint32_t)demog_blocks_per_sm(arch.demogUnroll, arch.demogBlock);
     cudaGetLastError();
     s->l.pdl = 1;
+    if (const int e = share_carveout())
+        return fail_free(fail(ARBO_ERR_CUDA, std::string("step kernels: ") + cudaGetErrorString((cudaError_t)e)));
     s->l.demogPipeline = arch.demogPipeline ? 1u : 0u;
     s->l.demogTmaBlocksPerSM = (uint32_t)demog_tma_blocks_per_sm(arch.demogUnroll);
     cudaGetLastError();
@@ -914,7 +916,7 @@ static int census_ptr(arbo_sim* s, arbo_census_field f, void** ptr, size_t* coun
     return ARBO_OK;
 }
 
-// One field of the mosquitoes' life records (0 PLE, 1 birth time, 2 death time) between host and
+// One field of the mosquitoes' life records (0 birth time, 1 death time, 2 PLE) between host and
 // device, through a device array of M values.
 static int life_field(arbo_sim* s, int field, void* host, bool store, void* stream)
 {
@@ -952,8 +954,8 @@ static int census_derived(arbo_sim* s, arbo_census_field f, int32_t* out, size_t
         if ((e = copy_out(s, born.data(), d.n_born, count * 4, stream))) return e;
         if ((e = copy_out(s, dtime.data(), d.n_dtime, count * 4, stream))) return e;
     } else {
-        if ((e = life_field(s, 1, born.data(), false, stream))) return e;
-        if ((e = life_field(s, 2, dtime.data(), false, stream))) return e;
+        if ((e = life_field(s, 0, born.data(), false, stream))) return e;
+        if ((e = life_field(s, 1, dtime.data(), false, stream))) return e;
     }
     if (f == ARBO_CENSUS_M_AGE) {
         state.resize(count);
@@ -982,7 +984,7 @@ int arbo_sim_get_census(arbo_sim* s, arbo_census_field f, void* host, size_t byt
     if (e) return e;
     if (bytes != count * elem) return fail(ARBO_ERR_INVALID, "census size mismatch: expected " + std::to_string(count * elem));
     if (packed == 3) return census_derived(s, f, (int32_t*)host, count, stream);
-    if (packed == 4) return life_field(s, 0, host, false, stream);
+    if (packed == 4) return life_field(s, 2, host, false, stream);
     e = copy_out(s, host, ptr, bytes, stream);
     if (e || !packed) return e;
     uint8_t* h = (uint8_t*)host;
@@ -1071,7 +1073,7 @@ int arbo_sim_set_census(arbo_sim* s, arbo_census_field f, const void* host, size
         if (f == ARBO_CENSUS_M_EXPOSED) return refresh_mosquito_code(s, nullptr, stream);
         return ARBO_OK;
     }
-    if (packed == 4) return life_field(s, 0, const_cast<void*>(host), true, stream);
+    if (packed == 4) return life_field(s, 2, const_cast<void*>(host), true, stream);
     if (packed == 1) return refresh_mosquito_code(s, (const uint8_t*)host, stream);
     std::vector<uint8_t> cur(count);
     const uint8_t* h = (const uint8_t*)host;
@@ -1407,6 +1409,7 @@ struct arbo_batch {
     uint32_t direct = 0;  // steps launched kernel by kernel since the launch shapes changed
     bool phase_shapes = false;  // the caller chose launch shapes of the per-phase kernels
     uint32_t cluster = 0;       // CTAs per simulation of k_steps (0: the per-phase kernels)
+    uint32_t cluster_per_sm = 1;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> step_ev;
     void* flush = nullptr;
@@ -1488,11 +1491,11 @@ bool chooses_shapes(const arbo_arch_param& a)
 // 41, 128 of them 51 and 65, 200 of them 100 and 91, 304 of them 120 and 130; 32 of 2.1e5 agents 37 and
 // 50; 64 of 4e4 to 4e5 agents 92 and 67. The line falls where one simulation is much larger than the
 // others (its cluster works alone) or there are more than fit at once.
-uint32_t batch_cluster(const arbo_batch* b)
+uint32_t batch_cluster(const arbo_batch* b, uint32_t* per_sm)
 {
     if (b->phase_shapes) return 0;
     const uint32_t n = (uint32_t)b->sims.size();
-    const uint32_t C = steps_cluster(n);
+    const uint32_t C = steps_cluster(n, per_sm);
     if (!C) return 0;
     double total = 0.0, most = 0.0;
     for (const arbo_sim* s : b->sims) {
@@ -1500,7 +1503,7 @@ uint32_t batch_cluster(const arbo_batch* b)
         total += units;
         most = std::max(most, units);
     }
-    const double per = n * C <= b->l.numSM ? 0.45 : 0.85;
+    const double per = *per_sm == 1 ? 0.45 : 0.85;
     return 13.0 + std::max(per * most / C, 0.003 * total) < 35.0 + 0.003 * total ? C : 0;
 }
 
@@ -1609,7 +1612,7 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     b->bd = bd;
     b->l = l;
     b->arch = a;
-    b->cluster = batch_cluster(b);
+    b->cluster = batch_cluster(b, &b->cluster_per_sm);
     return ARBO_OK;
 }
 
@@ -1894,7 +1897,7 @@ int arbo_batch_step(arbo_batch* b, uint32_t nsteps, void* stream)
     }
     while (n > 0 && b->cluster) {
         const uint32_t chunk = std::min(n, kClusterSteps);
-        e = launch_steps(b->bd.devs, b->bd.n, b->cluster, chunk, st);
+        e = launch_steps(b->bd.devs, b->bd.n, b->cluster, b->cluster_per_sm, chunk, st);
         if (e) return fail(ARBO_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString((cudaError_t)e));
         n -= chunk;
         batch_advance_host(b, chunk);

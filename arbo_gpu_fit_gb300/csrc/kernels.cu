@@ -18,6 +18,7 @@
 // No tensor cores: the work is integer streaming and scattered events.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 
 #include "../../include/arbo.h"
@@ -249,21 +250,21 @@ __device__ __forceinline__ uint32_t mosq_comm(const Dev& d, uint32_t i)
 // new code. c, end, end2: the community of its tile's first slot and where that and the next one end.
 __device__ __forceinline__ uint32_t mosq_deep(const Dev& d, uint32_t i, int32_t tn, uint32_t c, uint32_t end, uint32_t end2)
 {
-    const int4 r = *reinterpret_cast<const int4*>(d.m_life + i);  // ple, born, dtime
+    const int2 r = *reinterpret_cast<const int2*>(d.m_life + i);  // born, dtime
     uint32_t st = d.m_stat[i] & 3u;
     const int32_t ex = d.m_exposed[i];
     const uint32_t s = d.m_strain[i];
     comm_forward(d, i, c, end, end2);
-    if (tn >= r.z) {
+    if (tn >= r.y) {
         if (st == 2) counter_dec(&d.infm[s * d.P + c], d.ctrl);
         return st ? (uint32_t)(kDead | kDeep) : (uint32_t)kDead;
     }
-    if (st == 1 && ex < tn - r.y) {
+    if (st == 1 && ex < tn - r.x) {
         st = 2;
         d.m_stat[i] = 2;
         atomicAdd(&d.infm[s * d.P + c], 1u);
     }
-    return mosq_code(mosq_next(st, r.z, r.y, ex), tn, st != 0);
+    return mosq_code(mosq_next(st, r.y, r.x, ex), tn, st != 0);
 }
 
 // Bit 7 of each byte of x (the other bits zero) gathered into a 4-bit mask (byte k -> bit k).
@@ -453,7 +454,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
             const float ple = u01(x);
             const uint32_t o = v * kTile + sm.slot[v][r], i = q * kQuad * kTile + o;
             const int32_t dt = death_time(tn, death_age_lut(d, ple));
-            *reinterpret_cast<int4*>(d.m_life + i) = make_int4(__float_as_int(ple), tn, dt, 0);
+            *reinterpret_cast<int4*>(d.m_life + i) = make_int4(tn, dt, __float_as_int(ple), 0);
             if (codes[o] & kDeep) d.m_stat[i] = 0;
             codes[o] = mosq_code(dt, tn, false);
         }
@@ -589,35 +590,26 @@ __global__ void __launch_bounds__(128, 4) k_demog_tma(Dev d, uint32_t koff)
     griddep_launch_dependents();
 }
 
-// Block b of the demographic pass of one simulation: blocks below hblocks run human groups, the others
-// run one mosquito quad per warp.
+// Demographic pass of one simulation, one warp item per warp: the mosquito quads first, then the rows of
+// 32 * U human groups. With `spread`, neighbouring items go to different blocks, so that every block has
+// its share of the long items (quads) and of the short ones; else blocks take consecutive items and the
+// human blocks, which are short but end in latency chains, come last and fill the SMs that the last
+// mosquito blocks leave idle.
 template <int U>
-__device__ __forceinline__ void demog_block(const Dev& d, uint32_t b, uint32_t hblocks, uint32_t koff, QuadSmem* wsm)
+__global__ void __launch_bounds__(256, 6) k_demog(Dev d, uint32_t spread, uint32_t koff)
 {
+    __shared__ QuadSmem wsm[8];
     const uint32_t t = d.ctrl->t + koff;
     const Key key = load_key(d.ctrl);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    if (b < hblocks) {
+    const uint32_t quads = (d.tiles + kQuad - 1) / kQuad, rows = (d.nvec + 32 * U - 1) / (32 * U);
+    const uint32_t it = spread ? warp * gridDim.x + blockIdx.x : blockIdx.x * (blockDim.x >> 5) + warp;
+    if (it < quads) {
+        demog_mosquito_quad<true>(d, key, it, lane, t, wsm[warp]);
+    } else if (it - quads < rows) {
         griddep_wait();
-        demog_humans<U>(d, key, b * blockDim.x * U + threadIdx.x, blockDim.x, t, wsm[warp]);
-    } else {
-        const uint32_t wpb = blockDim.x >> 5;
-        const uint32_t q = (b - hblocks) * wpb + warp;
-        if (q * kQuad < d.tiles) demog_mosquito_quad<true>(d, key, q, lane, t, wsm[warp]);
+        demog_humans<U>(d, key, (it - quads) * 32 * U + lane, 32, t, wsm[warp]);
     }
-}
-
-// The mosquito quads' blocks come first in the grid and the human groups' blocks last: the human
-// blocks are short but end in latency chains (the slow paths of humans with an event due), and in
-// the last wave they fill the SMs that the mosquito blocks leave idle (2.4 waves of mosquito blocks
-// on the large workload). Same results either way; 34.6-34.8 against 36.4-37.5 us mid-epidemic.
-template <int U>
-__global__ void __launch_bounds__(256, 6) k_demog(Dev d, uint32_t hblocks, uint32_t koff)
-{
-    __shared__ QuadSmem wsm[8];
-    const uint32_t mblocks = gridDim.x - hblocks;
-    const uint32_t b = blockIdx.x < mblocks ? blockIdx.x + hblocks : blockIdx.x - mblocks;
-    demog_block<U>(d, b, hblocks, koff, wsm);
     griddep_launch_dependents();
 }
 
@@ -849,16 +841,29 @@ __device__ __forceinline__ void infect_human(const Dev& d, uint32_t i, uint32_t 
     d.n_next[i] = human_next(1, dtime, born, ex);
 }
 
+// The same for mosquito slot i.
+__device__ __forceinline__ void infect_mosquito(const Dev& d, uint32_t i, uint32_t s, uint32_t r, uint32_t t, int32_t born,
+                                                int32_t dtime)
+{
+    d.m_stat[i] = 1;
+    d.m_strain[i] = (uint8_t)s;
+    const int32_t now = (int32_t)t + 1;
+    const int32_t ex = (int32_t)resolve(__fadd_rn((float)(now - born), d.mExposed), r);
+    d.m_exposed[i] = ex;
+    d.m_code[i] = mosq_code(mosq_next(1, dtime, born, ex), now, true);
+}
+
 // Target of mosquito event e: the first alive slot of its attempt sequence (dead slots are
 // retried, cpp/mepidemic.cu:206-235). Returns UINT_MAX when the attempts run out. The four
 // candidates of one Philox call are loaded together (one memory round trip) and the first alive
 // one in attempt order is taken; its status is left in *state (a live slot without kDeep is susceptible). `first` is the draw of the
-// first four attempts (the caller computes it together with other lanes' draws).
+// first four attempts (the caller computes it together with other lanes' draws); a0 (a multiple of
+// four): the first attempt.
 __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key, uint32_t pidx, uint32_t e,
                                                     uint32_t base, uint32_t size, uint32_t t, uint32_t* state,
-                                                    const U4& first)
+                                                    const U4& first, uint32_t a0 = 0)
 {
-    for (uint32_t a = 0; a < d.maxTarget; a += 4) {
+    for (uint32_t a = a0; a < d.maxTarget; a += 4) {
         const U4 r = a == 0 ? first : draw4(key, kInfMTarget, pidx, t, e, a >> 2);
         uint32_t slot[4], st[4];
 #pragma unroll
@@ -878,10 +883,15 @@ __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key
 // Per-warp tables of the infection pass: one community and its events of every serotype
 // flattened into one index space.
 constexpr uint32_t kIntroScan = 1024;   // humans of a community up to which failed introductions look at all of them
+constexpr uint32_t kFewItems = 32;
 constexpr uint32_t kTargetCache = 128;  // items whose targets Phase A keeps for Phase C
 
 struct InfectWarpSmem {
-    uint4 target[kTargetCache];         // per item: four human targets, or a mosquito slot in .x
+    union {
+        uint4 target[kTargetCache];     // per item: four human targets, or a mosquito slot in .x
+        uint2 bid[128];                 // of up to 32 items: eligible events, {target (mosquito slots with
+                                        // bit 31), low word of the order key}
+    };
     // First item of each serotype position and events by position, humans (groups of four) and
     // mosquitoes; positions past the last serotype start at UINT_MAX.
     uint4 hstart[2], mstart[2];
@@ -911,6 +921,12 @@ __device__ __forceinline__ uint32_t wrap(uint32_t x, uint32_t n) { return x >= n
 // Infection draws of community c, by one warp. Lanes 0..S-1 read the community's event counts
 // and draw its introduction counts, lanes 8 and 9 the first serotypes; the events (groups of
 // four human events, single mosquito events) then form one index space walked by the 32 lanes:
+// Up to 32 items (kFew), which is most communities in most steps, the warp resolves among its lanes: every
+// lane loads all that its event may need in one round trip, the eligible events are listed in shared
+// memory, and an event holds its target if no listed one with a smaller serial order has the same. The
+// two round trips that the bids in memory cost are gone: infection pass of 5e4 agents 5.1 -> 3.6 us, of
+// 7e6 9.1 -> 6.6. It takes 126 registers, so clusters that share SMs (64 registers) go without it.
+// More items go through the targets' winner keys in memory, three phases:
 //   A: every event whose target is eligible at the start of the pass bids its serial order
 //      (serotype position j, event index) for the target with atomicMin; the targets of the first
 //      kTargetCache items are kept in shared memory for phase C;
@@ -922,7 +938,7 @@ __device__ __forceinline__ uint32_t wrap(uint32_t x, uint32_t n) { return x >= n
 // other warp reads or writes them during the pass and warp barriers order the phases. One warp
 // per community with no block barrier: the pass is a chain of dependent round trips per
 // community, so the more communities in flight per SM the better.
-template <bool kWait>
+template <bool kWait, bool kFew>
 __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -1005,6 +1021,199 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
         idt = __ldcg(&d.n_dtime[ii]);
     }
 
+    // External introductions, position by position: open_to(i, j, a) says whether no event before attempt a
+    // of position j holds human i, took(i, a, j) notes that the attempt has taken i.
+    auto introductions = [&](auto open_to, auto took) {
+        uint32_t avail = 0xFFu;  // bit s clear: no human of the community can take serotype s
+        bool scanned = false;
+        for (unsigned left_pos = intro; left_pos; left_pos &= left_pos - 1) {
+            const uint32_t j = __ffs(left_pos) - 1, s = wrap(s0h + j, S), ph = s * P + c;
+            uint32_t left = __shfl_sync(kFull, nej, j);
+            uint32_t a0 = (avail >> s) & 1u ? 0u : d.maxIntro;
+            // The first 32 attempts one per lane (most introductions find someone there), later ones
+            // 128 at a time, four to a lane and to a Philox call.
+            for (uint32_t per = 1; left > 0 && a0 < d.maxIntro; per = 4) {
+                uint32_t i[4], im[4], elig = 0;
+                int32_t bn = 0, dt = 0;  // times of the lane's one attempt
+                const uint32_t av = a0 + per * lane;  // a0 is a multiple of four
+                if (per == 1) {
+                    i[1] = i[2] = i[3] = im[1] = im[2] = im[3] = 0;
+                    if (left_pos != intro) {
+                        const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
+                        ii = nbase + bounded(pick4(r, av & 3u), ns);
+                        if (av < d.maxIntro) {
+                            iim = __ldcg(&d.n_imm[ii]);
+                            ist = __ldcg(&d.n_status[ii]);
+                            ibn = __ldcg(&d.n_born[ii]);
+                            idt = __ldcg(&d.n_dtime[ii]);
+                        }
+                    }
+                    i[0] = ii, im[0] = iim, bn = ibn, dt = idt;
+                    if (av < d.maxIntro && ist == 0 && !((iim >> s) & 1u) &&
+                        open_to(ii, j, av))
+                        elig = 1;
+                } else {
+                    const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        i[q] = im[q] = 0;
+                        if (av + q < d.maxIntro) {
+                            i[q] = nbase + bounded(r.v[q], ns);
+                            im[q] = __ldcg(&d.n_imm[i[q]]);
+                            if (__ldcg(&d.n_status[i[q]]) == 0 && !((im[q] >> s) & 1u) &&
+                                open_to(i[q], j, av + q))
+                                elig |= 1u << q;
+                        }
+                    }
+                }
+                // The eligible attempts in order; a human taken by one is lost to the later ones.
+                while (left > 0) {
+                    const unsigned bal = __ballot_sync(kFull, elig != 0);
+                    if (!bal) break;
+                    const uint32_t first = __ffs(bal) - 1;
+                    uint32_t q = elig ? __ffs(elig) - 1 : 0;
+                    const uint32_t iq = q == 0 ? i[0] : q == 1 ? i[1] : q == 2 ? i[2] : i[3];
+                    const uint32_t mq = q == 0 ? im[0] : q == 1 ? im[1] : q == 2 ? im[2] : im[3];
+                    const uint32_t taken = __shfl_sync(kFull, iq, first);
+                    took(taken, __shfl_sync(kFull, av + q, first), j);
+                    if (lane == first) {
+                        if (per != 1) {
+                            bn = __ldcg(&d.n_born[iq]);
+                            dt = __ldcg(&d.n_dtime[iq]);
+                        }
+                        infect_human(d, iq, s, draw4(key, kIntroExposed, ph, t, av + q), t, mq, bn, dt);
+                    }
+#pragma unroll
+                    for (q = 0; q < 4; ++q)
+                        if (i[q] == taken) elig &= ~(1u << q);
+                    left -= 1;
+                }
+                __syncwarp();
+                a0 += 32 * per;
+                if (left > 0 && !scanned && ns <= kIntroScan) {
+                    // Is there anyone left to infect? In a small population the attempts would else run
+                    // to their limit (1,000) in every community that is immune, 32 a round trip: once a small
+                    // population was immune its step took 42 us (2,000 humans) and 27 us (10,000), now 18
+                    // and 19; 512 instances of 1e4 humans 300 -> 255 us.
+                    scanned = true;
+                    uint32_t open = 0;
+                    for (uint32_t h = lane; h < ns; h += 32)
+                        if (__ldcg(&d.n_status[nbase + h]) == 0) open |= ~(uint32_t)__ldcg(&d.n_imm[nbase + h]);
+                    avail = __reduce_or_sync(kFull, open & 0xFFu);
+                }
+                if (!((avail >> s) & 1u)) break;
+            }
+            if (left > 0 && lane == 0) atomicAdd(&d.ctrl->diag[1], 1u);
+        }
+    };
+    if (kFew && items <= kFewItems) {
+        // One item per lane.
+        const bool act = lane < items, hum = lane < H;
+        uint32_t idx = 0, sp = 0, pp = 0, j = 0, elig = 0, k = 0;
+        uint32_t tg[4] = {0, 0, 0, 0}, im[4] = {0, 0, 0, 0};
+        int32_t bn[4] = {0, 0, 0, 0}, dt[4] = {0, 0, 0, 0};
+        U4 rx;  // exposed-age draw of the lane's first human event, or of its mosquito event
+        if (act) {
+            j = item_position(hum ? sh.hstart : sh.mstart, hum ? lane : lane - H, &idx);
+            sp = wrap((hum ? s0h : s0m) + j, S);
+            pp = sp * P + c;
+            k = hum ? min(sh.kh[j] - 4 * idx, 4u) : min(d.maxTarget, 4u);  // targets or attempts of the lane
+            const U4 r = draw4(key, hum ? (uint32_t)kInfHTarget : (uint32_t)kInfMTarget, pp, t, idx);
+            // Both kinds of event load alike, so that they wait together: a human's status, immunity, birth
+            // and death time, a mosquito slot's code, status, birth and death time.
+            const uint8_t *pa = hum ? d.n_status : d.m_code, *pb = hum ? d.n_imm : d.m_stat;
+            const int32_t *pc = hum ? d.n_born : &d.m_life->born, *pd = hum ? d.n_dtime : &d.m_life->dtime;
+            const uint32_t step = hum ? 1u : sizeof(Life) / 4;
+            uint32_t st[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                tg[q] = (hum ? nbase : mbase) + bounded(r.v[q], hum ? ns : ms);
+                st[q] = kDead;
+                if (q < k) {
+                    st[q] = pa[tg[q]];
+                    im[q] = pb[tg[q]];
+                    bn[q] = pc[(size_t)tg[q] * step];
+                    dt[q] = pd[(size_t)tg[q] * step];
+                }
+            }
+            rx = draw4(key, hum ? (uint32_t)kInfHExposed : (uint32_t)kInfMExposed, pp, t, hum ? 4 * idx : idx >> 2);
+            if (hum) {
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q)
+                    if (st[q] == 0 && !((im[q] >> sp) & 1u)) elig |= 1u << q;
+            } else {
+                uint32_t slot = UINT_MAX, state = 0;
+                int32_t born = 0, dies = 0;
+#pragma unroll
+                for (int q = 3; q >= 0; --q)
+                    if (!(st[q] & kDead)) {
+                        slot = tg[q];
+                        state = im[q] & 3u;
+                        born = bn[q];
+                        dies = dt[q];
+                    }
+                if (slot == UINT_MAX) {
+                    slot = mosquito_target(d, key, pp, idx, mbase, ms, t, &state, r, 4);
+                    if (slot == UINT_MAX) atomicAdd(&d.ctrl->diag[0], 1u);
+                    else {
+                        born = d.m_life[slot].born;
+                        dies = d.m_life[slot].dtime;
+                    }
+                }
+                bn[0] = born;
+                dt[0] = dies;
+                tg[0] = slot | 0x80000000u;
+                if (slot != UINT_MAX && state == 0) elig = 1;
+            }
+        }
+        // The eligible events, and of them the first in serial order on each target.
+        uint32_t nb = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            const unsigned bal = __ballot_sync(kFull, (elig >> q) & 1u);
+            if ((elig >> q) & 1u)
+                sh.bid[nb + __popc(bal & ((1u << lane) - 1u))] =
+                    make_uint2(tg[q], (uint32_t)order_key(0, j, 0, hum ? 4 * idx + q : idx));
+            nb += __popc(bal);
+        }
+        __syncwarp();
+        uint32_t won = elig;
+        if (nb > 1)
+            for (uint32_t b = 0; b < nb; ++b) {
+                const uint2 x = sh.bid[b];
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q)
+                    if (x.x == tg[q] && x.y < (uint32_t)order_key(0, j, 0, hum ? 4 * idx + q : idx)) won &= ~(1u << q);
+            }
+        if (intro)
+            introductions(
+                [&](uint32_t i, uint32_t jj, uint32_t a) {
+                    bool open = true;
+                    for (uint32_t b = 0; b < nb; ++b) open &= sh.bid[b].x != i || sh.bid[b].y > (uint32_t)order_key(0, jj, 1, a);
+                    return open;
+                },
+                [&](uint32_t i, uint32_t, uint32_t) {
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q)
+                        if (tg[q] == i) won &= ~(1u << q);
+                });
+        if (won && !hum) {
+            infect_mosquito(d, tg[0] & 0x7FFFFFFFu, sp, pick4(rx, idx & 3u), t, bn[0], dt[0]);
+        } else {
+            while (won) {
+                const uint32_t q = __ffs(won) - 1;
+                won &= won - 1;
+                const uint32_t tq = q == 0 ? tg[0] : q == 1 ? tg[1] : q == 2 ? tg[2] : tg[3];
+                const uint32_t iq = q == 0 ? im[0] : q == 1 ? im[1] : q == 2 ? im[2] : im[3];
+                const int32_t bq = q == 0 ? bn[0] : q == 1 ? bn[1] : q == 2 ? bn[2] : bn[3];
+                const int32_t dq = q == 0 ? dt[0] : q == 1 ? dt[1] : q == 2 ? dt[2] : dt[3];
+                if (q) rx = draw4(key, kInfHExposed, pp, t, 4 * idx + q);
+                infect_human(d, tq, sp, rx, t, iq, bq, dq);
+            }
+        }
+        __syncwarp();  // the warp's tables are reused for its next community
+        return;
+    }
     // Phase A. Human groups and mosquito events draw their targets in one pass (the first four
     // attempts of a mosquito event).
     for (uint32_t it = lane; it < items; it += 32) {
@@ -1038,87 +1247,10 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
     __syncwarp();
     // Phase B
     if (intro) {
-        uint32_t avail = 0xFFu;  // bit s clear: no human of the community can take serotype s
-        bool scanned = false;
-        for (unsigned left_pos = intro; left_pos; left_pos &= left_pos - 1) {
-            const uint32_t j = __ffs(left_pos) - 1, s = wrap(s0h + j, S), ph = s * P + c;
-            uint32_t left = __shfl_sync(kFull, nej, j);
-            uint32_t a0 = (avail >> s) & 1u ? 0u : d.maxIntro;
-            // The first 32 attempts one per lane (most introductions find someone there), later ones
-            // 128 at a time, four to a lane and to a Philox call.
-            for (uint32_t per = 1; left > 0 && a0 < d.maxIntro; per = 4) {
-                uint32_t i[4], im[4], elig = 0;
-                int32_t bn = 0, dt = 0;  // times of the lane's one attempt
-                const uint32_t av = a0 + per * lane;  // a0 is a multiple of four
-                if (per == 1) {
-                    i[1] = i[2] = i[3] = im[1] = im[2] = im[3] = 0;
-                    if (left_pos != intro) {
-                        const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
-                        ii = nbase + bounded(pick4(r, av & 3u), ns);
-                        if (av < d.maxIntro) {
-                            iim = __ldcg(&d.n_imm[ii]);
-                            ist = __ldcg(&d.n_status[ii]);
-                            ibn = __ldcg(&d.n_born[ii]);
-                            idt = __ldcg(&d.n_dtime[ii]);
-                        }
-                    }
-                    i[0] = ii, im[0] = iim, bn = ibn, dt = idt;
-                    if (av < d.maxIntro && ist == 0 && !((iim >> s) & 1u) &&
-                        __ldcg(&d.winh[ii]) > order_key(hiword, j, 1, av))
-                        elig = 1;
-                } else {
-                    const U4 r = draw4(key, kIntroTarget, ph, t, av >> 2);
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) {
-                        i[q] = im[q] = 0;
-                        if (av + q < d.maxIntro) {
-                            i[q] = nbase + bounded(r.v[q], ns);
-                            im[q] = __ldcg(&d.n_imm[i[q]]);
-                            if (__ldcg(&d.n_status[i[q]]) == 0 && !((im[q] >> s) & 1u) &&
-                                __ldcg(&d.winh[i[q]]) > order_key(hiword, j, 1, av + q))
-                                elig |= 1u << q;
-                        }
-                    }
-                }
-                // The eligible attempts in order; a human taken by one is lost to the later ones.
-                while (left > 0) {
-                    const unsigned bal = __ballot_sync(kFull, elig != 0);
-                    if (!bal) break;
-                    const uint32_t first = __ffs(bal) - 1;
-                    uint32_t q = elig ? __ffs(elig) - 1 : 0;
-                    const uint32_t iq = q == 0 ? i[0] : q == 1 ? i[1] : q == 2 ? i[2] : i[3];
-                    const uint32_t mq = q == 0 ? im[0] : q == 1 ? im[1] : q == 2 ? im[2] : im[3];
-                    const uint32_t taken = __shfl_sync(kFull, iq, first);
-                    if (lane == first) {
-                        d.winh[iq] = order_key(hiword, j, 1, av + q);
-                        if (per != 1) {
-                            bn = __ldcg(&d.n_born[iq]);
-                            dt = __ldcg(&d.n_dtime[iq]);
-                        }
-                        infect_human(d, iq, s, draw4(key, kIntroExposed, ph, t, av + q), t, mq, bn, dt);
-                    }
-#pragma unroll
-                    for (q = 0; q < 4; ++q)
-                        if (i[q] == taken) elig &= ~(1u << q);
-                    left -= 1;
-                }
-                __syncwarp();
-                a0 += 32 * per;
-                if (left > 0 && !scanned && ns <= kIntroScan) {
-                    // Is there anyone left to infect? In a small population the attempts would else run
-                    // to their limit (1,000) in every community that is immune, 32 a round trip: once a small
-                    // population was immune its step took 42 us (2,000 humans) and 27 us (10,000), now 18
-                    // and 19; 512 instances of 1e4 humans 300 -> 255 us.
-                    scanned = true;
-                    uint32_t open = 0;
-                    for (uint32_t h = lane; h < ns; h += 32)
-                        if (__ldcg(&d.n_status[nbase + h]) == 0) open |= ~(uint32_t)__ldcg(&d.n_imm[nbase + h]);
-                    avail = __reduce_or_sync(kFull, open & 0xFFu);
-                }
-                if (!((avail >> s) & 1u)) break;
-            }
-            if (left > 0 && lane == 0) atomicAdd(&d.ctrl->diag[1], 1u);
-        }
+        introductions([&](uint32_t i, uint32_t j, uint32_t a) { return __ldcg(&d.winh[i]) > order_key(hiword, j, 1, a); },
+                      [&](uint32_t i, uint32_t a, uint32_t j) {
+                          if (lane == 0) d.winh[i] = order_key(hiword, j, 1, a);
+                      });
         __syncwarp();
     }
     // Phase C
@@ -1181,20 +1313,14 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
                                       ? sh.target[it].x
                                       : mosquito_target(d, key, pm, idx, mbase, ms, t, &st, draw4(key, kInfMTarget, pm, t, idx));
             unsigned long long wk = 0;
-            int4 life = make_int4(0, 0, 0, 0);
-            if (slot != UINT_MAX) {  // winner key and life record in one round trip
+            int2 life = make_int2(0, 0);
+            if (slot != UINT_MAX) {  // winner key and times in one round trip
                 wk = __ldcg(&d.winm[slot]);
-                life = __ldcg(reinterpret_cast<const int4*>(d.m_life + slot));
+                life = __ldcg(reinterpret_cast<const int2*>(d.m_life + slot));
             }
             const U4 r = draw4(key, kInfMExposed, pm, t, idx >> 2);  // while they are on their way
-            if (slot != UINT_MAX && wk == order_key(hiword, j, 0, idx)) {
-                d.m_stat[slot] = 1;
-                d.m_strain[slot] = (uint8_t)sm;
-                const int32_t age = (int32_t)t + 1 - life.y;
-                const int32_t ex = (int32_t)resolve(__fadd_rn((float)age, d.mExposed), r.v[idx & 3]);
-                d.m_exposed[slot] = ex;
-                d.m_code[slot] = mosq_code(mosq_next(1, life.z, life.y, ex), (int32_t)t + 1, true);
-            }
+            if (slot != UINT_MAX && wk == order_key(hiword, j, 0, idx))
+                infect_mosquito(d, slot, sm, pick4(r, idx & 3u), t, life.x, life.y);
         }
     }
     __syncwarp();  // the warp's tables are reused for its next community
@@ -1208,7 +1334,7 @@ __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp<true>(d, c, at, sh);
+    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp<true, true>(d, c, at, sh);
 }
 
 // ------------------------------------------------------------------ batched steps
@@ -1329,7 +1455,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
     unsigned long long* wdev =
         reinterpret_cast<unsigned long long*>(infect_dyn + K * sizeof(InfectWarpSmem)) + warp * (sizeof(Dev) / 8);
     batch_warp_items(bd, bd.infect_off, bd.infect_run, wdev,
-                     [&](const Dev& d, uint32_t c) { infect_warp<true>(d, c, load_step(d.ctrl, koff), sh); });
+                     [&](const Dev& d, uint32_t c) { infect_warp<true, true>(d, c, load_step(d.ctrl, koff), sh); });
 }
 
 static_assert(16 * (sizeof(InfectWarpSmem) + sizeof(Dev)) <= 48 * 1024 && 16 * (sizeof(FoiWarpSmem) + sizeof(Dev)) <= 48 * 1024,
@@ -1376,7 +1502,8 @@ static_assert(kStepsSmem + sizeof(Dev) + 64 <= 48 * 1024, "shared memory of k_st
 // slowest simulation at each phase and hand out items through one counter, which with few items is all
 // latency: 32 simulations of 7e4 agents took 39 us a step, now 20, 8 of them 35 and 17. The bodies are
 // the per-phase kernels' own. Sixteen warps of 64 registers to a CTA, two CTAs to an SM.
-__global__ void __launch_bounds__(kStepsWarps * 32, 2) k_steps(const Dev* devs, uint32_t C, uint32_t nsteps)
+template <uint32_t B>
+__global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, uint32_t C, uint32_t nsteps)
 {
     extern __shared__ __align__(16) unsigned char steps_dyn[];
     __shared__ __align__(16) unsigned long long dev_copy[sizeof(Dev) / 8];
@@ -1401,7 +1528,7 @@ __global__ void __launch_bounds__(kStepsWarps * 32, 2) k_steps(const Dev* devs, 
         cluster_barrier();
         for (uint32_t g = w; g < foi; g += nw) foi_item<false>(d, g, 0, at, scratch.foi);
         cluster_barrier();
-        for (uint32_t c = w; c < d.P; c += nw) infect_warp<false>(d, c, at, scratch.infect);
+        for (uint32_t c = w; c < d.P; c += nw) infect_warp<false, B == 1>(d, c, at, scratch.infect);
         cluster_barrier();
     }
     if (rank == 0 && threadIdx.x == 0) {
@@ -1482,7 +1609,7 @@ __device__ __forceinline__ void init_mosquito_tile(const Dev& d, const Key& key,
         d.m_stat[i] = 0;
         d.m_strain[i] = 0;
         d.m_exposed[i] = 0;
-        Life life{0.0f, 0, INT_MIN, 0};  // padding, or never alive: age 0, death age 0
+        Life life{0, INT_MIN, 0.0f, 0};  // padding, or never alive: age 0, death age 0
         uint32_t code = kPad;
         if (i < d.M) {
             const U4 r = draw4(key, kInitMosquito, i, 0);
@@ -1781,15 +1908,20 @@ int launch_demog(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
         else k_demog_tma<1><<<grid, 128, 0, st>>>(d, koff);
         return (int)cudaGetLastError();
     }
-    const uint32_t hblocks = cdiv(d.nvec, (uint64_t)l.demogBlock * U);
-    const uint32_t quads = cdiv(d.tiles, kQuad);
-    const uint32_t mblocks = cdiv(quads, l.demogBlock / 32);
-    const dim3 grid(hblocks + mblocks), block(l.demogBlock);
+    const uint32_t items = cdiv(d.tiles, kQuad) + cdiv(d.nvec, (uint64_t)32 * U), sms = l.numSM ? l.numSM : 152u;
+    // With blocks of 8 warps and fewer than two of them per SM, the items are spread and the blocks made
+    // smaller, down to 4 warps, so that no SM gets two full blocks while others have none: step of 7e5
+    // agents 11.5 -> 10.8 us (and up to 13 when the early start placed the blocks badly), of 5e4 10.6 ->
+    // 10.4. From there on larger blocks are better (128 threads: 18.6 -> 21.4 us at 7e6 agents), and a
+    // grid of resident blocks striding over the items is not (20.5 us).
+    uint32_t warps = l.demogBlock / 32;
+    const bool spread = items <= 2 * warps * sms;
+    if (spread && warps == 8) warps = std::min(8u, std::max(4u, cdiv(items, 2 * sms)));
     // Within a run of steps the previous kernel is the last step's infection pass, which leaves the step
     // control, the dead counts and the tables alone, so the pass may begin before it ends. At a run's
     // first step (koff 0) it may be the kernel that advances the step control.
-    return launch_pdl(U == 4 ? k_demog<4> : U == 2 ? k_demog<2> : k_demog<1>, grid, block, 0, st, l.pdl && koff > 0, d,
-                      hblocks, koff);
+    return launch_pdl(U == 4 ? k_demog<4> : U == 2 ? k_demog<2> : k_demog<1>, dim3(cdiv(items, warps)), dim3(32 * warps), 0,
+                      st, l.pdl && koff > 0, d, spread ? 1u : 0u, koff);
 }
 
 uint32_t foi_items(uint32_t S, uint32_t P) { return cdiv((uint64_t)S * P, kFoiPairs) + S * cdiv(P, 256); }
@@ -1841,6 +1973,18 @@ int launch_advance(const Dev& d, uint32_t n, void* stream)
 {
     k_advance<<<1, 32, 0, (cudaStream_t)stream>>>(d, n);
     return (int)cudaGetLastError();
+}
+
+int share_carveout()
+{
+    const int pct = 44;  // 100 KB of 228: five blocks of the demographic kernel, and 128 KB of L1
+    const void* f[] = {(const void*)k_demog<1>, (const void*)k_demog<2>, (const void*)k_demog<4>, (const void*)k_foi,
+                       (const void*)k_infect};
+    for (const void* k : f) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return 0;
 }
 
 uint32_t launches_per_step() { return 3; }
@@ -1935,27 +2079,40 @@ static cudaLaunchConfig_t steps_config(uint32_t n, uint32_t C, cudaLaunchAttribu
     return cfg;
 }
 
-uint32_t steps_cluster(uint32_t n)
+typedef void (*StepsKernel)(const Dev*, uint32_t, uint32_t);
+
+// Largest cluster of which n fit the device at once with kernel k (0: none).
+static uint32_t largest_cluster(StepsKernel k, uint32_t n)
 {
     // Sixteen CTAs per cluster are more than the portable eight.
-    const bool wide = cudaFuncSetAttribute(k_steps, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    const bool wide = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     uint32_t found = 0;
     for (uint32_t C = wide ? 16 : 8; C >= 1 && !found; C /= 2) {
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = steps_config(1, C, &attr);
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, k_steps, &cfg) == cudaSuccess && fit > 0 && (uint32_t)fit >= n) found = C;
+        if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) == cudaSuccess && fit > 0 && (uint32_t)fit >= n) found = C;
     }
     (void)cudaGetLastError();
     return found;
 }
 
-int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t nsteps, void* stream)
+// CTAs that have an SM each keep 128 registers a thread; two to an SM have 64.
+static StepsKernel steps_kernel(uint32_t per_sm) { return per_sm == 1 ? k_steps<1> : k_steps<2>; }
+
+uint32_t steps_cluster(uint32_t n, uint32_t* per_sm)
+{
+    const uint32_t one = largest_cluster(k_steps<1>, n), two = largest_cluster(k_steps<2>, n);
+    *per_sm = one && one >= two ? 1u : 2u;
+    return one && one >= two ? one : two;
+}
+
+int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t per_sm, uint32_t nsteps, void* stream)
 {
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = steps_config(n, C, &attr);
     cfg.stream = (cudaStream_t)stream;
-    return (int)cudaLaunchKernelEx(&cfg, k_steps, devs, C, nsteps);
+    return (int)cudaLaunchKernelEx(&cfg, steps_kernel(per_sm), devs, C, nsteps);
 }
 
 int launch_advance_batch(const BatchDev& bd, uint32_t n, void* stream)

@@ -76,8 +76,9 @@ __host__ __device__ inline int32_t mosq_next(uint32_t st, int32_t dtime, int32_t
 
 // A mosquito slot's life: one 16-byte record, so that a birth writes one sector.
 struct __align__(16) Life {
+    int32_t born, dtime;
     float ple;
-    int32_t born, dtime, unused;
+    int32_t unused;
 };
 
 constexpr uint32_t kLutWide = 0x80000000u;    // mlut: several ages in the bucket, search the CDF
@@ -209,21 +210,24 @@ uint32_t foi_items(uint32_t S, uint32_t P);
 int launch_step(const Dev& d, const Launch& l, void* stream, void* events, uint32_t koff);
 // Adds n to the step counter and the winner epoch (one thread).
 int launch_advance(const Dev& d, uint32_t n, void* stream);
-// field 0, 1, 2: PLE, birth time, death time of every slot, between the life records and an array.
+// field 0, 1, 2: birth time, death time, PLE of every slot, between the life records and an array.
 int launch_life_field(const Dev& d, int field, void* array, bool store, void* stream);
 // Writes the census in the reference's types into the caller's buffers (arbo_sim_export_census).
 int launch_export(const Dev& d, const arbo_census_export& x, void* stream);
 uint32_t launches_per_step();
+// The same split of L1 and shared memory for the step kernels of one simulation: a kernel that wants
+// another split than the one still running on an SM cannot start there before that one has ended.
+int share_carveout();
 // Loads the single-instance step kernels for the launch shape of l on the current device (their
 // attributes are queried, which loads a lazily loaded function), so that later launches load no
 // code. Returns the cudaError_t as int.
 int preload_step_kernels(const Launch& l);
 
 // Many whole steps of the n simulations of descriptors devs in one launch, one cluster of C CTAs each
-// (C as steps_cluster(n) gives it: the largest of 16, 8, 4, 2, 1 with all n clusters resident at
-// once on the current device; 0 when there is none).
-int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t nsteps, void* stream);
-uint32_t steps_cluster(uint32_t n);
+// (C as steps_cluster gives it: the largest of 16, 8, 4, 2, 1 with all n clusters resident at once on
+// the current device, one or two CTAs per SM; 0 when there is none).
+int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t per_sm, uint32_t nsteps, void* stream);
+uint32_t steps_cluster(uint32_t n, uint32_t* per_sm);
 
 // Batched steps (see BatchDev); the block shapes come from l, the grids from bd.
 int launch_step_batch(const BatchDev& bd, const Launch& l, void* stream, void* events, uint32_t koff);
