@@ -43,20 +43,22 @@ constexpr uint32_t kDirectSteps = 256;
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// x to the power of a Weibull shape; pow(x, 1) is x, so exponential lives need no call.
+double power(double x, float shape) { return shape == 1.0f ? x : std::pow(x, (double)shape); }
+
 // Human bi-Weibull CDF at an integer age (cpp/ndemographic.cu:13-29), in double, rounded once.
 float human_cdf(const arbo_sim_param& p, uint32_t a)
 {
-    double x = std::pow((double)a * (double)p.nScaleInfantMortality, (double)p.nShapeInfantMortality);
+    double x = power((double)a * (double)p.nScaleInfantMortality, p.nShapeInfantMortality);
     if ((double)a >= (double)p.nLocWeibull)
-        x += std::pow(((double)a - (double)p.nLocWeibull) / (double)p.nScaleLifeExpectancy,
-                      (double)p.nShapeLifeExpectancy);
+        x += power(((double)a - (double)p.nLocWeibull) / (double)p.nScaleLifeExpectancy, p.nShapeLifeExpectancy);
     return (float)(1.0 - std::exp(-x));
 }
 
 // Mosquito Weibull CDF (cpp/mdemographic.cu:13-17).
 float mosquito_cdf(const arbo_sim_param& p, uint32_t a)
 {
-    double x = std::pow((double)a / (double)p.mScaleLifeExpectancy, (double)p.mShapeLifeExpectancy);
+    const double x = power((double)a / (double)p.mScaleLifeExpectancy, p.mShapeLifeExpectancy);
     return (float)(1.0 - std::exp(-x));
 }
 
@@ -141,6 +143,8 @@ struct arbo_sim {
     bool inited = false;
     void* base = nullptr;
     size_t bytes = 0;
+    void* zeroed = nullptr;  // the arrays that initialisation zeroes, one range of the allocation
+    size_t zeroed_bytes = 0;
     std::vector<uint32_t> nsize, msize, nloc, mloc;
     std::vector<float> etab;
     cudaStream_t cap = nullptr;
@@ -334,14 +338,17 @@ static const char* param_error(const arbo_sim_param& p, uint32_t N, uint32_t M)
     return nullptr;
 }
 
-// FNV-1a fingerprint of a table's bytes and length (the key of the intern table below).
+// FNV-1a fingerprint of the 4-byte words and the length of two tables (the key of the intern table below).
 static uint64_t table_fingerprint(const void* a, size_t na, const void* b, size_t nb)
 {
     uint64_t h = 1469598103934665603ull;
     auto mix = [&](const void* p, size_t n) {
-        const unsigned char* c = (const unsigned char*)p;
-        for (size_t i = 0; i < n; ++i) h = (h ^ c[i]) * 1099511628211ull;
-        for (int k = 0; k < 8; ++k) h = (h ^ ((n >> (8 * k)) & 0xFF)) * 1099511628211ull;
+        for (size_t i = 0; i + 4 <= n; i += 4) {
+            uint32_t w;
+            std::memcpy(&w, (const char*)p + i, 4);
+            h = (h ^ w) * 1099511628211ull;
+        }
+        h = (h ^ n) * 1099511628211ull;
     };
     mix(a, na);
     mix(b, nb);
@@ -502,31 +509,56 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     apply_rates(p, d);
     d.recordSpatial = p.recordSpatial ? 1u : 0u;
 
-    // One allocation, every array 256-byte aligned.
+    const std::vector<uint32_t> tcomm = block_communities(s->mloc, P, M, kTile);
+    const std::vector<uint32_t> hcomm = block_communities(s->nloc, P, N, kHumanBlock);
+    s->tab_h = intern_tables(cdfh, minvh);
+    s->tab_m = intern_tables(cdfm, minv);
+    Ctrl c{};
+    c.k0 = (uint32_t)seed;
+    c.k1 = (uint32_t)(seed >> 32);
+    c.instance = instance;
+
+    // One allocation, every array 256-byte aligned. First the arrays that are filled here, in one copy
+    // from a host image (eighteen copies took 0.15 ms); then those that initialisation zeroes, in one
+    // memset (arbo_sim_init); then the winner keys; then the census.
     const size_t Np = (size_t)d.nvec * 4, Mp = (size_t)d.tiles * kTile, SP = (size_t)S * P, R = (size_t)T + 1;
     struct Item {
         void** ptr;
         size_t bytes;
+        const void* src;  // host contents (the first group)
     };
-    std::vector<Item> items = {
-        {(void**)&d.n_born, Np * 4}, {(void**)&d.n_dtime, Np * 4}, {(void**)&d.n_next, Np * 4}, {(void**)&d.n_status, Np}, {(void**)&d.n_exposed, Np * 4},
+    const std::vector<Item> filled = {
+        {(void**)&d.nloc, (P + 1) * (size_t)4, s->nloc.data()}, {(void**)&d.mloc, (P + 1) * (size_t)4, s->mloc.data()},
+        {(void**)&d.nsize, P * (size_t)4, s->nsize.data()}, {(void**)&d.msize, P * (size_t)4, s->msize.data()},
+        {(void**)&d.ncnt, P * (size_t)4, s->nsize.data()}, {(void**)&d.tcomm, (size_t)d.tiles * 4, tcomm.data()},
+        {(void**)&d.csr_loc, (P + 1) * (size_t)4, csr->loc}, {(void**)&d.csr_to, (size_t)csr->nnz * 4, csr->to},
+        {(void**)&d.cdfh, cdfh.size() * 4, cdfh.data()}, {(void**)&d.cdfm, cdfm.size() * 4, cdfm.data()},
+        {(void**)&d.minv, minv.size() * 4, minv.data()}, {(void**)&d.mlut, mlut.size() * sizeof(uint2), mlut.data()},
+        {(void**)&d.minvh, minvh.size() * 4, minvh.data()}, {(void**)&d.hcomm, hcomm.size() * 4, hcomm.data()},
+        {(void**)&d.survh, survh.size() * 4, survh.data()}, {(void**)&d.survm, survm.size() * 4, survm.data()},
+        {(void**)&d.etab, R * 4, s->etab.data()}, {(void**)&d.ctrl, sizeof(Ctrl), &c},
+    };
+    const std::vector<Item> zeroed = {
+        {(void**)&d.infh, SP * 4}, {(void**)&d.infm, SP * 4}, {(void**)&d.inc, SP * 4}, {(void**)&d.transh, SP * 4},
+        {(void**)&d.transm, SP * 4}, {(void**)&d.s_ninc, R * S * 4}, {(void**)&d.s_ninf, R * S * 4},
+        {(void**)&d.s_one, R * S * 4}, {(void**)&d.s_minf, R * S * 4}, {(void**)&d.s_ncount, R * 4},
+        {(void**)&d.s_mcount, R * 4}, {(void**)&d.s_spatial, d.recordSpatial ? R * SP * 4 : 0},
+    };
+    const std::vector<Item> keys = {{(void**)&d.winh, Np * 8}, {(void**)&d.winm, Mp * 8}};
+    const std::vector<Item> census = {
+        {(void**)&d.mcnt, P * (size_t)4}, {(void**)&d.n_born, Np * 4}, {(void**)&d.n_dtime, Np * 4},
+        {(void**)&d.n_next, Np * 4}, {(void**)&d.n_status, Np}, {(void**)&d.n_exposed, Np * 4},
         {(void**)&d.n_recovery, Np * 4}, {(void**)&d.n_ple, Np * 4}, {(void**)&d.n_strain, Np}, {(void**)&d.n_imm, Np},
-        {(void**)&d.m_code, Mp}, {(void**)&d.m_stat, Mp}, {(void**)&d.m_life, Mp * sizeof(Life)}, {(void**)&d.m_exposed, Mp * 4},
-        {(void**)&d.m_strain, Mp}, {(void**)&d.ledger, (size_t)d.tiles * 4},
-        {(void**)&d.nloc, (P + 1) * 4}, {(void**)&d.mloc, (P + 1) * 4}, {(void**)&d.nsize, P * 4},
-        {(void**)&d.msize, P * 4}, {(void**)&d.tcomm, (size_t)d.tiles * 4}, {(void**)&d.csr_loc, (P + 1) * 4},
-        {(void**)&d.csr_to, std::max<size_t>(csr->nnz, 1) * 4}, {(void**)&d.infh, SP * 4}, {(void**)&d.infm, SP * 4},
-        {(void**)&d.inc, SP * 4}, {(void**)&d.ncnt, P * 4}, {(void**)&d.mcnt, P * 4}, {(void**)&d.transh, SP * 4},
-        {(void**)&d.transm, SP * 4}, {(void**)&d.cdfh, cdfh.size() * 4}, {(void**)&d.cdfm, cdfm.size() * 4}, {(void**)&d.minv, minv.size() * 4}, {(void**)&d.mlut, mlut.size() * sizeof(uint2)}, {(void**)&d.minvh, minvh.size() * 4},
-        {(void**)&d.hcomm, (size_t)cdiv(N, kHumanBlock) * 4},
-        {(void**)&d.survh, survh.size() * 4}, {(void**)&d.survm, survm.size() * 4}, {(void**)&d.etab, R * 4},
-        {(void**)&d.winh, Np * 8}, {(void**)&d.winm, Mp * 8}, {(void**)&d.s_ninc, R * S * 4},
-        {(void**)&d.s_ninf, R * S * 4}, {(void**)&d.s_one, R * S * 4}, {(void**)&d.s_ncount, R * 4},
-        {(void**)&d.s_mcount, R * 4}, {(void**)&d.s_minf, R * S * 4},
-        {(void**)&d.s_spatial, d.recordSpatial ? R * SP * 4 : 0}, {(void**)&d.ctrl, sizeof(Ctrl)},
+        {(void**)&d.m_code, Mp}, {(void**)&d.m_stat, Mp}, {(void**)&d.m_life, Mp * sizeof(Life)},
+        {(void**)&d.m_exposed, Mp * 4}, {(void**)&d.m_strain, Mp}, {(void**)&d.ledger, (size_t)d.tiles * 4},
     };
-    size_t total = 0;
-    for (auto& it : items) total += align256(it.bytes);
+    auto extent = [](const std::vector<Item>& v) {
+        size_t n = 0;
+        for (const Item& it : v) n += align256(it.bytes);
+        return n;
+    };
+    const size_t n_filled = extent(filled), n_zeroed = extent(zeroed), n_keys = extent(keys);
+    const size_t total = n_filled + n_zeroed + n_keys + extent(census);
     cudaError_t ce = cudaMalloc(&s->base, total);
     if (ce != cudaSuccess) {
         delete s;
@@ -535,50 +567,28 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     }
     s->bytes = total;
     size_t off = 0;
-    for (auto& it : items) {
-        *it.ptr = it.bytes ? (void*)((char*)s->base + off) : nullptr;
-        off += align256(it.bytes);
-    }
-
-    const std::vector<uint32_t> tcomm = block_communities(s->mloc, P, M, kTile);
+    for (const auto* group : {&filled, &zeroed, &keys, &census})
+        for (const Item& it : *group) {
+            *it.ptr = it.bytes ? (void*)((char*)s->base + off) : nullptr;
+            off += align256(it.bytes);
+        }
+    s->zeroed = (char*)s->base + n_filled;
+    s->zeroed_bytes = n_zeroed;
     auto fail_free = [&](int code) {
         arbo_sim_destroy(s);
         return code;
     };
-#define UP(dst, src, n)                                                                          \
-    do {                                                                                         \
-        cudaError_t e_ = cudaMemcpy((dst), (src), (n), cudaMemcpyHostToDevice);                  \
-        if (e_ != cudaSuccess) return fail_free(fail(ARBO_ERR_CUDA, cudaGetErrorString(e_)));    \
-        s->h2d += (n);                                                                           \
-    } while (0)
-    UP(d.nloc, s->nloc.data(), (P + 1) * 4);
-    UP(d.mloc, s->mloc.data(), (P + 1) * 4);
-    UP(d.nsize, s->nsize.data(), P * 4);
-    UP(d.msize, s->msize.data(), P * 4);
-    UP(d.ncnt, s->nsize.data(), P * 4);
-    UP(d.tcomm, tcomm.data(), (size_t)d.tiles * 4);
-    UP(d.csr_loc, csr->loc, (P + 1) * 4);
-    if (csr->nnz) UP(d.csr_to, csr->to, (size_t)csr->nnz * 4);
-    s->tab_h = intern_tables(cdfh, minvh);
-    s->tab_m = intern_tables(cdfm, minv);
-    UP(d.cdfh, cdfh.data(), cdfh.size() * 4);
-    UP(d.cdfm, cdfm.data(), cdfm.size() * 4);
-    UP(d.minv, minv.data(), minv.size() * 4);
-    UP(d.mlut, mlut.data(), mlut.size() * sizeof(uint2));
-    UP(d.minvh, minvh.data(), minvh.size() * 4);
-    const std::vector<uint32_t> hcomm = block_communities(s->nloc, P, N, kHumanBlock);
-    UP(d.hcomm, hcomm.data(), hcomm.size() * 4);
-    UP(d.survh, survh.data(), survh.size() * 4);
-    UP(d.survm, survm.data(), survm.size() * 4);
-    UP(d.etab, s->etab.data(), R * 4);
-    Ctrl c{};
-    c.k0 = (uint32_t)seed;
-    c.k1 = (uint32_t)(seed >> 32);
-    c.instance = instance;
-    UP(d.ctrl, &c, sizeof(Ctrl));
-#undef UP
-    if (cudaMemset(d.winh, 0xFF, Np * 8) != cudaSuccess || cudaMemset(d.winm, 0xFF, Mp * 8) != cudaSuccess ||
-        cudaMemset(d.transh, 0, SP * 4) != cudaSuccess || cudaMemset(d.transm, 0, SP * 4) != cudaSuccess)
+    std::vector<char> image(n_filled);
+    off = 0;
+    for (const Item& it : filled) {
+        if (it.bytes) std::memcpy(image.data() + off, it.src, it.bytes);
+        off += align256(it.bytes);
+        s->h2d += it.bytes;
+    }
+    ce = cudaMemcpy(s->base, image.data(), n_filled, cudaMemcpyHostToDevice);
+    if (ce != cudaSuccess) return fail_free(fail(ARBO_ERR_CUDA, cudaGetErrorString(ce)));
+    // Events (counters among the zeroed arrays) start at none, winner keys at the largest.
+    if (cudaMemset(s->zeroed, 0, n_zeroed) != cudaSuccess || cudaMemset(d.winh, 0xFF, n_keys) != cudaSuccess)
         return fail_free(fail(ARBO_ERR_CUDA, "cudaMemset at create"));
 
     s->l.demogBlock = arch.demogBlock;
@@ -706,19 +716,7 @@ int arbo_sim_init(arbo_sim* s, void* stream)
     CUDA_TRY(cudaSetDevice(s->device));
     cudaStream_t st = (cudaStream_t)stream;
     const Dev& d = s->d;
-    const size_t SP = (size_t)d.S * d.P, R = (size_t)d.T + 1;
-    CUDA_TRY(cudaMemsetAsync(d.infh, 0, SP * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.infm, 0, SP * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.inc, 0, SP * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.transh, 0, SP * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.transm, 0, SP * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.s_ninc, 0, R * d.S * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.s_ninf, 0, R * d.S * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.s_one, 0, R * d.S * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.s_minf, 0, R * d.S * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.s_ncount, 0, R * 4, st));
-    CUDA_TRY(cudaMemsetAsync(d.s_mcount, 0, R * 4, st));
-    if (d.s_spatial) CUDA_TRY(cudaMemsetAsync(d.s_spatial, 0, R * SP * 4, st));
+    CUDA_TRY(cudaMemsetAsync(s->zeroed, 0, s->zeroed_bytes, st));
     CUDA_TRY(cudaMemcpyAsync(d.mcnt, d.msize, (size_t)d.P * 4, cudaMemcpyDeviceToDevice, st));
     const int e = launch_init(d, s->l, st);
     if (e) return fail(ARBO_ERR_CUDA, std::string("init launch: ") + cudaGetErrorString((cudaError_t)e));
@@ -1337,7 +1335,7 @@ static __device__ __align__(256) unsigned long long g_noalloc_scratch[ARBO_NOALL
 // not surface in an unrelated later call.
 static void noalloc_prepare(arbo_sim* s)
 {
-    s->noalloc = nullptr;
+    if (s->noalloc) return;  // prepared by an earlier initialisation
     s->noalloc_err = 0;
     const size_t Np = (size_t)s->d.nvec * 4, Mp = (size_t)s->d.tiles * kTile;
     if (Np + Mp > ARBO_NOALLOC_MAX_AGENTS) return;
