@@ -146,6 +146,7 @@ struct arbo_sim {
     void* zeroed = nullptr;  // the arrays that initialisation zeroes, one range of the allocation
     size_t zeroed_bytes = 0;
     std::vector<uint32_t> nsize, msize, nloc, mloc;
+    uint64_t comm_most = 0;  // agents of the largest community
     std::vector<float> etab;
     cudaStream_t cap = nullptr;
     cudaGraphExec_t gmulti = nullptr;
@@ -591,6 +592,7 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     if (cudaMemset(s->zeroed, 0, n_zeroed) != cudaSuccess || cudaMemset(d.winh, 0xFF, n_keys) != cudaSuccess)
         return fail_free(fail(ARBO_ERR_CUDA, "cudaMemset at create"));
 
+    for (uint32_t c = 0; c < P; ++c) s->comm_most = std::max(s->comm_most, (uint64_t)s->nsize[c] + s->msize[c]);
     s->l.demogBlock = arch.demogBlock;
     s->l.demogUnroll = arch.demogUnroll;
     s->l.foiBlock = arch.foiBlock;
@@ -1467,6 +1469,14 @@ Dev batch_desc(const arbo_batch* b, size_t i)
     return d;
 }
 
+// Agents of the largest community from which a batch's infection pass, where the caller leaves the default
+// block, takes 256 threads and works off communities with many events by block (k_infect_batch<true>), in
+// runs of two communities. Smaller communities seldom have that many events, and the search for them costs
+// 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us, at runs of 4, 2 and 1: 352, 289 and
+// 278 in blocks of 256, 398, 370 and 350 in blocks of 512, 456, 378 and 280 in blocks of 64; with few
+// events 83, 85 and 92. One simulation alone keeps k_infect: with this its step took 1 to 3 % longer.
+constexpr uint64_t kHeavyCommunity = 16384;
+
 // Steps per launch of k_steps.
 constexpr uint32_t kClusterSteps = 128;
 
@@ -1516,13 +1526,19 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     l.demogBlock = a.demogBlock;
     l.demogUnroll = a.demogUnroll;
     l.foiBlock = a.foiBlock;
-    l.infectBlock = a.infectBlock;
+    arbo_arch_param dflt;
+    arbo_arch_param_query(&dflt, -1);
+    uint64_t most = 0;  // largest community of any instance
+    for (const arbo_sim* s : b->sims) most = std::max(most, s->comm_most);
+    const bool heavy = most >= kHeavyCommunity && a.infectBlock == dflt.infectBlock;
+    l.infectBlock = heavy ? 256 : a.infectBlock;
+    l.infectHeavy = heavy;
     l.numSM = a.totalSM ? a.totalSM : 152u;
     l.pdl = 1;
     std::vector<uint32_t> demog_off(n + 1, 0), demog_h(n, 0), foi_off(n + 1, 0), infect_off(n + 1, 0);
     std::vector<uint32_t> init_off[4];
     for (auto& v : init_off) v.assign(n + 1, 0);
-    const uint32_t K = a.infectBlock / 32;  // communities (warps) per infection CTA
+    const uint32_t K = l.infectBlock / 32;  // communities (warps) per infection CTA
     for (uint32_t i = 0; i < n; ++i) {
         const Dev& d = b->sims[i]->d;
         // Initialisation blocks of 256 threads (at least one per instance and kernel): humans,
@@ -1604,8 +1620,9 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     // Runs of consecutive communities per warp (fewer descriptor restagings), as long as every
     // resident warp still gets one.
     const uint32_t warps = l.numSM * occ[2] * K;
-    bd.infect_run = std::max(1u, std::min(kInfectRunMax, b->blocks[2] / std::max(warps, 1u)));
-    bd.grid_infect = std::max(1u, std::min(cdiv(cdiv(b->blocks[2], bd.infect_run), K), l.numSM * occ[2]));
+    const uint32_t run_max = heavy ? 2u : kInfectRunMax;
+    bd.infect_run = std::max(1u, std::min(run_max, b->blocks[2] / std::max(warps, 1u)));
+    bd.grid_infect = std::max(1u, std::min(cdiv(cdiv(b->blocks[2], bd.infect_run), heavy ? 1u : K), l.numSM * occ[2]));
     batch_drop_graphs(b);
     b->bd = bd;
     b->l = l;

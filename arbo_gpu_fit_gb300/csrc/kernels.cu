@@ -884,6 +884,11 @@ __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key
 // flattened into one index space.
 constexpr uint32_t kIntroScan = 1024;   // humans of a community up to which failed introductions look at all of them
 constexpr uint32_t kFewItems = 32;
+// Items past which a block of a batch works off a community together. Infection phase of 64 uneven
+// instances of a heavy epidemic (2.3e5 human infections a step) at 64, 128, 256 and 512: 369, 353, 340 and
+// 415 us, of 16 smaller ones 32, 29, 33 and 41.
+constexpr uint32_t kHeavyItems = 128;
+constexpr uint32_t kHeavyList = 64;     // such communities that a block can list
 constexpr uint32_t kTargetCache = 128;  // items whose targets Phase A keeps for Phase C
 
 struct InfectWarpSmem {
@@ -938,10 +943,29 @@ __device__ __forceinline__ uint32_t wrap(uint32_t x, uint32_t n) { return x >= n
 // other warp reads or writes them during the pass and warp barriers order the phases. One warp
 // per community with no block barrier: the pass is a chain of dependent round trips per
 // community, so the more communities in flight per SM the better.
-template <bool kWait, bool kFew>
-__device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh)
+//
+// By: one warp alone; one warp that leaves a community of more than kHeavyItems items untouched and lists it
+// (works it off itself when the list is full); or a whole block (every warp calls with the same community
+// and the same tables).
+// Communities that the warps of a block leave to the whole block: {instance, community}.
+struct HeavyList {
+    uint32_t n;
+    uint2 at[kHeavyList];
+};
+
+enum InfectBy : int { kByWarp = 0, kByWarpDefer = 1, kByBlock = 2 };
+
+template <bool kWait, bool kFew, int kBy>
+__device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh,
+                                            HeavyList* heavy = nullptr, uint32_t inst = 0)
 {
     const uint32_t lane = threadIdx.x & 31u;
+    const bool lead = kBy != kByBlock || threadIdx.x < 32;
+    const uint32_t gl = kBy == kByBlock ? threadIdx.x : lane, gt = kBy == kByBlock ? blockDim.x : 32u;
+    auto sync = [] {
+        if (kBy == kByBlock) __syncthreads();
+        else __syncwarp();
+    };
     const uint32_t t = at.t;
     const uint32_t hiword = ~at.epoch;
     const Key key = at.key;
@@ -964,10 +988,9 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
     const uint32_t mc = d.mcnt[c];
     uint32_t kh = lane < S ? d.transh[pl] : 0u;
     uint32_t km = lane < S ? d.transm[pl] : 0u;
+    const bool had_h = kh != 0, had_m = km != 0;
     uint32_t sv = 0, ne = 0;
     if (lane < S) {
-        if (kh) d.transh[pl] = 0;
-        if (km) d.transm[pl] = 0;
         if (ns == 0) kh = 0;
         else ne = (uint32_t)resolve(ext, rd.v[0]);
         if (mc == 0) km = 0;
@@ -996,22 +1019,33 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
             mi += x;
         }
     }
-    if (lane < 8) {
+    const uint32_t H = __shfl_sync(kFull, hi, 7), Mt = __shfl_sync(kFull, mi, 7);
+    const uint32_t items = H + Mt;
+    if (kBy == kByWarpDefer && items > kHeavyItems) {
+        uint32_t i = 0;
+        if (lane == 0) {
+            i = atomicAdd(&heavy->n, 1u);
+            if (i < kHeavyList) heavy->at[i] = make_uint2(inst, c);
+        }
+        if (__shfl_sync(kFull, i, 0) < kHeavyList) return;
+    }
+    if (kBy == kByBlock) __syncthreads();  // every warp has read the event counts
+    if (lead && had_h) d.transh[pl] = 0;
+    if (lead && had_m) d.transm[pl] = 0;
+    if (lead && lane < 8) {
         reinterpret_cast<uint32_t*>(sh.hstart)[lane] = lane < S ? hi - h0 : UINT_MAX;
         reinterpret_cast<uint32_t*>(sh.mstart)[lane] = lane < S ? mi - m0 : UINT_MAX;
         sh.kh[lane] = khj;
         sh.km[lane] = kmj;
     }
-    const uint32_t H = __shfl_sync(kFull, hi, 7), Mt = __shfl_sync(kFull, mi, 7);
     const unsigned intro = __ballot_sync(kFull, nej != 0);  // positions with introductions
-    __syncwarp();
-    const uint32_t items = H + Mt;
+    sync();
     if (items == 0 && !intro) return;
     // The first introduction's first 32 attempts load everything but the bids together with the events'
     // targets: nothing before them changes it.
     uint32_t ii = 0, iim = 0, ist = 1;
     int32_t ibn = 0, idt = 0;
-    if (intro && lane < d.maxIntro) {
+    if (lead && intro && lane < d.maxIntro) {
         const uint32_t ph = wrap(s0h + __ffs(intro) - 1, S) * P + c;
         const U4 r = draw4(key, kIntroTarget, ph, t, lane >> 2);
         ii = nbase + bounded(pick4(r, lane & 3u), ns);
@@ -1216,7 +1250,7 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
     }
     // Phase A. Human groups and mosquito events draw their targets in one pass (the first four
     // attempts of a mosquito event).
-    for (uint32_t it = lane; it < items; it += 32) {
+    for (uint32_t it = gl; it < items; it += gt) {
         const bool hum = it < H;
         const uint32_t rel = hum ? it : it - H;
         uint32_t idx;
@@ -1244,17 +1278,18 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
             else if (st == 0) atomicMin(&d.winm[slot], order_key(hiword, j, 0, idx));
         }
     }
-    __syncwarp();
+    sync();
     // Phase B
-    if (intro) {
+    if (intro && lead) {
         introductions([&](uint32_t i, uint32_t j, uint32_t a) { return __ldcg(&d.winh[i]) > order_key(hiword, j, 1, a); },
                       [&](uint32_t i, uint32_t a, uint32_t j) {
                           if (lane == 0) d.winh[i] = order_key(hiword, j, 1, a);
                       });
         __syncwarp();
     }
+    if (kBy == kByBlock && intro) __syncthreads();
     // Phase C
-    for (uint32_t it = lane; it < items; it += 32) {
+    for (uint32_t it = gl; it < items; it += gt) {
         if (it < H) {
             uint32_t idx;
             const uint32_t j = item_position(sh.hstart, it, &idx);
@@ -1323,18 +1358,18 @@ __device__ __forceinline__ void infect_warp(const Dev& d, uint32_t c, const Step
                 infect_mosquito(d, slot, sm, pick4(r, idx & 3u), t, life.x, life.y);
         }
     }
-    __syncwarp();  // the warp's tables are reused for its next community
+    sync();  // the tables are reused for the next community
 }
 
-// One warp per community: warp w of block b takes communities b*K + w, + gridDim.x*K, ...
-// (K = blockDim.x / 32; K per-warp tables in dynamic shared memory).
+// One warp per community: warp w of block b takes communities b*K + w (per-warp tables in dynamic shared
+// memory).
 __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
 {
     extern __shared__ __align__(16) unsigned char infect_dyn[];
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_warp<true, true>(d, c, at, sh);
+    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_unit<true, true, kByWarp>(d, c, at, sh);
 }
 
 // ------------------------------------------------------------------ batched steps
@@ -1353,8 +1388,9 @@ __device__ __forceinline__ uint32_t batch_instance(const uint32_t* __restrict__ 
 // Warp runs over the concatenated items of a batch's instances (off[i] = first item of instance
 // i): warps take runs of `run` consecutive items, strided over the grid, so that a warp restages
 // its instance descriptor (per-warp copy in shared memory, wdev) about once per run while every
-// instance is spread over many warps; fn(dev, item within the instance) runs each item.
-template <typename Fn>
+// instance is spread over many warps; fn(dev, item within the instance, instance) runs each item.
+// kAcross: consecutive runs go to different blocks.
+template <bool kAcross, typename Fn>
 __device__ __forceinline__ void batch_warp_items(const BatchDev& bd, const uint32_t* __restrict__ off, uint32_t run,
                                                  unsigned long long* wdev, Fn fn)
 {
@@ -1362,7 +1398,8 @@ __device__ __forceinline__ void batch_warp_items(const BatchDev& bd, const uint3
     const Dev& d = *reinterpret_cast<const Dev*>(wdev);
     const uint32_t total = __ldg(&off[bd.n]);
     const uint32_t runs = (total + run - 1) / run;
-    const uint32_t gw = blockIdx.x * W + (threadIdx.x >> 5), nw = gridDim.x * W;
+    const uint32_t w = threadIdx.x >> 5, gw = kAcross ? w * gridDim.x + blockIdx.x : blockIdx.x * W + w;
+    const uint32_t nw = gridDim.x * W;
     uint32_t inst = UINT_MAX, lo = 0, hi = 0;  // current instance and its item range
     for (uint32_t r = gw; r < runs; r += nw) {
         const uint32_t end = min(total, (r + 1) * run);
@@ -1376,7 +1413,7 @@ __device__ __forceinline__ void batch_warp_items(const BatchDev& bd, const uint3
                 for (uint32_t i = lane; i < sizeof(Dev) / 8; i += 32) wdev[i] = src[i];
                 __syncwarp();
             }
-            fn(d, it - lo);
+            fn(d, it - lo, inst);
         }
     }
 }
@@ -1441,21 +1478,48 @@ __global__ void __launch_bounds__(512) k_foi_batch(BatchDev bd, int collect_only
         *bd.work = 0u;
     }
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
-    batch_warp_items(bd, bd.foi_off, bd.foi_run, wdev,
-                     [&](const Dev& d, uint32_t item) { foi_item<true>(d, item, collect_only, load_step(d.ctrl, koff), sh); });
+    batch_warp_items<false>(bd, bd.foi_off, bd.foi_run, wdev, [&](const Dev& d, uint32_t item, uint32_t) {
+        foi_item<true>(d, item, collect_only, load_step(d.ctrl, koff), sh);
+    });
 }
 
 // Infection pass of a batch: one warp per community over the concatenated communities of all
-// instances (bd.infect_off counts communities), in runs of bd.infect_run communities per warp.
+// instances (bd.infect_off counts communities), in runs of bd.infect_run communities per warp. kHeavy: the
+// block then works off together those with more than kHeavyItems items, of which a warp alone takes 32 in
+// some 4 us, and neighbouring runs, mostly of one instance with many events or with few, go to different
+// blocks. 64 uneven instances (1.9e8 agents) in the steps of a heavy epidemic: phase 631 -> 202, 896 -> 270
+// and 775 -> 288 us; with few events 79 -> 85, and 24 such instances 38 -> 41.
+template <bool kHeavy>
 __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff)
 {
     extern __shared__ __align__(16) unsigned char infect_dyn[];
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
-    InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
-    unsigned long long* wdev =
-        reinterpret_cast<unsigned long long*>(infect_dyn + K * sizeof(InfectWarpSmem)) + warp * (sizeof(Dev) / 8);
-    batch_warp_items(bd, bd.infect_off, bd.infect_run, wdev,
-                     [&](const Dev& d, uint32_t c) { infect_warp<true, true>(d, c, load_step(d.ctrl, koff), sh); });
+    InfectWarpSmem* tables = reinterpret_cast<InfectWarpSmem*>(infect_dyn);
+    unsigned long long* descs = reinterpret_cast<unsigned long long*>(infect_dyn + K * sizeof(InfectWarpSmem));
+    unsigned long long* wdev = descs + warp * (sizeof(Dev) / 8);
+    if constexpr (!kHeavy) {
+        batch_warp_items<false>(bd, bd.infect_off, bd.infect_run, wdev, [&](const Dev& d, uint32_t c, uint32_t) {
+            infect_unit<true, true, kByWarp>(d, c, load_step(d.ctrl, koff), tables[warp]);
+        });
+    } else {
+        __shared__ HeavyList heavy;
+        if (threadIdx.x == 0) heavy.n = 0;
+        __syncthreads();
+        batch_warp_items<true>(bd, bd.infect_off, bd.infect_run, wdev, [&](const Dev& d, uint32_t c, uint32_t inst) {
+            const StepAt at = load_step(d.ctrl, koff);
+            infect_unit<true, true, kByWarpDefer>(d, c, at, tables[warp], &heavy, inst);
+        });
+        __syncthreads();
+        const uint32_t n = min(heavy.n, kHeavyList);
+        for (uint32_t i = 0; i < n; ++i) {
+            const uint2 h = heavy.at[i];
+            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(bd.devs + h.x);
+            for (uint32_t j = threadIdx.x; j < sizeof(Dev) / 8; j += blockDim.x) descs[j] = src[j];
+            __syncthreads();
+            const Dev& d = *reinterpret_cast<const Dev*>(descs);
+            infect_unit<true, false, kByBlock>(d, h.y, load_step(d.ctrl, koff), tables[0]);
+        }
+    }
 }
 
 static_assert(16 * (sizeof(InfectWarpSmem) + sizeof(Dev)) <= 48 * 1024 && 16 * (sizeof(FoiWarpSmem) + sizeof(Dev)) <= 48 * 1024,
@@ -1528,7 +1592,7 @@ __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, 
         cluster_barrier();
         for (uint32_t g = w; g < foi; g += nw) foi_item<false>(d, g, 0, at, scratch.foi);
         cluster_barrier();
-        for (uint32_t c = w; c < d.P; c += nw) infect_warp<false, B == 1>(d, c, at, scratch.infect);
+        for (uint32_t c = w; c < d.P; c += nw) infect_unit<false, B == 1, kByWarp>(d, c, at, scratch.infect);
         cluster_barrier();
     }
     if (rank == 0 && threadIdx.x == 0) {
@@ -2020,7 +2084,8 @@ int batch_blocks_per_sm(const Launch& l, uint32_t out[3])
         cudaSuccess)
         return (int)e;
     out[1] = n > 0 ? (uint32_t)n : 1u;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_infect_batch, (int)l.infectBlock,
+    const auto infect = l.infectHeavy ? k_infect_batch<true> : k_infect_batch<false>;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, infect, (int)l.infectBlock,
                                                             infect_smem(l.infectBlock, true))) != cudaSuccess)
         return (int)e;
     out[2] = n > 0 ? (uint32_t)n : 1u;
@@ -2043,8 +2108,8 @@ int launch_step_batch(const BatchDev& bd, const Launch& l, void* stream, void* e
                         0, koff)))
         return e;
     if (ev) cudaEventRecord(ev[2], st);
-    if ((e = launch_pdl(k_infect_batch, dim3(bd.grid_infect), dim3(l.infectBlock), infect_smem(l.infectBlock, true), st,
-                        l.pdl != 0, bd, koff)))
+    if ((e = launch_pdl(l.infectHeavy ? k_infect_batch<true> : k_infect_batch<false>, dim3(bd.grid_infect),
+                        dim3(l.infectBlock), infect_smem(l.infectBlock, true), st, l.pdl != 0, bd, koff)))
         return e;
     if (ev) cudaEventRecord(ev[3], st);
     return 0;

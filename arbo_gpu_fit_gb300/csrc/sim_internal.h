@@ -193,6 +193,7 @@ struct BatchDev {
 
 struct Launch {
     uint32_t demogBlock, demogUnroll, foiBlock, infectBlock, numSM, demogBlocksPerSM;
+    uint32_t infectHeavy;  // whole blocks work off communities with many events
     uint32_t pdl;  // 1: k_foi and k_infect use programmatic dependent launch
     uint32_t demogPipeline;       // 1: persistent TMA-staged demographic kernel
     uint32_t demogTmaBlocksPerSM;
