@@ -5,10 +5,13 @@
 // FP32 master weights and writes the BF16 copies. No reference counterpart: the reference has no
 // surrogate (include/arbo.h, section "surrogate").
 //
-// Products, all C = A * B^T with K-major BF16 operands (row-major A [M][K], B [N][K]):
-//   forward  Z_l  = H_{l-1} W_l^T          A = H_{l-1} [B][in],  B = W_l  [out][in]
-//   backward dH   = dZ_l W_l               A = dZ_l    [B][out], B = W_l^T [in][out]
-//   weights  dW_l = dZ_l^T H_{l-1}         A = dZ_l^T  [out][B], B = H_{l-1}^T [in][B]
+// Products, all C = A * B^T with K-major BF16 operands (row-major A [M][K], B [N][K]), C written
+// transposed (row-major [N][M]):
+//   forward  Z_l^T  = W_l H_{l-1}^T        A = W_l   [out][in],      B = H_{l-1} [rows][in]
+//   backward dH^T   = W_l^T dZ_l^T         A = W_l^T [in][out],      B = dZ_l    [rows][out]
+//   weights  dW_l^T = H_{l-1}^T dZ_l       A = H_{l-1}^T [in][rows], B = dZ_l^T  [out][rows]
+// A is at least two launches old in each, which lets the kernel fetch it before the launch that it
+// depends on has ended (k_gemm_tn).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -34,22 +37,23 @@ typedef __nv_bfloat16 bf16;
 
 enum Epi : int { kEpiHidden = 0, kEpiLinear = 1, kEpiBackward = 2, kEpiStore = 3, kEpiLoss = 4 };
 
-// One product C = A B^T and its epilogue.
+// One product C = A B^T, M a multiple of 16, and its epilogue, which writes C transposed. A, bias, zprev and
+// target were written before the launch that precedes this one began (they are read before it has ended).
 struct GemmArgs {
     const bf16* A;
     const bf16* B;
     uint32_t lda, ldb, M, N, K;
     int epi;
-    const float* bias;   // [N]
-    const float* zprev;  // [M][ldz] pre-activation whose derivative scales the product (backward)
+    const float* bias;   // [M]
+    const float* zprev;  // [N][ldz] pre-activation whose derivative scales the product (backward)
     uint32_t ldz;
-    float* outf;         // [M][ldof]
+    float* outf;         // [N][ldof]
     uint32_t ldof;
-    bf16* outb;          // [M][ldob]
+    bf16* outb;          // [N][ldob]; with it N is a multiple of 16
     uint32_t ldob;
-    bf16* outt;          // [N][ldot] transposed copy
+    bf16* outt;          // [M][ldot] copy of outb the other way round
     uint32_t ldot;
-    const float* target;  // [M][nout] (loss)
+    const float* target;  // [N][nout] (loss)
     uint32_t nout;
     float* loss;
 };
@@ -66,21 +70,20 @@ struct GemmLaunch {
     CUtensorMap map[2][2];  // A and B of each product
     GemmArgs g[2];
     uint32_t tn[2], tiles[2];
-    uint32_t stages, stage_size, acc_cols;  // operand ring; columns of one tensor-memory accumulator
+    // Operand ring: stages of `group` K chunks; columns of one tensor-memory accumulator.
+    uint32_t stages, group, stage_size, acc_cols;
     ColumnSums cs;
     uint32_t* err;  // bit 0: an mbarrier wait ran out
 };
 
 constexpr uint32_t kTileM = 128, kTileK = 64, kMaxStages = 8;
-constexpr uint32_t kMinTileN = 32, kMaxTileN = 256;
+constexpr uint32_t kMinTileN = 16, kMaxTileN = 256;
 constexpr uint32_t kStageBudget = 192 * 1024;  // shared memory of the operand ring
 constexpr uint32_t kEpiWarps = 16;  // four per quarter of the 128 tensor-memory lanes
-constexpr uint32_t kEpiPitch = 12;  // words per staged row of 8 columns
-constexpr uint32_t kEpiBytes = kEpiWarps * 32 * kEpiPitch * 4;  // one staging block per epilogue warp
 constexpr uint32_t kGemmThreads = 64 + kEpiWarps * 32 + 64;
 
-// Dynamic shared memory: the ring, the epilogue's staging and 1 KB of alignment slack.
-constexpr uint32_t kGemmSmemMax = kStageBudget + kEpiBytes + 1024;
+// Dynamic shared memory: the ring and 1 KB of alignment slack.
+constexpr uint32_t kGemmSmemMax = kStageBudget + 1024;
 static_assert(kGemmSmemMax <= 232448 - 256, "dynamic and static shared memory of one CTA");
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
@@ -96,73 +99,103 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
            ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
 }
 
-// The epilogue's copies between a warp's block of 32 rows (one per lane) and 8 columns and row-major
-// FP32 memory, through the warp's staging block, so that a warp instruction touches sixteen whole
-// 32-byte sectors. `rows` is the number of live rows.
-__device__ __forceinline__ void block_store_f32(float* st, const float (&v)[8], float* out, uint32_t ld, uint32_t rows,
-                                                uint32_t lane)
+// The epilogue's copies between a warp's block of the accumulator, 32 lanes (rows of C) by C columns, and
+// row-major FP32 memory that holds the matrix transposed: an instruction touches 128 consecutive bytes. Lanes
+// from M on and columns from N on are left out.
+template <int C>
+__device__ __forceinline__ void block_store_f32(const float (&v)[C], float* out, uint32_t ld, bool live, uint32_t cols)
 {
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-        *reinterpret_cast<float4*>(st + lane * kEpiPitch + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-    __syncwarp();
-    const uint32_t c = (lane & 1u) * 4;
+    for (uint32_t k = 0; k < C; ++k)
+        if (live && k < cols) out[(size_t)k * ld] = v[k];
+}
+
+template <int C>
+__device__ __forceinline__ void block_fetch_f32(float (&v)[C], const float* in, uint32_t ld, bool live)
+{
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const uint32_t r = it * 16 + (lane >> 1);
-        if (r < rows)
-            *reinterpret_cast<float4*>(out + (size_t)r * ld + c) = *reinterpret_cast<const float4*>(st + r * kEpiPitch + c);
+    for (uint32_t k = 0; k < C; ++k) v[k] = live ? __ldcg(in + (size_t)k * ld) : 0.0f;
+}
+
+// The block as BF16, w[j] packing columns 2j and 2j+1 of the lane's row: the lane's columns in one store to
+// `outt`, and transposed to `out` (row k of it is column k), where neighbouring lanes swap halves so that a
+// store carries two lanes of one column.
+template <int C>
+__device__ __forceinline__ void block_store_bf16(const uint32_t (&w)[C / 2], bf16* out, uint32_t ld, bf16* outt, bool live,
+                                                 uint32_t lane)
+{
+    if (live) {
+        if constexpr (C == 8) *reinterpret_cast<uint4*>(outt) = make_uint4(w[0], w[1], w[2], w[3]);
+        else *reinterpret_cast<uint2*>(outt) = make_uint2(w[0], w[1]);
     }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void block_fetch_f32(float4 (&f)[2], const float* in, uint32_t ld, uint32_t rows, uint32_t lane)
-{
-    const uint32_t c = (lane & 1u) * 4;
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        const uint32_t r = it * 16 + (lane >> 1);
-        f[it] = r < rows ? *reinterpret_cast<const float4*>(in + (size_t)r * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-}
-
-__device__ __forceinline__ void block_row_f32(const float* st, float (&v)[8], uint32_t lane)
-{
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const float4 x = *reinterpret_cast<const float4*>(st + lane * kEpiPitch + 4 * k);
-        v[4 * k] = x.x;
-        v[4 * k + 1] = x.y;
-        v[4 * k + 2] = x.z;
-        v[4 * k + 3] = x.w;
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void block_spread_f32(float* st, const float4 (&f)[2], float (&v)[8], uint32_t lane)
-{
-    const uint32_t c = (lane & 1u) * 4;
-#pragma unroll
-    for (int it = 0; it < 2; ++it) *reinterpret_cast<float4*>(st + (it * 16 + (lane >> 1)) * kEpiPitch + c) = f[it];
-    __syncwarp();
-    block_row_f32(st, v, lane);
-}
-
-// The block as BF16: row-major to `out`, transposed to `outt` (column n of the block at outt + n * ldt,
-// the lane's row advancing along it). w[j] packs columns 2j and 2j+1 of the lane's row; neighbouring
-// lanes swap halves so that each store of the transposed copy carries two rows of one column. Rows come
-// in pairs: the products with a transposed copy have a multiple of 16 of them.
-__device__ __forceinline__ void block_store_bf16(const uint32_t (&w)[4], bf16* out, uint32_t ld, bf16* outt, uint32_t ldt,
-                                                 uint32_t rows, uint32_t lane)
-{
-    if (lane < rows) *reinterpret_cast<uint4*>(out + (size_t)lane * ld) = make_uint4(w[0], w[1], w[2], w[3]);
     const uint32_t c = lane & 1u;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < C / 2; ++j) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, w[j], 1);
         const uint32_t v = c ? __byte_perm(other, w[j], 0x7632) : __byte_perm(w[j], other, 0x5410);
-        if (lane < rows) *reinterpret_cast<uint32_t*>(outt + (size_t)(2 * j + c) * ldt + lane - c) = v;
+        if (live) *reinterpret_cast<uint32_t*>(out + (size_t)(2 * j + c) * ld - c) = v;
     }
+}
+
+// Epilogue of one tile by one of the warps of a quarter of its rows (lane: row m): blocks of C columns, block
+// `part` and every (kEpiWarps / 4)-th after it. `ready` waits for the accumulator (tensor-memory address d) and
+// returns false when the wait ran out; what else the first block needs is fetched before it. Returns the
+// lane's sum of squared errors (loss).
+template <int C, typename Ready>
+__device__ __forceinline__ float tile_epilogue(const GemmArgs& g, uint32_t m, uint32_t n0, uint32_t nt, uint32_t part,
+                                               uint32_t d, uint32_t lane, Ready ready)
+{
+    constexpr uint32_t kStep = C * (kEpiWarps / 4);
+    const bool live = m < g.M;
+    float z[C] = {};
+    const float* zin = g.epi == kEpiBackward ? g.zprev : g.target;
+    const uint32_t ldz = g.epi == kEpiBackward ? g.ldz : g.nout;
+    const bool zlive = g.epi == kEpiBackward ? live : g.epi == kEpiLoss && m < g.nout;
+    if (part * C < nt) block_fetch_f32(z, zin + (size_t)(n0 + part * C) * ldz + m, ldz, zlive);
+    const float bias = live && g.bias ? __ldcg(g.bias + m) : 0.0f;
+    float e2 = 0.0f;
+    if (!ready()) return 0.0f;
+    for (uint32_t c0 = part * C; c0 < nt; c0 += kStep) {
+        const uint32_t n = n0 + c0;
+        float v[C];
+        uint32_t w[C / 2];
+        tc_ld(d + c0, v);
+        if (g.epi != kEpiBackward && g.epi != kEpiStore) {
+#pragma unroll
+            for (int k = 0; k < C; ++k) v[k] += bias;
+        }
+        if (g.epi == kEpiHidden) {
+            block_store_f32(v, g.outf + (size_t)n * g.ldof + m, g.ldof, live, C);
+#pragma unroll
+            for (int j = 0; j < C / 2; ++j) w[j] = pack_bf16(silu(v[2 * j]), silu(v[2 * j + 1]));
+        } else if (g.epi == kEpiBackward) {
+#pragma unroll
+            for (int j = 0; j < C / 2; ++j)
+                w[j] = pack_bf16(v[2 * j] * dsilu(z[2 * j]), v[2 * j + 1] * dsilu(z[2 * j + 1]));
+        } else if (g.epi == kEpiLoss) {
+            // Mean squared error over the real outputs and its gradient 2 (Y - T) / (rows * nout).
+            const float cells = (float)(g.N * g.nout);
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+                float grad = 0.0f;
+                if (m < g.nout) {
+                    const float e = v[j] - z[j];
+                    e2 += e * e;
+                    grad = 2.0f * e / cells;
+                }
+                v[j] = grad;
+            }
+#pragma unroll
+            for (int j = 0; j < C / 2; ++j) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
+        } else {
+            block_store_f32(v, g.outf + (size_t)n * g.ldof + m, g.ldof, live, n < g.N ? g.N - n : 0u);
+        }
+        if (g.epi == kEpiHidden || g.epi == kEpiBackward || g.epi == kEpiLoss) {
+            if (c0 + kStep < nt) block_fetch_f32(z, zin + (size_t)(n + kStep) * ldz + m, ldz, zlive);
+            block_store_bf16<C>(w, g.outb + (size_t)n * g.ldob + m, g.ldob, g.outt + (size_t)m * g.ldot + n, live, lane);
+        }
+    }
+    return e2;
 }
 
 // Column sums by the warps w, w + nw, ... of the launch, two columns at a time so that a warp keeps
@@ -206,46 +239,51 @@ __device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
     x.tn = p.tn[x.q];
     x.m0 = (i % mtiles) * kTileM;
     x.n0 = (i / mtiles) * x.tn;
-    x.nt = min(x.tn, g.N - x.n0);
+    x.nt = min(x.tn, (g.N - x.n0 + 15u) & ~15u);
     x.nk = (g.K + kTileK - 1) / kTileK;
     return x;
 }
 
 // Persistent, warp-specialised product: each CTA (640 threads) walks output tiles of kTileM x tn
-// (tn = 32, 64, 128 or 256) in a grid-stride loop over the tiles of one or two independent products.
-//   warp 0, one thread: TMA producer. Each 64-wide K chunk of A and B is one box per operand in
-//     the 128-byte-swizzled K-major layout; up to eight chunks are in flight ("full" / "empty"
-//     mbarriers per stage), which for the narrow tiles is the whole K of a 512-wide layer.
-//   warp 1, one thread: issues the four K=16 tcgen05 products of each chunk into one of two
-//     tensor-memory accumulators (tile parity), commits each chunk to the stage's "empty" barrier
-//     and each finished tile to the accumulator's "full" barrier.
-//   warps 2-17: epilogue. Warp w reads tensor-memory lanes 32*(w mod 4) .. +31 with tcgen05.ld, 8
-//     columns at a time (four warps share a lane quarter's columns: the activation's exponential and
-//     division are one long chain per output, which only other warps hide),
-//     applies the fused epilogue and writes whole sectors through shared memory (block_store_*), then
-//     releases the accumulator ("empty"), so the products of the next tile overlap the epilogue of
-//     this one.
+// (tn = 16, 32, 64, 128 or 256) in a grid-stride loop over the tiles of one or two independent products.
+//   warp 0: TMA producer. Each 64-wide K chunk of A and B is one box per operand in the
+//     128-byte-swizzled K-major layout. A stage of the operand ring ("full" / "empty" mbarriers) holds
+//     one to four chunks: a wait on an mbarrier costs some 180 cycles even when its phase is over, more
+//     than the products of a narrow chunk (4 x 20 cycles).
+//   warp 1: issues the four K=16 tcgen05 products of each chunk into one of two tensor-memory
+//     accumulators (tile parity), commits each stage that is filled again to its "empty" barrier
+//     and each finished tile to the accumulator's "full" barrier. The whole warp runs the loop and an
+//     elected lane issues: from a branch on the lane, an issue took some 100 cycles.
+//   warps 2-17: epilogue (tile_epilogue). Warp w reads tensor-memory lanes 32*(w mod 4) .. +31 with
+//     tcgen05.ld, 8 columns at a time, or 4 of a tile of 16 (four warps share a lane quarter's columns: the
+//     activation's exponential and division are one long chain per output, which only other warps hide),
+//     applies the fused epilogue, writes, and releases the accumulator ("empty"), so the products of the
+//     next tile overlap the epilogue of this one. A's rows are the lanes, so the row-major outputs are
+//     written 128 bytes an instruction straight from registers.
 //   warps 18-19: the launch's column sums (bias gradients), beside the products.
 // The backward pass of a layer is one launch: its weight gradient, the signal of the layer below and
-// its bias gradient all read the same dZ. Launched with programmatic serialization: barriers and
-// tensor memory are set up while the previous launch ends. The next launch is let in only after this
-// CTA holds its tensor memory, so a later CTA can never take columns that an earlier one waits for.
+// its bias gradient all read the same dZ.
+// Launched with programmatic serialization: barriers and tensor memory are set up and A, the larger operand
+// of a narrow tile, and the epilogue's first inputs are fetched while the previous launch runs. That is sound
+// because a launch lets the next one in only after its own wait: when a CTA starts, every launch but the
+// previous one has ended, and A, bias, zprev and target are older than that (GemmArgs). By then the CTA also
+// holds its tensor memory, so a later CTA can never take columns that an earlier one waits for.
 // Every wait is bounded; a role that runs out records the error and stops, which bounds the waits
 // of the others; tensor memory is freed at the end in every case.
 //
-// What bounds it: the small products of training (256 x 512 x 512) one tile's chain of load, product
-// and epilogue; the large ones (4096 x 1024 x 1024) the epilogue's traffic (FP32 pre-activation, BF16
-// activation and its transpose, 33.6 MB) and the operand loads from L2. With one column per store
-// instruction (32 rows apart) and tiles of 128 columns the first took 41.7 us and a
-// training step of the second shape 85 us a product; now 10.7 and 34 us (profiler, cold caches), and the
-// fit network's training step 573 -> 245 us.
+// What bounds it: the small products of training (256 x 512 x 512, one tile a CTA) the chain of B's load
+// (0.4 us), products (0.6), epilogue (1.0) and the hand-over to the next launch (1.2): 6.5 us a layer with A
+// loaded after the wait, the roles of A and B exchanged and one chunk a stage, now 3.5 (backward 4.1); the fit
+// network's training step 103 -> 71.5 us. The large ones (4096 x 1024 x 1024) the epilogue, issue of the
+// activation's instructions and 33.6 MB of outputs (FP32 pre-activation, BF16 activation and its transpose):
+// the step of a 1024-wide network at 4,096 rows 399 -> 304 us. 4096^3 alone 165 -> 104 us.
 __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_constant__ GemmLaunch p)
 {
     extern __shared__ uint8_t smem_raw[];
     __shared__ unsigned long long full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     constexpr uint32_t aBytes = kTileM * kTileK * 2;
     const uint32_t tiles = p.tiles[0] + p.tiles[1], S = p.stages;
     if (warp == 0) tc_alloc(&tmem_slot, 2 * p.acc_cols);
@@ -262,139 +300,126 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    griddep_launch_dependents();
-    griddep_wait();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     bool ok = true;
-    if (warp == 0 && lane == 0) {  // producer
-        uint32_t s = 0, round = 0;
-        for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-            const TileAt x = tile_at(p, t);
-            const uint32_t bytes = aBytes + x.tn * kTileK * 2;
-            for (uint32_t c = 0; c < x.nk && ok; ++c) {
-                if (round > 0) ok = tc_bar_wait(&empty[s], (round - 1) & 1u);
-                if (!ok) break;
-                uint8_t* sa = smem + s * p.stage_size;
-                tc_bar_expect_tx(&full[s], bytes);
-                tc_tma_load_2d(sa, &p.map[x.q][0], (int32_t)(c * kTileK), (int32_t)x.m0, &full[s]);
-                tc_tma_load_2d(sa + aBytes, &p.map[x.q][1], (int32_t)(c * kTileK), (int32_t)x.n0, &full[s]);
-                if (++s == S) {
-                    s = 0;
-                    ++round;
+    const uint32_t ring = tc_smem(smem), stage = p.stage_size, ring_end = ring + S * stage, G = p.group;
+    const uint32_t full0 = tc_smem(full), empty0 = tc_smem(empty);
+    if (warp == 0) {  // producer
+        uint32_t t = blockIdx.x;
+        TileAt x = tile_at(p, min(t, tiles - 1));
+        const CUtensorMap *ma = &p.map[x.q][0], *mb = &p.map[x.q][1];
+        uint32_t early = t < tiles ? min(x.nk, S * G) : 0;
+        const bool one = tc_elect();
+        auto load = [&](const CUtensorMap* map, uint32_t to, uint32_t pitch, uint32_t c, uint32_t end, uint32_t row, uint32_t bar) {
+            for (; c < end; ++c, to += pitch) tc_tma_load_2d(to, map, (int32_t)(c * kTileK), (int32_t)row, bar);
+        };
+        // A of the first tile's chunks that the ring holds; after the wait their B.
+        if (one)
+            for (uint32_t c = 0, s = 0; c < early; c += G, ++s) {
+                const uint32_t end = min(c + G, x.nk);
+                tc_bar_expect_tx(full0 + 8 * s, (end - c) * (aBytes + x.tn * kTileK * 2));
+                load(ma, ring + s * stage, aBytes, c, end, x.m0, full0 + 8 * s);
+            }
+        griddep_wait();
+        if (one) {
+            uint32_t s = 0, round = 0;
+            for (uint32_t c = 0; c < early; c += G, ++s)
+                load(mb, ring + s * stage + G * aBytes, x.tn * kTileK * 2, c, min(c + G, x.nk), x.n0, full0 + 8 * s);
+            griddep_launch_dependents();
+            if (s == S) {
+                s = 0;
+                round = 1;
+            }
+            // The rest, as stages come free.
+            while (t < tiles && ok) {
+                for (uint32_t c = early; c < x.nk; c += G) {
+                    if (round > 0) ok = tc_bar_wait(empty0 + 8 * s, (round - 1) & 1u);
+                    if (!ok) break;
+                    const uint32_t bar = full0 + 8 * s, sa = ring + s * stage, end = min(c + G, x.nk);
+                    tc_bar_expect_tx(bar, (end - c) * (aBytes + x.tn * kTileK * 2));
+                    load(ma, sa, aBytes, c, end, x.m0, bar);
+                    load(mb, sa + G * aBytes, x.tn * kTileK * 2, c, end, x.n0, bar);
+                    if (++s == S) {
+                        s = 0;
+                        ++round;
+                    }
+                }
+                early = 0;
+                t += gridDim.x;
+                if (t < tiles) {
+                    x = tile_at(p, t);
+                    ma = &p.map[x.q][0];
+                    mb = &p.map[x.q][1];
                 }
             }
         }
-    } else if (warp == 1 && lane == 0) {  // tensor-core issuer
-        uint32_t s = 0, round = 0, li = 0;
+    } else if (warp == 1) {  // tensor-core issuer
+        uint32_t sa = ring, bar = full0, phase = 0, li = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++li) {
             const TileAt x = tile_at(p, t);
-            const uint32_t a = li & 1u, K = p.g[x.q].K;
-            if (li >= 2) ok = tc_bar_wait(&acc_empty[a], ((li >> 1) - 1) & 1u);
+            const uint32_t a = li & 1u, idesc = tc_idesc_bf16(kTileM, x.nt), d = tmem + a * p.acc_cols;
+            if (li >= 2) ok = __all_sync(0xffffffffu, tc_bar_wait(tc_smem(&acc_empty[a]), ((li >> 1) - 1) & 1u));
             if (!ok) break;
             tc_fence_after();
-            const uint32_t idesc = tc_idesc_bf16(kTileM, x.nt), d = tmem + a * p.acc_cols;
-            for (uint32_t c = 0; c < x.nk; ++c) {
-                ok = tc_bar_wait(&full[s], round & 1u);
+            // Steps whose stage is filled again: all but the CTA's last S.
+            const uint32_t steps = (x.nk + G - 1) / G, refilled = t + gridDim.x < tiles ? x.nk : (steps - min(steps, S)) * G;
+            const uint32_t bstep = x.tn * kTileK * 2 / 16;
+            for (uint32_t c = 0; c < x.nk; c += G) {
+                ok = __all_sync(0xffffffffu, tc_bar_wait(bar, phase));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t sa = tc_smem(smem + s * p.stage_size), sb = sa + aBytes;
-                const uint32_t ks = min(4u, (K - c * kTileK + 15) / 16);
-                for (uint32_t kk = 0; kk < ks; ++kk)
-                    tc_mma(d, tc_desc_sw128(sa + kk * 32), tc_desc_sw128(sb + kk * 32), idesc, c > 0 || kk > 0);
-                tc_commit(&empty[s]);
-                if (++s == S) {
-                    s = 0;
-                    ++round;
+                const uint64_t da = tc_desc_sw128(sa), db = tc_desc_sw128(sa + G * aBytes);
+                const uint32_t n = min(G, x.nk - c);
+                if (tc_elect()) {
+                    uint64_t ag = da, bg = db;
+                    uint32_t g = 0;
+                    do {
+#pragma unroll
+                        for (uint32_t kk = 0; kk < 4; ++kk)  // a K=16 slice is 32 bytes on: 2 in the descriptor
+                            tc_mma(d, ag + 2 * kk, bg + 2 * kk, idesc, c + g + kk > 0);
+                        ag += aBytes / 16;
+                        bg += bstep;
+                    } while (++g < n);
+                    if (c < refilled) tc_commit(bar + (empty0 - full0));
+                }
+                sa += stage;
+                bar += 8;
+                if (sa == ring_end) {
+                    sa = ring;
+                    bar = full0;
+                    phase ^= 1u;
                 }
             }
-            tc_commit(&acc_full[a]);
+            if (tc_elect() && ok) tc_commit(tc_smem(&acc_full[a]));
         }
     } else if (warp >= 2 && warp < 2 + kEpiWarps) {  // epilogue
         const uint32_t quarter = warp & 3u, part = (warp - 2) >> 2;
-        float* st = reinterpret_cast<float*>(smem + S * p.stage_size) + (warp - 2) * 32 * kEpiPitch;
-        constexpr uint32_t kStep = 8 * (kEpiWarps / 4);  // columns between a warp's blocks
         uint32_t li = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++li) {
             const TileAt x = tile_at(p, t);
             const GemmArgs& g = p.g[x.q];
-            const uint32_t a = li & 1u, n0 = x.n0, nt = x.nt;
-            const uint32_t r0 = x.m0 + quarter * 32;
-            const uint32_t rows = r0 < g.M ? min(32u, g.M - r0) : 0u;
-            float4 zf[2];  // pre-activations of the next block, in flight while the current one is done
-            if (g.epi == kEpiBackward && part * 8 < nt)
-                block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n0 + part * 8, g.ldz, rows, lane);
-            float e2 = 0.0f;
-            ok = __all_sync(0xffffffffu, tc_bar_wait(&acc_full[a], (li >> 1) & 1u));  // warp-uniform
+            const uint32_t a = li & 1u, m = x.m0 + quarter * 32 + lane;
+            const uint32_t d = tmem + a * p.acc_cols + ((quarter * 32u) << 16);
+            auto ready = [&] {
+                if (li == 0) griddep_wait();
+                ok = __all_sync(0xffffffffu, tc_bar_wait(tc_smem(&acc_full[a]), (li >> 1) & 1u));  // warp-uniform
+                tc_fence_after();
+                return ok;
+            };
+            // A tile of 16 columns gives each of the four warps four.
+            float e2 = x.tn < 32 ? tile_epilogue<4>(g, m, x.n0, x.nt, part, d, lane, ready)
+                                 : tile_epilogue<8>(g, m, x.n0, x.nt, part, d, lane, ready);
             if (!ok) break;
-            tc_fence_after();
-            for (uint32_t c0 = part * 8; c0 < nt; c0 += kStep) {
-                const uint32_t n = n0 + c0;
-                float v[8], z[8];
-                uint32_t w[4];
-                if (g.epi == kEpiLoss) {  // targets of the block, four rows per instruction
-#pragma unroll
-                    for (int it = 0; it < 8; ++it) {
-                        const uint32_t r = 4 * it + (lane >> 3), c = n + (lane & 7u);
-                        z[it] = (r < rows && c < g.nout) ? g.target[(size_t)(r0 + r) * g.nout + c] : 0.0f;
-                    }
-                }
-                tc_ld8(tmem + a * p.acc_cols + ((quarter * 32u) << 16) + c0, v);
-                if (g.epi == kEpiHidden || g.epi == kEpiLinear || g.epi == kEpiLoss) {
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + n) + k);
-                        v[4 * k] += b.x;
-                        v[4 * k + 1] += b.y;
-                        v[4 * k + 2] += b.z;
-                        v[4 * k + 3] += b.w;
-                    }
-                }
-                if (g.epi == kEpiHidden) {
-                    block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, lane);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) w[j] = pack_bf16(silu(v[2 * j]), silu(v[2 * j + 1]));
-                } else if (g.epi == kEpiBackward) {
-                    block_spread_f32(st, zf, z, lane);
-                    if (c0 + kStep < nt)
-                        block_fetch_f32(zf, g.zprev + (size_t)r0 * g.ldz + n + kStep, g.ldz, rows, lane);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        w[j] = pack_bf16(v[2 * j] * dsilu(z[2 * j]), v[2 * j + 1] * dsilu(z[2 * j + 1]));
-                } else if (g.epi == kEpiLoss) {
-                    // Mean squared error over the real outputs and its gradient 2 (Y - T) / (rows * nout).
-                    const float cells = (float)(g.M * g.nout);
-#pragma unroll
-                    for (int it = 0; it < 8; ++it) st[(4 * it + (lane >> 3)) * kEpiPitch + (lane & 7u)] = z[it];
-                    __syncwarp();
-                    block_row_f32(st, z, lane);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float grad = 0.0f;
-                        if (lane < rows && n + j < g.nout) {
-                            const float e = v[j] - z[j];
-                            e2 += e * e;
-                            grad = 2.0f * e / cells;
-                        }
-                        v[j] = grad;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) w[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
-                } else {
-                    block_store_f32(st, v, g.outf + (size_t)r0 * g.ldof + n, g.ldof, rows, lane);
-                }
-                if (g.epi == kEpiHidden || g.epi == kEpiBackward || g.epi == kEpiLoss)
-                    block_store_bf16(w, g.outb + (size_t)r0 * g.ldob + n, g.ldob, g.outt + (size_t)n * g.ldot + r0,
-                                     g.ldot, rows, lane);
-            }
             if (g.epi == kEpiLoss) {
                 for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-                if (lane == 0 && e2 != 0.0f) atomicAdd(g.loss, e2 / (float)(g.M * g.nout));
+                if (lane == 0 && e2 != 0.0f) atomicAdd(g.loss, e2 / (float)(g.N * g.nout));
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) tc_bar_arrive(&acc_empty[a]);
+            if (lane == 0) tc_bar_arrive(tc_smem(&acc_empty[a]));
         }
     } else if (warp >= 2 + kEpiWarps && p.cs.cols) {
+        griddep_wait();
         column_sums(p.cs, blockIdx.x * 2 + (warp - 2 - kEpiWarps), gridDim.x * 2, lane);
     }
     if (!ok) atomicOr(p.err, 1u);
@@ -437,30 +462,47 @@ uint32_t tile_count(const GemmArgs& g, uint32_t tn)
     return ((g.M + kTileM - 1) / kTileM) * ((g.N + tn - 1) / tn);
 }
 
-// Model of a CTA's time on one tile (cycles): its operand loads, (128 + tn) rows of 128 bytes per K
-// chunk, and its epilogue, 32 columns at a time.
-uint64_t tile_cost(const GemmArgs& g, uint32_t tn)
+// Model of a CTA's time on one tile, in cycles: its operands and products, (128 + tn) rows of 128 bytes per K
+// chunk at 90 bytes a cycle, and its epilogue, by 32 columns: 2,500 with an activation or a loss and BF16
+// copies (16 columns 1,700), 900 for a plain store.
+struct TileCost {
+    double main, epi;
+};
+TileCost tile_cost(const GemmArgs& g, uint32_t tn)
 {
-    return (uint64_t)((g.K + kTileK - 1) / kTileK) * (kTileM + tn) * 2 + 500ull * (tn / 32);
+    const bool plain = g.epi == kEpiStore || g.epi == kEpiLinear;
+    const double per = plain ? 900.0 : 2500.0;
+    return {(g.K + kTileK - 1) / kTileK * (kTileM + tn) * 1.4,
+            tn < 32 ? (plain ? 700.0 : 1700.0) : per * tn / 32};
 }
 
 // Columns per tile of each of the n products of a launch on num_sm SMs: the pair with the smallest
-// modelled time. Narrow tiles win while wide ones leave SMs idle (a 256 x 512 layer: 32 tiles of 32
-// columns instead of 8 of 128), wide ones once every SM has work (fewer operand loads per output):
-// the step of a 1024-wide network at 4,096 rows took 570, 522, 496 and 450 us with forward tiles and
-// backward pairs of 32, 64, 128 and 256 columns, and 480 us with the long weight-gradient tiles first.
+// modelled time. Narrow tiles win while wide ones leave SMs idle, wide ones once every SM has work (fewer
+// operand loads per output) up to where the epilogue of a CTA's last tile, which nothing overlaps, weighs
+// more. Measured with forward and signal tiles of a columns and weight-gradient tiles of b (a/b): training
+// step of the fit network (256 x 512) 71.8 us at 16/32, 71.8 at 16/64, 75.5 at 32/32, 83 at 32/128 and 97 at
+// 64/64; of a 1024-wide network at 4,096 rows 304 at 128/64, 314 at 128/128, 326 at 64/64 and 256/64, 335 at
+// 256/256.
 void choose_tiles(const GemmArgs* g, uint32_t n, uint32_t num_sm, uint32_t (&tn)[2])
 {
-    uint64_t best = ~0ull;
+    constexpr double kPerTile = 1500.0;  // barriers and hand-over of a tile
+    double best = 1e300;
     for (uint32_t a = kMinTileN; a <= kMaxTileN; a *= 2)
         for (uint32_t b = kMinTileN; b <= (n > 1 ? kMaxTileN : kMinTileN); b *= 2) {
-            const uint64_t ca = tile_cost(g[0], a), cb = n > 1 ? tile_cost(g[1], b) : 0;
-            const uint64_t ta = tile_count(g[0], a), tb = n > 1 ? tile_count(g[1], b) : 0;
-            const uint64_t waves = (ta + tb + num_sm - 1) / num_sm;
+            double work = 0.0, longest = 0.0;
+            uint32_t tiles = 0;
+            for (uint32_t i = 0; i < n; ++i) {
+                const TileCost c = tile_cost(g[i], i ? b : a);
+                const uint32_t t = tile_count(g[i], i ? b : a);
+                tiles += t;
+                work += t * (std::max(c.main, c.epi) + kPerTile);  // loads overlap the epilogue before them
+                longest = std::max(longest, c.main + c.epi + kPerTile);
+            }
+            const uint32_t waves = (tiles + num_sm - 1) / num_sm;
             // One product fills whole waves; two of different cost fill the gaps of each other.
-            const uint64_t cost = waves <= 1 ? std::max(ca, cb)
-                                  : n == 1   ? waves * ca
-                                             : (ta * ca + tb * cb) / num_sm + std::max(ca, cb) / 2;
+            const double cost = waves <= 1 ? longest
+                                : n == 1   ? waves * work / tiles + std::min(tile_cost(g[0], a).main, tile_cost(g[0], a).epi)
+                                           : work / num_sm + 0.75 * longest;
             if (cost < best) {
                 best = cost;
                 tn[0] = a;
@@ -487,14 +529,16 @@ int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* e
         p.acc_cols = std::max(p.acc_cols, p.tn[i]);
         nk = std::max(nk, (g[i].K + kTileK - 1) / kTileK);
     }
-    p.stage_size = (kTileM + p.acc_cols) * kTileK * 2;
-    p.stages = std::min({kStageBudget / p.stage_size, kMaxStages, nk * (p.tiles[0] + p.tiles[1] > num_sm ? 2u : 1u)});
+    p.group = std::min(p.acc_cols <= 64 ? 4u : p.acc_cols <= 128 ? 2u : 1u, nk);
+    p.stage_size = p.group * (kTileM + p.acc_cols) * kTileK * 2;
+    p.stages = std::min({kStageBudget / p.stage_size, kMaxStages,
+                         (nk + p.group - 1) / p.group * (p.tiles[0] + p.tiles[1] > num_sm ? 2u : 1u)});
     p.cs = cs;
     p.err = err;
     // CTAs without a tile only add column sums (four columns each pass).
     const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 3) / 4), num_sm);
     return launch_pdl(k_gemm_tn, dim3(ctas), dim3(kGemmThreads),
-                      p.stages * p.stage_size + kEpiBytes + 1024, st, pdl, p);
+                      p.stages * p.stage_size + 1024, st, pdl, p);
 }
 
 // Inputs: FP32 [n][nin] -> BF16 [n][ldx] (zero padded) and transposed [ldx][ldt]; the loss is zeroed
@@ -636,11 +680,11 @@ int mlp_forward(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
     for (uint32_t l = 0; l < L && !e; ++l) {
         const uint32_t in = n->dim[l], out = n->dim[l + 1];
         GemmArgs g{};
-        g.A = l == 0 ? n->x : n->h[l - 1];
-        g.B = n->wb[l];
+        g.A = n->wb[l];
+        g.B = l == 0 ? n->x : n->h[l - 1];
         g.lda = g.ldb = in;
-        g.M = rows;
-        g.N = out;
+        g.M = out;
+        g.N = rows;
         g.K = in;
         g.bias = n->b[l];
         g.ldof = g.ldob = out;
@@ -666,8 +710,8 @@ int mlp_forward(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
     return e;
 }
 
-// One launch per layer: dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}) (M = rows, N = in, K = out), dW_l =
-// dZ_l^T H_{l-1} (M = out, N = in, K = rows) and db_l = column sums of dZ_l.
+// One launch per layer: dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}) (M = in, N = rows, K = out), dW_l =
+// dZ_l^T H_{l-1} (M = in, N = out, K = rows) and db_l = column sums of dZ_l.
 int mlp_backward(arbo_mlp* n, uint32_t rows, cudaStream_t st)
 {
     const uint32_t ld = n->maxb, L = n->L;
@@ -677,21 +721,21 @@ int mlp_backward(arbo_mlp* n, uint32_t rows, cudaStream_t st)
         const uint32_t in = n->dim[l], out = n->dim[l + 1];
         GemmArgs g[2] = {};
         GemmArgs& w = g[l > 0 ? 1 : 0];
-        w.A = dzt;
-        w.B = l == 0 ? n->xt : n->ht[l - 1];
+        w.A = l == 0 ? n->xt : n->ht[l - 1];
+        w.B = dzt;
         w.lda = w.ldb = ld;
-        w.M = out;
-        w.N = in;
+        w.M = in;
+        w.N = out;
         w.K = rows;
         w.epi = kEpiStore;
         w.outf = n->dw[l];
         w.ldof = in;
         if (l > 0) {
-            g[0].A = dz;
-            g[0].B = n->wt[l];
+            g[0].A = n->wt[l];
+            g[0].B = dz;
             g[0].lda = g[0].ldb = out;
-            g[0].M = rows;
-            g[0].N = in;
+            g[0].M = in;
+            g[0].N = rows;
             g[0].K = out;
             g[0].epi = kEpiBackward;
             g[0].zprev = n->z[l - 1];
@@ -1027,11 +1071,11 @@ int arbo_tc_gemm(const float* a, const float* b, uint32_t M, uint32_t N, uint32_
     cudaMemcpy(db, hb.data(), hb.size() * 2, cudaMemcpyHostToDevice);
     cudaMemset(derr, 0, 4);
     GemmArgs g{};
-    g.A = da;
-    g.B = db;
+    g.A = db;
+    g.B = da;
     g.lda = g.ldb = K;
-    g.M = M;
-    g.N = g.ldof = N;
+    g.M = g.ldof = N;
+    g.N = M;
     g.K = K;
     g.epi = kEpiStore;
     g.outf = dc;

@@ -53,6 +53,14 @@ __device__ __forceinline__ void tc_dealloc(uint32_t taddr, uint32_t ncols)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool tc_elect()
+{
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
+
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accum)
 {
     asm volatile(
@@ -63,9 +71,9 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
 }
 
 // Arrives once on the mbarrier when every tcgen05.mma issued so far by this thread has completed.
-__device__ __forceinline__ void tc_commit(unsigned long long* bar)
+__device__ __forceinline__ void tc_commit(uint32_t bar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem(bar))
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
 
@@ -81,15 +89,14 @@ __device__ __forceinline__ void tc_bar_init(unsigned long long* bar, uint32_t co
 }
 
 // Bounded wait for the phase of `bar` with the given parity; false when the bound ran out.
-__device__ __forceinline__ bool tc_bar_wait(unsigned long long* bar, uint32_t parity)
+__device__ __forceinline__ bool tc_bar_wait(uint32_t bar, uint32_t parity)
 {
-    const uint32_t a = tc_smem(bar);
     for (uint32_t it = 0; it < kTcMaxPolls; ++it) {
         uint32_t ok;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(ok)
-            : "r"(a), "r"(parity)
+            : "r"(bar), "r"(parity)
             : "memory");
         if (ok) return true;
     }
@@ -97,7 +104,7 @@ __device__ __forceinline__ bool tc_bar_wait(unsigned long long* bar, uint32_t pa
 }
 
 // Eight consecutive FP32 accumulator columns of the calling thread's tensor-memory lane.
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8])
+__device__ __forceinline__ void tc_ld(uint32_t taddr, float (&v)[8])
 {
     uint32_t r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -109,27 +116,40 @@ __device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8])
     for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// One arrival on `bar` that also announces `bytes` of asynchronous transfers for its current phase.
-__device__ __forceinline__ void tc_bar_expect_tx(unsigned long long* bar, uint32_t bytes)
+// Four of them.
+__device__ __forceinline__ void tc_ld(uint32_t taddr, float (&v)[4])
 {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem(bar)), "r"(bytes) : "memory");
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// One arrival on `bar` that also announces `bytes` of asynchronous transfers for its current phase.
+__device__ __forceinline__ void tc_bar_expect_tx(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
 // Plain arrival (count 1) on an mbarrier.
-__device__ __forceinline__ void tc_bar_arrive(unsigned long long* bar)
+__device__ __forceinline__ void tc_bar_arrive(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(bar)) : "memory");
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // Tiled TMA load of a 2-D box at element coordinates (x innermost, y) into shared memory,
 // completing on `bar`. x times the element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tc_tma_load_2d(void* dst, const CUtensorMap* map, int32_t x, int32_t y,
-                                               unsigned long long* bar)
+__device__ __forceinline__ void tc_tma_load_2d(uint32_t dst, const CUtensorMap* map, int32_t x, int32_t y,
+                                               uint32_t bar)
 {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            tc_smem(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(tc_smem(bar))
+            dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
 

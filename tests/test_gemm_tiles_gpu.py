@@ -24,7 +24,7 @@ def test_product_matches_numpy(gpu, M, N, K):
     assert np.all(err <= np.maximum(bound, 1e-30))
 
 
-@pytest.mark.parametrize("hidden,layers,n_out,rows", [(16, 1, 1, 16), (48, 2, 7, 144), (272, 1, 100, 400)])
+@pytest.mark.parametrize("hidden,layers,n_out,rows", [(16, 1, 1, 16), (48, 2, 7, 144), (272, 1, 100, 400), (656, 2, 33, 208)])
 def test_epilogues_match_restatement(gpu, hidden, layers, n_out, rows):
     rng = np.random.default_rng(hidden + rows)
     net = MLP(6, hidden, layers, n_out, max_batch=rows + 32, seed=7)
@@ -42,3 +42,20 @@ def test_epilogues_match_restatement(gpu, hidden, layers, n_out, rows):
         assert np.linalg.norm(dw - dws[l]) <= 2e-3 * np.linalg.norm(dws[l])
         assert np.linalg.norm(db - dbs[l]) <= 2e-3 * np.linalg.norm(dbs[l])
     assert np.abs(net.forward(x) - y[:, :n_out]).max() <= 1e-3 * max(1.0, np.abs(y).max())
+
+
+def test_row_counts_past_the_captured_ones(gpu):
+    """More row counts than captured sequences are kept: the first, the captured and the evicted call of each
+    give the same outputs and gradients, bit for bit."""
+    rng = np.random.default_rng(5)
+    net = MLP(6, 64, 2, 30, max_batch=192, seed=3)
+    x = rng.uniform(-1, 1, (192, 6)).astype(np.float32)
+    t = rng.standard_normal((192, 30)).astype(np.float32)
+    first = {}
+    for turn in range(3):
+        for rows in range(16, 192, 16):
+            for _ in range(1 + turn):
+                net.gradients(x[:rows], t[:rows])
+                got = [net.forward(x[:rows])] + [net.layer(l)[k] for l in range(net.layers) for k in (2, 3)]
+                for a, b in zip(first.setdefault(rows, got), got):
+                    np.testing.assert_array_equal(a, b)
