@@ -1571,7 +1571,9 @@ __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, 
 {
     extern __shared__ __align__(16) unsigned char steps_dyn[];
     __shared__ __align__(16) unsigned long long dev_copy[sizeof(Dev) / 8];
+    __shared__ uint32_t next[2];  // items taken, by parity of the step
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 2) next[threadIdx.x] = 0;
     {
         const unsigned long long* src = reinterpret_cast<const unsigned long long*>(devs + blockIdx.x / C);
         for (uint32_t i = threadIdx.x; i < sizeof(Dev) / 8; i += blockDim.x) dev_copy[i] = src[i];
@@ -1584,12 +1586,23 @@ __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, 
     StepAt at = load_step(d.ctrl, 0);
     const uint32_t quads = (d.tiles + kQuad - 1) / kQuad, hw = (d.nvec + 31) / 32;
     const uint32_t foi = foi_event_items(d) + d.S * series_chunks(d.P);
+    // Demographic items are of uneven cost. With four or more to a warp a CTA's warps take its share of them
+    // from a counter (step of 128 simulations of 7e4 agents 65.4 -> 62.8 us, later 38.2 -> 36.1); with
+    // fewer the counter costs more than it evens out (8 of them, half an item to a warp: 17.8 -> 18.4).
+    const bool by_counter = quads + hw >= 4 * nw;
     for (uint32_t k = 0; k < nsteps; ++k, ++at.t, ++at.epoch) {
-        for (uint32_t it = w; it < quads + hw; it += nw) {
+        auto after = [&](uint32_t it) {
+            if (!by_counter) return it + nw;
+            uint32_t i = 0;
+            if (lane == 0) i = atomicAdd(&next[k & 1u], 1u);
+            return __shfl_sync(kFull, i, 0) * C + rank;
+        };
+        for (uint32_t it = by_counter ? after(0) : w; it < quads + hw; it = after(it)) {
             if (it < quads) demog_mosquito_quad<false>(d, at.key, it, lane, at.t, scratch.demog);
             else demog_humans<1>(d, at.key, (it - quads) * 32 + lane, 32, at.t, scratch.demog);
         }
         cluster_barrier();
+        if (threadIdx.x == 0) next[(k + 1) & 1u] = 0;
         for (uint32_t g = w; g < foi; g += nw) foi_item<false>(d, g, 0, at, scratch.foi);
         cluster_barrier();
         for (uint32_t c = w; c < d.P; c += nw) infect_unit<false, B == 1, kByWarp>(d, c, at, scratch.infect);

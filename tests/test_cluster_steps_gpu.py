@@ -58,3 +58,17 @@ def test_clusters_and_phases_agree_and_alternate(gpu):
             b.step(30)
         for i in range(len(ws)):
             same(a[i], p[i], f"instance {i}, new seeds")
+
+
+def test_items_by_counter_equal_single_steps(gpu):
+    # Enough demographic items to a warp that a CTA's warps take them from a counter, in odd numbers.
+    ws = [small_case(n=5_003 + 97 * (i % 5), m=20_011 + 613 * (i % 3), side=3, T=9, seed=i) for i in range(160)]
+    together, check = make(ws), [0, 77, 159]
+    with Batch(together) as b:
+        b.init()
+        b.step(3)
+        b.step(6)
+        for i, s in zip(check, make([ws[i] for i in check])):
+            s.init()
+            s.step(9)
+            same(s, together[i], f"instance {i}")
