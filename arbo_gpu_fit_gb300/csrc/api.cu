@@ -598,7 +598,6 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     s->l.foiBlock = arch.foiBlock;
     s->l.infectBlock = arch.infectBlock;
     s->l.numSM = arch.totalSM;
-    s->l.demogBlocksPerSM = (uint32_t)demog_blocks_per_sm(arch.demogUnroll, arch.demogBlock);
     cudaGetLastError();
     s->l.pdl = 1;
     if (const int e = share_carveout())
@@ -1469,9 +1468,9 @@ Dev batch_desc(const arbo_batch* b, size_t i)
     return d;
 }
 
-// Agents of the largest community from which a batch's infection pass, where the caller leaves the default
-// block, takes 256 threads and works off communities with many events by block (k_infect_batch<true>), in
-// runs of two communities. Smaller communities seldom have that many events, and the search for them costs
+// Agents of the largest community from which a batch's infection pass works off communities with many events
+// by block (k_infect_batch<true>), in runs of two communities and, where the caller leaves the default block,
+// in blocks of 256 threads. Smaller communities seldom have that many events, and the search for them costs
 // 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us, at runs of 4, 2 and 1: 352, 289 and
 // 278 in blocks of 256, 398, 370 and 350 in blocks of 512, 456, 378 and 280 in blocks of 64; with few
 // events 83, 85 and 92. One simulation alone keeps k_infect: with this its step took 1 to 3 % longer.
@@ -1480,8 +1479,8 @@ constexpr uint64_t kHeavyCommunity = 16384;
 // Steps per launch of k_steps.
 constexpr uint32_t kClusterSteps = 128;
 
-// Whether `a` chooses launch shapes of the per-phase kernels (the human unroll aside, which chain
-// batches set for them): a caller who does gets those kernels.
+// Whether `a` chooses launch shapes of the per-phase kernels (the human unroll aside): a caller who does
+// gets those kernels.
 bool chooses_shapes(const arbo_arch_param& a)
 {
     arbo_arch_param q;
@@ -1530,8 +1529,8 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     arbo_arch_param_query(&dflt, -1);
     uint64_t most = 0;  // largest community of any instance
     for (const arbo_sim* s : b->sims) most = std::max(most, s->comm_most);
-    const bool heavy = most >= kHeavyCommunity && a.infectBlock == dflt.infectBlock;
-    l.infectBlock = heavy ? 256 : a.infectBlock;
+    const bool heavy = most >= kHeavyCommunity;
+    l.infectBlock = heavy && a.infectBlock == dflt.infectBlock ? 256 : a.infectBlock;
     l.infectHeavy = heavy;
     l.numSM = a.totalSM ? a.totalSM : 152u;
     l.pdl = 1;

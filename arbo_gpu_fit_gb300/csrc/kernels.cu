@@ -1951,16 +1951,6 @@ int launch_l2_flush(const void* buf, size_t bytes, uint32_t* sink, uint32_t num_
     return (int)cudaGetLastError();
 }
 
-int demog_blocks_per_sm(uint32_t unroll, uint32_t block)
-{
-    int n = 0;
-    cudaError_t e;
-    if (unroll == 4) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_demog<4>, (int)block, 0);
-    else if (unroll == 2) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_demog<2>, (int)block, 0);
-    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_demog<1>, (int)block, 0);
-    return (e == cudaSuccess && n > 0) ? n : 1;
-}
-
 int demog_tma_blocks_per_sm(uint32_t unroll)
 {
     int n = 0;

@@ -192,17 +192,16 @@ struct BatchDev {
 };
 
 struct Launch {
-    uint32_t demogBlock, demogUnroll, foiBlock, infectBlock, numSM, demogBlocksPerSM;
+    uint32_t demogBlock, demogUnroll, foiBlock, infectBlock, numSM;
     uint32_t infectHeavy;  // whole blocks work off communities with many events
-    uint32_t pdl;  // 1: k_foi and k_infect use programmatic dependent launch
+    uint32_t pdl;  // 1: the kernels of a step use programmatic dependent launch
     uint32_t demogPipeline;       // 1: persistent TMA-staged demographic kernel
     uint32_t demogTmaBlocksPerSM;
 };
 
 // Kernel launchers (kernels.cu). Each returns the cudaError_t of the launch as int.
 int launch_init(const Dev& d, const Launch& l, void* stream);
-// Resident CTAs per SM of the demographic kernel for the given unroll and block size.
-int demog_blocks_per_sm(uint32_t unroll, uint32_t block);
+// Resident CTAs per SM of the TMA-staged demographic kernel.
 int demog_tma_blocks_per_sm(uint32_t unroll);
 // Warp items of the force-of-infection kernel for S serotypes and P communities.
 uint32_t foi_items(uint32_t S, uint32_t P);

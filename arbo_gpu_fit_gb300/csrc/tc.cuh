@@ -1,12 +1,6 @@
 // tc.cuh — fifth-generation tensor-core building blocks for sm_103a (inline PTX): tensor-memory
 // allocation, shared-memory matrix descriptors, tcgen05.mma of BF16 operands into an FP32
 // accumulator in tensor memory, completion through an mbarrier, and accumulator loads.
-//
-// Operand layout (both operands K-major, no swizzle): the tile is stored as 8-row x 16-byte core
-// matrices; element (r, k) of a tile with KT columns sits at byte
-//     (r / 8) * SBO + (k / 8) * 128 + (r % 8) * 16 + (k % 8) * 2,    SBO = (KT / 8) * 128,
-// i.e. core matrices adjacent along K are 128 bytes apart (the descriptor's leading-dimension
-// offset) and groups of 8 rows are SBO apart (its stride offset).
 #pragma once
 #include <cuda.h>
 #include <stdint.h>
@@ -16,14 +10,6 @@ namespace arbo {
 constexpr uint32_t kTcMaxPolls = 1u << 22;  // bound of every mbarrier wait
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Shared-memory matrix descriptor: start address, leading (K) and stride (row-group) byte
-// offsets, descriptor version 1, no swizzle.
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
 
 // Descriptor of a K-major operand in the 128-byte-swizzled layout that a TMA copy with
 // CU_TENSOR_MAP_SWIZZLE_128B writes: rows of 128 bytes (64 BF16 along K), the 16-byte chunks of
@@ -79,8 +65,6 @@ __device__ __forceinline__ void tc_commit(uint32_t bar)
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Generic-proxy shared-memory writes made visible to the tensor core (async proxy).
-__device__ __forceinline__ void tc_fence_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void tc_bar_init(unsigned long long* bar, uint32_t count)
 {

@@ -1,5 +1,5 @@
 """Communities with many events a step, which a warp works off alone in one simulation and the whole block
-in a batch of large communities: the first against the serial oracle, the second against the first."""
+in a batch with large communities: the first against the serial oracle, the second against the first."""
 
 import pytest
 
@@ -22,7 +22,7 @@ def test_heavy_communities_match_oracle(gpu, n, m, side, shape):
     assert sim.series("n_incidence").sum() > 2000
 
 
-# The default block (by block from 16,384 agents a community) and set ones (by warp).
+# The default block (256 threads for communities of 16,384 agents) and set ones.
 @pytest.mark.parametrize("block", [None, 32, 512])
 def test_heavy_communities_in_a_batch(gpu, block):
     arch = ArchitectureParam(0, **({"infectBlock": block} if block else {}))
