@@ -1,6 +1,6 @@
 // kernels.cu — sm_103a kernels of one simulation time step and of its initialisation.
 //
-// One step is three launches (captured in a CUDA graph by the host):
+// One step is three launches (after a handle's first steps captured in CUDA graphs by the host):
 //   k_demog   human and mosquito demographic passes over the whole census (HBM stream: a
 //             human's next event time, a mosquito slot's event code; ages are birth times,
 //             so a survivor without a transition writes nothing), per-tile
@@ -12,7 +12,7 @@
 //             mVisitingInfected (cpp/datacollect.cu:10-189, cpp/epidemic.cu:12-29,
 //             cpp/nepidemic.cu:28-142, cpp/mepidemic.cu:28-138).
 //   k_infect  one warp per community: event-parallel infection draws resolved to the
-//             reference's serial order by a minimum order key per target, external
+//             reference's serial order among the warp's lanes or by a minimum order key per target, external
 //             introductions, application of the winners; replaces nmTransmission +
 //             mnTransmission (cpp/mepidemic.cu:143-246, cpp/nepidemic.cu:146-319).
 // No tensor cores: the work is integer streaming and scattered events.

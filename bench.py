@@ -8,7 +8,7 @@ communities on a 50x50 rook lattice, lognormal(0, 0.8) community sizes, 4 seroty
 A "step" is one simulation time step over the whole census (human and mosquito demographic
 passes, force of infection with dispersal, infection draws, series row). ``value`` =
 (humans + mosquito slots) * timed steps * ranks / max-over-ranks device time, with the census
-resident in HBM. The census read per step (63 MB) is smaller than L2, so every timed step is
+resident in HBM. The census read per step (10 MB) is smaller than L2, so every timed step is
 preceded by an untimed kernel that reads a 320 MiB buffer (cold L2 at each step start).
 
 Arms:
@@ -35,20 +35,20 @@ sys.path.insert(0, str(ROOT))
 # Algorithmic bytes per agent-step of the demographic pass, the roofline figure: what the
 # reference's algorithm moves per agent (read age 4 + death age 4 + status 1, write age 4).
 BYTES_PER_AGENT_STEP = 13
-# What this library's layout moves instead: ages are kept as birth times, so a mosquito slot costs
-# its state byte and death time (5) and a human its next event time (4), and a survivor without a
-# transition writes nothing; each birth writes the newborn's PLE, birth time and death time (12)
-# and a status byte, plus the status byte of the death that freed its slot.
+# What this library's layout moves instead: ages are kept as birth times and a slot's next event as one
+# byte, so a mosquito slot costs that byte (1) and a human its next event time (4), and a survivor
+# without a transition writes nothing; each birth writes the newborn's life record (16: birth and death
+# time, PLE) and its byte, plus the byte of the death that freed its slot.
 LAYOUT_BYTES_PER_HUMAN_STEP = 4
-LAYOUT_BYTES_PER_SLOT_STEP = 5
-LAYOUT_BYTES_PER_BIRTH = 14
+LAYOUT_BYTES_PER_SLOT_STEP = 1
+LAYOUT_BYTES_PER_BIRTH = 18
 FLUSH_MB = 320
 PEAKS_FILE = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6800.0
 # Per-launch DRAM traffic of the demographic kernel on this workload, from one ncu capture of a
 # launch at step 5 (the command is kept with its summary under profiles/):
-# dram__bytes_read.sum + dram__bytes_write.sum (42,747,136 + 8,205,824 bytes).
-DEMOG_TRAFFIC_BYTES = 50_952_960
+# dram__bytes_read.sum + dram__bytes_write.sum (15,225,344 + 4,442,624 bytes).
+DEMOG_TRAFFIC_BYTES = 19_667_968
 
 
 def parse():

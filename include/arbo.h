@@ -402,7 +402,7 @@ int arbo_sim_weekly_incidence(arbo_sim* s, uint32_t max_week, uint32_t* out, voi
  * it — a step loop running under a framework whose memory pool owns the device, an embedded or
  * real-time driver that forbids allocation after set-up, or code that must not trigger the device
  * memory that building a CUDA graph can take. arbo_sim_step captures and instantiates CUDA graphs
- * on first use, and the handle's own per-agent scratch was allocated at create; this entry point
+ * once a handle has made some hundred steps, and the handle's own per-agent scratch was allocated at create; this entry point
  * launches the same step kernels one by one and takes the infection pass's per-agent scratch from
  * a fixed array compiled into the library instead.
  *
@@ -425,9 +425,10 @@ int arbo_sim_step_noalloc(arbo_sim* s, uint32_t nsteps, void* stream);
 
 /* ------------------------------------------------------------------ batches */
 
-/* Many simulation handles stepped together: one persistent kernel per phase (demographic, force
- * of infection, infection) walks the blocks of every instance, with the step loop captured in a
- * CUDA graph. Replaces the reference's serial loop over replicates and MCMC proposals
+/* Many simulation handles stepped together: few and small ones as one thread-block cluster per
+ * simulation that runs many steps in a launch; others by one persistent kernel per phase
+ * (demographic, force of infection, infection) that walks the items of every instance, with long
+ * step loops captured in CUDA graphs. Replaces the reference's serial loop over replicates and MCMC proposals
  * (cpp/main.cpp:262-280, one simulation() call each). Instances may differ in every size and
  * parameter; each keeps its own buffers, key and counters, and its results are bit-identical to
  * stepping it alone, so arbo_sim_get_* read them as usual. Instances are stepped only through the
@@ -435,7 +436,8 @@ int arbo_sim_step_noalloc(arbo_sim* s, uint32_t nsteps, void* stream);
 typedef struct arbo_batch arbo_batch;
 
 /* Builds a batch of n handles (one device; each handle at most once). arch: launch shapes of the
- * batched kernels (NULL: those of sims[0]); the grids are one wave of resident CTAs. */
+ * batched kernels (NULL: those of sims[0]); the grids are one wave of resident CTAs. Shapes other than
+ * the defaults (the human unroll aside) select the per-phase kernels. */
 int arbo_batch_create(arbo_sim* const* sims, uint32_t n, const arbo_arch_param* arch, arbo_batch** out);
 int arbo_batch_destroy(arbo_batch* b);
 /* Number of instances and their total agents (humans + mosquito slots). */
