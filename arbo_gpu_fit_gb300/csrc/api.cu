@@ -1432,6 +1432,7 @@ struct arbo_batch {
     bool phase_shapes = false;  // the caller chose launch shapes of the per-phase kernels
     uint32_t cluster = 0;       // CTAs per simulation of k_steps (0: the per-phase kernels)
     uint32_t cluster_per_sm = 1;
+    uint64_t cluster_items = 0;  // demographic warp items of all simulations in k_steps
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> step_ev;
     void* flush = nullptr;
@@ -1650,6 +1651,8 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     b->l = l;
     b->arch = a;
     b->cluster = batch_cluster(b, &b->cluster_per_sm);
+    b->cluster_items = 0;
+    for (const arbo_sim* s : b->sims) b->cluster_items += cdiv(s->d.tiles, kQuad) + cdiv(s->d.nvec, 32);
     return ARBO_OK;
 }
 
@@ -1934,7 +1937,7 @@ int arbo_batch_step(arbo_batch* b, uint32_t nsteps, void* stream)
     }
     while (n > 0 && b->cluster) {
         const uint32_t chunk = std::min(n, kClusterSteps);
-        e = launch_steps(b->bd.devs, b->bd.n, b->cluster, b->cluster_per_sm, chunk, st);
+        e = launch_steps(b->bd.devs, b->bd.n, b->cluster, b->cluster_per_sm, b->cluster_items, chunk, st);
         if (e) return fail(ARBO_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString((cudaError_t)e));
         n -= chunk;
         batch_advance_host(b, chunk);

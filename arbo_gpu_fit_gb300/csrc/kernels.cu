@@ -466,14 +466,49 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
     }
 }
 
-// Quad with its codes loaded straight from global memory. With kWait, the wait for the previous kernel
+// What a phase's work waits for once it has done what does not depend on the previous phase: nothing, the
+// previous kernel of the stream, or (PendingWait) the previous phase of a cluster, once per warp and phase.
+struct NoWait {
+    __device__ __forceinline__ void operator()() const {}
+};
+struct GridWait {
+    __device__ __forceinline__ void operator()() const { griddep_wait(); }
+};
+// In the infection pass the next step's demographic pass may be scheduled only then: before its own wait it
+// reads the dead counts, which this step's pass (finished before the grid waited for) writes.
+struct GridWaitRelease {
+    __device__ __forceinline__ void operator()() const
+    {
+        griddep_wait();
+        griddep_launch_dependents();
+    }
+};
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Its two halves, for warps whose lanes the compiler may have apart.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+struct PendingWait {
+    bool& pending;  // warp-uniform
+    __device__ __forceinline__ void operator()() const
+    {
+        if (pending) cluster_wait();
+        pending = false;
+    }
+};
+
+// Quad with its codes loaded straight from global memory. The wait for the previous phase
 // stands between what does not depend on it and the codes, which its infections change.
-template <bool kWait>
+template <typename Wait>
 __device__ __forceinline__ void demog_mosquito_quad(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
-                                                    QuadSmem& sm)
+                                                    QuadSmem& sm, Wait wait)
 {
     const QuadStart at = quad_start(d, key, q, lane, t, sm);
-    if (kWait) griddep_wait();
+    wait();
     uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
     if (q * kQuad + (lane >> 3) < d.tiles) A = reinterpret_cast<const uint4*>(d.m_code)[q * 32 + lane];
     mosquito_quad_core(d, key, q, lane, t, sm, at, A);
@@ -605,7 +640,7 @@ __global__ void __launch_bounds__(256, 6) k_demog(Dev d, uint32_t spread, uint32
     const uint32_t quads = (d.tiles + kQuad - 1) / kQuad, rows = (d.nvec + 32 * U - 1) / (32 * U);
     const uint32_t it = spread ? warp * gridDim.x + blockIdx.x : blockIdx.x * (blockDim.x >> 5) + warp;
     if (it < quads) {
-        demog_mosquito_quad<true>(d, key, it, lane, t, wsm[warp]);
+        demog_mosquito_quad(d, key, it, lane, t, wsm[warp], GridWait{});
     } else if (it - quads < rows) {
         griddep_wait();
         demog_humans<U>(d, key, (it - quads) * 32 * U + lane, 32, t, wsm[warp]);
@@ -655,8 +690,8 @@ __device__ __forceinline__ uint32_t checked_count(uint32_t x, uint32_t* bad)
 // that spread the events, the row stood between their counters and their events.
 __device__ __forceinline__ uint32_t series_chunks(uint32_t P) { return (P + 255) / 256; }
 
-template <bool kWait>
-__device__ __forceinline__ void foi_series(const Dev& d, uint32_t item, int collect_only, const StepAt& at)
+template <typename Wait>
+__device__ __forceinline__ void foi_series(const Dev& d, uint32_t item, int collect_only, const StepAt& at, Wait wait)
 {
     const uint32_t lane = threadIdx.x & 31u, S = d.S, P = d.P, chunks = series_chunks(P);
     const uint32_t s = item / chunks, c0 = (item - s * chunks) * 256 + lane;
@@ -666,7 +701,7 @@ __device__ __forceinline__ void foi_series(const Dev& d, uint32_t item, int coll
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k)
             if (c0 + 32 * k < P) humans += __ldg(&d.ncnt[c0 + 32 * k]);
-    if (kWait) griddep_wait();
+    wait();
     uint32_t ih[8], im[8], ic[8], mc[8];
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k) {
@@ -709,7 +744,7 @@ __device__ __forceinline__ void foi_series(const Dev& d, uint32_t item, int coll
 // the events of pair l mod 16 in one direction (below 16 human to mosquito, else mosquito to human);
 // then the 32 lanes spread the flattened events of the warp's 64 (lane, kind) entries, four per Philox
 // call. No block barrier: a warp is a chain of two dependent round trips and its draws, so the more warps
-// in flight the better. With kWait, the wait for the previous kernel stands between the loads of static
+// in flight the better. The wait for the previous phase stands between the loads of static
 // data and those of its results.
 constexpr uint32_t kFoiPairs = 16;
 
@@ -721,8 +756,8 @@ struct __align__(16) FoiWarpSmem {
     uint32_t pad[3];
 };
 
-template <bool kWait>
-__device__ __forceinline__ void foi_events(const Dev& d, uint32_t p0, const StepAt& at, FoiWarpSmem& sh)
+template <typename Wait>
+__device__ __forceinline__ void foi_events(const Dev& d, uint32_t p0, const StepAt& at, FoiWarpSmem& sh, Wait wait)
 {
     const uint32_t lane = threadIdx.x & 31u, SP = d.S * d.P, P = d.P;
     const uint32_t slot = lane & (kFoiPairs - 1), p = p0 + slot;
@@ -744,7 +779,7 @@ __device__ __forceinline__ void foi_events(const Dev& d, uint32_t p0, const Step
         }
         r = draw4(at.key, hm ? kFoiHM : kFoiMH, p, at.t);
     }
-    if (kWait) griddep_wait();
+    wait();
     uint32_t nlocal = 0, nfar = 0;
     if (valid) {
         uint32_t bad = 0;
@@ -801,12 +836,12 @@ __device__ __forceinline__ void foi_events(const Dev& d, uint32_t p0, const Step
 // Items of the pass of one simulation: the event items first, then those of the series row.
 __device__ __forceinline__ uint32_t foi_event_items(const Dev& d) { return (d.S * d.P + kFoiPairs - 1) / kFoiPairs; }
 
-template <bool kWait>
-__device__ __forceinline__ void foi_item(const Dev& d, uint32_t item, int collect_only, const StepAt& at, FoiWarpSmem& sh)
+template <typename Wait>
+__device__ __forceinline__ void foi_item(const Dev& d, uint32_t item, int collect_only, const StepAt& at, FoiWarpSmem& sh, Wait wait)
 {
     const uint32_t ev = foi_event_items(d);
-    if (item >= ev) foi_series<kWait>(d, item - ev, collect_only, at);
-    else if (!collect_only) foi_events<kWait>(d, kFoiPairs * item, at, sh);
+    if (item >= ev) foi_series(d, item - ev, collect_only, at, wait);
+    else if (!collect_only) foi_events(d, kFoiPairs * item, at, sh, wait);
 }
 
 // Warp w of block b takes item b * W + w, then every gridDim.x * W further (W = blockDim.x / 32; W
@@ -819,7 +854,7 @@ __global__ void __launch_bounds__(512) k_foi(Dev d, int collect_only, uint32_t k
     const uint32_t items = foi_event_items(d) + d.S * series_chunks(d.P);
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t g = blockIdx.x * W + warp; g < items; g += gridDim.x * W) foi_item<true>(d, g, collect_only, at, sh);
+    for (uint32_t g = blockIdx.x * W + warp; g < items; g += gridDim.x * W) foi_item(d, g, collect_only, at, sh, GridWait{});
 }
 
 // ------------------------------------------------------------------ infection draws
@@ -955,8 +990,8 @@ struct HeavyList {
 
 enum InfectBy : int { kByWarp = 0, kByWarpDefer = 1, kByBlock = 2 };
 
-template <bool kWait, bool kFew, int kBy>
-__device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh,
+template <bool kFew, int kBy, typename Wait>
+__device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh, Wait wait,
                                             HeavyList* heavy = nullptr, uint32_t inst = 0)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -979,12 +1014,7 @@ __device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const Step
     // One draw per lane in one pass: introduction counts (lanes < S), first serotypes (8, 9).
     const U4 rd = draw4(key, lane < S ? (uint32_t)kIntroCount : lane == 8 ? (uint32_t)kInfMStart : (uint32_t)kInfHStart,
                         lane < S ? pl : c, t);
-    if (kWait) {
-        griddep_wait();
-        // Only now may the next step's demographic pass be scheduled: before its own wait it reads the
-        // dead counts, which this step's pass (finished before the grid waited for) writes.
-        griddep_launch_dependents();
-    }
+    wait();
     const uint32_t mc = d.mcnt[c];
     uint32_t kh = lane < S ? d.transh[pl] : 0u;
     uint32_t km = lane < S ? d.transm[pl] : 0u;
@@ -1369,7 +1399,7 @@ __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_unit<true, true, kByWarp>(d, c, at, sh);
+    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_unit<true, kByWarp>(d, c, at, sh, GridWaitRelease{});
 }
 
 // ------------------------------------------------------------------ batched steps
@@ -1458,7 +1488,7 @@ __global__ void __launch_bounds__(256, 5) k_demog_batch(BatchDev bd, uint32_t ko
             const uint32_t t = d.ctrl->t + koff;
             const Key key = load_key(d.ctrl);
             if (local < hw) demog_humans<U>(d, key, local * 32 * U + lane, 32, t, wsm[warp]);
-            else demog_mosquito_quad<false>(d, key, local - hw, lane, t, wsm[warp]);
+            else demog_mosquito_quad(d, key, local - hw, lane, t, wsm[warp], NoWait{});
         }
     }
     griddep_launch_dependents();
@@ -1479,7 +1509,7 @@ __global__ void __launch_bounds__(512) k_foi_batch(BatchDev bd, int collect_only
     }
     griddep_launch_dependents();  // the infection kernel may be scheduled; it waits for this grid
     batch_warp_items<false>(bd, bd.foi_off, bd.foi_run, wdev, [&](const Dev& d, uint32_t item, uint32_t) {
-        foi_item<true>(d, item, collect_only, load_step(d.ctrl, koff), sh);
+        foi_item(d, item, collect_only, load_step(d.ctrl, koff), sh, GridWait{});
     });
 }
 
@@ -1499,7 +1529,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
     unsigned long long* wdev = descs + warp * (sizeof(Dev) / 8);
     if constexpr (!kHeavy) {
         batch_warp_items<false>(bd, bd.infect_off, bd.infect_run, wdev, [&](const Dev& d, uint32_t c, uint32_t) {
-            infect_unit<true, true, kByWarp>(d, c, load_step(d.ctrl, koff), tables[warp]);
+            infect_unit<true, kByWarp>(d, c, load_step(d.ctrl, koff), tables[warp], GridWaitRelease{});
         });
     } else {
         __shared__ HeavyList heavy;
@@ -1507,7 +1537,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
         __syncthreads();
         batch_warp_items<true>(bd, bd.infect_off, bd.infect_run, wdev, [&](const Dev& d, uint32_t c, uint32_t inst) {
             const StepAt at = load_step(d.ctrl, koff);
-            infect_unit<true, true, kByWarpDefer>(d, c, at, tables[warp], &heavy, inst);
+            infect_unit<true, kByWarpDefer>(d, c, at, tables[warp], GridWaitRelease{}, &heavy, inst);
         });
         __syncthreads();
         const uint32_t n = min(heavy.n, kHeavyList);
@@ -1517,7 +1547,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
             for (uint32_t j = threadIdx.x; j < sizeof(Dev) / 8; j += blockDim.x) descs[j] = src[j];
             __syncthreads();
             const Dev& d = *reinterpret_cast<const Dev*>(descs);
-            infect_unit<true, false, kByBlock>(d, h.y, load_step(d.ctrl, koff), tables[0]);
+            infect_unit<false, kByBlock>(d, h.y, load_step(d.ctrl, koff), tables[0], NoWait{});
         }
     }
 }
@@ -1538,11 +1568,6 @@ size_t foi_smem(uint32_t threads, bool batch)
 }
 
 // ------------------------------------------------------------------ many steps of small simulations
-
-__device__ __forceinline__ void cluster_barrier()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 __device__ __forceinline__ uint32_t cluster_rank()
 {
@@ -1565,8 +1590,15 @@ static_assert(kStepsSmem + sizeof(Dev) + 64 <= 48 * 1024, "shared memory of k_st
 // nothing from one another, so each cluster goes on by itself; the per-phase batch kernels wait for the
 // slowest simulation at each phase and hand out items through one counter, which with few items is all
 // latency: 32 simulations of 7e4 agents took 39 us a step, now 20, 8 of them 35 and 17. The bodies are
-// the per-phase kernels' own. Sixteen warps of 64 registers to a CTA, two CTAs to an SM.
-template <uint32_t B>
+// the per-phase kernels' own. Sixteen warps to a CTA and B CTAs to an SM (64 registers at two).
+//
+// Two forms. With few demographic items to a warp (kMany false) they go in a fixed order, and each phase's
+// first item does what does not depend on the phase before (draws, constant tables) before it waits for
+// that phase: 8 simulations of 7e4 agents 17.4 -> 16.8 us a step, 32 of them 21.5 -> 21.0. With many (items
+// are of uneven cost) a CTA's warps take its share of them from a counter: 128 of them 65.4 -> 62.8 us,
+// later 38.2 -> 36.1; half an item to a warp by the counter took 18.4 for 17.8. Both together, in one
+// kernel of 64 registers, took 64.5 and 37.5 on 128.
+template <uint32_t B, bool kMany>
 __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, uint32_t C, uint32_t nsteps)
 {
     extern __shared__ __align__(16) unsigned char steps_dyn[];
@@ -1586,28 +1618,48 @@ __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, 
     StepAt at = load_step(d.ctrl, 0);
     const uint32_t quads = (d.tiles + kQuad - 1) / kQuad, hw = (d.nvec + 31) / 32;
     const uint32_t foi = foi_event_items(d) + d.S * series_chunks(d.P);
-    // Demographic items are of uneven cost. With four or more to a warp a CTA's warps take its share of them
-    // from a counter (step of 128 simulations of 7e4 agents 65.4 -> 62.8 us, later 38.2 -> 36.1); with
-    // fewer the counter costs more than it evens out (8 of them, half an item to a warp: 17.8 -> 18.4).
-    const bool by_counter = quads + hw >= 4 * nw;
     for (uint32_t k = 0; k < nsteps; ++k, ++at.t, ++at.epoch) {
-        auto after = [&](uint32_t it) {
-            if (!by_counter) return it + nw;
-            uint32_t i = 0;
-            if (lane == 0) i = atomicAdd(&next[k & 1u], 1u);
-            return __shfl_sync(kFull, i, 0) * C + rank;
-        };
-        for (uint32_t it = by_counter ? after(0) : w; it < quads + hw; it = after(it)) {
-            if (it < quads) demog_mosquito_quad<false>(d, at.key, it, lane, at.t, scratch.demog);
-            else demog_humans<1>(d, at.key, (it - quads) * 32 + lane, 32, at.t, scratch.demog);
+        auto human = [&](uint32_t it) { demog_humans<1>(d, at.key, (it - quads) * 32 + lane, 32, at.t, scratch.demog); };
+        if constexpr (kMany) {
+            auto take = [&] {
+                uint32_t i = 0;
+                if (lane == 0) i = atomicAdd(&next[k & 1u], 1u);
+                return __shfl_sync(kFull, i, 0) * C + rank;
+            };
+            for (uint32_t it = take(); it < quads + hw; it = take()) {
+                if (it < quads) demog_mosquito_quad(d, at.key, it, lane, at.t, scratch.demog, NoWait{});
+                else human(it);
+            }
+            cluster_barrier();
+            if (threadIdx.x == 0) next[(k + 1) & 1u] = 0;
+            for (uint32_t g = w; g < foi; g += nw) foi_item(d, g, 0, at, scratch.foi, NoWait{});
+            cluster_barrier();
+            for (uint32_t c = w; c < d.P; c += nw) infect_unit<B == 1, kByWarp>(d, c, at, scratch.infect, NoWait{});
+            cluster_barrier();
+        } else {
+            bool pending = k > 0;
+            const PendingWait later{pending};
+            auto end_phase = [&] {
+                later();  // a warp without items has not waited for the phase before
+                cluster_arrive();
+                pending = true;
+            };
+            for (uint32_t it = w; it < quads + hw; it += nw) {
+                if (it < quads) {
+                    demog_mosquito_quad(d, at.key, it, lane, at.t, scratch.demog, later);
+                } else {
+                    later();
+                    human(it);
+                }
+            }
+            end_phase();
+            for (uint32_t g = w; g < foi; g += nw) foi_item(d, g, 0, at, scratch.foi, later);
+            end_phase();
+            for (uint32_t c = w; c < d.P; c += nw) infect_unit<B == 1, kByWarp>(d, c, at, scratch.infect, later);
+            end_phase();
         }
-        cluster_barrier();
-        if (threadIdx.x == 0) next[(k + 1) & 1u] = 0;
-        for (uint32_t g = w; g < foi; g += nw) foi_item<false>(d, g, 0, at, scratch.foi);
-        cluster_barrier();
-        for (uint32_t c = w; c < d.P; c += nw) infect_unit<false, B == 1, kByWarp>(d, c, at, scratch.infect);
-        cluster_barrier();
     }
+    if (!kMany && nsteps) cluster_wait();
     if (rank == 0 && threadIdx.x == 0) {
         d.ctrl->t = at.t;
         d.ctrl->epoch = at.epoch;
@@ -2166,21 +2218,30 @@ static uint32_t largest_cluster(StepsKernel k, uint32_t n)
 }
 
 // CTAs that have an SM each keep 128 registers a thread; two to an SM have 64.
-static StepsKernel steps_kernel(uint32_t per_sm) { return per_sm == 1 ? k_steps<1> : k_steps<2>; }
+static StepsKernel steps_kernel(uint32_t per_sm, bool many)
+{
+    if (many) return per_sm == 1 ? k_steps<1, true> : k_steps<2, true>;
+    return per_sm == 1 ? k_steps<1, false> : k_steps<2, false>;
+}
 
 uint32_t steps_cluster(uint32_t n, uint32_t* per_sm)
 {
-    const uint32_t one = largest_cluster(k_steps<1>, n), two = largest_cluster(k_steps<2>, n);
+    // The larger of the two forms, so that either fits (each sets its own attribute).
+    const uint32_t one = std::min(largest_cluster(k_steps<1, false>, n), largest_cluster(k_steps<1, true>, n));
+    const uint32_t two = std::min(largest_cluster(k_steps<2, false>, n), largest_cluster(k_steps<2, true>, n));
     *per_sm = one && one >= two ? 1u : 2u;
     return one && one >= two ? one : two;
 }
 
-int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t per_sm, uint32_t nsteps, void* stream)
+int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t per_sm, uint64_t items, uint32_t nsteps,
+                 void* stream)
 {
+    const bool many = items >= 4ull * n * C * kStepsWarps;
+
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = steps_config(n, C, &attr);
     cfg.stream = (cudaStream_t)stream;
-    return (int)cudaLaunchKernelEx(&cfg, steps_kernel(per_sm), devs, C, nsteps);
+    return (int)cudaLaunchKernelEx(&cfg, steps_kernel(per_sm, many), devs, C, nsteps);
 }
 
 int launch_advance_batch(const BatchDev& bd, uint32_t n, void* stream)
