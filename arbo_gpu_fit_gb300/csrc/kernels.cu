@@ -918,7 +918,7 @@ __device__ __forceinline__ uint32_t mosquito_target(const Dev& d, const Key& key
 // Per-warp tables of the infection pass: one community and its events of every serotype
 // flattened into one index space.
 constexpr uint32_t kIntroScan = 1024;   // humans of a community up to which failed introductions look at all of them
-constexpr uint32_t kFewItems = 32;
+constexpr uint32_t kFewEvents = 32;
 // Items past which a block of a batch works off a community together. Infection phase of 64 uneven
 // instances of a heavy epidemic (2.3e5 human infections a step) at 64, 128, 256 and 512: 369, 353, 340 and
 // 415 us, of 16 smaller ones 32, 29, 33 and 41.
@@ -929,8 +929,8 @@ constexpr uint32_t kTargetCache = 128;  // items whose targets Phase A keeps for
 struct InfectWarpSmem {
     union {
         uint4 target[kTargetCache];     // per item: four human targets, or a mosquito slot in .x
-        uint2 bid[128];                 // of up to 32 items: eligible events, {target (mosquito slots with
-                                        // bit 31), low word of the order key}
+        uint2 bid[kFewEvents];          // of few events the eligible ones: {target (mosquito slots with bit
+                                        // 31), serotype position}
     };
     // First item of each serotype position and events by position, humans (groups of four) and
     // mosquitoes; positions past the last serotype start at UINT_MAX.
@@ -961,11 +961,14 @@ __device__ __forceinline__ uint32_t wrap(uint32_t x, uint32_t n) { return x >= n
 // Infection draws of community c, by one warp. Lanes 0..S-1 read the community's event counts
 // and draw its introduction counts, lanes 8 and 9 the first serotypes; the events (groups of
 // four human events, single mosquito events) then form one index space walked by the 32 lanes:
-// Up to 32 items (kFew), which is most communities in most steps, the warp resolves among its lanes: every
-// lane loads all that its event may need in one round trip, the eligible events are listed in shared
-// memory, and an event holds its target if no listed one with a smaller serial order has the same. The
-// two round trips that the bids in memory cost are gone: infection pass of 5e4 agents 5.1 -> 3.6 us, of
-// 7e6 9.1 -> 6.6. It takes 126 registers, so clusters that share SMs (64 registers) go without it.
+// Up to 32 events, which is most communities in most steps, the warp resolves among its lanes, one event to
+// a lane: every lane loads all that its event may need in one round trip, and the eligible events on a
+// target are found by matching the lanes' targets; lanes are in serial order, so the lowest one holds it.
+// The two round trips that the bids in memory cost are gone: infection pass of 5e4 agents 5.1 -> 3.6 us, of
+// 7e6 9.1 -> 6.6. One item (four human events) to a lane, which covers more of them, took twice the
+// registers: 64 leave twice the warps in flight in batches (phase of 512 instances of 7e4 agents 104 -> 90
+// us, of 64 uneven ones 228 -> 200) and fit the clusters that share SMs, which had gone without (step of
+// 128 such instances 63.4 -> 56.3 us at the peak, of 32 21.0 -> 19.8, of 8 16.9 -> 15.2).
 // More items go through the targets' winner keys in memory, three phases:
 //   A: every event whose target is eligible at the start of the pass bids its serial order
 //      (serotype position j, event index) for the target with atomicMin; the targets of the first
@@ -990,10 +993,11 @@ struct HeavyList {
 
 enum InfectBy : int { kByWarp = 0, kByWarpDefer = 1, kByBlock = 2 };
 
-template <bool kFew, int kBy, typename Wait>
+template <int kBy, typename Wait>
 __device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const StepAt& at, InfectWarpSmem& sh, Wait wait,
                                             HeavyList* heavy = nullptr, uint32_t inst = 0)
 {
+    constexpr bool kFew = kBy != kByBlock;  // may find few events
     const uint32_t lane = threadIdx.x & 31u;
     const bool lead = kBy != kByBlock || threadIdx.x < 32;
     const uint32_t gl = kBy == kByBlock ? threadIdx.x : lane, gt = kBy == kByBlock ? blockDim.x : 32u;
@@ -1039,18 +1043,21 @@ __device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const Step
     const uint32_t hs = wrap(s0h + (lane & 7u), S), ms_ = wrap(s0m + (lane & 7u), S);
     uint32_t khj = __shfl_sync(kFull, kh, hs), kmj = __shfl_sync(kFull, km, ms_), nej = __shfl_sync(kFull, ne, hs);
     if (lane >= S) khj = kmj = nej = 0;
-    uint32_t hi = (khj + 3) >> 2, mi = kmj;
+    uint32_t hi = (khj + 3) >> 2, mi = kmj, he = khj;  // groups of human events, mosquito events, human events
     const uint32_t h0 = hi, m0 = mi;
 #pragma unroll
     for (int off = 1; off < 8; off <<= 1) {
         const uint32_t y = __shfl_up_sync(kFull, hi, off), x = __shfl_up_sync(kFull, mi, off);
+        const uint32_t z = kFew ? __shfl_up_sync(kFull, he, off) : 0u;
         if (lane >= (uint32_t)off) {
             hi += y;
             mi += x;
+            he += z;
         }
     }
     const uint32_t H = __shfl_sync(kFull, hi, 7), Mt = __shfl_sync(kFull, mi, 7);
-    const uint32_t items = H + Mt;
+    const uint32_t items = H + Mt, Hev = kFew ? __shfl_sync(kFull, he, 7) : 0u;
+    const bool few = kFew && Hev + Mt <= kFewEvents;
     if (kBy == kByWarpDefer && items > kHeavyItems) {
         uint32_t i = 0;
         if (lane == 0) {
@@ -1063,7 +1070,7 @@ __device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const Step
     if (lead && had_h) d.transh[pl] = 0;
     if (lead && had_m) d.transm[pl] = 0;
     if (lead && lane < 8) {
-        reinterpret_cast<uint32_t*>(sh.hstart)[lane] = lane < S ? hi - h0 : UINT_MAX;
+        reinterpret_cast<uint32_t*>(sh.hstart)[lane] = lane < S ? (few ? he - khj : hi - h0) : UINT_MAX;
         reinterpret_cast<uint32_t*>(sh.mstart)[lane] = lane < S ? mi - m0 : UINT_MAX;
         sh.kh[lane] = khj;
         sh.km[lane] = kmj;
@@ -1170,110 +1177,75 @@ __device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const Step
             if (left > 0 && lane == 0) atomicAdd(&d.ctrl->diag[1], 1u);
         }
     };
-    if (kFew && items <= kFewItems) {
-        // One item per lane.
-        const bool act = lane < items, hum = lane < H;
-        uint32_t idx = 0, sp = 0, pp = 0, j = 0, elig = 0, k = 0;
-        uint32_t tg[4] = {0, 0, 0, 0}, im[4] = {0, 0, 0, 0};
-        int32_t bn[4] = {0, 0, 0, 0}, dt[4] = {0, 0, 0, 0};
-        U4 rx;  // exposed-age draw of the lane's first human event, or of its mosquito event
+    if (few) {
+        // One event per lane.
+        const bool act = lane < Hev + Mt, hum = lane < Hev;
+        uint32_t idx = 0, sp = 0, pp = 0, tg = 0, j = 0, im = 0;
+        int32_t bn = 0, dt = 0;
+        bool elig = false;
+        U4 rx;  // exposed-age draw
         if (act) {
-            j = item_position(hum ? sh.hstart : sh.mstart, hum ? lane : lane - H, &idx);
+            j = item_position(hum ? sh.hstart : sh.mstart, hum ? lane : lane - Hev, &idx);
             sp = wrap((hum ? s0h : s0m) + j, S);
             pp = sp * P + c;
-            k = hum ? min(sh.kh[j] - 4 * idx, 4u) : min(d.maxTarget, 4u);  // targets or attempts of the lane
-            const U4 r = draw4(key, hum ? (uint32_t)kInfHTarget : (uint32_t)kInfMTarget, pp, t, idx);
+            const U4 r = draw4(key, hum ? (uint32_t)kInfHTarget : (uint32_t)kInfMTarget, pp, t, hum ? idx >> 2 : idx);
             // Both kinds of event load alike, so that they wait together: a human's status, immunity, birth
-            // and death time, a mosquito slot's code, status, birth and death time.
-            const uint8_t *pa = hum ? d.n_status : d.m_code, *pb = hum ? d.n_imm : d.m_stat;
-            const int32_t *pc = hum ? d.n_born : &d.m_life->born, *pd = hum ? d.n_dtime : &d.m_life->dtime;
+            // and death time, a mosquito slot's code, status, birth and death time; of the slots of a
+            // mosquito event's further attempts, which few events get to, the codes.
+            const uint32_t base = hum ? nbase : mbase, size = hum ? ns : ms;
+            tg = base + bounded(hum ? pick4(r, idx & 3u) : r.v[0], size);
             const uint32_t step = hum ? 1u : sizeof(Life) / 4;
-            uint32_t st[4];
+            uint32_t st[4] = {kDead, kDead, kDead, kDead};
+            if (hum || d.maxTarget) st[0] = (hum ? d.n_status : d.m_code)[tg];
+            im = (hum ? d.n_imm : d.m_stat)[tg];
+            bn = (hum ? d.n_born : &d.m_life->born)[(size_t)tg * step];
+            dt = (hum ? d.n_dtime : &d.m_life->dtime)[(size_t)tg * step];
 #pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                tg[q] = (hum ? nbase : mbase) + bounded(r.v[q], hum ? ns : ms);
-                st[q] = kDead;
-                if (q < k) {
-                    st[q] = pa[tg[q]];
-                    im[q] = pb[tg[q]];
-                    bn[q] = pc[(size_t)tg[q] * step];
-                    dt[q] = pd[(size_t)tg[q] * step];
-                }
-            }
-            rx = draw4(key, hum ? (uint32_t)kInfHExposed : (uint32_t)kInfMExposed, pp, t, hum ? 4 * idx : idx >> 2);
+            for (uint32_t q = 1; q < 4; ++q)
+                if (!hum && q < d.maxTarget) st[q] = d.m_code[mbase + bounded(r.v[q], ms)];
+            rx = draw4(key, hum ? (uint32_t)kInfHExposed : (uint32_t)kInfMExposed, pp, t, hum ? idx : idx >> 2);
             if (hum) {
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q)
-                    if (st[q] == 0 && !((im[q] >> sp) & 1u)) elig |= 1u << q;
+                elig = st[0] == 0 && !((im >> sp) & 1u);
             } else {
-                uint32_t slot = UINT_MAX, state = 0;
-                int32_t born = 0, dies = 0;
+                uint32_t state = im & 3u;
+                if (st[0] & kDead) {
+                    tg = UINT_MAX;
 #pragma unroll
-                for (int q = 3; q >= 0; --q)
-                    if (!(st[q] & kDead)) {
-                        slot = tg[q];
-                        state = im[q] & 3u;
-                        born = bn[q];
-                        dies = dt[q];
-                    }
-                if (slot == UINT_MAX) {
-                    slot = mosquito_target(d, key, pp, idx, mbase, ms, t, &state, r, 4);
-                    if (slot == UINT_MAX) atomicAdd(&d.ctrl->diag[0], 1u);
-                    else {
-                        born = d.m_life[slot].born;
-                        dies = d.m_life[slot].dtime;
+                    for (int q = 3; q >= 1; --q)
+                        if (!(st[q] & kDead)) tg = mbase + bounded(r.v[q], ms);
+                    if (tg == UINT_MAX) tg = mosquito_target(d, key, pp, idx, mbase, ms, t, &state, r, 4);
+                    if (tg == UINT_MAX) {
+                        atomicAdd(&d.ctrl->diag[0], 1u);
+                    } else {
+                        state = d.m_stat[tg] & 3u;
+                        bn = d.m_life[tg].born;
+                        dt = d.m_life[tg].dtime;
                     }
                 }
-                bn[0] = born;
-                dt[0] = dies;
-                tg[0] = slot | 0x80000000u;
-                if (slot != UINT_MAX && state == 0) elig = 1;
+                elig = tg != UINT_MAX && state == 0;
+                tg |= 0x80000000u;
             }
         }
-        // The eligible events, and of them the first in serial order on each target.
-        uint32_t nb = 0;
-#pragma unroll
-        for (uint32_t q = 0; q < 4; ++q) {
-            const unsigned bal = __ballot_sync(kFull, (elig >> q) & 1u);
-            if ((elig >> q) & 1u)
-                sh.bid[nb + __popc(bal & ((1u << lane) - 1u))] =
-                    make_uint2(tg[q], (uint32_t)order_key(0, j, 0, hum ? 4 * idx + q : idx));
-            nb += __popc(bal);
-        }
-        __syncwarp();
-        uint32_t won = elig;
-        if (nb > 1)
-            for (uint32_t b = 0; b < nb; ++b) {
-                const uint2 x = sh.bid[b];
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q)
-                    if (x.x == tg[q] && x.y < (uint32_t)order_key(0, j, 0, hum ? 4 * idx + q : idx)) won &= ~(1u << q);
-            }
-        if (intro)
+        // Lanes are in serial order within a species, so of the eligible events on a target the lowest lane
+        // holds it.
+        const unsigned open_events = __ballot_sync(kFull, elig);
+        const unsigned same = __match_any_sync(kFull, tg) & open_events;
+        bool won = elig && __ffs(same) - 1 == (int)lane;
+        if (intro) {
+            const uint32_t nb = __popc(open_events);
+            if (elig) sh.bid[__popc(open_events & ((1u << lane) - 1u))] = make_uint2(tg, j);
+            __syncwarp();
             introductions(
-                [&](uint32_t i, uint32_t jj, uint32_t a) {
-                    bool open = true;
-                    for (uint32_t b = 0; b < nb; ++b) open &= sh.bid[b].x != i || sh.bid[b].y > (uint32_t)order_key(0, jj, 1, a);
+                [&](uint32_t i, uint32_t jj, uint32_t) {
+                    bool open = true;  // no event of this position or an earlier one is on i
+                    for (uint32_t b = 0; b < nb; ++b) open &= sh.bid[b].x != i || sh.bid[b].y > jj;
                     return open;
                 },
-                [&](uint32_t i, uint32_t, uint32_t) {
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        if (tg[q] == i) won &= ~(1u << q);
-                });
-        if (won && !hum) {
-            infect_mosquito(d, tg[0] & 0x7FFFFFFFu, sp, pick4(rx, idx & 3u), t, bn[0], dt[0]);
-        } else {
-            while (won) {
-                const uint32_t q = __ffs(won) - 1;
-                won &= won - 1;
-                const uint32_t tq = q == 0 ? tg[0] : q == 1 ? tg[1] : q == 2 ? tg[2] : tg[3];
-                const uint32_t iq = q == 0 ? im[0] : q == 1 ? im[1] : q == 2 ? im[2] : im[3];
-                const int32_t bq = q == 0 ? bn[0] : q == 1 ? bn[1] : q == 2 ? bn[2] : bn[3];
-                const int32_t dq = q == 0 ? dt[0] : q == 1 ? dt[1] : q == 2 ? dt[2] : dt[3];
-                if (q) rx = draw4(key, kInfHExposed, pp, t, 4 * idx + q);
-                infect_human(d, tq, sp, rx, t, iq, bq, dq);
-            }
+                [&](uint32_t i, uint32_t, uint32_t) { won = won && tg != i; });
+        }
+        if (won) {
+            if (hum) infect_human(d, tg, sp, rx, t, im, bn, dt);
+            else infect_mosquito(d, tg & 0x7FFFFFFFu, sp, pick4(rx, idx & 3u), t, bn, dt);
         }
         __syncwarp();  // the warp's tables are reused for its next community
         return;
@@ -1399,7 +1371,7 @@ __global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_unit<true, kByWarp>(d, c, at, sh, GridWaitRelease{});
+    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_unit<kByWarp>(d, c, at, sh, GridWaitRelease{});
 }
 
 // ------------------------------------------------------------------ batched steps
@@ -1529,7 +1501,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
     unsigned long long* wdev = descs + warp * (sizeof(Dev) / 8);
     if constexpr (!kHeavy) {
         batch_warp_items<false>(bd, bd.infect_off, bd.infect_run, wdev, [&](const Dev& d, uint32_t c, uint32_t) {
-            infect_unit<true, kByWarp>(d, c, load_step(d.ctrl, koff), tables[warp], GridWaitRelease{});
+            infect_unit<kByWarp>(d, c, load_step(d.ctrl, koff), tables[warp], GridWaitRelease{});
         });
     } else {
         __shared__ HeavyList heavy;
@@ -1537,7 +1509,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
         __syncthreads();
         batch_warp_items<true>(bd, bd.infect_off, bd.infect_run, wdev, [&](const Dev& d, uint32_t c, uint32_t inst) {
             const StepAt at = load_step(d.ctrl, koff);
-            infect_unit<true, kByWarpDefer>(d, c, at, tables[warp], GridWaitRelease{}, &heavy, inst);
+            infect_unit<kByWarpDefer>(d, c, at, tables[warp], GridWaitRelease{}, &heavy, inst);
         });
         __syncthreads();
         const uint32_t n = min(heavy.n, kHeavyList);
@@ -1547,7 +1519,7 @@ __global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff
             for (uint32_t j = threadIdx.x; j < sizeof(Dev) / 8; j += blockDim.x) descs[j] = src[j];
             __syncthreads();
             const Dev& d = *reinterpret_cast<const Dev*>(descs);
-            infect_unit<false, kByBlock>(d, h.y, load_step(d.ctrl, koff), tables[0], NoWait{});
+            infect_unit<kByBlock>(d, h.y, load_step(d.ctrl, koff), tables[0], NoWait{});
         }
     }
 }
@@ -1634,7 +1606,7 @@ __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, 
             if (threadIdx.x == 0) next[(k + 1) & 1u] = 0;
             for (uint32_t g = w; g < foi; g += nw) foi_item(d, g, 0, at, scratch.foi, NoWait{});
             cluster_barrier();
-            for (uint32_t c = w; c < d.P; c += nw) infect_unit<B == 1, kByWarp>(d, c, at, scratch.infect, NoWait{});
+            for (uint32_t c = w; c < d.P; c += nw) infect_unit<kByWarp>(d, c, at, scratch.infect, NoWait{});
             cluster_barrier();
         } else {
             bool pending = k > 0;
@@ -1655,7 +1627,7 @@ __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, 
             end_phase();
             for (uint32_t g = w; g < foi; g += nw) foi_item(d, g, 0, at, scratch.foi, later);
             end_phase();
-            for (uint32_t c = w; c < d.P; c += nw) infect_unit<B == 1, kByWarp>(d, c, at, scratch.infect, later);
+            for (uint32_t c = w; c < d.P; c += nw) infect_unit<kByWarp>(d, c, at, scratch.infect, later);
             end_phase();
         }
     }
