@@ -1365,14 +1365,22 @@ __device__ __forceinline__ void infect_unit(const Dev& d, uint32_t c, const Step
 
 // One warp per community: warp w of block b takes communities b*K + w (per-warp tables in dynamic shared
 // memory).
-__global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff)
+__device__ __forceinline__ void infect_communities(const Dev& d, uint32_t koff)
 {
     extern __shared__ __align__(16) unsigned char infect_dyn[];
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
     InfectWarpSmem& sh = reinterpret_cast<InfectWarpSmem*>(infect_dyn)[warp];
     const StepAt at = load_step(d.ctrl, koff);
-    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K) infect_unit<kByWarp>(d, c, at, sh, GridWaitRelease{});
+    for (uint32_t c = blockIdx.x * K + warp; c < d.P; c += gridDim.x * K)
+        infect_unit<kByWarp>(d, c, at, sh, GridWaitRelease{});
 }
+
+// Few communities to an SM: the shortest chain per warp (116 registers). Many: 80 registers, so that more
+// warps are in flight and the next kernels' blocks find room beside them. Step with the first and the
+// second: 100 communities 10.2 and 10.35 us, 400 10.8 and 10.9, 900 11.65 and 11.4, 2,500 18.65 and 18.6,
+// 3,969 38.4 and 37.7.
+__global__ void __launch_bounds__(512) k_infect(Dev d, uint32_t koff) { infect_communities(d, koff); }
+__global__ void __maxnreg__(80) k_infect_many(Dev d, uint32_t koff) { infect_communities(d, koff); }
 
 // ------------------------------------------------------------------ batched steps
 
@@ -1491,8 +1499,10 @@ __global__ void __launch_bounds__(512) k_foi_batch(BatchDev bd, int collect_only
 // some 4 us, and neighbouring runs, mostly of one instance with many events or with few, go to different
 // blocks. 64 uneven instances (1.9e8 agents) in the steps of a heavy epidemic: phase 631 -> 202, 896 -> 270
 // and 775 -> 288 us; with few events 79 -> 85, and 24 such instances 38 -> 41.
+// 80 registers; phase of 512 instances of 7e4 agents and of 24 uneven ones at 64, 72, 80 and 96: 90, 82, 79
+// and 84 us, 40, 37, 35 and 39.
 template <bool kHeavy>
-__global__ void __launch_bounds__(512) k_infect_batch(BatchDev bd, uint32_t koff)
+__global__ void __maxnreg__(80) k_infect_batch(BatchDev bd, uint32_t koff)
 {
     extern __shared__ __align__(16) unsigned char infect_dyn[];
     const uint32_t warp = threadIdx.x >> 5, K = blockDim.x >> 5;
@@ -2023,14 +2033,20 @@ int launch_foi(const Dev& d, const Launch& l, cudaStream_t st, int collect_only,
                       l.pdl && !collect_only, d, collect_only, koff);
 }
 
+typedef void (*InfectKernel)(Dev, uint32_t);
+static InfectKernel infect_kernel(uint32_t P, const Launch& l)
+{
+    return P >= 4 * (l.numSM ? l.numSM : 152u) ? k_infect_many : k_infect;
+}
+
 int launch_infect(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
 {
     const uint32_t per = l.infectBlock / 32;
     uint32_t blocks = cdiv(d.P, per);
     const uint32_t cap = 16u * (l.numSM ? l.numSM : 152u);
     if (blocks > cap) blocks = cap;
-    return launch_pdl(k_infect, dim3(blocks), dim3(l.infectBlock), infect_smem(l.infectBlock, false), st, l.pdl != 0, d,
-                      koff);
+    return launch_pdl(infect_kernel(d.P, l), dim3(blocks), dim3(l.infectBlock), infect_smem(l.infectBlock, false), st,
+                      l.pdl != 0, d, koff);
 }
 
 int launch_init(const Dev& d, const Launch& l, void* stream)
@@ -2070,7 +2086,7 @@ int share_carveout()
 {
     const int pct = 44;  // 100 KB of 228: five blocks of the demographic kernel, and 128 KB of L1
     const void* f[] = {(const void*)k_demog<1>, (const void*)k_demog<2>, (const void*)k_demog<4>, (const void*)k_foi,
-                       (const void*)k_infect};
+                       (const void*)k_infect, (const void*)k_infect_many};
     for (const void* k : f) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
         if (e != cudaSuccess) return (int)e;
@@ -2094,6 +2110,7 @@ int preload_step_kernels(const Launch& l)
                                  : cudaFuncGetAttributes(&a, k_demog<1>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_foi);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_infect);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_infect_many);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_advance);
     return (int)e;
 }
