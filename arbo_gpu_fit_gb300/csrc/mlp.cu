@@ -73,7 +73,8 @@ struct GemmLaunch {
     // Operand ring: stages of `group` K chunks; columns of one tensor-memory accumulator.
     uint32_t stages, group, stage_size, acc_cols;
     ColumnSums cs;
-    uint32_t* err;  // bit 0: an mbarrier wait ran out
+    uint32_t* err;       // bit 0: an mbarrier wait ran out
+    uint32_t* host_err;  // the same in host memory, or null
 };
 
 constexpr uint32_t kTileM = 128, kTileK = 64, kMaxStages = 8;
@@ -422,7 +423,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
         griddep_wait();
         column_sums(p.cs, blockIdx.x * 2 + (warp - 2 - kEpiWarps), gridDim.x * 2, lane);
     }
-    if (!ok) atomicOr(p.err, 1u);
+    if (!ok) {
+        atomicOr(p.err, 1u);
+        if (p.host_err) *(volatile uint32_t*)p.host_err = 1u;
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -514,8 +518,8 @@ void choose_tiles(const GemmArgs* g, uint32_t n, uint32_t num_sm, uint32_t (&tn)
 // Launches one or two independent products (g[i]: C = A B^T with its epilogue) and optional column
 // sums on persistent CTAs, at most one per SM. Returns a cudaError_t (invalid value when a tensor map
 // cannot be built; the reason is then in arbo_last_error).
-int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* err, cudaStream_t st, uint32_t num_sm,
-                bool pdl)
+int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* err, uint32_t* host_err, cudaStream_t st,
+                uint32_t num_sm, bool pdl)
 {
     GemmLaunch p{};
     uint32_t nk = 0;
@@ -535,6 +539,7 @@ int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* e
                          (nk + p.group - 1) / p.group * (p.tiles[0] + p.tiles[1] > num_sm ? 2u : 1u)});
     p.cs = cs;
     p.err = err;
+    p.host_err = host_err;
     // CTAs without a tile only add column sums (four columns each pass).
     const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 3) / 4), num_sm);
     return launch_pdl(k_gemm_tn, dim3(ctas), dim3(kGemmThreads),
@@ -652,7 +657,8 @@ struct arbo_mlp {
     uint32_t num_sm = 152;
     AdamArray* adam = nullptr;         // device table of the optimiser's arrays
     uint32_t adam_arrays = 0, adam_blocks = 0;
-    // What the host reads back every call: loss and error word, device (adjacent) and pinned.
+    // Pinned: the loss and error word as copied back after a training pass; an error word that the products
+    // themselves write, for predictions, which copy nothing else back.
     uint32_t* back = nullptr;
     cudaEvent_t done = nullptr;
     // Captured kernel sequences of the row counts in use. A row count is launched directly the first
@@ -705,7 +711,7 @@ int mlp_forward(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
             g.epi = kEpiLinear;
             g.outf = n->y;
         }
-        e = gemm_launch(&g, 1, ColumnSums{}, n->err, st, n->num_sm, true);
+        e = gemm_launch(&g, 1, ColumnSums{}, n->err, &n->back[2], st, n->num_sm, true);
     }
     return e;
 }
@@ -744,7 +750,7 @@ int mlp_backward(arbo_mlp* n, uint32_t rows, cudaStream_t st)
             g[0].outt = ndt;
             g[0].ldot = ld;
         }
-        e = gemm_launch(g, l > 0 ? 2 : 1, ColumnSums{dzt, ld, rows, out, n->db[l]}, n->err, st, n->num_sm, true);
+        e = gemm_launch(g, l > 0 ? 2 : 1, ColumnSums{dzt, ld, rows, out, n->db[l]}, n->err, &n->back[2], st, n->num_sm, true);
         std::swap(dz, nd);
         std::swap(dzt, ndt);
     }
@@ -809,10 +815,10 @@ int mlp_read_back(arbo_mlp* n, cudaStream_t st)
     return ARBO_OK;
 }
 
-int mlp_check_err(arbo_mlp* n)
+int mlp_check_err(arbo_mlp* n, uint32_t word)
 {
     UCUDA(cudaEventSynchronize(n->done));
-    const uint32_t e = n->back[1];
+    const uint32_t e = n->back[word];
     if (e) return ufail(ARBO_ERR_CUDA, "tensor-core product: an mbarrier wait ran out (error word " + std::to_string(e) + ")");
     return ARBO_OK;
 }
@@ -918,11 +924,12 @@ int arbo_mlp_create(uint32_t n_in, uint32_t hidden, uint32_t hidden_layers, uint
     n->tin = F((size_t)B * n_out);
     n->loss = F(2);  // and the error word beside it
     n->err = (uint32_t*)n->loss + 1;
-    if (!okm || cudaMallocHost(&n->back, 8) != cudaSuccess ||
+    if (!okm || cudaMallocHost(&n->back, 16) != cudaSuccess ||
         cudaEventCreateWithFlags(&n->done, cudaEventDisableTiming) != cudaSuccess) {
         arbo_mlp_destroy(n);
         return ufail(ARBO_ERR_ALLOC, "arbo_mlp_create: device allocation failed");
     }
+    std::memset(n->back, 0, 16);
     std::vector<AdamArray> arrays;
     for (uint32_t l = 0; l < n->L; ++l) {
         const uint32_t in = n->dim[l], o = n->dim[l + 1];
@@ -980,8 +987,8 @@ int arbo_mlp_forward(arbo_mlp* n, const float* x, uint32_t rows, float* y, void*
     } else {
         UCUDA(cudaMemcpy2DAsync(y, n->nout * 4, n->y, w * 4, n->nout * 4, rows, cudaMemcpyDeviceToHost, st));
     }
-    if ((e = mlp_read_back(n, st))) return e;
-    return mlp_check_err(n);
+    UCUDA(cudaEventRecord(n->done, st));
+    return mlp_check_err(n, 2);
 }
 
 int arbo_mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t rows, float* loss, void* stream)
@@ -989,7 +996,7 @@ int arbo_mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t row
     if (!n || !x || !t) return ufail(ARBO_ERR_INVALID, "null argument");
     UCUDA(cudaSetDevice(n->device));
     int e = mlp_gradients(n, x, t, rows, (cudaStream_t)stream);
-    if (!e) e = mlp_check_err(n);
+    if (!e) e = mlp_check_err(n, 1);
     if (!e && loss) std::memcpy(loss, &n->back[0], 4);
     return e;
 }
@@ -1007,7 +1014,7 @@ int arbo_mlp_train_step(arbo_mlp* n, const float* x, const float* t, uint32_t ro
     const float c1 = 1.0f - std::pow(b1, step), c2 = 1.0f - std::pow(b2, step);
     k_adam<<<n->adam_blocks, 256, 0, st>>>(n->adam, n->adam_arrays, lr, b1, b2, eps, c1, c2, n->err);
     UCUDA(cudaGetLastError());
-    if ((e = mlp_check_err(n))) return e;
+    if ((e = mlp_check_err(n, 1))) return e;
     n->steps += 1;
     if (loss) std::memcpy(loss, &n->back[0], 4);
     return ARBO_OK;
@@ -1085,7 +1092,7 @@ int arbo_tc_gemm(const float* a, const float* b, uint32_t M, uint32_t N, uint32_
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    auto product = [&]() { return gemm_launch(&g, 1, ColumnSums{}, derr, nullptr, (uint32_t)sms, false); };
+    auto product = [&]() { return gemm_launch(&g, 1, ColumnSums{}, derr, nullptr, nullptr, (uint32_t)sms, false); };
     int le = product();
     const std::string map_err = le ? std::string(arbo_last_error()) : std::string();
     cudaEventRecord(e0);
