@@ -75,6 +75,8 @@ struct GemmLaunch {
     ColumnSums cs;
     uint32_t* err;       // bit 0: an mbarrier wait ran out
     uint32_t* host_err;  // the same in host memory, or null
+    const float* loss;   // if not null, a finished loss and where in host memory it goes
+    float* host_loss;
 };
 
 constexpr uint32_t kTileM = 128, kTileK = 64, kMaxStages = 8;
@@ -421,6 +423,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
         }
     } else if (warp >= 2 + kEpiWarps && p.cs.cols) {
         griddep_wait();
+        if (p.loss && blockIdx.x == 0 && warp == 2 + kEpiWarps && lane == 0) *(volatile float*)p.host_loss = __ldcg(p.loss);
         column_sums(p.cs, blockIdx.x * 2 + (warp - 2 - kEpiWarps), gridDim.x * 2, lane);
     }
     if (!ok) {
@@ -519,7 +522,7 @@ void choose_tiles(const GemmArgs* g, uint32_t n, uint32_t num_sm, uint32_t (&tn)
 // sums on persistent CTAs, at most one per SM. Returns a cudaError_t (invalid value when a tensor map
 // cannot be built; the reason is then in arbo_last_error).
 int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* err, uint32_t* host_err, cudaStream_t st,
-                uint32_t num_sm, bool pdl)
+                uint32_t num_sm, bool pdl, const float* loss = nullptr, float* host_loss = nullptr)
 {
     GemmLaunch p{};
     uint32_t nk = 0;
@@ -540,6 +543,8 @@ int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* e
     p.cs = cs;
     p.err = err;
     p.host_err = host_err;
+    p.loss = loss;
+    p.host_loss = host_loss;
     // CTAs without a tile only add column sums (four columns each pass).
     const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 3) / 4), num_sm);
     return launch_pdl(k_gemm_tn, dim3(ctas), dim3(kGemmThreads),
@@ -657,8 +662,7 @@ struct arbo_mlp {
     uint32_t num_sm = 152;
     AdamArray* adam = nullptr;         // device table of the optimiser's arrays
     uint32_t adam_arrays = 0, adam_blocks = 0;
-    // Pinned: the loss and error word as copied back after a training pass; an error word that the products
-    // themselves write, for predictions, which copy nothing else back.
+    // Pinned: loss and error word, written by the products.
     uint32_t* back = nullptr;
     cudaEvent_t done = nullptr;
     // Captured kernel sequences of the row counts in use. A row count is launched directly the first
@@ -711,7 +715,7 @@ int mlp_forward(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
             g.epi = kEpiLinear;
             g.outf = n->y;
         }
-        e = gemm_launch(&g, 1, ColumnSums{}, n->err, &n->back[2], st, n->num_sm, true);
+        e = gemm_launch(&g, 1, ColumnSums{}, n->err, &n->back[1], st, n->num_sm, true);
     }
     return e;
 }
@@ -750,7 +754,8 @@ int mlp_backward(arbo_mlp* n, uint32_t rows, cudaStream_t st)
             g[0].outt = ndt;
             g[0].ldot = ld;
         }
-        e = gemm_launch(g, l > 0 ? 2 : 1, ColumnSums{dzt, ld, rows, out, n->db[l]}, n->err, &n->back[2], st, n->num_sm, true);
+        e = gemm_launch(g, l > 0 ? 2 : 1, ColumnSums{dzt, ld, rows, out, n->db[l]}, n->err, &n->back[1], st, n->num_sm, true,
+                        l + 1 == L ? n->loss : nullptr, (float*)n->back);
         std::swap(dz, nd);
         std::swap(dzt, ndt);
     }
@@ -807,30 +812,24 @@ int mlp_enqueue(arbo_mlp* n, uint32_t rows, bool train, cudaStream_t st)
     return (int)cudaGraphLaunch(slot->exec, st);
 }
 
-// Waits for what was enqueued before (and for the copy of loss and error word, which it enqueues).
-int mlp_read_back(arbo_mlp* n, cudaStream_t st)
-{
-    UCUDA(cudaMemcpyAsync(n->back, n->loss, 8, cudaMemcpyDeviceToHost, st));
-    UCUDA(cudaEventRecord(n->done, st));
-    return ARBO_OK;
-}
-
-int mlp_check_err(arbo_mlp* n, uint32_t word)
+// Waits for the event recorded behind the products; the loss is in back[0] then.
+int mlp_check_err(arbo_mlp* n)
 {
     UCUDA(cudaEventSynchronize(n->done));
-    const uint32_t e = n->back[word];
+    const uint32_t e = n->back[1];
     if (e) return ufail(ARBO_ERR_CUDA, "tensor-core product: an mbarrier wait ran out (error word " + std::to_string(e) + ")");
     return ARBO_OK;
 }
 
-// Upload, forward and backward pass and the copy of the loss, all enqueued on st.
+// Upload, forward and backward pass, all enqueued on st with the event behind them.
 int mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t rows, cudaStream_t st)
 {
     int e = mlp_upload(n, x, t, rows, st);
     if (e) return e;
     if ((e = mlp_enqueue(n, rows, true, st)))
         return ufail(ARBO_ERR_CUDA, std::string("forward/backward: ") + cudaGetErrorString((cudaError_t)e));
-    return mlp_read_back(n, st);
+    UCUDA(cudaEventRecord(n->done, st));
+    return ARBO_OK;
 }
 
 }  // namespace
@@ -924,12 +923,12 @@ int arbo_mlp_create(uint32_t n_in, uint32_t hidden, uint32_t hidden_layers, uint
     n->tin = F((size_t)B * n_out);
     n->loss = F(2);  // and the error word beside it
     n->err = (uint32_t*)n->loss + 1;
-    if (!okm || cudaMallocHost(&n->back, 16) != cudaSuccess ||
+    if (!okm || cudaMallocHost(&n->back, 8) != cudaSuccess ||
         cudaEventCreateWithFlags(&n->done, cudaEventDisableTiming) != cudaSuccess) {
         arbo_mlp_destroy(n);
         return ufail(ARBO_ERR_ALLOC, "arbo_mlp_create: device allocation failed");
     }
-    std::memset(n->back, 0, 16);
+    std::memset(n->back, 0, 8);
     std::vector<AdamArray> arrays;
     for (uint32_t l = 0; l < n->L; ++l) {
         const uint32_t in = n->dim[l], o = n->dim[l + 1];
@@ -988,7 +987,7 @@ int arbo_mlp_forward(arbo_mlp* n, const float* x, uint32_t rows, float* y, void*
         UCUDA(cudaMemcpy2DAsync(y, n->nout * 4, n->y, w * 4, n->nout * 4, rows, cudaMemcpyDeviceToHost, st));
     }
     UCUDA(cudaEventRecord(n->done, st));
-    return mlp_check_err(n, 2);
+    return mlp_check_err(n);
 }
 
 int arbo_mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t rows, float* loss, void* stream)
@@ -996,7 +995,7 @@ int arbo_mlp_gradients(arbo_mlp* n, const float* x, const float* t, uint32_t row
     if (!n || !x || !t) return ufail(ARBO_ERR_INVALID, "null argument");
     UCUDA(cudaSetDevice(n->device));
     int e = mlp_gradients(n, x, t, rows, (cudaStream_t)stream);
-    if (!e) e = mlp_check_err(n, 1);
+    if (!e) e = mlp_check_err(n);
     if (!e && loss) std::memcpy(loss, &n->back[0], 4);
     return e;
 }
@@ -1014,7 +1013,7 @@ int arbo_mlp_train_step(arbo_mlp* n, const float* x, const float* t, uint32_t ro
     const float c1 = 1.0f - std::pow(b1, step), c2 = 1.0f - std::pow(b2, step);
     k_adam<<<n->adam_blocks, 256, 0, st>>>(n->adam, n->adam_arrays, lr, b1, b2, eps, c1, c2, n->err);
     UCUDA(cudaGetLastError());
-    if ((e = mlp_check_err(n, 1))) return e;
+    if ((e = mlp_check_err(n))) return e;
     n->steps += 1;
     if (loss) std::memcpy(loss, &n->back[0], 4);
     return ARBO_OK;
