@@ -1515,13 +1515,14 @@ bool chooses_shapes(const arbo_arch_param& a)
 
 // CTAs per simulation when the batch's steps run as one cluster per simulation (k_steps), or 0 for the
 // per-phase kernels. C: the largest cluster of which all the simulations' fit the device at once.
-// A step takes a cluster about 13 us plus 0.45 us per 1,000 work units of its simulation (agents, and
-// 300 per community for the infection pass) and CTA, 0.85 us once CTAs share SMs, and the device as a
-// whole 0.003 us per 1,000 units; the per-phase kernels take 35 us and the same throughput. Measured, us
-// per step, clusters against per-phase kernels: 8 simulations of 7e4 agents 17 and 38, 32 of them 20 and
-// 41, 128 of them 51 and 65, 200 of them 100 and 91, 304 of them 120 and 130; 32 of 2.1e5 agents 37 and
-// 50; 64 of 4e4 to 4e5 agents 92 and 67. The line falls where one simulation is much larger than the
-// others (its cluster works alone) or there are more than fit at once.
+// A step takes a cluster about 11 us plus 0.45 us per 1,000 work units of its simulation (agents, and
+// 300 per community for the infection pass) and CTA; once CTAs share SMs 0.36 to 0.66 us, the more the
+// larger the SM's other simulations are; and the device as a whole 0.003 us per 1,000 units. The per-phase
+// kernels take 33 us and 0.0025 us per 1,000 units. Measured over a year's steps, us per step, clusters against
+// per-phase kernels: 8 simulations of 7e4 agents 14 and 35, 32 of them 17 and 37, 128 of them 44 and 64, 200
+// of them 82 and 81, 304 of them 95 and 117; 32 of 2.1e5 agents 34 and 50; of 4e4 to 4e5 agents 24 29 and
+// 41, 64 69 and 61. The line falls where one simulation is much larger than the others (its cluster works
+// alone) or there are more than fit at once.
 uint32_t batch_cluster(const arbo_batch* b, uint32_t* per_sm)
 {
     if (b->phase_shapes) return 0;
@@ -1534,8 +1535,8 @@ uint32_t batch_cluster(const arbo_batch* b, uint32_t* per_sm)
         total += units;
         most = std::max(most, units);
     }
-    const double per = *per_sm == 1 ? 0.45 : 0.85;
-    return 13.0 + std::max(per * most / C, 0.003 * total) < 35.0 + 0.003 * total ? C : 0;
+    const double per = *per_sm == 1 ? 0.45 : 0.36 + 0.3 * total / (n * most);
+    return 11.0 + std::max(per * most / C, 0.003 * total) < 33.0 + 0.0025 * total ? C : 0;
 }
 
 // Block counts of every instance for the launch shapes of `a`; descriptors and tables uploaded.
