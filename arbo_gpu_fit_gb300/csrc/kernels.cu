@@ -1571,7 +1571,7 @@ static_assert(kStepsSmem + sizeof(Dev) + 64 <= 48 * 1024, "shared memory of k_st
 // simulation runs `nsteps` whole steps, its phases separated by cluster barriers. Simulations need
 // nothing from one another, so each cluster goes on by itself; the per-phase batch kernels wait for the
 // slowest simulation at each phase and hand out items through one counter, which with few items is all
-// latency: 32 simulations of 7e4 agents took 39 us a step, now 20, 8 of them 35 and 17. The bodies are
+// latency: 32 simulations of 7e4 agents took 39 us a step, now 17, 8 of them 35 and 14. The bodies are
 // the per-phase kernels' own. Sixteen warps to a CTA and B CTAs to an SM (64 registers at two).
 //
 // Two forms. With few demographic items to a warp (kMany false) they go in a fixed order, and each phase's
