@@ -33,13 +33,19 @@ int fail(int code, const std::string& msg)
         if (e_ != cudaSuccess) return fail(ARBO_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Steps that a handle or batch launches kernel by kernel before it captures graphs: the three launches
+// Steps that a handle or batch makes before it captures graphs of graphSteps: the three launches
 // of a step take the host less time (about 8 us) than the step takes the device, while a 64-step graph
 // costs half a millisecond to make, again after every change of parameters. What is left of a call
 // after its whole graphs is launched the same way (as one-step graphs each step paid for a graph launch
 // and could not overlap the one before: 30 steps of 1.2e4 agents with initialisation and results 775 ->
 // 662 us, and 440 to 500 us less for the first run of a handle).
 constexpr uint32_t kDirectSteps = 256;
+
+// From this step on until then a single simulation runs in graphs of 16 steps: launched one by one, a step
+// takes the device 1.2 us longer, and by then the device has more work queued than such a graph takes the
+// host to make (some 120 us). A year of 7e5 agents with the handle made and freed 5.50 -> 5.22 ms, a first
+// year of 5e4 4.31 -> 4.05, of 7e6 7.92 -> 7.70.
+constexpr uint32_t kShortAfter = 48, kShortSteps = 16;
 
 // The rest of a call after its whole graphs, where several calls in turn end with the same one of this many
 // steps or more (a handle run again and again over the same days), gets a graph of its own too: launched one
@@ -156,7 +162,7 @@ struct arbo_sim {
     uint64_t comm_most = 0;  // agents of the largest community
     std::vector<float> etab;
     cudaStream_t cap = nullptr;
-    cudaGraphExec_t gmulti = nullptr, grest = nullptr;  // graphSteps steps; the rest of a call
+    cudaGraphExec_t gmulti = nullptr, gshort = nullptr, grest = nullptr;  // graphSteps, kShortSteps, the rest of a call
     uint32_t rest = 0, rest_calls = 0;                  // steps of that rest; calls that ended with it
     uint32_t direct = 0;  // steps launched kernel by kernel since the parameters changed
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -626,6 +632,7 @@ int arbo_sim_destroy(arbo_sim* s)
     if (!s) return ARBO_OK;
     cudaSetDevice(s->device);
     if (s->gmulti) cudaGraphExecDestroy(s->gmulti);
+    if (s->gshort) cudaGraphExecDestroy(s->gshort);
     if (s->grest) cudaGraphExecDestroy(s->grest);
     for (int k = 0; k < 4; ++k)
         if (s->ev[k]) cudaEventDestroy(s->ev[k]);
@@ -687,8 +694,9 @@ static void param_change_host(arbo_sim* s, const arbo_sim_param& p)
     apply_rates(p, s->d);
     fill_expected(p, s->d.M, s->d.T, s->etab);
     if (s->gmulti) cudaGraphExecDestroy(s->gmulti);
+    if (s->gshort) cudaGraphExecDestroy(s->gshort);
     if (s->grest) cudaGraphExecDestroy(s->grest);
-    s->gmulti = s->grest = nullptr;
+    s->gmulti = s->gshort = s->grest = nullptr;
     s->direct = 0;
     s->version += 1;
 }
@@ -773,13 +781,15 @@ int arbo_sim_step(arbo_sim* s, uint32_t nsteps, void* stream)
         }
         return ARBO_OK;
     }
+    bool tail = false;  // the rest of the call has been looked at
     while (n > 0) {
-        const uint32_t chunk = std::min(n, G);
-        cudaGraphExec_t* graph = nullptr;
+        uint32_t chunk = std::min(n, G);
+        cudaGraphExec_t* graph = nullptr;  // null: launched one by one
         if (s->direct >= kDirectSteps) {
             if (chunk == G) {
                 graph = &s->gmulti;
-            } else if (chunk >= kRestSteps) {
+            } else if (chunk >= kRestSteps && !tail) {
+                tail = true;
                 // The graph of a rest stays for the handle's life or until the parameters change.
                 if (!s->grest && chunk != s->rest) {
                     s->rest = chunk;
@@ -787,6 +797,11 @@ int arbo_sim_step(arbo_sim* s, uint32_t nsteps, void* stream)
                 }
                 if (chunk == s->rest && ++s->rest_calls >= kRestCalls) graph = &s->grest;
             }
+        }
+        if (!graph && s->direct >= kShortAfter && chunk >= kShortSteps) {
+            graph = &s->gshort;
+            chunk = kShortSteps;
+            s->direct += chunk;
         }
         if (graph) {
             if (!*graph) {
