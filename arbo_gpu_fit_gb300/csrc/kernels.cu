@@ -278,11 +278,10 @@ __device__ __forceinline__ uint32_t pick4(const U4& v, uint32_t i)
     return i == 0 ? v.v[0] : i == 1 ? v.v[1] : i == 2 ? v.v[2] : v.v[3];
 }
 
-// What a quad needs that does not depend on its codes, made while they are on their way: the tile's
-// carried dead count and community, the expected mosquitoes, and (left in the staging) the quad's quota
-// draws and the draws of the first 28 births of each tile, which are keyed by rank and not by slot.
+// What a quad needs that no step kernel writes, made while the previous pass ends: the tile's community,
+// the expected mosquitoes, and (left in the staging) the quad's quota draws and the draws of the first 28
+// births of each tile, which are keyed by rank and not by slot.
 struct QuadStart {
-    int32_t led;
     uint32_t c0, end, end2;
     float target;
 };
@@ -293,7 +292,6 @@ __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uin
     const uint32_t u = lane >> 3, b = q * kQuad + u;
     const bool live = b < d.tiles;
     QuadStart at;
-    at.led = live ? d.ledger[b] : 0;
     at.c0 = live ? __ldg(&d.tcomm[b]) : 0u;
     at.end = at.end2 = ~0u;
     if (at.c0 & kTileSpans) {
@@ -312,6 +310,14 @@ __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uin
     return at;
 }
 
+// The carried dead count of the lane's tile. The last step's pass wrote it, so it is loaded after the wait,
+// in the same round trip as the codes.
+__device__ __forceinline__ int32_t quad_ledger(const Dev& d, uint32_t q, uint32_t lane)
+{
+    const uint32_t b = q * kQuad + (lane >> 3);
+    return b < d.tiles ? d.ledger[b] : 0;
+}
+
 // One warp, tiles 4q..4q+3; lane l holds the codes of slots 16(l mod 8) .. +15 of tile 4q + l/8, four
 // words. Per tile: deaths (a live slot dies in the step that reaches its death time), the birth quota
 // (cpp/mdemographic.cu:104-129) from the carried dead count, rebirth of the lowest-index dead slots, the
@@ -326,7 +332,7 @@ __device__ __forceinline__ QuadStart quad_start(const Dev& d, const Key key, uin
 // reborn slot under its rank; one lane per reborn slot then draws its PLE and writes its life record
 // (one sector instead of three) and its code, which the owners write back with one 16-byte store.
 __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, uint32_t q, uint32_t lane, uint32_t t,
-                                                   QuadSmem& sm, const QuadStart& at, const uint4 A)
+                                                   QuadSmem& sm, const QuadStart& at, const int32_t led, const uint4 A)
 {
     const int32_t tn = (int32_t)t + 1;
     const uint32_t u = lane >> 3, seg = lane & 7u, b = q * kQuad + u;
@@ -402,7 +408,7 @@ __device__ __forceinline__ void mosquito_quad_core(const Dev& d, const Key key, 
     if (live) {
         const uint32_t start = b * kTile;
         const uint32_t bt = (d.M - start) < kTile ? (d.M - start) : kTile;
-        const uint32_t L = (uint32_t)at.led + died_tot;
+        const uint32_t L = (uint32_t)led + died_tot;
         const float fbt = (float)bt;
         float x = __fmul_rn(at.target, fbt);
         x = __fdiv_rn(x, (float)d.M);
@@ -474,8 +480,9 @@ struct NoWait {
 struct GridWait {
     __device__ __forceinline__ void operator()() const { griddep_wait(); }
 };
-// In the infection pass the next step's demographic pass may be scheduled only then: before its own wait it
-// reads the dead counts, which this step's pass (finished before the grid waited for) writes.
+// In the infection pass the next step's demographic pass may be scheduled only then, so that when a pass
+// starts, every kernel but the one before it has ended. What a pass reads before its own wait (step control,
+// tables, network) no step kernel writes: an early start is promised earlier kernels' writes only after it.
 struct GridWaitRelease {
     __device__ __forceinline__ void operator()() const
     {
@@ -511,7 +518,7 @@ __device__ __forceinline__ void demog_mosquito_quad(const Dev& d, const Key key,
     wait();
     uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
     if (q * kQuad + (lane >> 3) < d.tiles) A = reinterpret_cast<const uint4*>(d.m_code)[q * 32 + lane];
-    mosquito_quad_core(d, key, q, lane, t, sm, at, A);
+    mosquito_quad_core(d, key, q, lane, t, sm, at, quad_ledger(d, q, lane), A);
 }
 
 // ------------------------------------------------------------------ TMA-staged pipeline
@@ -620,7 +627,8 @@ __global__ void __launch_bounds__(128, 4) k_demog_tma(Dev d, uint32_t koff)
         uint4 A = make_uint4(~0u, ~0u, ~0u, ~0u);
         if (q * kQuad + (lane >> 3) < d.tiles) A = ws.stage[sidx][lane];
         __syncwarp();  // every lane has its words before the buffer is refilled next iteration
-        mosquito_quad_core(d, key, q, lane, t, ws.qs, quad_start(d, key, q, lane, t, ws.qs), A);
+        const int32_t led = quad_ledger(d, q, lane);
+        mosquito_quad_core(d, key, q, lane, t, ws.qs, quad_start(d, key, q, lane, t, ws.qs), led, A);
     }
     griddep_launch_dependents();
 }
@@ -2019,7 +2027,7 @@ int launch_demog(const Dev& d, const Launch& l, cudaStream_t st, uint32_t koff)
     const bool spread = items <= 2 * warps * sms;
     if (spread && warps == 8) warps = std::min(8u, std::max(4u, cdiv(items, 2 * sms)));
     // Within a run of steps the previous kernel is the last step's infection pass, which leaves the step
-    // control, the dead counts and the tables alone, so the pass may begin before it ends. At a run's
+    // control and the tables alone, so the pass may begin before it ends. At a run's
     // first step (koff 0) it may be the kernel that advances the step control.
     return launch_pdl(U == 4 ? k_demog<4> : U == 2 ? k_demog<2> : k_demog<1>, dim3(cdiv(items, warps)), dim3(32 * warps), 0,
                       st, l.pdl && koff > 0, d, spread ? 1u : 0u, koff);
