@@ -54,6 +54,10 @@ constexpr uint32_t kShortAfter = 48, kShortSteps = 16;
 // of 30 steps takes a quarter of a millisecond to make.
 constexpr uint32_t kRestSteps = 8, kRestCalls = 4;
 
+// Words that a handle keeps for its census accessors. All 12e6 PLE of the largest population in chunks of 2^20
+// take 0.52 ms, of 2^18 0.94, as one copy of a dense array 0.26.
+constexpr size_t kLifeStage = 1u << 20;
+
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // x to the power of a Weibull shape; pow(x, 1) is x, so exponential lives need no call.
@@ -158,6 +162,9 @@ struct arbo_sim {
     size_t bytes = 0;
     void* zeroed = nullptr;  // the arrays that initialisation zeroes, one range of the allocation
     size_t zeroed_bytes = 0;
+    void* life_stage = nullptr;  // staging of census accessors (life_words); used under life_mu
+    size_t life_stage_bytes = 0;
+    std::mutex life_mu;
     std::vector<uint32_t> nsize, msize, nloc, mloc;
     uint64_t comm_most = 0;  // agents of the largest community
     std::vector<float> etab;
@@ -533,6 +540,7 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
     c.k1 = (uint32_t)(seed >> 32);
     c.instance = instance;
 
+    s->life_stage_bytes = std::max<size_t>(8, std::min<size_t>(M, kLifeStage) * 4);
     // One allocation, every array 256-byte aligned. First the arrays that are filled here, in one copy
     // from a host image (eighteen copies took 0.15 ms); then those that initialisation zeroes, in one
     // memset (arbo_sim_init); then the winner keys; then the census.
@@ -566,6 +574,7 @@ int arbo_sim_create(const arbo_sim_param* sp, const arbo_arch_param* ap, const a
         {(void**)&d.n_recovery, Np * 4}, {(void**)&d.n_ple, Np * 4}, {(void**)&d.n_strain, Np}, {(void**)&d.n_imm, Np},
         {(void**)&d.m_code, Mp}, {(void**)&d.m_stat, Mp}, {(void**)&d.m_life, Mp * sizeof(Life)},
         {(void**)&d.m_exposed, Mp * 4}, {(void**)&d.m_strain, Mp}, {(void**)&d.ledger, (size_t)d.tiles * 4},
+        {&s->life_stage, s->life_stage_bytes},
     };
     auto extent = [](const std::vector<Item>& v) {
         size_t n = 0;
@@ -953,24 +962,25 @@ static int census_ptr(arbo_sim* s, arbo_census_field f, void** ptr, size_t* coun
     return ARBO_OK;
 }
 
-// One field of the mosquitoes' life records (0 birth time, 1 death time, 2 PLE) between host and
-// device, through a device array of M values.
-static int life_field(arbo_sim* s, int field, void* host, bool store, void* stream)
+// Words of the mosquitoes' life records (1 or 2 from `word` on: birth time, death time, PLE) between host and
+// device, in chunks through the handle's staging array. Allocating one here would make the call wait for the
+// whole device and fail when memory is short.
+static int life_words(arbo_sim* s, int word, int words, void* host, bool store, void* stream)
 {
-    const size_t bytes = (size_t)s->d.M * 4;
-    cudaStream_t st = (cudaStream_t)stream;
+    std::lock_guard<std::mutex> lk(s->life_mu);  // until the stream is done with the staging array
     CUDA_TRY(cudaSetDevice(s->device));
-    void* buf = nullptr;
-    cudaError_t e = cudaMalloc(&buf, bytes);
-    if (e != cudaSuccess)
-        return fail(ARBO_ERR_ALLOC, std::string("cudaMalloc of a census field: ") + cudaGetErrorString(e));
-    if (store) e = cudaMemcpyAsync(buf, host, bytes, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = (cudaError_t)launch_life_field(s->d, field, buf, store, stream);
-    if (e == cudaSuccess && !store) e = cudaMemcpyAsync(host, buf, bytes, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(buf);
-    if (e != cudaSuccess) return fail(ARBO_ERR_CUDA, std::string("census field: ") + cudaGetErrorString(e));
-    (store ? s->h2d : s->d2h) += bytes;
+    cudaStream_t st = (cudaStream_t)stream;
+    const size_t chunk = s->life_stage_bytes / (4 * (size_t)words);
+    for (size_t i = 0; i < s->d.M; i += chunk) {
+        const size_t n = std::min<size_t>(chunk, s->d.M - i), bytes = n * 4 * words;
+        char* h = (char*)host + i * 4 * words;
+        if (store) CUDA_TRY(cudaMemcpyAsync(s->life_stage, h, bytes, cudaMemcpyHostToDevice, st));
+        const int e = launch_life_words(s->d, (uint32_t)i, (uint32_t)n, word, words, s->life_stage, store, stream);
+        if (e) return fail(ARBO_ERR_CUDA, std::string("census field: ") + cudaGetErrorString((cudaError_t)e));
+        if (!store) CUDA_TRY(cudaMemcpyAsync(h, s->life_stage, bytes, cudaMemcpyDeviceToHost, st));
+        (store ? s->h2d : s->d2h) += bytes;
+    }
+    CUDA_TRY(cudaStreamSynchronize(st));
     return ARBO_OK;
 }
 
@@ -985,14 +995,14 @@ static int census_derived(arbo_sim* s, arbo_census_field f, int32_t* out, size_t
     int e = arbo_sim_status(s, stream, &err, &now);
     if (e) return e;
     const bool human = f == ARBO_CENSUS_N_AGE || f == ARBO_CENSUS_N_DEATH_AGE;
-    std::vector<int32_t> born(count), dtime(count);
+    // Birth and death times: two arrays of the humans, pairs of the mosquitoes.
+    std::vector<int32_t> times(2 * count);
     std::vector<uint8_t> state;
     if (human) {
-        if ((e = copy_out(s, born.data(), d.n_born, count * 4, stream))) return e;
-        if ((e = copy_out(s, dtime.data(), d.n_dtime, count * 4, stream))) return e;
-    } else {
-        if ((e = life_field(s, 0, born.data(), false, stream))) return e;
-        if ((e = life_field(s, 1, dtime.data(), false, stream))) return e;
+        if ((e = copy_out(s, times.data(), d.n_born, count * 4, stream))) return e;
+        if ((e = copy_out(s, times.data() + count, d.n_dtime, count * 4, stream))) return e;
+    } else if ((e = life_words(s, 0, 2, times.data(), false, stream))) {
+        return e;
     }
     if (f == ARBO_CENSUS_M_AGE) {
         state.resize(count);
@@ -1000,7 +1010,7 @@ static int census_derived(arbo_sim* s, arbo_census_field f, int32_t* out, size_t
     }
     const int32_t tn = (int32_t)now;
     for (size_t i = 0; i < count; ++i) {
-        const int32_t b = born[i], x = dtime[i];
+        const int32_t b = human ? times[i] : times[2 * i], x = human ? times[count + i] : times[2 * i + 1];
         if (f == ARBO_CENSUS_N_AGE) out[i] = tn - b;
         else if (f == ARBO_CENSUS_M_AGE) {
             if (!(state[i] & kDead)) out[i] = tn - b;
@@ -1021,7 +1031,7 @@ int arbo_sim_get_census(arbo_sim* s, arbo_census_field f, void* host, size_t byt
     if (e) return e;
     if (bytes != count * elem) return fail(ARBO_ERR_INVALID, "census size mismatch: expected " + std::to_string(count * elem));
     if (packed == 3) return census_derived(s, f, (int32_t*)host, count, stream);
-    if (packed == 4) return life_field(s, 2, host, false, stream);
+    if (packed == 4) return life_words(s, 2, 1, host, false, stream);
     e = copy_out(s, host, ptr, bytes, stream);
     if (e || !packed) return e;
     uint8_t* h = (uint8_t*)host;
@@ -1060,34 +1070,6 @@ static int refresh_human_next(arbo_sim* s, void* stream)
     return ARBO_OK;
 }
 
-// Recomputes every mosquito slot's event code from its dead flag (dead[i], or the present code's when
-// dead is null), status, life and exposed age (after a census write that changed any of them).
-static int refresh_mosquito_code(arbo_sim* s, const uint8_t* dead, void* stream)
-{
-    const Dev& d = s->d;
-    const size_t M = d.M;
-    std::vector<uint8_t> code(M), stat(M);
-    std::vector<Life> life(M);
-    std::vector<int32_t> ex(M);
-    uint32_t err = 0, now = 0;
-    int e;
-    if ((e = arbo_sim_status(s, stream, &err, &now)) || (e = copy_out(s, code.data(), d.m_code, M, stream)) ||
-        (e = copy_out(s, stat.data(), d.m_stat, M, stream)) ||
-        (e = copy_out(s, life.data(), d.m_life, M * sizeof(Life), stream)) ||
-        (e = copy_out(s, ex.data(), d.m_exposed, M * 4, stream)))
-        return e;
-    for (size_t i = 0; i < M; ++i) {
-        const uint32_t st = stat[i] & 3u;
-        if (dead ? dead[i] != 0 : (code[i] & kDead) != 0) code[i] = (uint8_t)(kDead | (st ? kDeep : 0u));
-        else code[i] = mosq_code(mosq_next(st, life[i].dtime, life[i].born, ex[i]), (int32_t)now, st != 0);
-    }
-    cudaStream_t cs = (cudaStream_t)stream;
-    CUDA_TRY(cudaMemcpyAsync(d.m_code, code.data(), M, cudaMemcpyHostToDevice, cs));
-    CUDA_TRY(cudaStreamSynchronize(cs));
-    s->h2d += M;
-    return ARBO_OK;
-}
-
 int arbo_sim_set_census(arbo_sim* s, arbo_census_field f, const void* host, size_t bytes, void* stream)
 {
     if (!s || !host) return fail(ARBO_ERR_INVALID, "null argument");
@@ -1101,24 +1083,18 @@ int arbo_sim_set_census(arbo_sim* s, arbo_census_field f, const void* host, size
         return fail(ARBO_ERR_INVALID, "ages and death ages are derived from birth and death times and cannot be set");
     CUDA_TRY(cudaSetDevice(s->device));
     cudaStream_t st = (cudaStream_t)stream;
-    if (!packed) {
-        CUDA_TRY(cudaMemcpyAsync(ptr, host, bytes, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        s->h2d += bytes;
-        if (f == ARBO_CENSUS_N_STATUS || f == ARBO_CENSUS_N_EXPOSED || f == ARBO_CENSUS_N_RECOVERY)
-            return refresh_human_next(s, stream);
-        if (f == ARBO_CENSUS_M_EXPOSED) return refresh_mosquito_code(s, nullptr, stream);
-        return ARBO_OK;
-    }
-    if (packed == 4) return life_field(s, 2, const_cast<void*>(host), true, stream);
-    if (packed == 1) return refresh_mosquito_code(s, (const uint8_t*)host, stream);
-    std::vector<uint8_t> cur(count);
-    const uint8_t* h = (const uint8_t*)host;
-    for (size_t i = 0; i < count; ++i) cur[i] = (uint8_t)(h[i] & 3u);
-    CUDA_TRY(cudaMemcpyAsync(ptr, cur.data(), count, cudaMemcpyHostToDevice, st));
+    if (packed == 4) return life_words(s, 2, 1, const_cast<void*>(host), true, stream);
+    // A mosquito's status, exposed age and dead flag move its next event. Dead flags go where the codes are,
+    // which are then made from them.
+    const bool event = packed || f == ARBO_CENSUS_M_EXPOSED;
+    CUDA_TRY(cudaMemcpyAsync(ptr, host, bytes, cudaMemcpyHostToDevice, st));
+    e = event ? launch_refresh_codes(s->d, packed == 1, stream) : 0;
+    if (e) return fail(ARBO_ERR_CUDA, std::string("census write: ") + cudaGetErrorString((cudaError_t)e));
     CUDA_TRY(cudaStreamSynchronize(st));
-    s->h2d += count;
-    return refresh_mosquito_code(s, nullptr, stream);
+    s->h2d += bytes;
+    if (f == ARBO_CENSUS_N_STATUS || f == ARBO_CENSUS_N_EXPOSED || f == ARBO_CENSUS_N_RECOVERY)
+        return refresh_human_next(s, stream);
+    return ARBO_OK;
 }
 
 int arbo_sim_dims(const arbo_sim* s, uint32_t* n, uint32_t* m, uint32_t* p, uint32_t* strains, uint32_t* max_time,

@@ -210,8 +210,13 @@ uint32_t foi_items(uint32_t S, uint32_t P);
 int launch_step(const Dev& d, const Launch& l, void* stream, void* events, uint32_t koff);
 // Adds n to the step counter and the winner epoch (one thread).
 int launch_advance(const Dev& d, uint32_t n, void* stream);
-// field 0, 1, 2: birth time, death time, PLE of every slot, between the life records and an array.
-int launch_life_field(const Dev& d, int field, void* array, bool store, void* stream);
+// `words` (1 or 2) consecutive words of the life records of slots first .. first + n - 1, from word `word` on
+// (0, 1, 2: birth time, death time, PLE), to or from a dense device array.
+int launch_life_words(const Dev& d, uint32_t first, uint32_t n, int word, int words, void* array, bool store,
+                      void* stream);
+// Every slot's event code from its status, life and exposed age after one of them was written. `flags`: the
+// code array holds dead flags (0 or not) instead of codes.
+int launch_refresh_codes(const Dev& d, bool flags, void* stream);
 // Writes the census in the reference's types into the caller's buffers (arbo_sim_export_census).
 int launch_export(const Dev& d, const arbo_census_export& x, void* stream);
 uint32_t launches_per_step();
