@@ -1484,24 +1484,42 @@ Dev batch_desc(const arbo_batch* b, size_t i)
 }
 
 // Agents of the largest community from which a batch's infection pass works off communities with many events
-// by block (k_infect_batch<true>), in runs of two communities and, where the caller leaves the default block,
-// in blocks of 256 threads. Smaller communities seldom have that many events, and the search for them costs
+// by block (k_infect_batch<true>), in runs of two communities (one in blocks of one or two warps) and, where the
+// batch takes its handles' default shape, in blocks of kHeavyBlock threads. Smaller communities seldom have that many events, and the search for them costs
 // 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us, at runs of 4, 2 and 1: 352, 289 and
 // 278 in blocks of 256, 398, 370 and 350 in blocks of 512, 456, 378 and 280 in blocks of 64; with few
 // events 83, 85 and 92. One simulation alone keeps k_infect: with this its step took 1 to 3 % longer.
 constexpr uint64_t kHeavyCommunity = 16384;
+constexpr uint32_t kHeavyBlock = 256;
+
+bool batch_heavy(const arbo_batch* b)
+{
+    uint64_t most = 0;  // largest community of any instance
+    for (const arbo_sim* s : b->sims) most = std::max(most, s->comm_most);
+    return most >= kHeavyCommunity;
+}
+
+// Launch shapes of a batch whose caller gives none.
+arbo_arch_param batch_default_arch(const arbo_batch* b)
+{
+    arbo_arch_param a = b->sims[0]->arch, q;
+    arbo_arch_param_query(&q, -1);
+    if (a.infectBlock == q.infectBlock && batch_heavy(b)) a.infectBlock = kHeavyBlock;
+    return a;
+}
 
 // Steps per launch of k_steps.
 constexpr uint32_t kClusterSteps = 128;
 
 // Whether `a` chooses launch shapes of the per-phase kernels (the human unroll aside): a caller who does
 // gets those kernels.
-bool chooses_shapes(const arbo_arch_param& a)
+bool chooses_shapes(const arbo_batch* b, const arbo_arch_param& a)
 {
     arbo_arch_param q;
     arbo_arch_param_query(&q, -1);
-    return a.demogBlock != q.demogBlock || a.foiBlock != q.foiBlock || a.infectBlock != q.infectBlock ||
-           a.graphSteps != q.graphSteps || a.demogPipeline != q.demogPipeline;
+    const bool infect = a.infectBlock != q.infectBlock && !(a.infectBlock == kHeavyBlock && batch_heavy(b));
+    return a.demogBlock != q.demogBlock || a.foiBlock != q.foiBlock || infect || a.graphSteps != q.graphSteps ||
+           a.demogPipeline != q.demogPipeline;
 }
 
 // CTAs per simulation when the batch's steps run as one cluster per simulation (k_steps), or 0 for the
@@ -1541,12 +1559,8 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     l.demogBlock = a.demogBlock;
     l.demogUnroll = a.demogUnroll;
     l.foiBlock = a.foiBlock;
-    arbo_arch_param dflt;
-    arbo_arch_param_query(&dflt, -1);
-    uint64_t most = 0;  // largest community of any instance
-    for (const arbo_sim* s : b->sims) most = std::max(most, s->comm_most);
-    const bool heavy = most >= kHeavyCommunity;
-    l.infectBlock = heavy && a.infectBlock == dflt.infectBlock ? 256 : a.infectBlock;
+    const bool heavy = batch_heavy(b);
+    l.infectBlock = a.infectBlock;
     l.infectHeavy = heavy;
     l.numSM = a.totalSM ? a.totalSM : 152u;
     l.pdl = 1;
@@ -1635,7 +1649,7 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     // Runs of consecutive communities per warp (fewer descriptor restagings), as long as every
     // resident warp still gets one.
     const uint32_t warps = l.numSM * occ[2] * K;
-    const uint32_t run_max = heavy ? 2u : kInfectRunMax;
+    const uint32_t run_max = heavy ? (K > 2 ? 2u : 1u) : kInfectRunMax;
     bd.infect_run = std::max(1u, std::min(run_max, b->blocks[2] / std::max(warps, 1u)));
     bd.grid_infect = std::max(1u, std::min(cdiv(cdiv(b->blocks[2], bd.infect_run), heavy ? 1u : K), l.numSM * occ[2]));
     batch_drop_graphs(b);
@@ -1782,8 +1796,9 @@ int arbo_batch_create(arbo_sim* const* sims, uint32_t n, const arbo_arch_param* 
         return bail(fail(ARBO_ERR_CUDA, "cudaStreamCreate"));
     for (int k = 0; k < 4; ++k)
         if (cudaEventCreate(&b->ev[k]) != cudaSuccess) return bail(fail(ARBO_ERR_CUDA, "cudaEventCreate"));
-    b->phase_shapes = chooses_shapes(arch ? *arch : sims[0]->arch);
-    const int e = batch_configure(b, arch ? *arch : sims[0]->arch);
+    const arbo_arch_param a = arch ? *arch : batch_default_arch(b);
+    b->phase_shapes = chooses_shapes(b, a);
+    const int e = batch_configure(b, a);
     if (e) return bail(e);
     *out = b;
     return ARBO_OK;
@@ -1821,7 +1836,7 @@ int arbo_batch_set_arch(arbo_batch* b, const arbo_arch_param* arch)
     CUDA_TRY(cudaSetDevice(b->device));
     CUDA_TRY(cudaDeviceSynchronize());  // graphs of the old shape may still run
     const bool before = b->phase_shapes;
-    b->phase_shapes = chooses_shapes(*arch);
+    b->phase_shapes = chooses_shapes(b, *arch);
     const int e = batch_configure(b, *arch);
     if (e) b->phase_shapes = before;
     return e;

@@ -436,8 +436,9 @@ int arbo_sim_step_noalloc(arbo_sim* s, uint32_t nsteps, void* stream);
 typedef struct arbo_batch arbo_batch;
 
 /* Builds a batch of n handles (one device; each handle at most once). arch: launch shapes of the
- * batched kernels (NULL: those of sims[0]); the grids are one wave of resident CTAs. Shapes other than
- * the defaults (the human unroll aside) select the per-phase kernels. */
+ * batched kernels (NULL: those of sims[0], with 256 for the default infectBlock in a batch with a
+ * community of 16,384 agents or more); the grids are one wave of resident CTAs. Shapes other than
+ * those defaults (the human unroll aside) select the per-phase kernels. */
 int arbo_batch_create(arbo_sim* const* sims, uint32_t n, const arbo_arch_param* arch, arbo_batch** out);
 int arbo_batch_destroy(arbo_batch* b);
 /* Number of instances and their total agents (humans + mosquito slots). */

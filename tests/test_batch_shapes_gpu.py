@@ -1,0 +1,39 @@
+"""Launch shapes of a batch: the ones asked for are the ones that run, read back and kept, also where a batch
+with large communities would take others by itself, and the results do not depend on them."""
+import pytest
+
+from arbo_gpu_fit_gb300.simulation import ArchitectureParam, Batch
+from tests.helpers import small_case
+from tests.test_batch_gpu import make, same
+
+pytestmark = pytest.mark.gpu
+
+
+def workloads(T):
+    # One large community, and more small ones than the infection pass has warps.
+    return [small_case(n=20_000, m=60_000, side=1, T=T, seed=3), small_case(n=20_000, m=50_000, side=80, T=T, seed=4),
+            small_case(n=500, m=2_000, side=3, T=T, seed=5)]
+
+
+def test_infection_block_of_a_batch_with_large_communities(gpu):
+    ws = workloads(12)
+    alone, together = make(ws), make(ws)
+    got = {}
+    for name, arch in (("default", None), ("64", ArchitectureParam(0, infectBlock=64)),
+                       ("256", ArchitectureParam(0, infectBlock=256))):
+        with Batch(together, arch) as b:
+            shape, grids = b.arch()
+            got[name] = (shape.infectBlock, grids[2])
+            b.set_arch(shape)  # what is read back selects the same again
+            again, grids = b.arch()
+            assert (again.infectBlock, grids[2]) == got[name], name
+    assert got["64"][0] == 64 and got["256"][0] == 256 and got["default"] == got["256"]
+    # Blocks of two warps leave room for more of them on an SM.
+    assert got["64"][1] > got["256"][1]
+    with Batch(together, ArchitectureParam(0, infectBlock=64, foiBlock=128)) as b:
+        b.init()
+        b.step(12)
+    for i, s in enumerate(alone):
+        s.init()
+        s.step(12)
+        same(s, together[i], f"instance {i}")
