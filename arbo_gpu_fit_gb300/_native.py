@@ -155,6 +155,7 @@ SIGNATURES = {
     "arbo_batch_step": (c_int, [c_void_p, c_uint32, c_void_p]),
     "arbo_batch_run": (c_int, [c_void_p, c_void_p]),
     "arbo_batch_set_arch": (c_int, [c_void_p, POINTER(ArchParamStruct)]),
+    "arbo_batch_get_cluster": (c_int, [c_void_p, POINTER(c_uint32), POINTER(c_uint32)]),
     "arbo_batch_get_arch": (c_int, [c_void_p, POINTER(ArchParamStruct), POINTER(c_uint32)]),
     "arbo_batch_autotune": (c_int, [c_void_p, c_uint32, POINTER(ArchParamStruct), POINTER(c_float), c_void_p]),
     "arbo_batch_time_phases": (c_int, [c_void_p, c_uint32, c_uint32, POINTER(c_float), c_void_p]),

@@ -1485,8 +1485,8 @@ Dev batch_desc(const arbo_batch* b, size_t i)
 
 // Agents of the largest community from which a batch's infection pass works off communities with many events
 // by block (k_infect_batch<true>), in runs of two communities (one in blocks of one or two warps) and, where the
-// batch takes its handles' default shape, in blocks of kHeavyBlock threads. Smaller communities seldom have that many events, and the search for them costs
-// 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us, at runs of 4, 2 and 1: 352, 289 and
+// batch takes its handles' default shape, in blocks of kHeavyBlock threads. Smaller communities seldom have that
+// many events, and the search for them costs 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us, at runs of 4, 2 and 1: 352, 289 and
 // 278 in blocks of 256, 398, 370 and 350 in blocks of 512, 456, 378 and 280 in blocks of 64; with few
 // events 83, 85 and 92. One simulation alone keeps k_infect: with this its step took 1 to 3 % longer.
 constexpr uint64_t kHeavyCommunity = 16384;
@@ -1523,7 +1523,8 @@ bool chooses_shapes(const arbo_batch* b, const arbo_arch_param& a)
 }
 
 // CTAs per simulation when the batch's steps run as one cluster per simulation (k_steps), or 0 for the
-// per-phase kernels. C: the largest cluster of which all the simulations' fit the device at once.
+// per-phase kernels. C: the largest cluster of which all the simulations' fit the device at once and, as the
+// grids of the per-phase kernels do, the batch's SMs (b->l.numSM).
 // A step takes a cluster about 11 us plus 0.45 us per 1,000 work units of its simulation (agents, and
 // 300 per community for the infection pass) and CTA; once CTAs share SMs 0.36 to 0.66 us, the more the
 // larger the SM's other simulations are; and the device as a whole 0.003 us per 1,000 units. The per-phase
@@ -1536,7 +1537,7 @@ uint32_t batch_cluster(const arbo_batch* b, uint32_t* per_sm)
 {
     if (b->phase_shapes) return 0;
     const uint32_t n = (uint32_t)b->sims.size();
-    const uint32_t C = steps_cluster(n, per_sm);
+    const uint32_t C = steps_cluster(n, b->l.numSM, per_sm);
     if (!C) return 0;
     double total = 0.0, most = 0.0;
     for (const arbo_sim* s : b->sims) {
@@ -1840,6 +1841,14 @@ int arbo_batch_set_arch(arbo_batch* b, const arbo_arch_param* arch)
     const int e = batch_configure(b, *arch);
     if (e) b->phase_shapes = before;
     return e;
+}
+
+int arbo_batch_get_cluster(const arbo_batch* b, uint32_t* ctas, uint32_t* per_sm)
+{
+    if (!b || !ctas) return fail(ARBO_ERR_INVALID, "null argument");
+    *ctas = b->cluster;
+    if (per_sm) *per_sm = b->cluster ? b->cluster_per_sm : 0u;
+    return ARBO_OK;
 }
 
 int arbo_batch_get_arch(const arbo_batch* b, arbo_arch_param* arch, uint32_t grids[3])

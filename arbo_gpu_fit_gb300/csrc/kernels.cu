@@ -2221,13 +2221,14 @@ static cudaLaunchConfig_t steps_config(uint32_t n, uint32_t C, cudaLaunchAttribu
 
 typedef void (*StepsKernel)(const Dev*, uint32_t, uint32_t);
 
-// Largest cluster of which n fit the device at once with kernel k (0: none).
-static uint32_t largest_cluster(StepsKernel k, uint32_t n)
+// Largest cluster of which n fit the device at once with kernel k and have `ctas` CTAs at most (0: none).
+static uint32_t largest_cluster(StepsKernel k, uint32_t n, uint64_t ctas)
 {
     // Sixteen CTAs per cluster are more than the portable eight.
     const bool wide = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     uint32_t found = 0;
     for (uint32_t C = wide ? 16 : 8; C >= 1 && !found; C /= 2) {
+        if ((uint64_t)n * C > ctas) continue;
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = steps_config(1, C, &attr);
         int fit = 0;
@@ -2244,11 +2245,13 @@ static StepsKernel steps_kernel(uint32_t per_sm, bool many)
     return per_sm == 1 ? k_steps<1, false> : k_steps<2, false>;
 }
 
-uint32_t steps_cluster(uint32_t n, uint32_t* per_sm)
+uint32_t steps_cluster(uint32_t n, uint32_t num_sm, uint32_t* per_sm)
 {
     // The larger of the two forms, so that either fits (each sets its own attribute).
-    const uint32_t one = std::min(largest_cluster(k_steps<1, false>, n), largest_cluster(k_steps<1, true>, n));
-    const uint32_t two = std::min(largest_cluster(k_steps<2, false>, n), largest_cluster(k_steps<2, true>, n));
+    const uint64_t sms = num_sm;
+    const uint32_t one = std::min(largest_cluster(k_steps<1, false>, n, sms), largest_cluster(k_steps<1, true>, n, sms));
+    const uint32_t two =
+        std::min(largest_cluster(k_steps<2, false>, n, 2 * sms), largest_cluster(k_steps<2, true>, n, 2 * sms));
     *per_sm = one && one >= two ? 1u : 2u;
     return one && one >= two ? one : two;
 }

@@ -230,11 +230,11 @@ int preload_step_kernels(const Launch& l);
 
 // Many whole steps of the n simulations of descriptors devs in one launch, one cluster of C CTAs each
 // (C as steps_cluster gives it: the largest of 16, 8, 4, 2, 1 with all n clusters resident at once on
-// the current device, one or two CTAs per SM; 0 when there is none). items: demographic warp items of all
-// simulations.
+// the current device, one or two CTAs per SM, and no more CTAs than num_sm SMs take; 0 when there is none).
+// items: demographic warp items of all simulations.
 int launch_steps(const Dev* devs, uint32_t n, uint32_t C, uint32_t per_sm, uint64_t items, uint32_t nsteps,
                  void* stream);
-uint32_t steps_cluster(uint32_t n, uint32_t* per_sm);
+uint32_t steps_cluster(uint32_t n, uint32_t num_sm, uint32_t* per_sm);
 
 // Batched steps (see BatchDev); the block shapes come from l, the grids from bd.
 int launch_step_batch(const BatchDev& bd, const Launch& l, void* stream, void* events, uint32_t koff);

@@ -348,6 +348,12 @@ class Batch:
         check(self._lib.arbo_batch_get_arch(self._h, byref(a), grids))
         return a, list(grids)
 
+    def cluster(self):
+        """(CTAs of each simulation's cluster, CTAs to an SM); (0, 0) where the per-phase kernels step the batch."""
+        ctas, per_sm = c_uint32(), c_uint32()
+        check(self._lib.arbo_batch_get_cluster(self._h, byref(ctas), byref(per_sm)))
+        return ctas.value, per_sm.value
+
     def set_arch(self, arch: ArchitectureParam) -> None:
         check(self._lib.arbo_batch_set_arch(self._h, byref(arch)))
 

@@ -462,6 +462,9 @@ int arbo_batch_run(arbo_batch* b, void* stream);
  * three persistent kernels). */
 int arbo_batch_set_arch(arbo_batch* b, const arbo_arch_param* arch);
 int arbo_batch_get_arch(const arbo_batch* b, arbo_arch_param* arch, uint32_t grids[3]);
+/* How arbo_batch_step steps the batch: CTAs of each simulation's cluster, 0 for the per-phase kernels; CTAs
+ * to an SM (optional). Clusters, like the grids, take no more CTAs than totalSM SMs hold. */
+int arbo_batch_get_cluster(const arbo_batch* b, uint32_t* ctas, uint32_t* per_sm);
 /* Autotuner: tries demographic (block, unroll), force-of-infection block and infection block
  * shapes in turn, each for steps_per_candidate real steps of the batch (the results do not depend
  * on the shape), keeps the fastest per phase and applies it. Consumes 13*steps_per_candidate

@@ -37,3 +37,23 @@ def test_infection_block_of_a_batch_with_large_communities(gpu):
         s.init()
         s.step(12)
         same(s, together[i], f"instance {i}")
+
+
+def test_clusters_leave_the_other_sms_free(gpu):
+    ws = [small_case(n=300 + 40 * i, m=1_000 + 200 * i, side=2, T=30, seed=i) for i in range(8)]
+    alone, together = make(ws), make(ws)
+    for s in alone:
+        s.init()
+        s.step(30)
+    for sms in (None, 64, 16, 4, 3, 1):
+        with Batch(together, ArchitectureParam(0, totalSM=sms) if sms else None) as b:
+            ctas, per_sm = b.cluster()
+            if sms is None:
+                assert 8 * ctas > 64, "more than the limits below allow"
+            else:
+                assert 8 * ctas <= sms * per_sm
+                assert ctas or 8 > 2 * sms, "clusters where they fit"
+            b.init()
+            b.step(30)
+            for i, s in enumerate(alone):
+                same(s, together[i], f"instance {i} on {sms} SMs")
