@@ -1657,6 +1657,7 @@ int batch_configure(arbo_batch* b, const arbo_arch_param& a)
     b->bd = bd;
     b->l = l;
     b->arch = a;
+    b->phase_shapes = chooses_shapes(b, a);
     b->cluster = batch_cluster(b, &b->cluster_per_sm);
     b->cluster_items = 0;
     for (const arbo_sim* s : b->sims) b->cluster_items += cdiv(s->d.tiles, kQuad) + cdiv(s->d.nvec, 32);
@@ -1747,6 +1748,32 @@ int batch_flush(arbo_batch* b, uint32_t flush_mb, cudaStream_t st)
     return e ? fail(ARBO_ERR_CUDA, std::string("flush launch: ") + cudaGetErrorString((cudaError_t)e)) : ARBO_OK;
 }
 
+// One step by the kernels that arbo_batch_step uses.
+int batch_one_step(arbo_batch* b, cudaStream_t st)
+{
+    return b->cluster ? launch_steps(b->bd.devs, b->bd.n, b->cluster, b->cluster_per_sm, b->cluster_items, 1, st)
+                      : launch_step_batch(b->bd, b->l, st, nullptr, 0);
+}
+
+// Fastest of n such steps, each launched by itself, ms (the first launch of a kernel may load it).
+int batch_fastest_step(arbo_batch* b, uint32_t n, cudaStream_t st, float* ms)
+{
+    *ms = 1e30f;
+    for (uint32_t k = 0; k < n; ++k) {
+        CUDA_TRY(cudaEventRecord(b->ev[0], st));
+        int e = batch_one_step(b, st);
+        CUDA_TRY(cudaEventRecord(b->ev[3], st));
+        if (!e && !b->cluster) e = launch_advance_batch(b->bd, 1, st);
+        if (e) return fail(ARBO_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString((cudaError_t)e));
+        batch_advance_host(b, 1);
+        CUDA_TRY(cudaEventSynchronize(b->ev[3]));
+        float x = 0.0f;
+        CUDA_TRY(cudaEventElapsedTime(&x, b->ev[0], b->ev[3]));
+        *ms = std::min(*ms, x);
+    }
+    return ARBO_OK;
+}
+
 // Mean ms per phase over n directly launched steps: [demographic, force of infection, infection, step].
 int batch_phases(arbo_batch* b, uint32_t n, uint32_t flush_mb, cudaStream_t st, double acc[4])
 {
@@ -1797,9 +1824,7 @@ int arbo_batch_create(arbo_sim* const* sims, uint32_t n, const arbo_arch_param* 
         return bail(fail(ARBO_ERR_CUDA, "cudaStreamCreate"));
     for (int k = 0; k < 4; ++k)
         if (cudaEventCreate(&b->ev[k]) != cudaSuccess) return bail(fail(ARBO_ERR_CUDA, "cudaEventCreate"));
-    const arbo_arch_param a = arch ? *arch : batch_default_arch(b);
-    b->phase_shapes = chooses_shapes(b, a);
-    const int e = batch_configure(b, a);
+    const int e = batch_configure(b, arch ? *arch : batch_default_arch(b));
     if (e) return bail(e);
     *out = b;
     return ARBO_OK;
@@ -1836,11 +1861,7 @@ int arbo_batch_set_arch(arbo_batch* b, const arbo_arch_param* arch)
     if (!b || !arch) return fail(ARBO_ERR_INVALID, "null argument");
     CUDA_TRY(cudaSetDevice(b->device));
     CUDA_TRY(cudaDeviceSynchronize());  // graphs of the old shape may still run
-    const bool before = b->phase_shapes;
-    b->phase_shapes = chooses_shapes(b, *arch);
-    const int e = batch_configure(b, *arch);
-    if (e) b->phase_shapes = before;
-    return e;
+    return batch_configure(b, *arch);
 }
 
 int arbo_batch_get_cluster(const arbo_batch* b, uint32_t* ctas, uint32_t* per_sm)
@@ -2009,13 +2030,14 @@ int arbo_batch_time_steps(arbo_batch* b, uint32_t nsteps, uint32_t flush_mb, flo
         CUDA_TRY(cudaEventCreate(&ev));
         b->step_ev.push_back(ev);
     }
-    // One graph-launched step at a time, each between its own events (optional L2 flush first).
+    // One step at a time, each between its own events (optional L2 flush first): one launch of the cluster
+    // kernel, or a graph of the per-phase kernels.
     cudaGraphExec_t one = nullptr;
-    if ((e = batch_capture(b, 1, &one))) return e;
+    if (!b->cluster && (e = batch_capture(b, 1, &one))) return e;
     for (uint32_t k = 0; k < n; ++k) {
         if ((e = batch_flush(b, flush_mb, st))) break;
         cudaError_t ce = cudaEventRecord(b->step_ev[0], st);
-        if (ce == cudaSuccess) ce = cudaGraphLaunch(one, st);
+        if (ce == cudaSuccess) ce = one ? cudaGraphLaunch(one, st) : (cudaError_t)batch_one_step(b, st);
         if (ce == cudaSuccess) ce = cudaEventRecord(b->step_ev[1], st);
         if (ce == cudaSuccess) ce = cudaEventSynchronize(b->step_ev[1]);
         if (ce == cudaSuccess) ce = cudaEventElapsedTime(&step_ms[k], b->step_ev[0], b->step_ev[1]);
@@ -2025,7 +2047,7 @@ int arbo_batch_time_steps(arbo_batch* b, uint32_t nsteps, uint32_t flush_mb, flo
         }
         batch_advance_host(b, 1);
     }
-    cudaGraphExecDestroy(one);
+    if (one) cudaGraphExecDestroy(one);
     return e;
 }
 
@@ -2045,13 +2067,24 @@ int arbo_batch_autotune(arbo_batch* b, uint32_t steps_per_candidate, arbo_arch_p
     if (batch_room(b, t) < need)
         return fail(ARBO_ERR_STATE, "arbo_batch_autotune: " + std::to_string(need) + " steps needed, " +
                                         std::to_string(batch_room(b, t)) + " left");
+    // The default shapes, which clusters go with (chooses_shapes), and whether they would be taken.
+    arbo_arch_param cur = b->arch, q, plain = cur;
+    arbo_arch_param_query(&q, -1);
+    plain.demogBlock = q.demogBlock;
+    plain.foiBlock = q.foiBlock;
+    plain.infectBlock = batch_heavy(b) ? kHeavyBlock : q.infectBlock;
+    float by_cluster = 1e30f, by_phase = 1e30f;
+    if ((e = batch_configure(b, plain))) return e;
+    const bool clusters = b->cluster != 0;
+    if (clusters && (e = batch_fastest_step(b, steps_per_candidate, st, &by_cluster))) return e;
     // Coordinate search: every candidate runs real steps (results do not depend on the launch
-    // shape), each phase keeps the shape with the smallest mean time.
-    arbo_arch_param cur = b->arch;
+    // shape), each phase keeps the shape with the smallest mean time. Where clusters are an option, their steps
+    // and those that compare the search's pick with them stand in for its last two demographic shapes.
     double acc[4];
     double bd = 1e30, bf = 1e30, bi = 1e30;
     arbo_arch_param pick = cur;
     for (const auto& c : demog) {
+        if (clusters && &c >= demog + 4) break;
         arbo_arch_param a = cur;
         a.demogBlock = c[0];
         a.demogUnroll = c[1];
@@ -2062,6 +2095,8 @@ int arbo_batch_autotune(arbo_batch* b, uint32_t steps_per_candidate, arbo_arch_p
             pick.demogUnroll = c[1];
         }
     }
+    double other = 1e30;  // of the force-of-infection blocks that are not the default
+    uint32_t other_foi = 0;
     for (uint32_t f : foi) {
         arbo_arch_param a = pick;
         a.foiBlock = f;
@@ -2069,6 +2104,10 @@ int arbo_batch_autotune(arbo_batch* b, uint32_t steps_per_candidate, arbo_arch_p
         if (acc[1] < bf) {
             bf = acc[1];
             pick.foiBlock = f;
+        }
+        if (f != q.foiBlock && acc[1] < other) {
+            other = acc[1];
+            other_foi = f;
         }
     }
     for (uint32_t f : infect) {
@@ -2079,6 +2118,15 @@ int arbo_batch_autotune(arbo_batch* b, uint32_t steps_per_candidate, arbo_arch_p
             bi = acc[2];
             pick.infectBlock = f;
         }
+    }
+    if (clusters) {
+        // The shapes say which kernels step a batch: default ones would select the clusters again.
+        if (!chooses_shapes(b, pick)) {
+            pick.foiBlock = other_foi;
+            bf = other;
+        }
+        if ((e = batch_configure(b, pick)) || (e = batch_fastest_step(b, steps_per_candidate, st, &by_phase))) return e;
+        if (by_cluster <= by_phase) pick = plain;
     }
     if ((e = batch_configure(b, pick))) return e;
     if (best) *best = pick;

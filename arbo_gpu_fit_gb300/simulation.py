@@ -358,7 +358,8 @@ class Batch:
         check(self._lib.arbo_batch_set_arch(self._h, byref(arch)))
 
     def autotune(self, steps_per_candidate: int = 2):
-        """Picks the launch shapes (coordinate search over real steps); returns (arch, phase ms)."""
+        """Picks the launch shapes, or the clusters of the default ones (over real steps); returns (arch, ms of
+        the fastest shape of each phase)."""
         a = ArchitectureParam.__new__(ArchitectureParam)
         ArchParamStruct.__init__(a)
         ms = (c_float * 3)()
@@ -366,11 +367,13 @@ class Batch:
         return a, np.array(ms[:], np.float64)
 
     def time_phases(self, nsteps: int, flush_mb: int = 0) -> np.ndarray:
+        """Mean ms of the three per-phase kernels and of the step by them, however the batch is stepped."""
         out = (c_float * 4)()
         check(self._lib.arbo_batch_time_phases(self._h, int(nsteps), int(flush_mb), out, self.stream))
         return np.array(out[:], np.float64)
 
     def time_steps(self, nsteps: int, flush_mb: int = 0) -> np.ndarray:
+        """Per-step ms by the kernels that step the batch, one step a launch."""
         out = np.zeros(int(nsteps), np.float32)
         check(self._lib.arbo_batch_time_steps(self._h, int(nsteps), int(flush_mb), _f32p(out), self.stream))
         return out.astype(np.float64)

@@ -467,11 +467,16 @@ int arbo_batch_get_arch(const arbo_batch* b, arbo_arch_param* arch, uint32_t gri
 int arbo_batch_get_cluster(const arbo_batch* b, uint32_t* ctas, uint32_t* per_sm);
 /* Autotuner: tries demographic (block, unroll), force-of-infection block and infection block
  * shapes in turn, each for steps_per_candidate real steps of the batch (the results do not depend
- * on the shape), keeps the fastest per phase and applies it. Consumes 13*steps_per_candidate
- * steps. best / best_ms (3 phase times of the choice, ms) are optional. */
+ * on the shape), keeps the fastest per phase and applies it. Where clusters are an option their step
+ * is timed against that choice (and two demographic shapes fewer are tried): if it is the faster, the
+ * default shapes are applied, which select the clusters. Consumes 13*steps_per_candidate steps. best:
+ * the shapes applied; given to arbo_batch_set_arch or arbo_batch_create they select the same kernels
+ * again. best_ms: the times of the fastest shape of each of the three phases, ms. Both optional. */
 int arbo_batch_autotune(arbo_batch* b, uint32_t steps_per_candidate, arbo_arch_param* best, float* best_ms,
                         void* stream);
-/* Measurement, as arbo_sim_time_phases / arbo_sim_time_steps for the whole batch. */
+/* Measurement, as arbo_sim_time_phases / arbo_sim_time_steps for the whole batch. time_steps times the
+ * kernels that arbo_batch_step uses, a step a launch (clusters run up to 128 steps a launch there);
+ * time_phases always the per-phase kernels. */
 int arbo_batch_time_phases(arbo_batch* b, uint32_t nsteps, uint32_t flush_mb, float* ms_out, void* stream);
 int arbo_batch_time_steps(arbo_batch* b, uint32_t nsteps, uint32_t flush_mb, float* step_ms, void* stream);
 

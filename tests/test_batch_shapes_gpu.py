@@ -57,3 +57,48 @@ def test_clusters_leave_the_other_sms_free(gpu):
             b.step(30)
             for i, s in enumerate(alone):
                 same(s, together[i], f"instance {i} on {sms} SMs")
+
+
+def small_batch(T):
+    return [small_case(n=3_000 + 400 * i, m=10_000 + 900 * i, side=5, T=T, seed=i) for i in range(8)]
+
+
+def test_timed_steps_are_those_of_the_batch(gpu):
+    # A step of eight such simulations takes clusters about half the time of the per-phase kernels.
+    together = make(small_batch(60))
+    fastest = {}
+    for name, arch in (("clusters", None), ("phases", ArchitectureParam(0, graphSteps=32))):
+        with Batch(together, arch) as b:
+            assert (b.cluster()[0] > 0) == (name == "clusters")
+            b.init()
+            fastest[name] = b.time_steps(30).min()
+            assert all(s.status() == (0, 30) for s in together)
+    assert fastest["clusters"] < 0.8 * fastest["phases"], fastest
+
+
+@pytest.mark.parametrize("case", ["clusters", "phases"])
+def test_tuned_shapes_select_what_was_tuned(gpu, case):
+    ws = small_batch(60) if case == "clusters" else workloads(60)
+    alone, together = make(ws), make(ws)
+    for s in alone:
+        s.init()
+    with Batch(together) as b:
+        assert (b.cluster()[0] > 0) == (case == "clusters")
+        b.init()
+        best, ms = b.autotune(2)
+        assert all(s.status() == (0, 26) for s in together) and (ms > 0).all()
+        how = b.cluster()
+        applied, _ = b.arch()
+        names = [f for f, _ in best._fields_]
+        assert [getattr(applied, f) for f in names] == [getattr(best, f) for f in names]
+        b.step(10)
+        b.set_arch(best)
+        assert b.cluster() == how
+        b.step(5)
+    if case == "clusters":
+        assert how[0] > 0, "twice as fast as the phases on this workload"
+    for i, s in enumerate(alone):
+        s.step(41)
+        same(s, together[i], f"instance {i}")
+    with Batch(make(ws), best) as b:
+        assert b.cluster() == how
