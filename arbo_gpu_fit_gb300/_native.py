@@ -162,6 +162,7 @@ SIGNATURES = {
     "arbo_batch_time_steps": (c_int, [c_void_p, c_uint32, c_uint32, POINTER(c_float), c_void_p]),
     "arbo_selftest_philox": (c_int, [POINTER(c_uint32), c_uint32, POINTER(c_uint32)]),
     "arbo_selftest_curand_philox": (c_int, [c_uint64, c_uint32, POINTER(c_uint32)]),
+    "arbo_selftest_stalled_product": (c_int, [c_uint32, c_uint32, c_uint32, POINTER(c_uint32)]),
 }
 
 _lock = threading.Lock()

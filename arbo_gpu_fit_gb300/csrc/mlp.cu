@@ -77,6 +77,7 @@ struct GemmLaunch {
     uint32_t* host_err;  // the same in host memory, or null
     const float* loss;   // if not null, a finished loss and where in host memory it goes
     float* host_loss;
+    uint32_t polls;      // bound of the roles' waits (kTcMaxPolls; 0 in the self-test: every wait runs out)
 };
 
 constexpr uint32_t kTileM = 128, kTileK = 64, kMaxStages = 8;
@@ -272,7 +273,8 @@ __device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
 // previous one has ended, and A, bias, zprev and target are older than that (GemmArgs). By then the CTA also
 // holds its tensor memory, so a later CTA can never take columns that an earlier one waits for.
 // Every wait is bounded; a role that runs out records the error and stops, which bounds the waits
-// of the others; tensor memory is freed at the end in every case.
+// of the others. The CTA then waits, bounded again, for its copies and products in flight, which write its
+// shared and tensor memory; tensor memory is freed at the end in every case.
 //
 // What bounds it: the small products of training (256 x 512 x 512, one tile a CTA) the chain of B's load
 // (0.4 us), products (0.6), epilogue (1.0) and the hand-over to the next launch (1.2): 6.5 us a layer with A
@@ -283,7 +285,7 @@ __device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
 __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_constant__ GemmLaunch p)
 {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ unsigned long long full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2];
+    __shared__ unsigned long long full[kMaxStages], empty[kMaxStages], acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t tmem_slot;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -299,6 +301,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
             tc_bar_init(&acc_full[a], 1);
             tc_bar_init(&acc_empty[a], kEpiWarps);
         }
+        tc_bar_init(&drained, 1);
     }
     tc_fence_before();
     __syncthreads();
@@ -306,7 +309,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     bool ok = true;
     const uint32_t ring = tc_smem(smem), stage = p.stage_size, ring_end = ring + S * stage, G = p.group;
-    const uint32_t full0 = tc_smem(full), empty0 = tc_smem(empty);
+    const uint32_t full0 = tc_smem(full), empty0 = tc_smem(empty), polls = p.polls;
+    uint32_t fills = 0;  // of ring stages, by the producing lane
     if (warp == 0) {  // producer
         uint32_t t = blockIdx.x;
         TileAt x = tile_at(p, min(t, tiles - 1));
@@ -336,7 +340,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
             // The rest, as stages come free.
             while (t < tiles && ok) {
                 for (uint32_t c = early; c < x.nk; c += G) {
-                    if (round > 0) ok = tc_bar_wait(empty0 + 8 * s, (round - 1) & 1u);
+                    if (round > 0) ok = tc_bar_wait(empty0 + 8 * s, (round - 1) & 1u, polls);
                     if (!ok) break;
                     const uint32_t bar = full0 + 8 * s, sa = ring + s * stage, end = min(c + G, x.nk);
                     tc_bar_expect_tx(bar, (end - c) * (aBytes + x.tn * kTileK * 2));
@@ -355,20 +359,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
                     mb = &p.map[x.q][1];
                 }
             }
+            fills = round * S + s;
         }
     } else if (warp == 1) {  // tensor-core issuer
         uint32_t sa = ring, bar = full0, phase = 0, li = 0;
         for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++li) {
             const TileAt x = tile_at(p, t);
             const uint32_t a = li & 1u, idesc = tc_idesc_bf16(kTileM, x.nt), d = tmem + a * p.acc_cols;
-            if (li >= 2) ok = __all_sync(0xffffffffu, tc_bar_wait(tc_smem(&acc_empty[a]), ((li >> 1) - 1) & 1u));
+            if (li >= 2) ok = __all_sync(0xffffffffu, tc_bar_wait(tc_smem(&acc_empty[a]), ((li >> 1) - 1) & 1u, polls));
             if (!ok) break;
             tc_fence_after();
             // Steps whose stage is filled again: all but the CTA's last S.
             const uint32_t steps = (x.nk + G - 1) / G, refilled = t + gridDim.x < tiles ? x.nk : (steps - min(steps, S)) * G;
             const uint32_t bstep = x.tn * kTileK * 2 / 16;
             for (uint32_t c = 0; c < x.nk; c += G) {
-                ok = __all_sync(0xffffffffu, tc_bar_wait(bar, phase));
+                ok = __all_sync(0xffffffffu, tc_bar_wait(bar, phase, polls));
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t da = tc_desc_sw128(sa), db = tc_desc_sw128(sa + G * aBytes);
@@ -405,7 +410,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
             const uint32_t d = tmem + a * p.acc_cols + ((quarter * 32u) << 16);
             auto ready = [&] {
                 if (li == 0) griddep_wait();
-                ok = __all_sync(0xffffffffu, tc_bar_wait(tc_smem(&acc_full[a]), (li >> 1) & 1u));  // warp-uniform
+                ok = __all_sync(0xffffffffu, tc_bar_wait(tc_smem(&acc_full[a]), (li >> 1) & 1u, polls));  // warp-uniform
                 tc_fence_after();
                 return ok;
             };
@@ -431,7 +436,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_tn(const __grid_consta
         if (p.host_err) *(volatile uint32_t*)p.host_err = 1u;
     }
     tc_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        for (uint32_t f = fills - min(fills, S); f < fills; ++f) tc_bar_wait(full0 + 8 * (f % S), (f / S) & 1u);
+        if (warp == 1 && tc_elect()) {
+            tc_commit(tc_smem(&drained));
+            tc_bar_wait(tc_smem(&drained), 0u);
+        }
+        tc_fence_before();
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 0) tc_dealloc(tmem, 2 * p.acc_cols);
 }
@@ -522,7 +535,8 @@ void choose_tiles(const GemmArgs* g, uint32_t n, uint32_t num_sm, uint32_t (&tn)
 // sums on persistent CTAs, at most one per SM. Returns a cudaError_t (invalid value when a tensor map
 // cannot be built; the reason is then in arbo_last_error).
 int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* err, uint32_t* host_err, cudaStream_t st,
-                uint32_t num_sm, bool pdl, const float* loss = nullptr, float* host_loss = nullptr)
+                uint32_t num_sm, bool pdl, const float* loss = nullptr, float* host_loss = nullptr,
+                uint32_t polls = kTcMaxPolls)
 {
     GemmLaunch p{};
     uint32_t nk = 0;
@@ -545,6 +559,7 @@ int gemm_launch(const GemmArgs* g, uint32_t n, const ColumnSums& cs, uint32_t* e
     p.host_err = host_err;
     p.loss = loss;
     p.host_loss = host_loss;
+    p.polls = polls;
     // CTAs without a tile only add column sums (four columns each pass).
     const uint32_t ctas = std::min(std::max(p.tiles[0] + p.tiles[1], (cs.cols + 3) / 4), num_sm);
     return launch_pdl(k_gemm_tn, dim3(ctas), dim3(kGemmThreads),
@@ -641,6 +656,7 @@ int ufail(int code, const std::string& msg) { return set_error(code, msg); }
     } while (0)
 
 uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; }
+size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
 
@@ -1110,6 +1126,37 @@ int arbo_tc_gemm(const float* a, const float* b, uint32_t M, uint32_t N, uint32_
     if (le) return ufail(ARBO_ERR_CUDA, "arbo_tc_gemm: launch failed: " + map_err + " " + cudaGetErrorString((cudaError_t)le));
     if (ce != cudaSuccess) return ufail(ARBO_ERR_CUDA, std::string("arbo_tc_gemm: ") + cudaGetErrorString(ce));
     if (herr) return ufail(ARBO_ERR_CUDA, "arbo_tc_gemm: an mbarrier wait ran out");
+    return ARBO_OK;
+}
+
+// A product of zeros whose waits all run out at once, with the first copies in flight: its error word.
+int arbo_selftest_stalled_product(uint32_t M, uint32_t N, uint32_t K, uint32_t* err)
+{
+    if (!err || M == 0 || N == 0 || K == 0 || N % 16 || K % 16)
+        return ufail(ARBO_ERR_INVALID, "arbo_selftest_stalled_product: N and K multiples of 16");
+    UCUDA(cudaFuncSetAttribute(k_gemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmemMax));
+    const size_t na = up256((size_t)N * K * 2), nb = up256((size_t)M * K * 2), nc = up256((size_t)M * N * 4);
+    char* base = nullptr;
+    UCUDA(cudaMalloc(&base, na + nb + nc + 256));
+    GemmArgs g{};
+    g.A = (const bf16*)base;
+    g.B = (const bf16*)(base + na);
+    g.lda = g.ldb = K;
+    g.M = g.ldof = N;
+    g.N = M;
+    g.K = K;
+    g.epi = kEpiStore;
+    g.outf = (float*)(base + na + nb);
+    uint32_t* derr = (uint32_t*)(base + na + nb + nc);
+    int sms = 152, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaMemset(base, 0, na + nb + nc + 256);
+    if (e == cudaSuccess)
+        e = (cudaError_t)gemm_launch(&g, 1, ColumnSums{}, derr, nullptr, nullptr, (uint32_t)sms, false, nullptr, nullptr, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(err, derr, 4, cudaMemcpyDeviceToHost);
+    cudaFree(base);
+    if (e != cudaSuccess) return ufail(ARBO_ERR_CUDA, std::string("stalled product: ") + cudaGetErrorString(e));
     return ARBO_OK;
 }
 

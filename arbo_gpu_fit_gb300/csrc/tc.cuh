@@ -73,9 +73,9 @@ __device__ __forceinline__ void tc_bar_init(unsigned long long* bar, uint32_t co
 }
 
 // Bounded wait for the phase of `bar` with the given parity; false when the bound ran out.
-__device__ __forceinline__ bool tc_bar_wait(uint32_t bar, uint32_t parity)
+__device__ __forceinline__ bool tc_bar_wait(uint32_t bar, uint32_t parity, uint32_t polls = kTcMaxPolls)
 {
-    for (uint32_t it = 0; it < kTcMaxPolls; ++it) {
+    for (uint32_t it = 0; it < polls; ++it) {
         uint32_t ok;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"

@@ -614,6 +614,12 @@ int arbo_selftest_philox(const uint32_t* ctr_key, uint32_t n, uint32_t* out);
  * computed on the device. No reference counterpart: a library cross-check of the Philox rounds. */
 int arbo_selftest_curand_philox(uint64_t seed, uint32_t n, uint32_t* out);
 
+/* The error word of one tensor-core product of zeros (A [M][K], B [N][K]; N and K multiples of 16) whose
+ * waits are all given a limit of zero, so that each runs out at once with the first operand copies in
+ * flight. No reference counterpart: checks that a product which gives up says so and leaves the device fit
+ * for the next one. */
+int arbo_selftest_stalled_product(uint32_t M, uint32_t N, uint32_t K, uint32_t* err);
+
 #ifdef __cplusplus
 }
 #endif
