@@ -754,6 +754,16 @@ int arbo_sim_init(arbo_sim* s, void* stream)
     return ARBO_OK;
 }
 
+// Whether a caller records st into a graph of its own. Steps are not recorded: the host counts a step when it
+// launches it, so a graph run again would step past the end of the series. (Steps by this library's graphs
+// cannot be recorded anyhow; graphSteps 0 and arbo_sim_step_noalloc leave it to the caller.)
+static bool recording(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) (void)cudaGetLastError();
+    return c != cudaStreamCaptureStatusNone;
+}
+
 static int capture_graph(arbo_sim* s, uint32_t steps, cudaGraphExec_t* out)
 {
     cudaGraph_t g = nullptr;
@@ -790,6 +800,7 @@ int arbo_sim_step(arbo_sim* s, uint32_t nsteps, void* stream)
         }
         return ARBO_OK;
     }
+    if (n > 0 && recording(st)) return fail(ARBO_ERR_CUDA, "arbo_sim_step: not permitted when the stream is capturing");
     bool tail = false;  // the rest of the call has been looked at
     while (n > 0) {
         uint32_t chunk = std::min(n, G);
@@ -1972,6 +1983,7 @@ int arbo_batch_step(arbo_batch* b, uint32_t nsteps, void* stream)
         }
         return ARBO_OK;
     }
+    if (n > 0 && recording(st)) return fail(ARBO_ERR_CUDA, "arbo_batch_step: not permitted when the stream is capturing");
     while (n > 0 && b->cluster) {
         const uint32_t chunk = std::min(n, kClusterSteps);
         e = launch_steps(b->bd.devs, b->bd.n, b->cluster, b->cluster_per_sm, b->cluster_items, chunk, st);
