@@ -33,9 +33,10 @@ int fail(int code, const std::string& msg)
         if (e_ != cudaSuccess) return fail(ARBO_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Steps that a handle or batch makes before it captures graphs of graphSteps: the three launches
-// of a step take the host less time (about 8 us) than the step takes the device, while a 64-step graph
-// costs half a millisecond to make, again after every change of parameters. What is left of a call
+// Steps that a handle or a batch stepped by phases makes before it captures graphs of graphSteps (a handle
+// makes shorter ones before, kShortAfter): the three launches of a step take the host less time (about 8 us)
+// than the step takes the device, while a 64-step graph costs half a millisecond to make, again after every
+// change of a handle's parameters. What is left of a call
 // after its whole graphs is launched the same way (as one-step graphs each step paid for a graph launch
 // and could not overlap the one before: 30 steps of 1.2e4 agents with initialisation and results 775 ->
 // 662 us, and 440 to 500 us less for the first run of a handle).

@@ -1,6 +1,6 @@
 // kernels.cu — sm_103a kernels of one simulation time step and of its initialisation.
 //
-// One step is three launches (after a handle's first steps captured in CUDA graphs by the host):
+// One step is three launches (captured in CUDA graphs by the host after a handle's first steps):
 //   k_demog   human and mosquito demographic passes over the whole census (HBM stream: a
 //             human's next event time, a mosquito slot's event code; ages are birth times,
 //             so a survivor without a transition writes nothing), per-tile
@@ -637,7 +637,8 @@ __global__ void __launch_bounds__(128, 4) k_demog_tma(Dev d, uint32_t koff)
 // 32 * U human groups. With `spread`, neighbouring items go to different blocks, so that every block has
 // its share of the long items (quads) and of the short ones; else blocks take consecutive items and the
 // human blocks, which are short but end in latency chains, come last and fill the SMs that the last
-// mosquito blocks leave idle.
+// mosquito blocks leave idle. 40 registers, so that six blocks fit an SM; the body takes a little more and
+// spills 8 bytes a thread.
 template <int U>
 __global__ void __launch_bounds__(256, 6) k_demog(Dev d, uint32_t spread, uint32_t koff)
 {
@@ -758,10 +759,9 @@ constexpr uint32_t kFoiPairs = 16;
 
 struct __align__(16) FoiWarpSmem {
     uint32_t to[kFoiPairs][8];  // CSR row of each pair's source community (degree <= 8)
-    uint32_t base[33];          // first group of four events of each lane; base[32]: groups in the warp
+    uint32_t base[32];          // first group of four events of each lane
     uint32_t local[32], far[32];  // a lane's events to neighbours and to any community
     uint32_t loc[kFoiPairs], deg[kFoiPairs], row[kFoiPairs];  // CSR row, its length, first counter of the serotype
-    uint32_t pad[3];
 };
 
 template <typename Wait>
@@ -1587,7 +1587,8 @@ static_assert(kStepsSmem + sizeof(Dev) + 64 <= 48 * 1024, "shared memory of k_st
 // that phase: 8 simulations of 7e4 agents 17.4 -> 16.8 us a step, 32 of them 21.5 -> 21.0. With many (items
 // are of uneven cost) a CTA's warps take its share of them from a counter: 128 of them 65.4 -> 62.8 us,
 // later 38.2 -> 36.1; half an item to a warp by the counter took 18.4 for 17.8. Both together, in one
-// kernel of 64 registers, took 64.5 and 37.5 on 128.
+// kernel of 64 registers, took 64.5 and 37.5 on 128. At 64 registers the infection body spills: 104 bytes a
+// thread in the first form, 64 in the second; at 128 (CTAs with an SM each) nothing.
 template <uint32_t B, bool kMany>
 __global__ void __launch_bounds__(kStepsWarps * 32, B) k_steps(const Dev* devs, uint32_t C, uint32_t nsteps)
 {

@@ -270,7 +270,9 @@ __device__ __forceinline__ TileAt tile_at(const GemmLaunch& p, uint32_t t)
 // Launched with programmatic serialization: barriers and tensor memory are set up and A, the larger operand
 // of a narrow tile, and the epilogue's first inputs are fetched while the previous launch runs. That is sound
 // because a launch lets the next one in only after its own wait: when a CTA starts, every launch but the
-// previous one has ended, and A, bias, zprev and target are older than that (GemmArgs). By then the CTA also
+// previous one has ended, and A, bias, zprev and target are older than that (GemmArgs). What the passes of
+// the same step wrote among them (activations and pre-activations, read by the backward launches) is in L2 by
+// then, and the early reads are TMA copies and ld.cg, which go to L2 and not through L1. By then the CTA also
 // holds its tensor memory, so a later CTA can never take columns that an earlier one waits for.
 // Every wait is bounded; a role that runs out records the error and stops, which bounds the waits
 // of the others. The CTA then waits, bounded again, for its copies and products in flight, which write its

@@ -278,9 +278,9 @@ class Simulation:
 
 
 class Batch:
-    """Many Simulation handles stepped together (arbo_batch_* of include/arbo.h): one persistent
-    kernel per phase over the blocks of every instance, the step loop in a CUDA graph. Each
-    instance's results equal stepping it alone; read them through the Simulation objects, which
+    """Many Simulation handles stepped together (arbo_batch_* of include/arbo.h): few and small ones as
+    one thread-block cluster per simulation, others by one persistent kernel per phase over the items
+    of every instance. Each instance's results equal stepping it alone; read them through the Simulation objects, which
     must outlive the batch and be stepped only through it."""
 
     def __init__(self, sims, arch: Optional[ArchitectureParam] = None, stream: int = 0):

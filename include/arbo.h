@@ -126,7 +126,8 @@ typedef struct arbo_arch_param {
     uint32_t totalSM;
     uint32_t demogBlock;     /* threads per CTA of the demographic kernel (multiple of 32) */
     uint32_t demogUnroll;    /* 4-agent groups per thread (1, 2 or 4)                      */
-    uint32_t foiBlock;       /* threads per CTA of the force-of-infection kernel (one warp per 32 pairs) */
+    uint32_t foiBlock;       /* threads per CTA of the force-of-infection kernel (one warp per 16 pairs,
+                                a lane per pair and direction) */
     uint32_t infectBlock;    /* threads per CTA of the infection kernel (one warp per community) */
     uint32_t graphSteps;     /* steps captured per CUDA graph (0: no graph)                */
     uint32_t demogPipeline;  /* 1: persistent demographic kernel with TMA-staged mosquito tiles
@@ -281,7 +282,8 @@ int arbo_sim_init(arbo_sim* s, void* stream);
 /* Advance nsteps time steps: per step the human and mosquito demographic passes, the
  * series row of the next time point, the force of infection with dispersal, and the
  * infection draws. Replaces the body of the time loop of simulation (cpp/simulation.cpp:
- * 115-155): nDemographic, mDemographic, epidemic, dataCollect. Asynchronous on `stream`. */
+ * 115-155): nDemographic, mDemographic, epidemic, dataCollect. Asynchronous on `stream`, which must not
+ * be capturing (unless graphSteps is 0): ARBO_ERR_CUDA. */
 int arbo_sim_step(arbo_sim* s, uint32_t nsteps, void* stream);
 
 /* Run the remaining steps up to max_time and synchronise; returns ARBO_ERR_DEVICE if the
@@ -401,10 +403,11 @@ int arbo_sim_weekly_incidence(arbo_sim* s, uint32_t max_week, uint32_t* out, voi
  * Who needs it: callers that hold a handle created earlier but must not allocate while they step
  * it — a step loop running under a framework whose memory pool owns the device, an embedded or
  * real-time driver that forbids allocation after set-up, or code that must not trigger the device
- * memory that building a CUDA graph can take. arbo_sim_step captures and instantiates CUDA graphs
- * once a handle has made some hundred steps, and the handle's own per-agent scratch was allocated at create; this entry point
- * launches the same step kernels one by one and takes the infection pass's per-agent scratch from
- * a fixed array compiled into the library instead.
+ * memory that building a CUDA graph can take. arbo_sim_step captures and instantiates CUDA graphs from
+ * the 48th step after a handle's creation or a change of its parameters on, and again from the 256th and
+ * for a rest of steps that calls keep ending with, and the handle's own per-agent scratch was allocated at
+ * create; this entry point launches the same step kernels one by one and takes the infection pass's
+ * per-agent scratch from a fixed array compiled into the library instead.
  *
  * Limits and behaviour:
  *  - The handle's padded humans plus padded mosquito slots must not exceed ARBO_NOALLOC_MAX_AGENTS;
@@ -428,8 +431,8 @@ int arbo_sim_step_noalloc(arbo_sim* s, uint32_t nsteps, void* stream);
 /* Many simulation handles stepped together: few and small ones as one thread-block cluster per
  * simulation that runs many steps in a launch; others by one persistent kernel per phase
  * (demographic, force of infection, infection) that walks the items of every instance, with long
- * step loops captured in CUDA graphs. Replaces the reference's serial loop over replicates and MCMC proposals
- * (cpp/main.cpp:262-280, one simulation() call each). Instances may differ in every size and
+ * step loops captured in CUDA graphs. Replaces the reference's serial loop over replicates and MCMC
+ * proposals (cpp/main.cpp:262-280, one simulation() call each). Instances may differ in every size and
  * parameter; each keeps its own buffers, key and counters, and its results are bit-identical to
  * stepping it alone, so arbo_sim_get_* read them as usual. Instances are stepped only through the
  * batch once it exists (they must stay at one step count) and outlive it. */
