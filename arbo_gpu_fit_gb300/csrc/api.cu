@@ -36,10 +36,9 @@ int fail(int code, const std::string& msg)
 // Steps that a handle or a batch stepped by phases makes before it captures graphs of graphSteps (a handle
 // makes shorter ones before, kShortAfter): the three launches of a step take the host less time (about 8 us)
 // than the step takes the device, while a 64-step graph costs half a millisecond to make, again after every
-// change of a handle's parameters. What is left of a call
-// after its whole graphs is launched the same way (as one-step graphs each step paid for a graph launch
-// and could not overlap the one before: 30 steps of 1.2e4 agents with initialisation and results 775 ->
-// 662 us, and 440 to 500 us less for the first run of a handle).
+// change of a handle's parameters. What is left of a call after its whole graphs is launched the same way (as
+// one-step graphs each step paid for a graph launch and could not overlap the one before: 30 steps of 1.2e4
+// agents with initialisation and results 775 -> 662 us, and 440 to 500 us less for the first run of a handle).
 constexpr uint32_t kDirectSteps = 256;
 
 // From this step on until then a single simulation runs in graphs of 16 steps: launched one by one, a step
@@ -1498,9 +1497,11 @@ Dev batch_desc(const arbo_batch* b, size_t i)
 // Agents of the largest community from which a batch's infection pass works off communities with many events
 // by block (k_infect_batch<true>), in runs of two communities (one in blocks of one or two warps) and, where the
 // batch takes its handles' default shape, in blocks of kHeavyBlock threads. Smaller communities seldom have that
-// many events, and the search for them costs 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us, at runs of 4, 2 and 1: 352, 289 and
-// 278 in blocks of 256, 398, 370 and 350 in blocks of 512, 456, 378 and 280 in blocks of 64; with few
-// events 83, 85 and 92. One simulation alone keeps k_infect: with this its step took 1 to 3 % longer.
+// many events, and the search for them costs 2 % of a step. Phase of 64 uneven instances in a heavy epidemic, us,
+// at runs of 4, 2 and 1: 352, 289 and 278 in blocks of 256, 398, 370 and 350 in blocks of 512, 456, 378 and 280
+// in blocks of 64; with few events 83, 85 and 92. With the present kernels, days 60 to 90: 240 in blocks of 256,
+// in blocks of 64 331 at runs of 2 and 255 at 1. One simulation alone keeps k_infect: with this form always on its
+// step took 1 to 3 % longer.
 constexpr uint64_t kHeavyCommunity = 16384;
 constexpr uint32_t kHeavyBlock = 256;
 
