@@ -47,8 +47,8 @@ PEAKS_FILE = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6800.0
 # Per-launch DRAM traffic of the demographic kernel on this workload, from one ncu capture of a
 # launch at step 5 (the command is kept with its summary under profiles/):
-# dram__bytes_read.sum + dram__bytes_write.sum (15,225,344 + 4,442,624 bytes).
-DEMOG_TRAFFIC_BYTES = 19_667_968
+# dram__bytes_read.sum + dram__bytes_write.sum (15,236,608 + 4,463,104 bytes).
+DEMOG_TRAFFIC_BYTES = 19_699_712
 
 
 def parse():
